@@ -352,6 +352,38 @@ def test_sample_matches_oracle():
         assert int(got.max()) < V
 
 
+@pytest.mark.parametrize("V,ld,form", [(320, 320, "plain"), (4096, 4099, "plain"), (5121, 5121, "plain"), (50257, 50257, "plain"),
+                                       (50257, 50260, "ties"), (32001, 32003, "masked"), (32000, 32000, "lowest"), (60001, 60001, "plain")])
+def test_sample_selection_edges(V, ld, form):
+    """Candidate selection by value bins: rows too short for it, rows whose start is off the 16-byte lines, ties at the threshold,
+    hidden tokens (-inf, and the type's lowest value: both leave the bins to the radix select), rows too long for shared memory.
+    The draw's uncertainty is the oracle's own (_oracle_choices)."""
+    cu = _cu()
+    torch.manual_seed(V)
+    B = 12
+    logits = (torch.randn(B, ld, device="cuda") * 2.5).float()
+    if form == "ties":
+        logits = (logits * 25).round() / 25
+    elif form != "plain":
+        hidden = torch.rand(B, ld, device="cuda") < 0.9
+        logits.masked_fill_(hidden, float("-inf") if form == "masked" else torch.finfo(torch.float32).min)
+        logits[:, 7] = 1.0
+    logits = logits[:, :V]
+    greedy = torch.tensor([1, 0, 0, 0] * (B // 4), dtype=torch.int32, device="cuda")
+    temp = torch.tensor([1.0, 0.7, 1.3] * (B // 3), device="cuda")
+    top_k = torch.tensor([0, 50, 0, 1, 7, 300] * (B // 6), dtype=torch.int32, device="cuda")
+    if form == "ties":      # tied values at the 1024th place are more than the 1024 candidates that the kernel keeps
+        top_k = top_k + 100 * (top_k == 0).int()
+    top_p = torch.tensor([0.9, 1.0, 0.9, 0.5] * (B // 4), device="cuda")
+    for step in range(4):
+        rng = torch.tensor([[91 + 13 * b, step] for b in range(B)], dtype=torch.int32, device="cuda")
+        want, lo, hi = _oracle_choices(lambda r, sh: R.sample(logits, greedy, temp, top_k, top_p, r, vocab=V, u_shift=sh), rng)
+        got = cu.sample(logits, greedy, temp, top_k, top_p, rng, vocab=V)
+        _check_tokens(got, want, lo, hi, f"step {step}")
+        g = greedy.bool()
+        assert torch.equal(got.long()[g], logits[g].argmax(-1))
+
+
 def test_sample_plain_multinomial_never_falls_through():
     """top_k = 0, top_p = 1: every thread must see the same draw (the RNG counter is advanced only after all
     threads have read it) and the per-thread CDF intervals must tile [0, total) without gaps -- before the fix a
