@@ -3,14 +3,12 @@
 //   per head and token:  S <- g_t S ;  u = beta_t (v_t - S^T k_t) ;  S <- S + k_t u^T ;  o_t = S^T q_t
 //
 // Every value column of the state is a recurrence of its own (S^T k, the write and the read-out only couple the rows of one
-// column), so thread (j, r) keeps rows [r * KPT, r * KPT + KPT) of column j in registers and the R threads of a column meet
-// in two warp-shuffle sums per token.  One block = one (sequence, head, slice of value columns); the block that reads a
-// slot's old state is the block that writes its new one.  Tokens are staged 16 at a time through shared memory: q and k in
-// strips of KPT + 4 floats (the strips a warp reads together lie in different banks, every read a 16-byte one; strips beyond
-// dk hold zeros), copied asynchronously one stage ahead, made unit vectors there (x / sqrt(sum x^2 + eps), q times its scale), decays exp(log g) and write
-// strengths (sigmoid taken here if asked) beside them.  The state lies in memory column-major per head ([dv][dk]).
-// KPT is the key size itself up to 64 (R = 1): the lanes of a warp then differ only in their value column, every staged q / k
-// read is one address for the whole warp (a shared-memory broadcast), and no shuffle is needed; larger keys split over R lanes.
+// column), so a thread keeps KPT rows of two columns in registers and the R threads of a column pair meet in warp-shuffle sums.
+// One block = one (sequence, head, slice of value columns); the block that reads a slot's old state is the block that writes its new
+// one.  Tokens are staged 16 at a time through shared memory: q and k in strips of KPT + 4 floats (the strips a warp reads together
+// lie in different banks, every read a 16-byte one; strips beyond dk hold zeros), copied asynchronously one stage ahead; the numbers
+// per token (decay, write strength, the norms 1 / sqrt(sum x^2 + eps), k . q) lie beside them.  The state lies in memory
+// column-major per head ([dv][dk]).
 //
 // A batch of single tokens (decode) runs the row-split form instead (delta_step_kernel): one warp per value column, lanes over
 // the key rows, so that every state access is one contiguous column (512 bytes at dk = 128) -- a decode step is bound by
@@ -31,7 +29,7 @@ struct DeltaArgs {
   float* out;                            // [T, H * dv]
   float* state;                          // [slots, H, dv, dk]
   const int* cu_q; const int* seq_lens; const int* slots;
-  int H, rep, dk, dv, dvt, R;
+  int H, rep, dk, dv, dvt;
   float unit_eps, q_scale;
   int unit, beta_sigmoid;
   int vec16;       // q / k / v rows, the key size and the value slices allow 16-byte copies
@@ -47,40 +45,75 @@ __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commi
 template <int N>
 __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
 
+// Two 32-bit numbers per instruction: half the issue slots of the same arithmetic (148 SMs, 8 warps each: 126 against 116 multiply-adds
+// per clock and SM when nothing else is issued, and the slots left over take the shared-memory loads).
+__device__ __forceinline__ uint64_t fma_pair(uint64_t a, uint64_t b, uint64_t c) {
+  uint64_t d;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+  return d;
+}
+__device__ __forceinline__ uint64_t mul_pair(uint64_t a, uint64_t b) {
+  uint64_t d;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+  return d;
+}
+__device__ __forceinline__ uint64_t pair_of(float lo, float hi) {
+  uint64_t d;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(d) : "f"(lo), "f"(hi));
+  return d;
+}
+__device__ __forceinline__ float sum_of_pair(uint64_t v) {
+  float lo, hi;
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v));
+  return lo + hi;
+}
+
+// Portions.  Per token a thread makes two dot products with its rows of the OLD state (S^T k and S^T q) and then writes; the
+// read-out is decay * S^T q + u * (k . q), so only S^T k stands in the chain from token to token, and the norms of q and k and k . q
+// are numbers per token that the staging computes (8 lanes a token), never rescaled rows.
+// The 32-bit pipe wants 4 operations per state element and token.  Shared memory delivers 128 bytes a clock to an SM's registers
+// whether the lanes read one address or 32, so rows that feed one column (64 rows x 1 column: 48 16-byte reads per thread and token in
+// the form before this one) bound the kernel; 32 rows x 2 columns read a third of that.  16 rows x 4 columns read less still and lost
+// it to shuffles and selects.  16 heads of 128 x 128 on B200: 8 prompts of 1024 tokens 764 -> 666 us, of 576 .. 1472 1083 -> 934,
+// one of 1500 1100 -> 633; 32 heads of 64 x 64: 713 -> 407, 1007 -> 572, 1017 -> 578.  A lone block now waits on its own chain
+// (about 800 clocks a token), a full SM on issue.  Blocks of 64 threads (32 columns at key size 128): a sequence's chain is as long as its portion, and with
+// small blocks every SM holds several sequences at once.
 // Stages of 16 tokens are double-buffered: the asynchronous copies of stage s + 1 (global -> shared, no registers) run behind the
 // arithmetic of stage s, so the dependent chain of a long portion never waits for memory.
-template <int KPT>
+template <int KPT, int R>
 __global__ void __launch_bounds__(256) delta_scan_kernel(DeltaArgs a) {
-  constexpr int STRIP = KPT + 4;
+  constexpr int STRIP = KPT + 4, row = R * STRIP, COLS = 2;
   extern __shared__ __align__(16) float sm[];
   const int b = blockIdx.x;
   const int q0 = a.cu_q[b], ql = a.cu_q[b + 1] - q0, ctx = a.seq_lens[b] - ql, slot = a.slots[b];
   if (slot < 0 || ctx < 0 || ql <= 0) return;
   const int h = blockIdx.y, hk = h / a.rep;
   const int j0 = blockIdx.z * a.dvt, nj = min(a.dvt, a.dv - j0);
-  const int dk = a.dk, R = a.R, row = R * STRIP, nthr = blockDim.x;
-  const int jl = threadIdx.x / R, r = threadIdx.x % R;
-  const bool live = jl < nj;
-  const int j = j0 + jl, i0 = r * KPT;
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarp = nthr >> 5;
-  const int stage_floats = 2 * DTCH * row + DTCH * a.dvt + 2 * DTCH;     // q, k [DTCH][row]; v [DTCH][dvt]; decays, strengths [DTCH]
-  float S[KPT];
-  float* sp = a.state + (((int64_t)slot * a.H + h) * a.dv + (live ? j : 0)) * dk;
+  const int dk = a.dk, nthr = blockDim.x;
+  const int r = threadIdx.x % R, c0 = threadIdx.x / R * COLS;          // key strip, first column (inside the slice)
+  const int i0 = r * KPT;
+  const int stage_floats = 2 * DTCH * row + DTCH * a.dvt + 8 * DTCH;     // q, k [DTCH][row]; v [DTCH][dvt]; eight numbers per token
+  uint64_t S[COLS][KPT / 2];
+  float* sp = a.state + (((int64_t)slot * a.H + h) * a.dv + j0 + c0) * dk;      // column c0 + c at sp + c * dk
   const bool vec = (dk & 3) == 0;        // every column of the state starts on a 16-byte boundary
 #pragma unroll
-  for (int ii = 0; ii < KPT; ii += 4) {
-    float4 t4 = make_float4(0.f, 0.f, 0.f, 0.f);
-    if (live && ctx > 0) {
-      if (vec && i0 + ii + 4 <= dk) t4 = *reinterpret_cast<const float4*>(sp + i0 + ii);
-      else {
-        if (i0 + ii < dk) t4.x = sp[i0 + ii];
-        if (i0 + ii + 1 < dk) t4.y = sp[i0 + ii + 1];
-        if (i0 + ii + 2 < dk) t4.z = sp[i0 + ii + 2];
-        if (i0 + ii + 3 < dk) t4.w = sp[i0 + ii + 3];
+  for (int c = 0; c < COLS; ++c)
+#pragma unroll
+    for (int ii = 0; ii < KPT; ii += 4) {
+      float4 t4 = make_float4(0.f, 0.f, 0.f, 0.f);
+      if (c0 + c < nj && ctx > 0) {
+        const float* p = sp + (int64_t)c * dk;
+        if (vec && i0 + ii + 4 <= dk) t4 = *reinterpret_cast<const float4*>(p + i0 + ii);
+        else {
+          if (i0 + ii < dk) t4.x = p[i0 + ii];
+          if (i0 + ii + 1 < dk) t4.y = p[i0 + ii + 1];
+          if (i0 + ii + 2 < dk) t4.z = p[i0 + ii + 2];
+          if (i0 + ii + 3 < dk) t4.w = p[i0 + ii + 3];
+        }
       }
+      S[c][ii / 2] = pair_of(t4.x, t4.y);
+      S[c][ii / 2 + 1] = pair_of(t4.z, t4.w);
     }
-    S[ii] = t4.x; S[ii + 1] = t4.y; S[ii + 2] = t4.z; S[ii + 3] = t4.w;
-  }
   // the strips' padding (beyond dk, and between strips) is read by the arithmetic and never copied into: zero it once
   for (int idx = threadIdx.x; idx < 2 * stage_floats; idx += nthr) sm[idx] = 0.f;
   __syncthreads();
@@ -89,7 +122,7 @@ __global__ void __launch_bounds__(256) delta_scan_kernel(DeltaArgs a) {
     float* qs = B;
     float* ks = B + DTCH * row;
     float* vs = ks + DTCH * row;
-    float* gs = vs + DTCH * a.dvt;
+    float* gs = vs + DTCH * a.dvt + 6 * DTCH;
     if (a.vec16) {
       const int n4 = dk >> 2;
       for (int idx = threadIdx.x; idx < nt * n4; idx += nthr) {
@@ -125,14 +158,17 @@ __global__ void __launch_bounds__(256) delta_scan_kernel(DeltaArgs a) {
     cp_async_commit();
   };
   issue(0, sm);
+  const int64_t ldo = (int64_t)a.H * a.dv;
+  float* op = a.out + q0 * ldo + (int64_t)h * a.dv + j0 + c0;
   int cur = 0;
   for (int t0 = 0; t0 < ql; t0 += DTCH, cur ^= 1) {
     const int nt = min(DTCH, ql - t0);
     float* qs = sm + cur * stage_floats;
     float* ks = qs + DTCH * row;
     float* vs = ks + DTCH * row;
-    float* gs = vs + DTCH * a.dvt;
-    float* bs = gs + DTCH;
+    float4* f4 = reinterpret_cast<float4*>(vs + DTCH * a.dvt);      // [DTCH] strength; strength * decay / |k|; 1 / |k|; decay
+    float2* f2 = reinterpret_cast<float2*>(f4 + DTCH);              // [DTCH] decay * q_scale / |q|; k . q of the scaled vectors
+    const float* raw = reinterpret_cast<const float*>(f2 + DTCH);   // [2][DTCH] log decays, write strengths as given
     if (t0 + DTCH < ql) {
       issue(t0 + DTCH, sm + (cur ^ 1) * stage_floats);
       cp_async_wait<1>();
@@ -140,64 +176,100 @@ __global__ void __launch_bounds__(256) delta_scan_kernel(DeltaArgs a) {
       cp_async_wait<0>();
     }
     __syncthreads();
-    if (threadIdx.x < nt) {
-      gs[threadIdx.x] = expf(gs[threadIdx.x]);
-      if (a.beta_sigmoid) bs[threadIdx.x] = 1.f / (1.f + expf(-bs[threadIdx.x]));
-    }
-    if (a.unit || a.q_scale != 1.f) {
-      for (int tt = warp; tt < nt; tt += nwarp) {
-        float sq = 0.f, sk = 0.f;
-        for (int w = lane; w < row; w += 32) {
-          sq = fmaf(qs[tt * row + w], qs[tt * row + w], sq);
-          sk = fmaf(ks[tt * row + w], ks[tt * row + w], sk);
-        }
-        sq = warp_sum(sq);
-        sk = warp_sum(sk);
-        const float rq = (a.unit ? rsqrtf(sq + a.unit_eps) : 1.f) * a.q_scale, rk = a.unit ? rsqrtf(sk + a.unit_eps) : 1.f;
-        for (int w = lane; w < row; w += 32) {
-          qs[tt * row + w] *= rq;
-          ks[tt * row + w] *= rk;
-        }
+    // (whole warps: the shuffles name all lanes; padding and rows past nt are zeros or older numbers that nobody reads)
+    for (int t8 = threadIdx.x >> 3; t8 < DTCH; t8 += nthr >> 3) {
+      const int l8 = threadIdx.x & 7;
+      float sq = 0.f, sk = 0.f, skq = 0.f;
+#pragma unroll
+      for (int w = 0; w < row; w += 32) {
+        if (w + l8 * 4 >= row) break;
+        const float4 x = *reinterpret_cast<const float4*>(qs + t8 * row + w + l8 * 4), y = *reinterpret_cast<const float4*>(ks + t8 * row + w + l8 * 4);
+        sq = fmaf(x.x, x.x, fmaf(x.y, x.y, fmaf(x.z, x.z, fmaf(x.w, x.w, sq))));
+        sk = fmaf(y.x, y.x, fmaf(y.y, y.y, fmaf(y.z, y.z, fmaf(y.w, y.w, sk))));
+        skq = fmaf(x.x, y.x, fmaf(x.y, y.y, fmaf(x.z, y.z, fmaf(x.w, y.w, skq))));
+      }
+      __syncwarp();
+#pragma unroll
+      for (int o = 4; o > 0; o >>= 1) {
+        sq += __shfl_xor_sync(0xffffffffu, sq, o);
+        sk += __shfl_xor_sync(0xffffffffu, sk, o);
+        skq += __shfl_xor_sync(0xffffffffu, skq, o);
+      }
+      if (l8 == 0 && t8 < nt) {
+        const float fq = (a.unit ? rsqrtf(sq + a.unit_eps) : 1.f) * a.q_scale, fk = a.unit ? rsqrtf(sk + a.unit_eps) : 1.f;
+        const float g = expf(raw[t8]), x = raw[DTCH + t8], be = a.beta_sigmoid ? 1.f / (1.f + expf(-x)) : x;
+        f4[t8] = make_float4(be, be * g * fk, fk, g);
+        f2[t8] = make_float2(g * fq, skq * fk * fq);
       }
     }
     __syncthreads();
-    for (int tt = 0; tt < nt; ++tt) {
-      const float g = gs[tt], be = bs[tt];
-      const float* kr = ks + tt * row + r * STRIP;
-      const float* qr = qs + tt * row + r * STRIP;
-      float d0 = 0.f, d1 = 0.f, d2 = 0.f, d3 = 0.f;
+    const float* kr = ks + r * STRIP;
+    const float* qr = qs + r * STRIP;
+    const float* vr = vs + c0;
+#pragma unroll 2
+    for (int tt = 0; tt < nt; ++tt, kr += row, qr += row, vr += a.dvt, op += ldo) {
+      const float4 f = f4[tt];
+      const float2 fo = f2[tt], v2 = *reinterpret_cast<const float2*>(vr);
+      uint64_t kk[KPT / 2], d0, d1, e0, e1;
 #pragma unroll
-      for (int ii = 0; ii < KPT; ii += 4) {
-        const float4 k4 = *reinterpret_cast<const float4*>(kr + ii);
-        d0 = fmaf(S[ii], k4.x, d0); d1 = fmaf(S[ii + 1], k4.y, d1); d2 = fmaf(S[ii + 2], k4.z, d2); d3 = fmaf(S[ii + 3], k4.w, d3);
+      for (int ii = 0; ii < KPT / 4; ++ii) {
+        const ulonglong2 k4 = *reinterpret_cast<const ulonglong2*>(kr + 4 * ii), q4 = *reinterpret_cast<const ulonglong2*>(qr + 4 * ii);
+        kk[2 * ii] = k4.x;
+        kk[2 * ii + 1] = k4.y;
+        if (ii == 0) {
+          d0 = mul_pair(S[0][0], k4.x); d1 = mul_pair(S[1][0], k4.x);
+          e0 = mul_pair(S[0][0], q4.x); e1 = mul_pair(S[1][0], q4.x);
+        } else {
+          d0 = fma_pair(S[0][2 * ii], k4.x, d0); d1 = fma_pair(S[1][2 * ii], k4.x, d1);
+          e0 = fma_pair(S[0][2 * ii], q4.x, e0); e1 = fma_pair(S[1][2 * ii], q4.x, e1);
+        }
+        d0 = fma_pair(S[0][2 * ii + 1], k4.y, d0); d1 = fma_pair(S[1][2 * ii + 1], k4.y, d1);
+        e0 = fma_pair(S[0][2 * ii + 1], q4.y, e0); e1 = fma_pair(S[1][2 * ii + 1], q4.y, e1);
       }
-      float d = (d0 + d1) + (d2 + d3);
-      for (int o = R >> 1; o > 0; o >>= 1) d += __shfl_xor_sync(0xffffffffu, d, o);
-      const float u = be * (vs[tt * a.dvt + jl] - g * d);
-      float e0 = 0.f, e1 = 0.f, e2 = 0.f, e3 = 0.f;
+      float x0 = sum_of_pair(d0), x1 = sum_of_pair(d1);
 #pragma unroll
-      for (int ii = 0; ii < KPT; ii += 4) {
-        const float4 k4 = *reinterpret_cast<const float4*>(kr + ii);
-        const float4 q4 = *reinterpret_cast<const float4*>(qr + ii);
-        S[ii] = fmaf(g, S[ii], k4.x * u); S[ii + 1] = fmaf(g, S[ii + 1], k4.y * u);
-        S[ii + 2] = fmaf(g, S[ii + 2], k4.z * u); S[ii + 3] = fmaf(g, S[ii + 3], k4.w * u);
-        e0 = fmaf(S[ii], q4.x, e0); e1 = fmaf(S[ii + 1], q4.y, e1); e2 = fmaf(S[ii + 2], q4.z, e2); e3 = fmaf(S[ii + 3], q4.w, e3);
+      for (int o = R >> 1; o > 0; o >>= 1) {
+        x0 += __shfl_xor_sync(0xffffffffu, x0, o);
+        x1 += __shfl_xor_sync(0xffffffffu, x1, o);
       }
-      float o = (e0 + e1) + (e2 + e3);
-      for (int s = R >> 1; s > 0; s >>= 1) o += __shfl_xor_sync(0xffffffffu, o, s);
-      if (live && r == 0) a.out[(int64_t)(q0 + t0 + tt) * a.H * a.dv + (int64_t)h * a.dv + j] = o;
+      const float u0 = fmaf(f.x, v2.x, -f.y * x0), u1 = fmaf(f.x, v2.y, -f.y * x1);
+      const float w0 = u0 * f.z, w1 = u1 * f.z;
+      const uint64_t g2 = pair_of(f.w, f.w), p0 = pair_of(w0, w0), p1 = pair_of(w1, w1);
+#pragma unroll
+      for (int ii = 0; ii < KPT / 2; ++ii) {
+        S[0][ii] = fma_pair(g2, S[0][ii], mul_pair(kk[ii], p0));
+        S[1][ii] = fma_pair(g2, S[1][ii], mul_pair(kk[ii], p1));
+      }
+      // S^T q of the old state: the first exchange leaves one column per lane
+      const float y0 = sum_of_pair(e0), y1 = sum_of_pair(e1);
+      if (R > 1) {
+        const bool hi = r & (R >> 1);
+        float y = (hi ? y1 : y0) + __shfl_xor_sync(0xffffffffu, hi ? y0 : y1, R >> 1);
+#pragma unroll
+        for (int o = R >> 2; o > 0; o >>= 1) y += __shfl_xor_sync(0xffffffffu, y, o);
+        if ((r & ((R >> 1) - 1)) == 0 && c0 + hi < nj) op[hi] = fmaf(fo.x, y, (hi ? u1 : u0) * fo.y);
+      } else {
+        if (c0 < nj) op[0] = fmaf(fo.x, y0, u0 * fo.y);
+        if (c0 + 1 < nj) op[1] = fmaf(fo.x, y1, u1 * fo.y);
+      }
     }
     __syncthreads();      // this buffer is copied into again at the start of the next round
   }
-  if (live) {
+#pragma unroll
+  for (int c = 0; c < COLS; ++c) {
+    if (c0 + c >= nj) continue;
+    float* p = sp + (int64_t)c * dk;
 #pragma unroll
     for (int ii = 0; ii < KPT; ii += 4) {
-      if (vec && i0 + ii + 4 <= dk) *reinterpret_cast<float4*>(sp + i0 + ii) = make_float4(S[ii], S[ii + 1], S[ii + 2], S[ii + 3]);
+      float4 t4;
+      asm("mov.b64 {%0, %1}, %2;" : "=f"(t4.x), "=f"(t4.y) : "l"(S[c][ii / 2]));
+      asm("mov.b64 {%0, %1}, %2;" : "=f"(t4.z), "=f"(t4.w) : "l"(S[c][ii / 2 + 1]));
+      if (vec && i0 + ii + 4 <= dk) *reinterpret_cast<float4*>(p + i0 + ii) = t4;
       else {
-        if (i0 + ii < dk) sp[i0 + ii] = S[ii];
-        if (i0 + ii + 1 < dk) sp[i0 + ii + 1] = S[ii + 1];
-        if (i0 + ii + 2 < dk) sp[i0 + ii + 2] = S[ii + 2];
-        if (i0 + ii + 3 < dk) sp[i0 + ii + 3] = S[ii + 3];
+        if (i0 + ii < dk) p[i0 + ii] = t4.x;
+        if (i0 + ii + 1 < dk) p[i0 + ii + 1] = t4.y;
+        if (i0 + ii + 2 < dk) p[i0 + ii + 2] = t4.z;
+        if (i0 + ii + 3 < dk) p[i0 + ii + 3] = t4.w;
       }
     }
   }
@@ -298,7 +370,7 @@ LLMSS_API int llmss_delta_scan(const float* q, int64_t ldq, const float* k, int6
   a.unit = unit_eps >= 0.f ? 1 : 0; a.unit_eps = unit_eps >= 0.f ? unit_eps : 0.f; a.q_scale = q_scale; a.beta_sigmoid = beta_sigmoid;
   if (max_q <= 1 && dk <= 256) {
     // every sequence brings one token: one warp per value column, lanes over the key rows
-    a.R = 1; a.dvt = 0;
+    a.dvt = 0;
     const int per_pass = STEP_WARPS * STEP_COLS;
     int groups = 1;
     while ((int64_t)B * heads * groups < 1024 && groups * per_pass < dv) groups *= 2;
@@ -314,32 +386,33 @@ LLMSS_API int llmss_delta_scan(const float* q, int64_t ldq, const float* k, int6
     LLMSS_CHECK_CUDA(cudaGetLastError());
     return 0;
   }
-  // key rows per thread: the key size itself up to 64 (a column per thread), 64 beyond (R lanes per column)
-  static const int kpt_max = [] { const char* e = getenv("LLMSS_DELTA_KPT"); const int v = e ? atoi(e) : 64; return v == 32 || v == 128 ? v : 64; }();
-  int kpt = dk <= 8 ? 8 : (dk <= 16 ? 16 : (dk <= 32 ? 32 : (dk <= 64 ? 64 : 128)));
-  if (kpt > kpt_max) kpt = kpt_max;
+  // up to 32 key rows per thread, R lanes (a power of two) to a column pair
+  const int kpt = dk <= 8 ? 8 : (dk <= 16 ? 16 : 32);
   int R = 1;
   while (R * kpt < dk) R *= 2;
-  a.R = R;
-  int threads = ((dv * R + 31) / 32) * 32;
-  threads = threads > 256 ? 256 : threads;
-  a.dvt = threads / R;
+  int threads = (((dv + 1) / 2 * R + 31) / 32) * 32;
+  const int most = R <= 4 ? 64 : 256;       // long keys: a stage of q and k is shared by more columns
+  threads = threads > most ? most : threads;
+  a.dvt = threads / R * 2;
   const dim3 grid(B, heads, (dv + a.dvt - 1) / a.dvt);
   LLMSS_REQUIRE(grid.y <= 65535 && grid.z <= 65535, "delta_scan: grid too large");
   a.vec16 = (dk % 4 == 0 && dv % 4 == 0 && a.dvt % 4 == 0 && ldq % 4 == 0 && ldk % 4 == 0 && ldv % 4 == 0 &&
              (((uintptr_t)q | (uintptr_t)k | (uintptr_t)v) & 15) == 0) ? 1 : 0;
-  const size_t smem = 2 * sizeof(float) * ((size_t)2 * DTCH * R * (kpt + 4) + (size_t)DTCH * a.dvt + 2 * DTCH);
-#define LLMSS_DS(K)                                                                     \
-  do {                                                                                  \
-    static PerDeviceSmem gsm;                                                           \
-    if (smem > 48 * 1024) LLMSS_CHECK_CUDA(gsm.ensure(delta_scan_kernel<K>, (int)smem)); \
-    delta_scan_kernel<K><<<grid, threads, smem, stream>>>(a);                           \
+  const size_t smem = 2 * sizeof(float) * ((size_t)2 * DTCH * R * (kpt + 4) + (size_t)DTCH * a.dvt + 8 * DTCH);
+#define LLMSS_DS(K, RR)                                                                     \
+  do {                                                                                      \
+    static PerDeviceSmem gsm;                                                               \
+    if (smem > 48 * 1024) LLMSS_CHECK_CUDA(gsm.ensure(delta_scan_kernel<K, RR>, (int)smem)); \
+    delta_scan_kernel<K, RR><<<grid, threads, smem, stream>>>(a);                           \
   } while (0)
-  if (kpt == 8) LLMSS_DS(8);
-  else if (kpt == 16) LLMSS_DS(16);
-  else if (kpt == 32) LLMSS_DS(32);
-  else if (kpt == 64) LLMSS_DS(64);
-  else LLMSS_DS(128);
+  if (kpt == 8) LLMSS_DS(8, 1);
+  else if (kpt == 16) LLMSS_DS(16, 1);
+  else if (R == 1) LLMSS_DS(32, 1);
+  else if (R == 2) LLMSS_DS(32, 2);
+  else if (R == 4) LLMSS_DS(32, 4);
+  else if (R == 8) LLMSS_DS(32, 8);
+  else if (R == 16) LLMSS_DS(32, 16);
+  else LLMSS_DS(32, 32);
 #undef LLMSS_DS
   LLMSS_CHECK_CUDA(cudaGetLastError());
   return 0;

@@ -1,0 +1,60 @@
+"""Prompt-side kernels at the edges of their tiles against the plain recurrences / sums in float64."""
+import pytest
+import torch
+
+from llmss_b200 import ops
+from llmss_b200.engine.batch import BatchInput
+
+pytestmark = pytest.mark.gpu
+
+F32, F64 = torch.float32, torch.float64
+
+
+def _batch(lens, ctxs, slots):
+    cu = torch.tensor([0] + list(lens)).cumsum(0).to(torch.int32)
+    i32 = dict(dtype=torch.int32, device="cuda")
+    z = torch.zeros(1, **i32)
+    return BatchInput(tokens=z, positions=z, slot_mapping=z, block_tables=z.view(1, 1), seq_lens=torch.tensor([a + b for a, b in zip(lens, ctxs)], **i32),
+                      cu_q=cu.cuda(), last_idx=z, num_seqs=len(lens), max_q=max(lens), max_kv=1, is_decode=False, is_fresh_prefill=False,
+                      state_slots=torch.tensor(slots, **i32))
+
+
+def _rel(got, want):
+    return float((got.double().cpu() - want).norm() / want.norm().clamp_min(1e-30))
+
+
+@pytest.mark.parametrize("dk,dv,heads,qk_heads,unit", [(128, 128, 2, 1, True), (64, 64, 2, 2, True), (24, 16, 2, 1, False), (8, 3, 3, 3, True),
+                                                       (100, 70, 2, 2, True), (200, 40, 1, 1, False), (300, 10, 1, 1, True)])
+@pytest.mark.parametrize("copies", [1, 40])
+def test_delta_portions(dk, dv, heads, qk_heads, unit, copies):
+    """Portions around the 16-token stages, states carried over; ``copies`` > 1 has enough columns in flight for 64 key rows per
+    thread.  Bound: 32-bit sums, 3e-6 of the norm."""
+    torch.manual_seed(dk + dv)
+    lens, ctxs = [16, 1, 33, 47][:4 if copies == 1 else 2] * copies, [0, 3, 8, 0][:4 if copies == 1 else 2] * copies
+    slots, T = list(range(len(lens))), sum(lens)
+    q, k, v = (torch.randn(T, n, device="cuda") for n in (qk_heads * dk, qk_heads * dk, heads * dv))
+    if not unit:        # keys of norm 1 keep the rule stable
+        k = torch.nn.functional.normalize(k.view(T, qk_heads, dk), dim=-1).reshape(T, -1)
+    g, b = -torch.rand(T, heads, device="cuda") * 0.3, torch.randn(T, heads, device="cuda")
+    state = torch.randn(len(lens), heads, dk, dv, device="cuda") * 0.1
+    S0 = state.reshape(len(lens), heads, dv, dk).transpose(2, 3).double().cpu()
+    rep = heads // qk_heads
+    qf, kf = (x.double().cpu().view(T, qk_heads, dk) for x in (q, k))
+    if unit:
+        qf, kf = (x * torch.rsqrt(x.square().sum(-1, keepdim=True) + 1e-6) for x in (qf, kf))
+    qf, kf, vf = (qf * 0.25).repeat_interleave(rep, 1), kf.repeat_interleave(rep, 1), v.double().cpu().view(T, heads, dv)
+    a, beta = torch.exp(g.double().cpu()), torch.sigmoid(b.double().cpu())
+    want, at, ends = torch.zeros_like(vf), 0, []
+    for i, n in enumerate(lens):
+        S = S0[i].clone() if ctxs[i] else torch.zeros(heads, dk, dv, dtype=F64)
+        for t in range(at, at + n):
+            S = S * a[t][:, None, None]
+            u = beta[t][:, None] * (vf[t] - torch.einsum("hkv,hk->hv", S, kf[t]))
+            S = S + kf[t][:, :, None] * u[:, None, :]
+            want[t] = torch.einsum("hkv,hk->hv", S, qf[t])
+        ends.append(S)
+        at += n
+    got = ops.delta_scan(q, k, v, g, b, _batch(lens, ctxs, slots), state, heads, qk_heads, dk, dv, unit_eps=1e-6 if unit else None, q_scale=0.25,
+                         beta_sigmoid=True)
+    assert _rel(got, want.reshape(T, -1)) < 3e-6
+    assert _rel(state.reshape(len(lens), heads, dv, dk).transpose(2, 3), torch.stack(ends)) < 3e-6
