@@ -101,6 +101,8 @@ struct GemmArgs {
   int64_t ag_ld;
   const CUtensorMap* ag_maps;  // ag: device array [2 parities] of maps over the gathered [M, K] activation (local)
   int tm_rot;                  // token-tile rotation: with ag, every rank starts on the tiles of its own shard
+  const int* groups;           // grouped pair kernel: [E + 1] first row of every group, then [E + 1] first token tile
+  int n_groups;                // E
   unsigned long long* dbg;  // optional per-CTA phase timestamps [grid][8] (globaltimer ns), see llmss_gemm_set_debug
   SymmWs ws;
 };
@@ -317,7 +319,8 @@ __device__ __forceinline__ void store_chunk_full_t(const GemmArgs& a, const floa
         r += 2 * a.ldr;
       }
   } else {
-    T* o = reinterpret_cast<T*>(a.out) + (int64_t)mb0 * a.ldo + n;
+    using TO = typename std::conditional<EPI == EPI_F32, float, T>::type;
+    TO* o = reinterpret_cast<TO*>(a.out) + (int64_t)mb0 * a.ldo + n;
     const T* r = reinterpret_cast<const T*>(a.residual) + (int64_t)mb0 * a.ldr + n;
     const bool do_act = n >= a.act_start;
 #pragma unroll
@@ -326,15 +329,15 @@ __device__ __forceinline__ void store_chunk_full_t(const GemmArgs& a, const floa
       for (int j = 0; j < 8; ++j) {
         const float x = v[u][j] + bval;
         const float y = do_act ? act_t<ACT>(x, a.act) : x;
-        *o = from_f32<T>(y + (has_res ? to_f32(*r) : 0.f));
+        *o = from_f32<TO>(y + (has_res ? to_f32(*r) : 0.f));
         o += a.ldo;
         r += a.ldr;
       }
   }
 }
-// Dispatch of the full-chunk stores; false = flavour without a fast form (fp32 output): use store_chunk.
+// Dispatch of the full-chunk stores.
 template <typename T, int CH>
-__device__ __forceinline__ bool store_chunk_full(const GemmArgs& a, const float (&v)[CH][8], int n, int mb0, int lane, float bval) {
+__device__ __forceinline__ void store_chunk_full(const GemmArgs& a, const float (&v)[CH][8], int n, int mb0, int lane, float bval) {
   if (a.epi == EPI_PLAIN) {
     store_chunk_plain_full<T, CH>(a, v, n, mb0, bval);
   } else if (a.epi == EPI_ACT) {
@@ -348,9 +351,10 @@ __device__ __forceinline__ bool store_chunk_full(const GemmArgs& a, const float 
     else if (a.act == LLMSS_ACT_GELU_TANH) store_chunk_full_t<T, CH, EPI_GATED, LLMSS_ACT_GELU_TANH>(a, v, n, mb0, lane, bval);
     else store_chunk_full_t<T, CH, EPI_GATED, ACT_RUNTIME>(a, v, n, mb0, lane, bval);
   } else {
-    return false;
+    if (a.act == LLMSS_ACT_NONE) store_chunk_full_t<T, CH, EPI_F32, LLMSS_ACT_NONE>(a, v, n, mb0, lane, bval);
+    else if (a.act == LLMSS_ACT_SILU) store_chunk_full_t<T, CH, EPI_F32, LLMSS_ACT_SILU>(a, v, n, mb0, lane, bval);
+    else store_chunk_full_t<T, CH, EPI_F32, ACT_RUNTIME>(a, v, n, mb0, lane, bval);
   }
-  return true;
 }
 
 // ---- thread-block-cluster helpers (split-K kernel) ----
@@ -1219,9 +1223,31 @@ struct PCfg2 {
   static constexpr int STAGE_BYTES = W_BYTES + X_BYTES;
   static constexpr int STAGES = 6;               // 192 KB ring; the parked fp32 tile of the split-K schedule (128 KB) reuses it
   static constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + 1024 /*align*/ + 512 /*barriers*/;
+  static constexpr int MAX_GROUPS = 256, GROUP_BYTES = 2 * (MAX_GROUPS + 1) * 4;   // grouped form: its table, behind the barriers
 };
 
-template <typename T>
+// Grouped form (routed experts): the rows of x are sorted into E contiguous groups of any size, group e is multiplied by its own
+// [N, K] weight (a 3-D tensor map [K, N, E]), and the row ranges are read from device memory, so nothing of the routing passes the
+// host.  Tiles run group by group, feature tile by feature tile, token tile fastest; a tile's token rows may reach into the next
+// group (their columns are computed and not stored).  8192 tokens, 4 of 16 experts of 1024, width 2048: the block's pass with every
+// expert for every token 963 us, with this 429 us.
+struct GroupTile {
+  int e, fn, row0, row_end;      // group, feature tile of the pair, first token row, end of the group's rows
+};
+struct GroupWalk {
+  const int* rows;               // [E + 1]
+  const int* tiles;              // [E + 1] token tiles in front of group e
+  int e = 0, ptn;
+  __device__ GroupWalk(const int* table, int E, int pair_tiles_n) : rows(table), tiles(table + E + 1), ptn(pair_tiles_n) {}
+  // tile < ptn * tiles[E], called with growing tiles
+  __device__ __forceinline__ GroupTile at(int tile) {
+    while (tile >= ptn * tiles[e + 1]) ++e;
+    const int local = tile - ptn * tiles[e], tm = tiles[e + 1] - tiles[e];
+    return GroupTile{e, local / tm, rows[e] + (local % tm) * PCfg2::BN, rows[e + 1]};
+  }
+};
+
+template <typename T, bool GROUPED>
 __global__ void __launch_bounds__(kNumThreads, 1)
 gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant__ CUtensorMap tmap_x,
                  const __grid_constant__ GemmArgs a) {
@@ -1241,7 +1267,8 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_consta
   const int CS = (int)cluster_nctarank(), r = (int)cluster_ctarank();
   const int S = CS >> 1, p = r >> 1, h = r & 1;
   const int pair_tiles_n = (a.tiles_n + 1) >> 1;
-  const int n_tiles = pair_tiles_n * a.tiles_m;
+  int n_tiles = pair_tiles_n * a.tiles_m;
+  int* group_table = reinterpret_cast<int*>(tmem_slot + 4);
   const int n_clusters = (int)gridDim.x / CS, cluster_id = (int)blockIdx.x / CS;   // S > 1: n_clusters == n_tiles
   const int kb0 = (int)(((int64_t)p * a.kb_total) / S), kb1 = (int)(((int64_t)(p + 1) * a.kb_total) / S);
   constexpr int NG = BN / 8;
@@ -1277,6 +1304,12 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_consta
   const uint32_t tmem_base = *tmem_slot;
   float4* staging = reinterpret_cast<float4*>(smem);  // split-K: [NG*2][128] float4, reuses the drained TMA ring
   pdl_wait();
+  if (GROUPED) {
+    for (int i = threadIdx.x; i < 2 * (a.n_groups + 1); i += kNumThreads) group_table[i] = a.groups[i];
+    __syncthreads();
+    n_tiles = pair_tiles_n * group_table[2 * a.n_groups + 1];
+  }
+  GroupWalk walk(group_table, a.n_groups, pair_tiles_n);     // each role walks the tiles on its own
   if (threadIdx.x == 0) LLMSS_STAMP(1);
 
   if (warp == 0) {
@@ -1287,14 +1320,23 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_consta
     for (int tile = cluster_id; tile < n_tiles && dbg_mode != 3; tile += n_clusters) {
       // token tile fastest: the pairs running at the same time share ONE weight tile (streamed from HBM once, L2 hits
       // for the others) and sweep the activation, which stays L2-resident across the weight tiles
-      const int tn = (tile / a.tiles_m) * 2 + h;        // this CTA's 128-feature tile (may lie past N: zero-filled, unstored)
-      const int xrow = (tile % a.tiles_m) * BN + (h ^ (a.aligned & 1)) * C::XH;   // a.aligned: bring-up switch for the half order
+      int tn, xrow, group = 0;        // tn: this CTA's 128-feature tile (may lie past N: zero-filled, unstored)
+      if (GROUPED) {
+        const GroupTile t = walk.at(tile);
+        tn = t.fn * 2 + h;
+        xrow = t.row0 + h * C::XH;
+        group = t.e;
+      } else {
+        tn = (tile / a.tiles_m) * 2 + h;
+        xrow = (tile % a.tiles_m) * BN + (h ^ (a.aligned & 1)) * C::XH;   // a.aligned: bring-up switch for the half order
+      }
       for (int kb = kb0; kb < kb1; ++kb) {
         mbar_wait(&empty_bar[stage], phase ^ 1, 60);
         uint8_t* sw = smem + stage * C::STAGE_BYTES;
         if (elect_one()) {
           mbar_arrive_expect_tx(&full_bar[stage], C::STAGE_BYTES);
-          tma_load_2d(sw, &tmap_w, &full_bar[stage], kb * BK, tn * BM, pol_w);
+          if (GROUPED) tma_load_3d(sw, &tmap_w, &full_bar[stage], kb * BK, tn * BM, group, pol_w);
+          else tma_load_2d(sw, &tmap_w, &full_bar[stage], kb * BK, tn * BM, pol_w);
           tma_load_2d(sw + C::W_BYTES, &tmap_x, &full_bar[stage], kb * BK, xrow, pol_x);
         }
         __syncwarp();
@@ -1358,26 +1400,35 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_consta
     uint32_t aphase = 0;
     const uint32_t tempty_leader = mapa_shared(smem_u32(&tempty_bar[0]), (uint32_t)(r & ~1));
     for (int tile = cluster_id; tile < n_tiles; tile += n_clusters) {
-      const int tn = (tile / a.tiles_m) * 2 + h, tm = tile % a.tiles_m;
-      const int n = tn * BM + f, m0 = tm * BN;
+      int tn, m0, m_end = a.M;
+      if (GROUPED) {
+        const GroupTile t = walk.at(tile);
+        tn = t.fn * 2 + h;
+        m0 = t.row0;
+        m_end = t.row_end;
+      } else {
+        tn = (tile / a.tiles_m) * 2 + h;
+        m0 = (tile % a.tiles_m) * BN;
+      }
+      const int n = tn * BM + f;
       const uint32_t t_addr = tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(as * BN);
       mbar_wait(&tfull_bar[as], aphase, 64);  // all MMAs of the tile retired => its stages of BOTH CTAs have been consumed
       tcgen05_fence_after();
       if (threadIdx.x == 64) LLMSS_STAMP(5);
-      if (S == 1) {
+      if (GROUPED || S == 1) {
         // ---- straight out of tensor memory, CH groups of 8 token columns at a time (residuals fetched ahead)
         constexpr int CH = 4;
         const float bval = (bias != nullptr && n < a.N) ? to_f32(bias[n]) : 0.f;
-        // fast stores need the warp's 32 features in range (warp-uniform: the gated flavour shuffles) and a flavour that
-        // has one; the row test below is per chunk
-        const bool plain_ok = a.epi != EPI_F32 && tn * BM + quarter * 32 + 32 <= a.N;
+        // fast stores need the warp's 32 features in range (warp-uniform: the gated flavour shuffles); the row test below is
+        // per chunk
+        const bool plain_ok = tn * BM + quarter * 32 + 32 <= a.N;
 #pragma unroll 1
         for (int cg0 = 0; cg0 < NG; cg0 += CH) {
           float v[CH][8], rv[CH][8];
-          const bool fast = plain_ok && m0 + (cg0 + CH) * 8 <= a.M;
+          const bool fast = plain_ok && m0 + (cg0 + CH) * 8 <= m_end;
           if (!fast) {
 #pragma unroll
-            for (int u = 0; u < CH; ++u) epilogue_load_res8<T>(a, rv[u], n, m0 + (cg0 + u) * 8, lane, a.M);
+            for (int u = 0; u < CH; ++u) epilogue_load_res8<T>(a, rv[u], n, m0 + (cg0 + u) * 8, lane, m_end);
           }
           {
             // one 32-column load and ONE wait per chunk: a tensor-memory round trip is ~0.3 us, and paying it per 8
@@ -1396,7 +1447,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_consta
             if (lane == 0) mbar_arrive_remote(tempty_leader + (uint32_t)(as * 8));
           }
           if (fast) store_chunk_full<T, CH>(a, v, n, m0 + cg0 * 8, lane, bval);
-          else store_chunk<T, CH>(a, v, rv, n, m0 + cg0 * 8, lane, bval, a.M);
+          else store_chunk<T, CH>(a, v, rv, n, m0 + cg0 * 8, lane, bval, m_end);
         }
       } else {
         // ---- split-K: park the partial accumulator in shared memory: [(cg*2 + half)][feature] float4, conflict-free
@@ -1414,7 +1465,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_consta
       if (++as == 2) { as = 0; aphase ^= 1; }
     }
   }
-  if (S > 1) {   // cluster-uniform: one tile per cluster, partials parked above
+  if (!GROUPED && S > 1) {   // cluster-uniform: one tile per cluster, partials parked above
     tcgen05_fence_before();
     __syncwarp();
     cluster_sync_all();  // every CTA's partial tile is parked and visible cluster-wide
@@ -1587,17 +1638,18 @@ int launch_cluster(const CUtensorMap& tw, const CUtensorMap& tx, const GemmArgs&
               : launch_cluster_ar<T, BN, false>(tw, tx, a, tiles, split, stream);
 }
 
-template <typename T>
+template <typename T, bool GROUPED = false>
 int launch_pair(const CUtensorMap& tw, const CUtensorMap& tx, const GemmArgs& a, int clusters, int split,
                 cudaStream_t stream) {
   static PerDeviceSmem configured;
-  auto kern = gemm_pair_kernel<T>;
-  LLMSS_CHECK_CUDA(configured.ensure(kern, PCfg2::SMEM_BYTES));
+  auto kern = gemm_pair_kernel<T, GROUPED>;
+  constexpr int smem = PCfg2::SMEM_BYTES + (GROUPED ? PCfg2::GROUP_BYTES : 0);
+  LLMSS_CHECK_CUDA(configured.ensure(kern, smem));
   cudaLaunchConfig_t cfg;
   memset(&cfg, 0, sizeof(cfg));
   cfg.gridDim = dim3(clusters * 2 * split);
   cfg.blockDim = dim3(kNumThreads);
-  cfg.dynamicSmemBytes = PCfg2::SMEM_BYTES;
+  cfg.dynamicSmemBytes = smem;
   cfg.stream = stream;
   cudaLaunchAttribute attr[2];
   attr[0].id = cudaLaunchAttributeClusterDimension;
@@ -1984,4 +2036,44 @@ LLMSS_API int llmss_gemm_ex(const void* x, int64_t ldx, const void* w, int64_t l
     }
   }
 #undef LLMSS_LAUNCH
+}
+
+// Grouped linear layers (routed experts): rows [rows[e], rows[e + 1]) of x [P, K] times w_e [N, K] (element (n, k) of group e at
+// w + e * w_group_stride + n * ldw + k) -> the same rows of out.  groups: device table [rows[0..E] | first token tile of 256
+// rows, [0..E]] as llmss_moe_group writes it.  Nothing is read on the host.  gated: rows of w_e interleave (gate, up).
+LLMSS_API int llmss_gemm_grouped(const void* x, int64_t ldx, const void* w, int64_t ldw, int64_t w_group_stride, const int* groups, int E,
+                                 void* out, int64_t ldo, int P, int N, int K, int dtype, int out_f32, int act, int gated,
+                                 cudaStream_t stream) {
+  LLMSS_REQUIRE(dtype == LLMSS_F16 || dtype == LLMSS_BF16, "gemm_grouped: dtype must be f16/bf16");
+  LLMSS_REQUIRE(P > 0 && N > 0 && K > 0 && K % 8 == 0 && E > 0 && E <= PCfg2::MAX_GROUPS, "gemm_grouped: bad shape P=%d N=%d K=%d E=%d", P, N, K, E);
+  LLMSS_REQUIRE(!(gated && out_f32) && (!gated || N % 2 == 0), "gemm_grouped: a gated product has an even N and a 16-bit result");
+  LLMSS_REQUIRE(((uintptr_t)w % 16) == 0 && ldw % 8 == 0 && w_group_stride % 8 == 0, "gemm_grouped: weights off the 16-byte lines");
+  PFN_encodeTiled enc = get_encode();
+  LLMSS_REQUIRE(enc != nullptr, "gemm_grouped: cuTensorMapEncodeTiled entry point not available");
+  CUtensorMap tw, tx;
+  cuuint64_t dims[3] = {(cuuint64_t)K, (cuuint64_t)N, (cuuint64_t)E};
+  cuuint64_t strides[2] = {(cuuint64_t)ldw * 2, (cuuint64_t)w_group_stride * 2};
+  cuuint32_t box[3] = {(cuuint32_t)BK, (cuuint32_t)BM, 1}, estr[3] = {1, 1, 1};
+  CUresult r = enc(&tw, dtype == LLMSS_BF16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 3, const_cast<void*>(w), dims,
+                   strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                   CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  LLMSS_REQUIRE(r == CUDA_SUCCESS, "gemm_grouped: cuTensorMapEncodeTiled failed with CUresult %d", (int)r);
+  if (int e = make_tmap(&tx, x, dtype, P, K, ldx, PCfg2::XH)) return e;
+  GemmArgs a;
+  memset(&a, 0, sizeof(a));
+  a.M = P; a.N = N; a.K = K;
+  a.tiles_n = (N + BM - 1) / BM;
+  a.kb_total = (K + BK - 1) / BK;
+  a.dtype = dtype;
+  a.out = out; a.ldo = ldo; a.out_f32 = out_f32;
+  a.act = act; a.gated = gated;
+  a.epi = gated ? EPI_GATED : (out_f32 ? EPI_F32 : (act != LLMSS_ACT_NONE ? EPI_ACT : EPI_PLAIN));
+  a.groups = groups; a.n_groups = E;
+  // as many persistent pairs as the machine holds; never more than there can be tiles
+  const int64_t most = (int64_t)((a.tiles_n + 1) / 2) * ((int64_t)P / PCfg2::BN + (P < E ? P : E));
+  int clusters = num_sms() / 2;
+  if (clusters > most) clusters = (int)most;
+  if (clusters < 1) clusters = 1;
+  return dtype == LLMSS_F16 ? launch_pair<__half, true>(tw, tx, a, clusters, 1, stream)
+                            : launch_pair<__nv_bfloat16, true>(tw, tx, a, clusters, 1, stream);
 }

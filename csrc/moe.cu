@@ -22,22 +22,24 @@ constexpr int kMaxGroupTop = 4;  // a group scores as the sum of at most this ma
 // score_kind 0: s = softmax(z); 1: s = sigmoid(z).  Experts are chosen by c = s + correction (correction may be null); the
 // weights are the chosen experts' s.  A group scores as the sum of its `group_top` largest c (1: its best expert).
 // renorm: weights / (their sum + 1e-20).  Experts outside the kept groups are never chosen, whatever the sign of c.
+// PL experts per lane: 32 * PL >= E
+template <int PL>
 __global__ void __launch_bounds__(128) moe_route_kernel(const float* __restrict__ z, int64_t ldz, int E, int top, int groups,
                                                         int keep, float route_scale, int score_kind,
                                                         const float* __restrict__ correction, int group_top, int renorm,
                                                         int* __restrict__ ids, float* __restrict__ wts,
                                                         float* __restrict__ dense, int T) {
-  __shared__ float cs_all[4][32 * kMaxPerLane];
+  __shared__ float cs_all[4][32 * PL];
   const int t = blockIdx.x * 4 + (threadIdx.x >> 5);
   const int lane = threadIdx.x & 31;
   if (t >= T) return;
   float* cs = cs_all[threadIdx.x >> 5];
   const float* zr = z + (int64_t)t * ldz;
-  float s[kMaxPerLane], c[kMaxPerLane];
-  bool ok[kMaxPerLane];
+  float s[PL], c[PL];
+  bool ok[PL];
   float mx = -INFINITY;
 #pragma unroll
-  for (int i = 0; i < kMaxPerLane; ++i) {
+  for (int i = 0; i < PL; ++i) {
     const int e = lane + i * 32;
     s[i] = e < E ? zr[e] : -INFINITY;
     mx = fmaxf(mx, s[i]);
@@ -46,20 +48,20 @@ __global__ void __launch_bounds__(128) moe_route_kernel(const float* __restrict_
     mx = warp_max(mx);
     float sum = 0.f;
 #pragma unroll
-    for (int i = 0; i < kMaxPerLane; ++i) {
+    for (int i = 0; i < PL; ++i) {
       const int e = lane + i * 32;
       s[i] = e < E ? expf(s[i] - mx) : 0.f;
       sum += s[i];
     }
     sum = warp_sum(sum);
 #pragma unroll
-    for (int i = 0; i < kMaxPerLane; ++i) s[i] /= sum;
+    for (int i = 0; i < PL; ++i) s[i] /= sum;
   } else {
 #pragma unroll
-    for (int i = 0; i < kMaxPerLane; ++i) s[i] = lane + i * 32 < E ? 1.f / (1.f + expf(-s[i])) : 0.f;
+    for (int i = 0; i < PL; ++i) s[i] = lane + i * 32 < E ? 1.f / (1.f + expf(-s[i])) : 0.f;
   }
 #pragma unroll
-  for (int i = 0; i < kMaxPerLane; ++i) {
+  for (int i = 0; i < PL; ++i) {
     const int e = lane + i * 32;
     c[i] = e < E ? s[i] + (correction != nullptr ? correction[e] : 0.f) : -INFINITY;
     ok[i] = false;
@@ -68,9 +70,9 @@ __global__ void __launch_bounds__(128) moe_route_kernel(const float* __restrict_
   __syncwarp();
   // group scores: lane l owns groups l, l + 32, ...
   const int gsz = E / groups;
-  float gs[kMaxPerLane];
+  float gs[PL];
 #pragma unroll
-  for (int j = 0; j < kMaxPerLane; ++j) {
+  for (int j = 0; j < PL; ++j) {
     const int g = lane + j * 32;
     gs[j] = -INFINITY;
     if (g >= groups) continue;
@@ -95,7 +97,7 @@ __global__ void __launch_bounds__(128) moe_route_kernel(const float* __restrict_
     float bv = -INFINITY;
     int bg = 0x7fffffff;
 #pragma unroll
-    for (int j = 0; j < kMaxPerLane; ++j) {
+    for (int j = 0; j < PL; ++j) {
       const int g = lane + j * 32;
       if (g >= groups) continue;
       const unsigned long long word = g < 64 ? taken_lo : g < 128 ? taken_hi : g < 192 ? taken_2 : taken_3;
@@ -112,7 +114,7 @@ __global__ void __launch_bounds__(128) moe_route_kernel(const float* __restrict_
     else if (bg < 192) taken_2 |= 1ull << (bg - 128); else if (bg < 256) taken_3 |= 1ull << (bg - 192);
   }
 #pragma unroll
-  for (int i = 0; i < kMaxPerLane; ++i) {
+  for (int i = 0; i < PL; ++i) {
     const int e = lane + i * 32;
     if (e >= E) continue;
     const int g = e / gsz;
@@ -128,7 +130,7 @@ __global__ void __launch_bounds__(128) moe_route_kernel(const float* __restrict_
     float bv = -INFINITY, bs = 0.f;
     int be = 0x7fffffff;
 #pragma unroll
-    for (int i = 0; i < kMaxPerLane; ++i) {
+    for (int i = 0; i < PL; ++i) {
       const int e = lane + i * 32;
       if (e < E && ok[i] && (be == 0x7fffffff || c[i] > bv || (c[i] == bv && e < be))) { bv = c[i]; be = e; bs = s[i]; }
     }
@@ -313,6 +315,121 @@ __global__ void __launch_bounds__(256) moe_combine_kernel(const float* __restric
   }
 }
 
+// ---- the same sorting without the host: per-block expert counts, then every block derives its own offsets from all counts and
+// places its pairs in pair order (the result does not depend on scheduling).  The table is what llmss_gemm_grouped reads.
+constexpr int PAIRS = 1024;      // pairs per block
+constexpr int GROUP_ROWS = 256;  // rows of a token tile of the grouped product
+
+__global__ void __launch_bounds__(256) moe_hist_kernel(const int* __restrict__ ids, int P, int E, int* __restrict__ hist) {
+  __shared__ int c[256];
+  c[threadIdx.x] = 0;
+  __syncthreads();
+  const int p0 = blockIdx.x * PAIRS;
+  for (int p = p0 + threadIdx.x; p < min(P, p0 + PAIRS); p += 256) atomicAdd(&c[ids[p]], 1);
+  __syncthreads();
+  if (threadIdx.x < E) hist[blockIdx.x * E + threadIdx.x] = c[threadIdx.x];
+}
+
+// exclusive sum over the block's 256 threads
+__device__ __forceinline__ int block_exclusive(int v, int* warps, int* total) {
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  int incl = v;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const int t = __shfl_up_sync(0xffffffffu, incl, o);
+    if (lane >= o) incl += t;
+  }
+  __syncthreads();
+  if (lane == 31) warps[w] = incl;
+  __syncthreads();
+  int before = 0, all = 0;
+#pragma unroll
+  for (int i = 0; i < 8; ++i) {
+    before += i < w ? warps[i] : 0;
+    all += warps[i];
+  }
+  *total = all;
+  return before + incl - v;
+}
+
+__global__ void __launch_bounds__(256) moe_place_kernel(const int* __restrict__ ids, int P, int E, const int* __restrict__ hist,
+                                                        int* __restrict__ table, int* __restrict__ inv) {
+  __shared__ int warps[8];
+  __shared__ int next[256];          // next free row of every expert for this block's pairs
+  __shared__ int wcount[8][256];     // a round's pairs per warp and expert
+  const int e = threadIdx.x, lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  int all = 0, mine = 0;
+  if (e < E) {
+#pragma unroll 4
+    for (int b = 0; b < (int)gridDim.x; ++b) {
+      const int v = hist[b * E + e];
+      all += v;
+      mine += b < (int)blockIdx.x ? v : 0;
+    }
+  }
+  int total, tiles;
+  const int first = block_exclusive(all, warps, &total);
+  const int tile0 = block_exclusive((all + GROUP_ROWS - 1) / GROUP_ROWS, warps, &tiles);
+  if (blockIdx.x == 0) {
+    if (e < E) { table[e] = first; table[E + 1 + e] = tile0; }
+    if (e == 0) { table[E] = total; table[2 * E + 1] = tiles; }
+  }
+  next[e] = first + mine;
+  for (int r = 0; r < PAIRS / 256; ++r) {
+    const int p = blockIdx.x * PAIRS + r * 256 + threadIdx.x;
+    const int id = p < P ? ids[p] : -1;
+#pragma unroll
+    for (int i = 0; i < 8; ++i) wcount[i][e] = 0;
+    __syncthreads();
+    const unsigned same = __match_any_sync(0xffffffffu, id);
+    if (id >= 0 && lane == __ffs(same) - 1) wcount[w][id] = __popc(same);
+    __syncthreads();
+    if (id >= 0) {
+      int pos = next[id] + __popc(same & ((1u << lane) - 1u));
+      for (int i = 0; i < w; ++i) pos += wcount[i][id];
+      inv[p] = pos;
+    }
+    __syncthreads();
+    int add = 0;
+#pragma unroll
+    for (int i = 0; i < 8; ++i) add += wcount[i][e];
+    next[e] += add;
+  }
+}
+
+// every token's row to its places in the sorted order: one read, `top` writes.  V: uint4 (rows of whole 16-byte pieces) or T
+template <typename V>
+__global__ void __launch_bounds__(128) moe_scatter_rows_kernel(const V* __restrict__ h, int64_t ldh, const int* __restrict__ inv, int top,
+                                                               V* __restrict__ xs, int n) {
+  const int64_t t = blockIdx.x;
+  for (int c = threadIdx.x; c < n; c += 128) {
+    const V v = h[t * ldh + c];
+    for (int k = 0; k < top; ++k) xs[(int64_t)inv[t * top + k] * n + c] = v;
+  }
+}
+
+// moe_combine_kernel on rows of whole 16-byte vectors
+__global__ void __launch_bounds__(256) moe_combine4_kernel(const float* __restrict__ y, const int* __restrict__ inv,
+                                                           const float* __restrict__ wts, float* __restrict__ out, int64_t ldo, int W,
+                                                           int top, int add) {
+  const int64_t t = blockIdx.x;
+  for (int c = threadIdx.x * 4; c < W; c += 1024) {
+    float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll 4
+    for (int k = 0; k < top; ++k) {
+      const float w = wts[t * top + k];
+      const float4 x = *reinterpret_cast<const float4*>(y + (int64_t)inv[t * top + k] * W + c);
+      v.x += w * x.x; v.y += w * x.y; v.z += w * x.z; v.w += w * x.w;
+    }
+    float4* o = reinterpret_cast<float4*>(out + t * ldo + c);
+    if (add) {
+      const float4 b = *o;
+      v = make_float4(b.x + v.x, b.y + v.y, b.z + v.z, b.w + v.w);
+    }
+    *o = v;
+  }
+}
+
 template <typename T>
 int launch_experts(const void* h, int64_t ldh, const int* ids, const float* wts, const void* w_up, const void* w_down,
                    int64_t ldd, void* act_scratch, float* out, int64_t ldo, int T_, int W, int F, int top, int act, int gated, int add,
@@ -339,8 +456,14 @@ LLMSS_API int llmss_moe_route_ex(const float* z, int64_t ldz, int T_, int E, int
   LLMSS_REQUIRE(score_kind == 0 || score_kind == 1, "moe_route: score kind %d (0 softmax, 1 sigmoid)", score_kind);
   LLMSS_REQUIRE(group_top >= 1 && group_top <= kMaxGroupTop, "moe_route: a group sums its %d best (1..%d)", group_top, kMaxGroupTop);
   if (T_ == 0) return 0;
-  moe_route_kernel<<<(T_ + 3) / 4, 128, 0, stream>>>(z, ldz, E, top, groups, keep, route_scale, score_kind, correction, group_top,
-                                                     renorm, ids, wts, dense, T_);
+#define LLMSS_ROUTE(PL) \
+  moe_route_kernel<PL><<<(T_ + 3) / 4, 128, 0, stream>>>(z, ldz, E, top, groups, keep, route_scale, score_kind, correction, group_top, renorm, \
+                                                         ids, wts, dense, T_)
+  if (E <= 32) LLMSS_ROUTE(1);
+  else if (E <= 64) LLMSS_ROUTE(2);
+  else if (E <= 128) LLMSS_ROUTE(4);
+  else LLMSS_ROUTE(kMaxPerLane);
+#undef LLMSS_ROUTE
   LLMSS_CHECK_CUDA(cudaGetLastError());
   return 0;
 }
@@ -407,6 +530,11 @@ LLMSS_API int llmss_moe_gather_rows(const void* h, int64_t ldh, const int* perm,
 LLMSS_API int llmss_moe_combine_ex(const float* y, const int* inv, const float* wts, float* out, int64_t ldo, int T_, int W, int top,
                                    int add, cudaStream_t stream) {
   if (T_ <= 0) return 0;
+  if (W % 4 == 0 && ldo % 4 == 0 && (((uintptr_t)y | (uintptr_t)out) & 15) == 0) {
+    moe_combine4_kernel<<<T_, 256, 0, stream>>>(y, inv, wts, out, ldo, W, top, add);
+    LLMSS_CHECK_CUDA(cudaGetLastError());
+    return 0;
+  }
   moe_combine_kernel<<<T_, 256, 0, stream>>>(y, inv, wts, out, ldo, W, top, add);
   LLMSS_CHECK_CUDA(cudaGetLastError());
   return 0;
@@ -415,4 +543,27 @@ LLMSS_API int llmss_moe_combine_ex(const float* y, const int* inv, const float* 
 LLMSS_API int llmss_moe_combine(const float* y, const int* inv, const float* wts, float* out, int64_t ldo, int T_, int W, int top,
                                 cudaStream_t stream) {
   return llmss_moe_combine_ex(y, inv, wts, out, ldo, T_, W, top, 0, stream);
+}
+
+// Sorts the P = T * top (token, expert) pairs by expert on the device.  inv[pair] = row in the sorted order; table [2 * (E + 1)]:
+// first row of every expert (and P), first token tile of 256 rows of every expert (and their number); hist: scratch of
+// ceil(P / 1024) * E numbers.
+LLMSS_API int llmss_moe_group(const int* ids, int P, int E, int* hist, int* table, int* inv, cudaStream_t stream) {
+  LLMSS_REQUIRE(P > 0 && E > 0 && E <= 256, "moe_group: %d pairs, %d experts (at most 256)", P, E);
+  const int blocks = (P + PAIRS - 1) / PAIRS;
+  moe_hist_kernel<<<blocks, 256, 0, stream>>>(ids, P, E, hist);
+  moe_place_kernel<<<blocks, 256, 0, stream>>>(ids, P, E, hist, table, inv);
+  LLMSS_CHECK_CUDA(cudaGetLastError());
+  return 0;
+}
+
+// xs[inv[t * top + k]] = h[t] for every token and choice; h, xs 16-bit
+LLMSS_API int llmss_moe_scatter_rows(const void* h, int64_t ldh, const int* inv, int top, void* xs, int T_, int W, cudaStream_t stream) {
+  if (T_ <= 0) return 0;
+  if (W % 8 == 0 && ldh % 8 == 0 && (((uintptr_t)h | (uintptr_t)xs) & 15) == 0)
+    moe_scatter_rows_kernel<uint4><<<T_, 128, 0, stream>>>((const uint4*)h, ldh / 8, inv, top, (uint4*)xs, W / 8);
+  else
+    moe_scatter_rows_kernel<uint16_t><<<T_, 128, 0, stream>>>((const uint16_t*)h, ldh, inv, top, (uint16_t*)xs, W);
+  LLMSS_CHECK_CUDA(cudaGetLastError());
+  return 0;
 }

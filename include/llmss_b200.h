@@ -221,6 +221,15 @@ int llmss_moe_count(const int* ids, int P, int E, int* counts, llmss_stream_t st
 int llmss_moe_permute(const int* ids, int P, int E, const int* offsets, int* perm, int* inv, llmss_stream_t stream);
 int llmss_moe_gather_rows(const void* h, int64_t ldh, const int* perm, int top, void* xs, int P, int W, int dtype,
                           llmss_stream_t stream);
+/* the same sorting without the host: inv[pair] = row in the order by expert, table [2 * (E + 1)] = first row of every expert (and P),
+ * first tile of 256 rows of every expert (and their number); hist: ceil(P / 1024) * E numbers of scratch */
+int llmss_moe_group(const int* ids, int P, int E, int* hist, int* table, int* inv, llmss_stream_t stream);
+/* xs[inv[t * top + k]] = h[t], 16-bit rows */
+int llmss_moe_scatter_rows(const void* h, int64_t ldh, const int* inv, int top, void* xs, int T, int W, llmss_stream_t stream);
+/* rows [table[e], table[e + 1]) of x [P, K] times w_e [N, K]^T (element (n, k) at w + e * w_group_stride + n * ldw + k), 16-bit operands
+ * with K, ldx, ldw and w_group_stride multiples of 8 */
+int llmss_gemm_grouped(const void* x, int64_t ldx, const void* w, int64_t ldw, int64_t w_group_stride, const int* table, int E, void* out,
+                       int64_t ldo, int P, int N, int K, int dtype, int out_f32, int act, int gated, llmss_stream_t stream);
 int llmss_moe_combine(const float* y, const int* inv, const float* wts, float* out, int64_t ldo, int T, int W, int top,
                       llmss_stream_t stream);
 int llmss_moe_scale(void* a, int64_t lda, const float* dense, int T, int E, int F, int dtype, llmss_stream_t stream);

@@ -117,6 +117,10 @@ _SIGS = {
     "llmss_moe_count": (c_int, [c_void_p, c_int, c_int, c_void_p, c_void_p]),
     "llmss_moe_permute": (c_int, [c_void_p, c_int, c_int, c_void_p, c_void_p, c_void_p, c_void_p]),
     "llmss_moe_gather_rows": (c_int, [c_void_p, c_int64, c_void_p, c_int, c_void_p, c_int, c_int, c_int, c_void_p]),
+    "llmss_moe_group": (c_int, [c_void_p, c_int, c_int, c_void_p, c_void_p, c_void_p, c_void_p]),
+    "llmss_moe_scatter_rows": (c_int, [c_void_p, c_int64, c_void_p, c_int, c_void_p, c_int, c_int, c_void_p]),
+    "llmss_gemm_grouped": (c_int, [c_void_p, c_int64, c_void_p, c_int64, c_int64, c_void_p, c_int, c_void_p, c_int64, c_int, c_int, c_int,
+                                   c_int, c_int, c_int, c_int, c_void_p]),
     "llmss_moe_combine": (c_int, [c_void_p, c_void_p, c_void_p, c_void_p, c_int64, c_int, c_int, c_int, c_void_p]),
     "llmss_moe_scale": (c_int, [c_void_p, c_int64, c_void_p, c_int, c_int, c_int, c_int, c_void_p]),
     "llmss_embed_bigram": (c_int, [c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int64, c_int64, c_int, c_void_p,

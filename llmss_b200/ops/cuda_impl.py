@@ -616,10 +616,20 @@ def moe_scale(a, dense, experts: int, ff: int):
     return a
 
 
+def moe_groups_on_device(h, w_up, w_down, gated: bool = False) -> bool:
+    """Whether the grouped form can sort and multiply without the host: 16-bit operands on the 16-byte lines of the tensor maps,
+    at most 256 experts."""
+    E, F, W = w_up.shape
+    F = F // 2 if gated else F
+    return (h.dtype != torch.float32 and E <= 256 and W % 8 == 0 and F % 8 == 0 and w_down.stride(0) % 8 == 0 and w_up.is_contiguous()
+            and w_up.data_ptr() % 16 == 0 and w_down.data_ptr() % 16 == 0)
+
+
 def moe_experts_grouped(h, ids, wts, w_up, w_down, act, gated: bool = False, base=None):
-    """Long prompts: sort the (token, expert) pairs by expert on the device and run every expert as one pair of tensor-core
-    GEMMs over its contiguous rows -- top / experts of the dense form's FLOPs.  Reads the per-expert counts on the host (one
-    small synchronising copy), so it is for prompt processing, not for graph-captured decode steps."""
+    """Long prompts: sort the (token, expert) pairs by expert and run every expert on its own contiguous rows -- top / experts of
+    the dense form's FLOPs.  Sorting, row ranges and tiles stay on the device: one tensor-core launch per projection walks the
+    experts (llmss_gemm_grouped).  Sizes that miss its tensor maps count on the host instead (one small synchronising copy) and
+    run a pair of linear layers per expert."""
     lib = _lib.load()
     T, W, ldh = _rows2d(h)
     E, F, _ = w_up.shape
@@ -627,27 +637,40 @@ def moe_experts_grouped(h, ids, wts, w_up, w_down, act, gated: bool = False, bas
         F //= 2
     top = ids.shape[1]
     P, dev = T * top, h.device
-    counts = torch.empty(E, dtype=torch.int32, device=dev)
-    _lib.check(lib.llmss_moe_count(_ptr(ids), P, E, _ptr(counts), _stream()), "llmss_moe_count")
-    cnt = counts.tolist()
-    offs, o = [], 0
-    for c in cnt:
-        offs.append(o)
-        o += c
-    offsets = torch.tensor(offs, dtype=torch.int32).to(dev)
-    perm = torch.empty(P, dtype=torch.int32, device=dev)
-    inv = torch.empty(P, dtype=torch.int32, device=dev)
-    _lib.check(lib.llmss_moe_permute(_ptr(ids), P, E, _ptr(offsets), _ptr(perm), _ptr(inv), _stream()), "llmss_moe_permute")
-    xs = torch.empty(P, W, dtype=h.dtype, device=dev)
-    _lib.check(lib.llmss_moe_gather_rows(_ptr(h), ldh, _ptr(perm), top, _ptr(xs), P, W, _DT[h.dtype], _stream()),
-               "llmss_moe_gather_rows")
-    _count(3)
+    assert ids.is_contiguous() and wts.is_contiguous() and w_down.stride(1) == 1 and h.dtype == w_up.dtype == w_down.dtype
     a = torch.empty(P, F, dtype=h.dtype, device=dev)
     y = torch.empty(P, W, dtype=torch.float32, device=dev)
-    for e, (lo, c) in enumerate(zip(offs, cnt)):
-        if c:
-            linear(xs[lo:lo + c], w_up[e], act=act, gated=gated, out=a[lo:lo + c])
-            linear(a[lo:lo + c], w_down[:, e * F:(e + 1) * F], out_dtype=torch.float32, out=y[lo:lo + c])
+    xs = torch.empty(P, W, dtype=h.dtype, device=dev)
+    if moe_groups_on_device(h, w_up, w_down, gated):
+        ints = torch.empty(P + 2 * (E + 1) + -(-P // 1024) * E, dtype=torch.int32, device=dev)
+        inv, table, hist = ints[:P], ints[P:P + 2 * (E + 1)], ints[P + 2 * (E + 1):]
+        _lib.check(lib.llmss_moe_group(_ptr(ids), P, E, _ptr(hist), _ptr(table), _ptr(inv), _stream()), "llmss_moe_group")
+        _lib.check(lib.llmss_moe_scatter_rows(_ptr(h), ldh, _ptr(inv), top, _ptr(xs), T, W, _stream()), "llmss_moe_scatter_rows")
+        rows = w_up.shape[1]
+        _lib.check(lib.llmss_gemm_grouped(_ptr(xs), W, _ptr(w_up), W, rows * W, _ptr(table), E, _ptr(a), F, P, rows, W, _DT[h.dtype], 0, act,
+                                          1 if gated else 0, _stream()), "llmss_gemm_grouped")
+        _lib.check(lib.llmss_gemm_grouped(_ptr(a), F, _ptr(w_down), w_down.stride(0), F, _ptr(table), E, _ptr(y), W, P, W, F, _DT[h.dtype], 1,
+                                          ACT_NONE, 0, _stream()), "llmss_gemm_grouped")
+        _count(5)
+    else:
+        counts = torch.empty(E, dtype=torch.int32, device=dev)
+        _lib.check(lib.llmss_moe_count(_ptr(ids), P, E, _ptr(counts), _stream()), "llmss_moe_count")
+        cnt = counts.tolist()
+        offs, o = [], 0
+        for c in cnt:
+            offs.append(o)
+            o += c
+        offsets = torch.tensor(offs, dtype=torch.int32).to(dev)
+        perm = torch.empty(P, dtype=torch.int32, device=dev)
+        inv = torch.empty(P, dtype=torch.int32, device=dev)
+        _lib.check(lib.llmss_moe_permute(_ptr(ids), P, E, _ptr(offsets), _ptr(perm), _ptr(inv), _stream()), "llmss_moe_permute")
+        _lib.check(lib.llmss_moe_gather_rows(_ptr(h), ldh, _ptr(perm), top, _ptr(xs), P, W, _DT[h.dtype], _stream()),
+                   "llmss_moe_gather_rows")
+        _count(3)
+        for e, (lo, c) in enumerate(zip(offs, cnt)):
+            if c:
+                linear(xs[lo:lo + c], w_up[e], act=act, gated=gated, out=a[lo:lo + c])
+                linear(a[lo:lo + c], w_down[:, e * F:(e + 1) * F], out_dtype=torch.float32, out=y[lo:lo + c])
     out = base if base is not None else torch.empty(T, W, dtype=torch.float32, device=dev)
     assert out.dtype == torch.float32 and out.shape == (T, W) and out.stride(1) == 1
     _lib.check(lib.llmss_moe_combine_ex(_ptr(y), _ptr(inv), _ptr(wts), _ptr(out), out.stride(0), T, W, top, 0 if base is None else 1,

@@ -58,3 +58,30 @@ def test_delta_portions(dk, dv, heads, qk_heads, unit, copies):
                          beta_sigmoid=True)
     assert _rel(got, want.reshape(T, -1)) < 3e-6
     assert _rel(state.reshape(len(lens), heads, dv, dk).transpose(2, 3), torch.stack(ends)) < 3e-6
+
+
+@pytest.mark.parametrize("T,W,E,top,F,gated,skew", [(300, 128, 16, 4, 64, False, False), (1500, 256, 8, 2, 136, True, False), (513, 72, 5, 1, 40, False, True),
+                                                    (1024, 64, 256, 8, 32, True, False), (700, 64, 3, 3, 264, False, False), (1, 64, 8, 2, 64, False, False)])
+def test_experts_sorted_on_the_device(T, W, E, top, F, gated, skew):
+    """Groups of no rows, of less and of more than a token tile, features off the 256-feature pairs, hidden sizes off the 64-column
+    k-blocks, down matrices as a view of wider rows, a sum onto another result.  Bound: bf16 operands and hidden rows, 1e-2."""
+    from llmss_b200.ops import cuda_impl as cu
+
+    torch.manual_seed(T + E)
+    dt = torch.bfloat16
+    rows = 2 * F if gated else F
+    h = torch.randn(T, W, device="cuda").to(dt)
+    up = (torch.randn(E, rows, W, device="cuda") * W ** -0.5).to(dt)
+    down = (torch.randn(W, 16 + E * F, device="cuda") * F ** -0.5).to(dt)[:, 16:]
+    z = torch.randn(T, E, device="cuda") + (8.0 * (torch.arange(E, device="cuda") == 2) if skew else 0.0)
+    ids, wts = ops.moe_route(z, E, top, 1, 1, 1.0)
+    base = torch.randn(T, W, device="cuda")
+    assert cu.moe_groups_on_device(h, up, down, gated)
+    got = cu.moe_experts_grouped(h, ids, wts, up, down, ops.ACT_SILU, gated, base=base.clone())
+    want = base.double()
+    for e in range(E):
+        t, j = torch.nonzero(ids == e, as_tuple=True)
+        x = h[t].double() @ up[e].double().t()
+        x = torch.nn.functional.silu(x[:, 0::2]) * x[:, 1::2] if gated else torch.nn.functional.silu(x)
+        want.index_add_(0, t, wts[t, j].double()[:, None] * (x @ down[:, e * F:(e + 1) * F].double().t()))
+    assert _rel(got, want.cpu()) < 1e-2
