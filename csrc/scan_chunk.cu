@@ -1,0 +1,601 @@
+// Long portions of the gated linear recurrence (csrc/recurrent.cu: linear_scan) as products over chunks of 64 tokens.
+//
+//   S_t = diag(a_t) S_(t-1) + k_t (c_t v_t)^T ;  o_t = S_t^T q_t   or, read before the update,  (S_(t-1) + diag(u) k_t (c_t v_t)^T)^T q_t
+//
+// Token by token a state element costs three operations and a share of a reduction, twice over (the two passes of the token-serial
+// form).  Over a chunk the same sums are products of tiles that live in shared memory, two multiply-adds per state element and token:
+//   1. scan_state_kernel   U_c = sum_j (prod_(t > j) a_t * k_j) v_j^T and the chunk's decay D_c, every chunk a block;
+//   2. scan_carry_kernel   S_(c+1) = D_c S_c + U_c along a sequence's chunks, an element per thread; U_c is replaced by S_c;
+//   3. scan_out_kernel     o = (decayed q) S_c + tril((decayed q) (decayed k)^T) v, every chunk a block.
+// Everything is 32-bit on the multiply-add pipe (two numbers per instruction where both operands lie in memory order): a 3-term
+// split on the tensor cores would run at 158 against 126 multiply-adds per clock and SM and round its sums differently.
+//
+// Decays without overflow: a sub-block of 16 tokens takes its middle as reference, q_i gets F(i) and k_j gets 1 / F(j) with F the
+// decay from the middle (products of at most 8 factors, one division); between sub-blocks the factor from middle to middle is at
+// most 1.  F and 1 / F stay finite while half a sub-block decays by no more than 2^-100 (or grows by 2^100) in any channel; a chunk
+// where one does more runs token by token (a column per thread).  Kernel 1 needs no reciprocals: its factors are suffix products.
+//
+// B200, 8 prompts of 1024 tokens, against the two passes of the token-serial form: 32 heads of 64 x 64, decay per channel and bonus
+// 618 -> 376 us (99 + 36 + 221, ncu: 44 % of the multiply-add pipe, shared memory 37 to 57 % of its bandwidth); 16 heads of 128 x 128, per
+// channel 979 -> 643 us, constant decay 846 -> 616 us; 32 heads of 128 x 64, decay per token 830 -> 612 us.  Kernel 3 is bound by shared
+// memory: a tile of 8 x 4 per thread reads 12 16-byte pieces for 64 packed multiply-adds, and every piece takes 4 clocks of the SM.
+#include "common.cuh"
+
+namespace {
+
+constexpr int C = 64, SB = 16, NS = C / SB, JT = 64;     // chunk, sub-block, value columns per block
+constexpr float kSafe = 7.888609e-31f;                   // 2^-100
+
+struct ChunkArgs {
+  const float* q; int64_t ldq;
+  const float* k; int64_t ldk;
+  const float* v; int64_t ldv;
+  const float* decay; int64_t ldd;     // kind 0: [H] decays; 1: [T, H] log decays; 2: [T, H * dk] log decays
+  const float* bonus;                  // [H, dk] or null
+  const float* vscale; int64_t ldvs;   // [T, H] or null
+  float* out;                          // [T, H * dv]
+  float* state;                        // [slots, H, dv, dk]
+  const int* cu_q; const int* seq_lens; const int* slots;
+  float* chunks;                       // [chunk slots][H][dv][dk]: U_c, then S_c
+  float* decays;                       // [chunk slots][H][dk]
+  int H, rep, dk, dv, nslices;
+};
+
+// rows and chunk slots of sequence b; the slots of all sequences take T / 64 + B places: cu_q[b] / 64 + b is the first of b's
+struct Rows {
+  int q0, ql, ctx, slot, first;
+};
+__device__ __forceinline__ Rows rows_of(const ChunkArgs& a, int b) {
+  Rows r;
+  r.q0 = a.cu_q[b];
+  r.ql = a.cu_q[b + 1] - r.q0;
+  r.ctx = a.seq_lens[b] - r.ql;
+  r.slot = a.slots[b];
+  r.first = r.q0 / C + b;
+  if (r.slot < 0 || r.ctx < 0) r.ql = 0;
+  return r;
+}
+
+__device__ __forceinline__ uint64_t pfma(uint64_t x, uint64_t y, uint64_t z) {
+  uint64_t d;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(x), "l"(y), "l"(z));
+  return d;
+}
+__device__ __forceinline__ uint64_t pmul(uint64_t x, uint64_t y) {
+  uint64_t d;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(x), "l"(y));
+  return d;
+}
+__device__ __forceinline__ uint64_t pack(float lo, float hi) {
+  uint64_t d;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(d) : "f"(lo), "f"(hi));
+  return d;
+}
+__device__ __forceinline__ float2 unpack(uint64_t v) {
+  float2 r;
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
+  return r;
+}
+__device__ __forceinline__ ulonglong2 lds2(const float* p) { return *reinterpret_cast<const ulonglong2*>(p); }
+
+// Loads never stand behind a branch: rows past the chunk's end and channels past dk are read from the last valid place and replaced
+// by a select, so that a thread's loads are all in flight together (behind branches, or moved behind one by the compiler, the same
+// loads were two thirds of the time; hence the volatile load).
+__device__ __forceinline__ float ld_f32(const float* p) {
+  float v;
+  asm volatile("ld.global.nc.f32 %0, [%1];" : "=f"(v) : "l"(p));
+  return v;
+}
+// SB rows of one column, from local row l0 of n; p: the column in the chunk's row 0
+__device__ __forceinline__ void load_rows(const float* p, int64_t ld, int l0, int n, float (&x)[SB]) {
+  const int first = min(l0, n - 1);
+  p += first * ld;
+#pragma unroll
+  for (int i = 0; i < SB; ++i) {
+    x[i] = ld_f32(p);
+    p += l0 + i + 1 < n ? ld : 0;
+  }
+}
+// 1 / x by one Newton-Raphson step on the approximate reciprocal; x lies in 2^-100 .. 2^100 wherever the result is used
+__device__ __forceinline__ float recip(float x) {
+  float y;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+  return fmaf(y, fmaf(-x, y, 1.f), y);
+}
+// decay factors of SB tokens of a channel (1 where `in` is false or past n); `table`: a chunk's per-token factors (kinds 0 and 1)
+template <int KIND>
+__device__ __forceinline__ void load_factors(const float* p, int64_t ld, const float* table, int l0, int n, bool in, float (&x)[SB]) {
+  if (KIND == 2) load_rows(p, ld, l0, n, x);
+#pragma unroll
+  for (int i = 0; i < SB; ++i) {
+    const float f = KIND == 2 ? expf(x[i]) : table[l0 + i];
+    x[i] = in && l0 + i < n ? f : 1.f;
+  }
+}
+// ROWS tokens of the chunk's value columns from local row l0, NT threads: element i of a thread is (its index + i NT) of [ROWS][JT]
+template <int NT, int ROWS>
+__device__ __forceinline__ void load_values(const ChunkArgs& a, int64_t t0, int l0, int n, int h, int j0, int nj, float (&x)[ROWS * JT / NT]) {
+  const int j = threadIdx.x % JT, t1 = l0 + threadIdx.x / JT;
+  constexpr int STEP = NT / JT, E = ROWS * JT / NT;
+  const float* p = a.v + t0 * a.ldv + (int64_t)h * a.dv + j0 + min(j, nj - 1);
+#pragma unroll
+  for (int i = 0; i < E; ++i) x[i] = ld_f32(p + (int64_t)min(t1 + i * STEP, n - 1) * a.ldv);
+  if (a.vscale != nullptr) {
+    float w[E];
+#pragma unroll
+    for (int i = 0; i < E; ++i) w[i] = ld_f32(a.vscale + (t0 + min(t1 + i * STEP, n - 1)) * a.ldvs + h);
+#pragma unroll
+    for (int i = 0; i < E; ++i) x[i] *= w[i];
+  }
+#pragma unroll
+  for (int i = 0; i < E; ++i)
+    if (j >= nj || t1 + i * STEP >= n) x[i] = 0.f;
+}
+template <int KIND>
+__device__ __forceinline__ void fill_table(const ChunkArgs& a, float* table, int64_t t0, int n, int h) {
+  if (KIND != 2 && threadIdx.x < C) {
+    float x = 1.f;
+    if ((int)threadIdx.x < n) x = KIND == 0 ? a.decay[h] : expf(a.decay[(t0 + threadIdx.x) * a.ldd + h]);
+    table[threadIdx.x] = x;
+  }
+  if (KIND != 2) __syncthreads();
+}
+
+// ---- 1: U_c and D_c, DK threads.  A thread owns 8 key rows x 8 value columns, both as two runs of 4 half a tile apart (the quarter
+// warps' 16-byte reads lie in different banks): 4 reads for 32 packed multiply-adds.
+template <int DK, int KIND>
+__global__ void __launch_bounds__(DK, DK == 64 ? 7 : 4) scan_state_kernel(ChunkArgs a) {
+  extern __shared__ __align__(16) float sm[];
+  float* ks = sm;                      // [C][DK] keys times the decay behind them, inside the sub-block
+  float* vs = ks + C * DK;             // [C][JT]
+  float* ds = vs + C * JT;             // [NS][DK] decay of a sub-block
+  float* table = ds + NS * DK;         // [C]
+  const Rows r = rows_of(a, blockIdx.z);
+  const int t_lo = blockIdx.x * C;
+  if (t_lo >= r.ql) return;
+  const int n = min(C, r.ql - t_lo), h = blockIdx.y / a.nslices, slice = blockIdx.y % a.nslices;
+  const int j0 = slice * JT, nj = min(JT, a.dv - j0);
+  const int64_t t0 = r.q0 + t_lo;
+  const int hq = h / a.rep;
+  fill_table<KIND>(a, table, t0, n, h);
+  {
+    const int c = threadIdx.x, cc = min(c, a.dk - 1);
+    const bool in = c < a.dk;
+    const float* kp = a.k + t0 * a.ldk + (int64_t)hq * a.dk + cc;
+    const float* dp = KIND == 2 ? a.decay + t0 * a.ldd + (int64_t)h * a.dk + cc : nullptr;
+#pragma unroll 1
+    for (int s = 0; s < NS; ++s) {
+      float kx[SB], x[SB], vr[C * JT / DK / NS];
+      load_rows(kp, a.ldk, s * SB, n, kx);
+      load_factors<KIND>(dp, a.ldd, table, s * SB, n, in, x);
+      load_values<DK, SB>(a, t0, s * SB, n, h, j0, nj, vr);
+      float p = 1.f;
+#pragma unroll
+      for (int i = SB - 1; i >= 0; --i) {
+        ks[(s * SB + i) * DK + c] = in && s * SB + i < n ? kx[i] * p : 0.f;
+        p *= x[i];
+      }
+      ds[s * DK + c] = p;
+#pragma unroll
+      for (int i = 0; i < C * JT / DK / NS; ++i) vs[s * SB * JT + threadIdx.x + i * DK] = vr[i];
+    }
+  }
+  __syncthreads();
+  constexpr int KG = DK / 8;
+  const int kg = threadIdx.x % KG, vg = threadIdx.x / KG;
+  const int i0 = kg * 4, i1 = DK / 2 + kg * 4, c0 = vg * 4, c1 = JT / 2 + vg * 4;
+  uint64_t acc[4][8];
+#pragma unroll
+  for (int p = 0; p < 4; ++p)
+#pragma unroll
+    for (int j = 0; j < 8; ++j) acc[p][j] = 0;
+#pragma unroll 1
+  for (int s = 0; s < NS; ++s) {
+    if (s > 0) {
+      const ulonglong2 d0 = lds2(ds + s * DK + i0), d1 = lds2(ds + s * DK + i1);
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+        acc[0][j] = pmul(acc[0][j], d0.x); acc[1][j] = pmul(acc[1][j], d0.y);
+        acc[2][j] = pmul(acc[2][j], d1.x); acc[3][j] = pmul(acc[3][j], d1.y);
+      }
+    }
+#pragma unroll 2
+    for (int i = 0; i < SB; ++i) {
+      const int t = s * SB + i;
+      const ulonglong2 k0 = lds2(ks + t * DK + i0), k1 = lds2(ks + t * DK + i1);
+      const float4 x = *reinterpret_cast<const float4*>(vs + t * JT + c0), y = *reinterpret_cast<const float4*>(vs + t * JT + c1);
+      const uint64_t vv[8] = {pack(x.x, x.x), pack(x.y, x.y), pack(x.z, x.z), pack(x.w, x.w), pack(y.x, y.x), pack(y.y, y.y), pack(y.z, y.z), pack(y.w, y.w)};
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+        acc[0][j] = pfma(k0.x, vv[j], acc[0][j]); acc[1][j] = pfma(k0.y, vv[j], acc[1][j]);
+        acc[2][j] = pfma(k1.x, vv[j], acc[2][j]); acc[3][j] = pfma(k1.y, vv[j], acc[3][j]);
+      }
+    }
+  }
+  const int64_t at = (int64_t)(r.first + blockIdx.x) * a.H + h;
+#pragma unroll
+  for (int j = 0; j < 8; ++j) {
+    const int col = (j < 4 ? c0 : c1) + (j & 3);
+    if (col >= nj) continue;
+    float* u = a.chunks + (at * a.dv + j0 + col) * a.dk;
+    const float2 p0 = unpack(acc[0][j]), p1 = unpack(acc[1][j]), p2 = unpack(acc[2][j]), p3 = unpack(acc[3][j]);
+    if (i0 < a.dk) *reinterpret_cast<float4*>(u + i0) = make_float4(p0.x, p0.y, p1.x, p1.y);     // (dk is a multiple of 4)
+    if (i1 < a.dk) *reinterpret_cast<float4*>(u + i1) = make_float4(p2.x, p2.y, p3.x, p3.y);
+  }
+  if (slice == 0 && (int)threadIdx.x < a.dk) {
+    float p = 1.f;
+#pragma unroll
+    for (int s = 0; s < NS; ++s) p *= ds[s * DK + threadIdx.x];
+    a.decays[at * a.dk + threadIdx.x] = p;
+  }
+}
+
+// ---- 2: chunk states, two neighbouring key rows of a value column per thread; grid (plane / 512, B).  Eight chunks' loads in flight
+__global__ void __launch_bounds__(256) scan_carry_kernel(ChunkArgs a) {
+  const Rows r = rows_of(a, blockIdx.y);
+  if (r.ql <= 0) return;
+  const int per_head = a.dv * a.dk, plane = a.H * per_head;          // (the host checks that it fits)
+  const int e = (blockIdx.x * 256 + threadIdx.x) * 2;
+  if (e >= plane) return;
+  const int h = e / per_head, i = e % a.dk;
+  float2* st = reinterpret_cast<float2*>(a.state + (int64_t)r.slot * plane + e);
+  float2 S = r.ctx > 0 ? *st : make_float2(0.f, 0.f);
+  const int nch = (r.ql + C - 1) / C, dstep = a.H * a.dk;
+  float* u = a.chunks + (int64_t)r.first * plane + e;
+  const float* d = a.decays + ((int64_t)r.first * a.H + h) * a.dk + i;
+  for (int c0 = 0; c0 < nch; c0 += 8) {
+    float2 uu[8], dd[8];
+#pragma unroll
+    for (int x = 0; x < 8; ++x) {
+      const int c = min(c0 + x, nch - 1);
+      asm volatile("ld.global.v2.f32 {%0, %1}, [%2];" : "=f"(uu[x].x), "=f"(uu[x].y) : "l"(u + (int64_t)c * plane));
+      asm volatile("ld.global.v2.f32 {%0, %1}, [%2];" : "=f"(dd[x].x), "=f"(dd[x].y) : "l"(d + (int64_t)c * dstep));
+    }
+#pragma unroll
+    for (int x = 0; x < 8; ++x)
+      if (c0 + x < nch) {
+        *reinterpret_cast<float2*>(u + (int64_t)(c0 + x) * plane) = S;
+        S = make_float2(fmaf(dd[x].x, S.x, uu[x].x), fmaf(dd[x].y, S.y, uu[x].y));
+      }
+  }
+  *st = S;
+}
+
+// ---- 3: outputs of a chunk, 128 threads.  Thread (tg, cg) owns tokens tg + 8 m and value columns cg + 16 m: every thread has rows of
+// every sub-block, so the triangular product is as much work for each.  Rows of q, k and S are padded by 4 floats: 16-byte reads of
+// neighbouring rows lie in different banks.  The scores reuse the keys' place, the values lie behind them.
+template <int DK> struct OutSmem {
+  static constexpr int LD = DK + 4, LA = C + 4;
+  static constexpr int Q = C * LD, S = JT * LD, KA = (C * LD > C * LA + C * JT) ? C * LD : C * LA + C * JT;
+  static constexpr int FLOATS = Q + KA + S + 2 * NS * DK + 10 * DK + (DK / 32 + 1) * C;
+};
+
+template <int DK, int KIND, bool BEFORE>
+__global__ void __launch_bounds__(128, DK == 64 ? 3 : 2) scan_out_kernel(ChunkArgs a) {
+  using M = OutSmem<DK>;
+  constexpr int LD = M::LD, LA = M::LA;
+  extern __shared__ __align__(16) float sm[];
+  float* qs = sm;                       // [C][LD]
+  float* ks = qs + M::Q;                // [C][LD], then scores [C][LA] and values [C][JT]
+  float* as = ks;
+  float* vs = ks + C * LA;
+  float* ss = ks + M::KA;               // [JT][LD] start state, columns as rows
+  float* halves = ss + M::S;            // [NS][2][DK] decay of the first and second half of a sub-block
+  float* mids = halves + 2 * NS * DK;   // [10][DK]: middle of s' to middle of s (pairs (1,0) (2,0) (2,1) (3,0) (3,1) (3,2)), start to middle of s
+  float* diag = mids + 10 * DK;         // [DK / 32][C] bonus products, a part per 32 channels
+  float* table = diag + (DK / 32) * C;  // [C]
+  const Rows r = rows_of(a, blockIdx.z);
+  const int t_lo = blockIdx.x * C;
+  if (t_lo >= r.ql) return;
+  const int n = min(C, r.ql - t_lo), h = blockIdx.y / a.nslices, slice = blockIdx.y % a.nslices;
+  const int j0 = slice * JT, nj = min(JT, a.dv - j0);
+  const int64_t t0 = r.q0 + t_lo;
+  const int hq = h / a.rep, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const float* S = a.chunks + (((int64_t)(r.first + blockIdx.x) * a.H + h) * a.dv + j0) * a.dk;
+  const float* qp = a.q + t0 * a.ldq + (int64_t)hq * a.dk;
+  const float* kp = a.k + t0 * a.ldk + (int64_t)hq * a.dk;
+  fill_table<KIND>(a, table, t0, n, h);
+  // start state -> shared memory (asynchronously; a column or channel that is not there is never copied into and zeroed instead)
+  for (int i = tid; i < JT * (DK / 4); i += 128) {
+    const int j = i / (DK / 4), c = (i % (DK / 4)) * 4;
+    if (j < nj && c < a.dk)
+      asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(ss + j * LD + c)), "l"(S + (int64_t)j * a.dk + c) : "memory");
+    else
+      *reinterpret_cast<float4*>(ss + j * LD + c) = make_float4(0.f, 0.f, 0.f, 0.f);
+  }
+  bool deep = false;                    // some half sub-block decays by more than 2^-100
+#pragma unroll 1
+  for (int task = tid; task < NS * DK; task += 128) {
+    const int c = task % DK, cc = min(c, a.dk - 1), s = task / DK, l0 = s * SB;
+    const bool in = c < a.dk;
+    float x[SB], qx[SB], kx[SB];
+    load_rows(qp + cc, a.ldq, l0, n, qx);
+    load_rows(kp + cc, a.ldk, l0, n, kx);
+    load_factors<KIND>(KIND == 2 ? a.decay + t0 * a.ldd + (int64_t)h * a.dk + cc : nullptr, a.ldd, table, l0, n, in, x);
+#pragma unroll
+    for (int i = 0; i < SB; ++i)
+      if (!in || l0 + i >= n) qx[i] = kx[i] = 0.f;
+    if (BEFORE) {
+      // bonus products of 16 tokens over this warp's 32 channels: four exchanges leave token (lane bits 4..1) per lane pair
+      float d[SB];
+      const float u = a.bonus != nullptr ? a.bonus[(int64_t)h * a.dk + cc] : 0.f;
+#pragma unroll
+      for (int i = 0; i < SB; ++i) d[i] = qx[i] * u * kx[i];
+#pragma unroll
+      for (int o = 16, w = SB / 2; o > 1; o >>= 1, w >>= 1) {
+        const bool hi = lane & o;
+#pragma unroll
+        for (int i = 0; i < w; ++i) d[i] = (hi ? d[i + w] : d[i]) + __shfl_xor_sync(0xffffffffu, hi ? d[i] : d[i + w], o);
+      }
+      d[0] += __shfl_xor_sync(0xffffffffu, d[0], 1);
+      if (!(lane & 1)) diag[(c >> 5) * C + l0 + (lane >> 1)] = d[0];
+    }
+    float f = 1.f;
+#pragma unroll
+    for (int i = SB / 2; i < SB; ++i) {
+      const float before = f;
+      f *= x[i];
+      qs[(l0 + i) * LD + c] = qx[i] * (BEFORE ? before : f);
+      ks[(l0 + i) * LD + c] = kx[i] * recip(f);
+    }
+    halves[(2 * s + 1) * DK + c] = f;
+    deep |= !(f >= kSafe && f <= 1.f / kSafe);
+    f = 1.f;
+#pragma unroll
+    for (int i = SB / 2 - 1; i >= 0; --i) {
+      const float after = f;
+      f *= x[i];
+      qs[(l0 + i) * LD + c] = qx[i] * recip(BEFORE ? f : after);
+      ks[(l0 + i) * LD + c] = kx[i] * after;
+    }
+    halves[2 * s * DK + c] = f;
+    deep |= !(f >= kSafe && f <= 1.f / kSafe);
+  }
+  asm volatile("cp.async.wait_all;" ::: "memory");
+  auto bonus_of = [&](int t) {
+    float d = 0.f;
+#pragma unroll
+    for (int g = 0; g < DK / 32; ++g) d += diag[g * C + t];
+    return d;
+  };
+  float* op = a.out + t0 * a.H * a.dv + (int64_t)h * a.dv + j0;
+  const int64_t ldo = (int64_t)a.H * a.dv;
+  if (__syncthreads_or(deep)) {
+    // ---- token by token: a value column per thread, raw q and k rows and the factors in shared memory
+    for (int i = tid; i < C * DK; i += 128) {
+      const int t = i / DK, c = i % DK;
+      const bool in = t < n && c < a.dk;
+      qs[t * DK + c] = in ? qp[(int64_t)t * a.ldq + c] : 0.f;
+      ks[t * DK + c] = in ? kp[(int64_t)t * a.ldk + c] : 0.f;
+    }
+    float col[DK];
+    if (tid < JT) {
+#pragma unroll
+      for (int c = 0; c < DK; ++c) col[c] = ss[tid * LD + c];
+    }
+    __syncthreads();
+    for (int i = tid; i < C * DK; i += 128) {
+      const int t = i / DK, c = i % DK;
+      ss[t * DK + c] = !(t < n && c < a.dk) ? 1.f : KIND == 2 ? expf(a.decay[(t0 + t) * a.ldd + (int64_t)h * a.dk + c]) : table[t];
+    }
+    __syncthreads();
+    if (tid < nj) {
+      for (int t = 0; t < n; ++t) {
+        float v = a.v[(t0 + t) * a.ldv + (int64_t)h * a.dv + j0 + tid];
+        if (a.vscale != nullptr) v *= a.vscale[(t0 + t) * a.ldvs + h];
+        float o0 = 0.f, o1 = 0.f;
+#pragma unroll
+        for (int c = 0; c < DK; c += 4) {
+          const float4 q4 = *reinterpret_cast<const float4*>(qs + t * DK + c), k4 = *reinterpret_cast<const float4*>(ks + t * DK + c),
+                       x4 = *reinterpret_cast<const float4*>(ss + t * DK + c);
+          if (BEFORE) {
+            o0 = fmaf(q4.x, col[c], o0); o1 = fmaf(q4.y, col[c + 1], o1); o0 = fmaf(q4.z, col[c + 2], o0); o1 = fmaf(q4.w, col[c + 3], o1);
+          }
+          col[c] = fmaf(x4.x, col[c], k4.x * v); col[c + 1] = fmaf(x4.y, col[c + 1], k4.y * v);
+          col[c + 2] = fmaf(x4.z, col[c + 2], k4.z * v); col[c + 3] = fmaf(x4.w, col[c + 3], k4.w * v);
+          if (!BEFORE) {
+            o0 = fmaf(q4.x, col[c], o0); o1 = fmaf(q4.y, col[c + 1], o1); o0 = fmaf(q4.z, col[c + 2], o0); o1 = fmaf(q4.w, col[c + 3], o1);
+          }
+        }
+        op[t * ldo + tid] = BEFORE ? fmaf(bonus_of(t), v, o0 + o1) : o0 + o1;
+      }
+    }
+    return;
+  }
+  // factors between middles, and from the chunk's start to the middles
+  for (int c = tid; c < DK; c += 128) {
+    float h1[NS], h2[NS];
+#pragma unroll
+    for (int s = 0; s < NS; ++s) { h1[s] = halves[2 * s * DK + c]; h2[s] = halves[(2 * s + 1) * DK + c]; }
+    float run = 1.f;
+#pragma unroll
+    for (int s = 0; s < NS; ++s) {
+      mids[(6 + s) * DK + c] = run * h1[s];
+      run *= h1[s] * h2[s];
+      float back = h1[s];
+#pragma unroll
+      for (int p = NS - 2; p >= 0; --p) {
+        if (p >= s) continue;
+        back *= h2[p];
+        mids[(s * (s - 1) / 2 + p) * DK + c] = back;
+        back *= h1[p];
+      }
+    }
+  }
+  // the values, held in registers until the keys' place is free
+  const int cg = tid & 15, tg = tid >> 4;
+  float vr[C * JT / 128];
+  load_values<128, C>(a, t0, 0, n, h, j0, nj, vr);
+  __syncthreads();
+  // ---- scores: 80 tiles of 4 x 8 (eight per 16 x 16 block of the lower triangle), 20 lanes of every warp
+  float sc[4][8];
+  int si = 0, sj = 0, sb = 0, sp = 0;
+  const bool scorer = lane < 20;
+  if (scorer) {
+    const int tile = warp * 20 + lane, blk = tile >> 3, w = tile & 7;
+    sb = blk < 1 ? 0 : blk < 3 ? 1 : blk < 6 ? 2 : 3;
+    sp = blk - sb * (sb + 1) / 2;
+    si = sb * SB + (w & 3);            // tokens si + 4 m, keys sj + 2 m: neighbouring lanes read neighbouring rows
+    sj = sp * SB + (w >> 2);
+    uint64_t acc[4][8];
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+      for (int j = 0; j < 8; ++j) acc[i][j] = 0;
+    const float* mid = mids + (sb * (sb - 1) / 2 + sp) * DK;
+#pragma unroll 1
+    for (int c = 0; c < DK; c += 4) {
+      ulonglong2 f;
+      f.x = f.y = pack(1.f, 1.f);
+      if (sb != sp) f = lds2(mid + c);
+      ulonglong2 q4[4];
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        q4[i] = lds2(qs + (si + 4 * i) * LD + c);
+        q4[i].x = pmul(q4[i].x, f.x);
+        q4[i].y = pmul(q4[i].y, f.y);
+      }
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+        const ulonglong2 k4 = lds2(ks + (sj + 2 * j) * LD + c);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) acc[i][j] = pfma(q4[i].y, k4.y, pfma(q4[i].x, k4.x, acc[i][j]));
+      }
+    }
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+        const float2 p = unpack(acc[i][j]);
+        const int ti = si + 4 * i, tj = sj + 2 * j;
+        float x = p.x + p.y;
+        if (tj > ti) x = 0.f;
+        else if (BEFORE && tj == ti) x = bonus_of(ti);
+        sc[i][j] = x;
+      }
+  }
+  __syncthreads();
+  // ---- scores over the keys, values behind them, q from its sub-block's middle to the chunk's start
+  if (scorer) {
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+      for (int j = 0; j < 8; ++j) as[(si + 4 * i) * LA + sj + 2 * j] = sc[i][j];
+  }
+#pragma unroll
+  for (int i = 0; i < C * JT / 128; ++i) vs[tid + i * 128] = vr[i];
+  for (int i = tid; i < C * (DK / 4); i += 128) {
+    const int t = i / (DK / 4), c = (i % (DK / 4)) * 4;
+    float4* p = reinterpret_cast<float4*>(qs + t * LD + c);
+    const float4 f = *reinterpret_cast<const float4*>(mids + (6 + t / SB) * DK + c), x = *p;
+    *p = make_float4(x.x * f.x, x.y * f.y, x.z * f.z, x.w * f.w);
+  }
+  __syncthreads();
+  // ---- o = q S: pairs along the key rows
+  float o[8][4];
+  {
+    uint64_t acc[8][4];
+#pragma unroll
+    for (int m = 0; m < 8; ++m)
+#pragma unroll
+      for (int j = 0; j < 4; ++j) acc[m][j] = 0;
+#pragma unroll 1
+    for (int c = 0; c < DK; c += 4) {
+      ulonglong2 s4[4];
+#pragma unroll
+      for (int j = 0; j < 4; ++j) s4[j] = lds2(ss + (cg + 16 * j) * LD + c);
+#pragma unroll
+      for (int m = 0; m < 8; ++m) {
+        const ulonglong2 q4 = lds2(qs + (tg + 8 * m) * LD + c);
+#pragma unroll
+        for (int j = 0; j < 4; ++j) acc[m][j] = pfma(q4.y, s4[j].y, pfma(q4.x, s4[j].x, acc[m][j]));
+      }
+    }
+#pragma unroll
+    for (int m = 0; m < 8; ++m)
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const float2 p = unpack(acc[m][j]);
+        o[m][j] = p.x + p.y;
+      }
+  }
+  // ---- o += scores v: rows of sub-blocks s and later see the keys of sub-block s
+#pragma unroll
+  for (int s = 0; s < NS; ++s) {
+#pragma unroll 1
+    for (int t = s * SB; t < (s + 1) * SB; t += 4) {
+      float v4[4][4];
+#pragma unroll
+      for (int x = 0; x < 4; ++x)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) v4[x][j] = vs[(t + x) * JT + cg + 16 * j];
+#pragma unroll
+      for (int m = 2 * s; m < 8; ++m) {
+        const float4 w = *reinterpret_cast<const float4*>(as + (tg + 8 * m) * LA + t);
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+          o[m][j] = fmaf(w.w, v4[3][j], fmaf(w.z, v4[2][j], fmaf(w.y, v4[1][j], fmaf(w.x, v4[0][j], o[m][j]))));
+      }
+    }
+  }
+#pragma unroll
+  for (int m = 0; m < 8; ++m) {
+    const int t = tg + 8 * m;
+    if (t >= n) continue;
+#pragma unroll
+    for (int j = 0; j < 4; ++j)
+      if (cg + 16 * j < nj) op[t * ldo + cg + 16 * j] = o[m][j];
+  }
+}
+
+template <int DK, int KIND, bool BEFORE>
+int launch_chunks(const ChunkArgs& a, int B, int nch, cudaStream_t stream) {
+  const dim3 grid(nch, a.H * a.nslices, B);
+  constexpr int s1 = (C * DK + C * JT + NS * DK + C) * 4, s3 = OutSmem<DK>::FLOATS * 4;
+  static PerDeviceSmem g1, g3;
+  LLMSS_CHECK_CUDA(g1.ensure(scan_state_kernel<DK, KIND>, s1));
+  LLMSS_CHECK_CUDA(g3.ensure(scan_out_kernel<DK, KIND, BEFORE>, s3));
+  scan_state_kernel<DK, KIND><<<grid, DK, s1, stream>>>(a);
+  const int plane = a.H * a.dv * a.dk;
+  scan_carry_kernel<<<dim3((plane + 511) / 512, B), 256, 0, stream>>>(a);
+  scan_out_kernel<DK, KIND, BEFORE><<<grid, 128, s3, stream>>>(a);
+  LLMSS_CHECK_CUDA(cudaGetLastError());
+  return 0;
+}
+
+}  // namespace
+
+// Floats of scratch for T packed tokens of B sequences.
+LLMSS_API int64_t llmss_linear_scan_chunked_floats(int T, int B, int H, int dk, int dv) {
+  return ((int64_t)T / C + B) * H * (int64_t)dk * (dv + 1);
+}
+
+// llmss_linear_scan over chunks of 64 tokens (see the head of this file): dk a multiple of 4 up to 128, the state and the scratch on
+// 16-byte lines; any strides, value size and sequence lengths.
+LLMSS_API int llmss_linear_scan_chunked(const float* q, int64_t ldq, const float* k, int64_t ldk, const float* v, int64_t ldv, const float* decay,
+                                        int64_t ldd, int decay_kind, const float* bonus, const float* vscale, int64_t ldvs, float* out,
+                                        float* state, const int* cu_q, const int* seq_lens, const int* slots, int B, int T, int max_q, int heads,
+                                        int qk_heads, int dk, int dv, int read_before, float* scratch, cudaStream_t stream) {
+  LLMSS_REQUIRE(heads > 0 && qk_heads > 0 && heads % qk_heads == 0, "linear_scan_chunked: %d heads over %d query/key heads", heads, qk_heads);
+  LLMSS_REQUIRE(dk > 0 && dk % 4 == 0 && dk <= 128 && dv > 0, "linear_scan_chunked: key size %d (a multiple of 4 up to 128), value size %d", dk, dv);
+  LLMSS_REQUIRE(decay_kind >= 0 && decay_kind <= 2 && scratch != nullptr, "linear_scan_chunked: decay kind %d", decay_kind);
+  LLMSS_REQUIRE((((uintptr_t)state | (uintptr_t)scratch) & 15) == 0, "linear_scan_chunked: state / scratch off the 16-byte lines");
+  if (B <= 0 || max_q <= 0) return 0;
+  ChunkArgs a{q, ldq, k, ldk, v, ldv, decay, ldd, bonus, vscale, ldvs, out, state, cu_q, seq_lens, slots, nullptr, nullptr, heads, heads / qk_heads,
+              dk, dv, (dv + JT - 1) / JT};
+  a.chunks = scratch;
+  a.decays = scratch + ((int64_t)T / C + B) * heads * (int64_t)dk * dv;
+  const int nch = (max_q + C - 1) / C;
+  LLMSS_REQUIRE((int64_t)heads * a.nslices <= 65535 && B <= 65535 && (int64_t)heads * dv * dk < (1ll << 30), "linear_scan_chunked: grid too large");
+#define LLMSS_LC(DK, KIND)                                                                      \
+  return read_before ? launch_chunks<DK, KIND, true>(a, B, nch, stream) : launch_chunks<DK, KIND, false>(a, B, nch, stream)
+  if (dk <= 64) {
+    if (decay_kind == 0) LLMSS_LC(64, 0);
+    if (decay_kind == 1) LLMSS_LC(64, 1);
+    LLMSS_LC(64, 2);
+  }
+  if (decay_kind == 0) LLMSS_LC(128, 0);
+  if (decay_kind == 1) LLMSS_LC(128, 1);
+  LLMSS_LC(128, 2);
+#undef LLMSS_LC
+}

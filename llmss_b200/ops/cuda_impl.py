@@ -767,6 +767,10 @@ def ssm_dt(dt_raw, dt_bias, a_log):
 
 _SCAN_CHUNK = int(os.environ.get("LLMSS_SCAN_CHUNK", "128"))          # tokens per chunk of the two-pass recurrence
 _SCAN_CHUNK_MIN = int(os.environ.get("LLMSS_SCAN_CHUNK_MIN", "256"))   # portions from this length on run in two passes
+# Portions from this length on run as products over chunks of 64 tokens.  Products / token by token on B200, us: 8 x 128 tokens 90 / 127
+# (32 heads of 64 x 64, decay per channel), 117 / 246 (16 of 128 x 128, per channel), 117 / 134 (constant decay), 116 / 130 (32 of
+# 128 x 64, decay per token); 8 x 64 tokens 94 / 77, 80 / 140, 86 / 80, 82 / 77.
+_SCAN_TILES_MIN = int(os.environ.get("LLMSS_SCAN_TILES_MIN", "96"))
 
 
 def linear_scan(q, k, v, decay, decay_kind, batch, state, heads, qk_heads, dk, dv, bonus=None, v_scale=None, read_before=False):
@@ -777,6 +781,17 @@ def linear_scan(q, k, v, decay, decay_kind, batch, state, heads, qk_heads, dk, d
     assert decay.dtype == torch.float32 and state.dtype == torch.float32 and state.is_contiguous()
     out = torch.empty(T, heads * dv, dtype=torch.float32, device=v.device)
     cu, sl, ss, B, mq = _bq(batch)
+    if (mq >= _SCAN_TILES_MIN and dk % 4 == 0 and dk <= 128 and state.data_ptr() % 16 == 0 and heads * -(-dv // 64) <= 65535 and B <= 65535
+            and not torch.cuda.is_current_stream_capturing()):
+        # portions: products of tiles over chunks of 64 tokens (csrc/scan_chunk.cu)
+        scratch = torch.empty(lib.llmss_linear_scan_chunked_floats(T, B, heads, dk, dv), dtype=torch.float32, device=v.device)
+        rc = lib.llmss_linear_scan_chunked(_ptr(q), ldq, _ptr(k), ldk, _ptr(v), ldv, _ptr(decay), decay.stride(0) if decay.dim() == 2 else 0,
+                                           decay_kind, _ptr(bonus), _ptr(v_scale), v_scale.stride(0) if v_scale is not None else 0, _ptr(out),
+                                           _ptr(state), cu, sl, ss, B, T, mq, heads, qk_heads, dk, dv, 1 if read_before else 0, _ptr(scratch),
+                                           _stream())
+        _lib.check(rc, "llmss_linear_scan_chunked")
+        _count(3)
+        return out
     # long portions of few sequences: two passes over chunks, every chunk a block (a recurrence is a chain per token)
     chunk, scratch = 0, None
     if mq >= _SCAN_CHUNK_MIN and not torch.cuda.is_current_stream_capturing():

@@ -85,3 +85,63 @@ def test_experts_sorted_on_the_device(T, W, E, top, F, gated, skew):
         x = torch.nn.functional.silu(x[:, 0::2]) * x[:, 1::2] if gated else torch.nn.functional.silu(x)
         want.index_add_(0, t, wts[t, j].double()[:, None] * (x @ down[:, e * F:(e + 1) * F].double().t()))
     assert _rel(got, want.cpu()) < 1e-2
+
+
+def _scan64(q, k, v, a, bonus, before, lens, S0):
+    """The recurrence of ops.reference.linear_scan in 64 bits; a [T, H, dk] decay factors; S0 per sequence [H, dk, dv]."""
+    out, ends, at = torch.zeros_like(v), [], 0
+    for n, S in zip(lens, S0):
+        S = S.clone()
+        for t in range(at, at + n):
+            kv = k[t][:, :, None] * v[t][:, None, :]
+            new = a[t][:, :, None] * S + kv
+            read = (S + (bonus[:, :, None] * kv if bonus is not None else 0)) if before else new
+            out[t] = torch.einsum("hkv,hk->hv", read, q[t])
+            S = new
+        ends.append(S)
+        at += n
+    return out, ends
+
+
+@pytest.mark.parametrize("kind,dk,dv,heads,qk_heads,before,deep", [
+    (2, 64, 64, 2, 2, True, 0), (2, 128, 128, 2, 2, False, 0), (1, 128, 64, 4, 2, False, 0), (0, 128, 128, 2, 2, False, 0), (2, 4, 1, 3, 3, False, 0),
+    (2, 60, 70, 2, 2, True, 0), (1, 100, 130, 2, 1, True, 0), (0, 68, 3, 2, 2, False, 0), (2, 64, 64, 2, 2, True, 1), (2, 128, 72, 1, 1, False, 1),
+    (1, 64, 16, 2, 2, False, 2)])
+def test_linear_scan_over_chunks(kind, dk, dv, heads, qk_heads, before, deep):
+    """Portions that end inside, at and behind a chunk, with and without a state, in packed order and with an inert sequence; strides
+    off the 16-byte lines; ``deep``: decays past 2^-100 within half a sub-block (1), growth (2) -- the token-by-token form of a chunk.
+    Bound: 32-bit sums, 2e-6 of the norm."""
+    torch.manual_seed(dk * 7 + dv)
+    lens, ctxs, slots = [64, 1, 130, 65, 200, 3], [0, 5, 7, 0, 64, 9], [4, 0, 2, 5, 1, -1]
+    T = sum(lens)
+    wide = lambda n: torch.randn(T, n + 3, device="cuda")[:, 1:n + 1]
+    q, k, v = wide(qk_heads * dk), wide(qk_heads * dk), wide(heads * dv)
+    bonus = torch.randn(heads, dk, device="cuda") * 0.5 if before else None
+    scale = None
+    if kind == 0:
+        dec = torch.rand(heads, device="cuda") * 0.5 + 0.5
+        a = dec.double().cpu().view(1, heads, 1).expand(T, heads, dk)
+    else:
+        n = heads if kind == 1 else heads * dk
+        dec = -torch.exp(wide(n) - 1.0)
+        if deep == 1:
+            dec = torch.where(torch.rand(T, n, device="cuda") < 0.02, -300.0, dec)
+        if deep == 2:
+            dec = torch.where(torch.rand(T, n, device="cuda") < 0.01, 8.0, dec * 2)
+        a = torch.exp(dec.double().cpu()).view(T, heads, -1).expand(T, heads, dk)
+        scale = torch.rand(T, heads, device="cuda") + 0.5 if kind == 1 else None
+    state = torch.randn(6, heads, dk, dv, device="cuda")
+    S0 = [state[s].reshape(heads, dv, dk).transpose(1, 2).double().cpu() if c else torch.zeros(heads, dk, dv, dtype=F64) for s, c in zip(slots, ctxs)]
+    rep = heads // qk_heads
+    d = lambda x, n, w: x.double().cpu().reshape(T, n, w)
+    vv = d(v, heads, dv) * (scale.double().cpu()[:, :, None] if scale is not None else 1.0)
+    want, ends = _scan64(d(q, qk_heads, dk).repeat_interleave(rep, 1), d(k, qk_heads, dk).repeat_interleave(rep, 1), vv, a,
+                         bonus.double().cpu() if before else None, before, lens, S0)
+    before_state = state.clone()
+    got = ops.linear_scan(q, k, v, dec, kind, _batch(lens, ctxs, slots), state, heads, qk_heads, dk, dv, bonus=bonus, v_scale=scale,
+                          read_before=before)
+    live = T - lens[-1]
+    assert _rel(got[:live], want.reshape(T, -1)[:live]) < 2e-6
+    for s, S in zip(slots[:-1], ends):
+        assert _rel(state[s].reshape(heads, dv, dk).transpose(1, 2), S) < 2e-6
+    assert torch.equal(state[3], before_state[3])        # a slot that no sequence names
