@@ -14,6 +14,8 @@
 // decay from the middle (products of at most 8 factors, one division); between sub-blocks the factor from middle to middle is at
 // most 1.  F and 1 / F stay finite while half a sub-block decays by no more than 2^-100 (or grows by 2^100) in any channel; a chunk
 // where one does more runs token by token (a column per thread).  Kernel 1 needs no reciprocals: its factors are suffix products.
+// Decays that are one number per token or head are multiplied out in 64 bits, once per chunk: with a constant decay every rounding has
+// the same sign, and the powers' error, not the sums', would be the result's (3.5e-7 of the norm against 7e-8 token by token).
 //
 // B200, 8 prompts of 1024 tokens, against the two passes of the token-serial form: 32 heads of 64 x 64, decay per channel and bonus
 // 618 -> 376 us (99 + 36 + 221, ncu: 44 % of the multiply-add pipe, shared memory 37 to 57 % of its bandwidth); 16 heads of 128 x 128, per
@@ -38,6 +40,7 @@ struct ChunkArgs {
   const int* cu_q; const int* seq_lens; const int* slots;
   float* chunks;                       // [chunk slots][H][dv][dk]: U_c, then S_c
   float* decays;                       // [chunk slots][H][dk]
+  float* decay_rest;                   // [chunk slots][H]: what rounding D_c to 32 bits left (kinds 0 and 1)
   int H, rep, dk, dv, nslices;
 };
 
@@ -102,13 +105,12 @@ __device__ __forceinline__ float recip(float x) {
   asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
   return fmaf(y, fmaf(-x, y, 1.f), y);
 }
-// decay factors of SB tokens of a channel (1 where `in` is false or past n); `table`: a chunk's per-token factors (kinds 0 and 1)
-template <int KIND>
-__device__ __forceinline__ void load_factors(const float* p, int64_t ld, const float* table, int l0, int n, bool in, float (&x)[SB]) {
-  if (KIND == 2) load_rows(p, ld, l0, n, x);
+// decay factors of SB tokens of a channel (1 where `in` is false or past n)
+__device__ __forceinline__ void load_factors(const float* p, int64_t ld, int l0, int n, bool in, float (&x)[SB]) {
+  load_rows(p, ld, l0, n, x);
 #pragma unroll
   for (int i = 0; i < SB; ++i) {
-    const float f = KIND == 2 ? expf(x[i]) : table[l0 + i];
+    const float f = expf(x[i]);
     x[i] = in && l0 + i < n ? f : 1.f;
   }
 }
@@ -131,14 +133,20 @@ __device__ __forceinline__ void load_values(const ChunkArgs& a, int64_t t0, int 
   for (int i = 0; i < E; ++i)
     if (j >= nj || t1 + i * STEP >= n) x[i] = 0.f;
 }
+// kinds 0 and 1: a chunk's factors per token in 64 bits
 template <int KIND>
-__device__ __forceinline__ void fill_table(const ChunkArgs& a, float* table, int64_t t0, int n, int h) {
-  if (KIND != 2 && threadIdx.x < C) {
-    float x = 1.f;
-    if ((int)threadIdx.x < n) x = KIND == 0 ? a.decay[h] : expf(a.decay[(t0 + threadIdx.x) * a.ldd + h]);
+__device__ __forceinline__ void fill_table(const ChunkArgs& a, double* table, int64_t t0, int n, int h) {
+  if (threadIdx.x < C) {
+    double x = 1.0;
+    if ((int)threadIdx.x < n) x = KIND == 0 ? (double)a.decay[h] : exp((double)a.decay[(t0 + threadIdx.x) * a.ldd + h]);
     table[threadIdx.x] = x;
   }
-  if (KIND != 2) __syncthreads();
+  __syncthreads();
+}
+__device__ __forceinline__ double product(const double* table, int lo, int hi) {
+  double p = 1.0;
+  for (int t = lo; t < hi; ++t) p *= table[t];
+  return p;
 }
 
 // ---- 1: U_c and D_c, DK threads.  A thread owns 8 key rows x 8 value columns, both as two runs of 4 half a tile apart (the quarter
@@ -148,8 +156,9 @@ __global__ void __launch_bounds__(DK, DK == 64 ? 7 : 4) scan_state_kernel(ChunkA
   extern __shared__ __align__(16) float sm[];
   float* ks = sm;                      // [C][DK] keys times the decay behind them, inside the sub-block
   float* vs = ks + C * DK;             // [C][JT]
-  float* ds = vs + C * JT;             // [NS][DK] decay of a sub-block
-  float* table = ds + NS * DK;         // [C]
+  float* ds = vs + C * JT;             // [NS][DK] decay of a sub-block (kind 2)
+  float* behind = ds;                  // [C] decay behind a token, to the chunk's end (kinds 0 and 1)
+  double* table = reinterpret_cast<double*>(ds + NS * DK);         // [C]
   const Rows r = rows_of(a, blockIdx.z);
   const int t_lo = blockIdx.x * C;
   if (t_lo >= r.ql) return;
@@ -157,7 +166,11 @@ __global__ void __launch_bounds__(DK, DK == 64 ? 7 : 4) scan_state_kernel(ChunkA
   const int j0 = slice * JT, nj = min(JT, a.dv - j0);
   const int64_t t0 = r.q0 + t_lo;
   const int hq = h / a.rep;
-  fill_table<KIND>(a, table, t0, n, h);
+  if (KIND != 2) {
+    fill_table<KIND>(a, table, t0, n, h);
+    if (threadIdx.x < C) behind[threadIdx.x] = (float)product(table, threadIdx.x + 1, C);
+    __syncthreads();
+  }
   {
     const int c = threadIdx.x, cc = min(c, a.dk - 1);
     const bool in = c < a.dk;
@@ -167,15 +180,15 @@ __global__ void __launch_bounds__(DK, DK == 64 ? 7 : 4) scan_state_kernel(ChunkA
     for (int s = 0; s < NS; ++s) {
       float kx[SB], x[SB], vr[C * JT / DK / NS];
       load_rows(kp, a.ldk, s * SB, n, kx);
-      load_factors<KIND>(dp, a.ldd, table, s * SB, n, in, x);
+      if (KIND == 2) load_factors(dp, a.ldd, s * SB, n, in, x);
       load_values<DK, SB>(a, t0, s * SB, n, h, j0, nj, vr);
       float p = 1.f;
 #pragma unroll
       for (int i = SB - 1; i >= 0; --i) {
-        ks[(s * SB + i) * DK + c] = in && s * SB + i < n ? kx[i] * p : 0.f;
-        p *= x[i];
+        ks[(s * SB + i) * DK + c] = in && s * SB + i < n ? kx[i] * (KIND == 2 ? p : behind[s * SB + i]) : 0.f;
+        if (KIND == 2) p *= x[i];
       }
-      ds[s * DK + c] = p;
+      if (KIND == 2) ds[s * DK + c] = p;
 #pragma unroll
       for (int i = 0; i < C * JT / DK / NS; ++i) vs[s * SB * JT + threadIdx.x + i * DK] = vr[i];
     }
@@ -191,7 +204,7 @@ __global__ void __launch_bounds__(DK, DK == 64 ? 7 : 4) scan_state_kernel(ChunkA
     for (int j = 0; j < 8; ++j) acc[p][j] = 0;
 #pragma unroll 1
   for (int s = 0; s < NS; ++s) {
-    if (s > 0) {
+    if (KIND == 2 && s > 0) {
       const ulonglong2 d0 = lds2(ds + s * DK + i0), d1 = lds2(ds + s * DK + i1);
 #pragma unroll
       for (int j = 0; j < 8; ++j) {
@@ -224,13 +237,20 @@ __global__ void __launch_bounds__(DK, DK == 64 ? 7 : 4) scan_state_kernel(ChunkA
   }
   if (slice == 0 && (int)threadIdx.x < a.dk) {
     float p = 1.f;
+    if (KIND == 2) {
 #pragma unroll
-    for (int s = 0; s < NS; ++s) p *= ds[s * DK + threadIdx.x];
+      for (int s = 0; s < NS; ++s) p *= ds[s * DK + threadIdx.x];
+    } else {
+      const double all = product(table, 0, C);
+      p = (float)all;
+      if (threadIdx.x == 0) a.decay_rest[at] = (float)(all - (double)p);
+    }
     a.decays[at * a.dk + threadIdx.x] = p;
   }
 }
 
 // ---- 2: chunk states, two neighbouring key rows of a value column per thread; grid (plane / 512, B).  Eight chunks' loads in flight
+template <bool REST>
 __global__ void __launch_bounds__(256) scan_carry_kernel(ChunkArgs a) {
   const Rows r = rows_of(a, blockIdx.y);
   if (r.ql <= 0) return;
@@ -243,18 +263,22 @@ __global__ void __launch_bounds__(256) scan_carry_kernel(ChunkArgs a) {
   const int nch = (r.ql + C - 1) / C, dstep = a.H * a.dk;
   float* u = a.chunks + (int64_t)r.first * plane + e;
   const float* d = a.decays + ((int64_t)r.first * a.H + h) * a.dk + i;
+  const float* rest = a.decay_rest + (int64_t)r.first * a.H + h;
   for (int c0 = 0; c0 < nch; c0 += 8) {
     float2 uu[8], dd[8];
+    float rr[8];
 #pragma unroll
     for (int x = 0; x < 8; ++x) {
       const int c = min(c0 + x, nch - 1);
       asm volatile("ld.global.v2.f32 {%0, %1}, [%2];" : "=f"(uu[x].x), "=f"(uu[x].y) : "l"(u + (int64_t)c * plane));
       asm volatile("ld.global.v2.f32 {%0, %1}, [%2];" : "=f"(dd[x].x), "=f"(dd[x].y) : "l"(d + (int64_t)c * dstep));
+      rr[x] = REST ? rest[(int64_t)c * a.H] : 0.f;
     }
 #pragma unroll
     for (int x = 0; x < 8; ++x)
       if (c0 + x < nch) {
         *reinterpret_cast<float2*>(u + (int64_t)(c0 + x) * plane) = S;
+        if (REST) uu[x] = make_float2(fmaf(rr[x], S.x, uu[x].x), fmaf(rr[x], S.y, uu[x].y));
         S = make_float2(fmaf(dd[x].x, S.x, uu[x].x), fmaf(dd[x].y, S.y, uu[x].y));
       }
   }
@@ -267,7 +291,7 @@ __global__ void __launch_bounds__(256) scan_carry_kernel(ChunkArgs a) {
 template <int DK> struct OutSmem {
   static constexpr int LD = DK + 4, LA = C + 4;
   static constexpr int Q = C * LD, S = JT * LD, KA = (C * LD > C * LA + C * JT) ? C * LD : C * LA + C * JT;
-  static constexpr int FLOATS = Q + KA + S + 2 * NS * DK + 10 * DK + (DK / 32 + 1) * C;
+  static constexpr int FLOATS = Q + KA + S + 2 * NS * DK + 10 * DK + (DK / 32 + 4) * C + 2 * 2 * NS;
 };
 
 template <int DK, int KIND, bool BEFORE>
@@ -283,7 +307,10 @@ __global__ void __launch_bounds__(128, DK == 64 ? 3 : 2) scan_out_kernel(ChunkAr
   float* halves = ss + M::S;            // [NS][2][DK] decay of the first and second half of a sub-block
   float* mids = halves + 2 * NS * DK;   // [10][DK]: middle of s' to middle of s (pairs (1,0) (2,0) (2,1) (3,0) (3,1) (3,2)), start to middle of s
   float* diag = mids + 10 * DK;         // [DK / 32][C] bonus products, a part per 32 channels
-  float* table = diag + (DK / 32) * C;  // [C]
+  double* table = reinterpret_cast<double*>(diag + (DK / 32) * C);   // [C] (kinds 0 and 1)
+  double* thalf = table + C;            // [NS][2]
+  float* tq = reinterpret_cast<float*>(thalf + 2 * NS);              // [C] factors on q and, [C], on k
+  float* tk = tq + C;
   const Rows r = rows_of(a, blockIdx.z);
   const int t_lo = blockIdx.x * C;
   if (t_lo >= r.ql) return;
@@ -294,7 +321,18 @@ __global__ void __launch_bounds__(128, DK == 64 ? 3 : 2) scan_out_kernel(ChunkAr
   const float* S = a.chunks + (((int64_t)(r.first + blockIdx.x) * a.H + h) * a.dv + j0) * a.dk;
   const float* qp = a.q + t0 * a.ldq + (int64_t)hq * a.dk;
   const float* kp = a.k + t0 * a.ldk + (int64_t)hq * a.dk;
-  fill_table<KIND>(a, table, t0, n, h);
+  if (KIND != 2) {
+    fill_table<KIND>(a, table, t0, n, h);
+    if (tid < C) {
+      const int mid = tid / SB * SB + SB / 2;          // F(t): from the middle to behind t
+      const double f = tid >= mid ? product(table, mid, tid + 1) : 1.0 / product(table, tid + 1, mid);
+      tq[tid] = (float)(BEFORE ? (tid >= mid ? product(table, mid, tid) : 1.0 / product(table, tid, mid)) : f);
+      tk[tid] = (float)(1.0 / f);
+    } else if (tid < C + 2 * NS) {
+      thalf[tid - C] = product(table, (tid - C) * (SB / 2), (tid - C + 1) * (SB / 2));
+    }
+    __syncthreads();
+  }
   // start state -> shared memory (asynchronously; a column or channel that is not there is never copied into and zeroed instead)
   for (int i = tid; i < JT * (DK / 4); i += 128) {
     const int j = i / (DK / 4), c = (i % (DK / 4)) * 4;
@@ -311,7 +349,7 @@ __global__ void __launch_bounds__(128, DK == 64 ? 3 : 2) scan_out_kernel(ChunkAr
     float x[SB], qx[SB], kx[SB];
     load_rows(qp + cc, a.ldq, l0, n, qx);
     load_rows(kp + cc, a.ldk, l0, n, kx);
-    load_factors<KIND>(KIND == 2 ? a.decay + t0 * a.ldd + (int64_t)h * a.dk + cc : nullptr, a.ldd, table, l0, n, in, x);
+    if (KIND == 2) load_factors(a.decay + t0 * a.ldd + (int64_t)h * a.dk + cc, a.ldd, l0, n, in, x);
 #pragma unroll
     for (int i = 0; i < SB; ++i)
       if (!in || l0 + i >= n) qx[i] = kx[i] = 0.f;
@@ -329,6 +367,14 @@ __global__ void __launch_bounds__(128, DK == 64 ? 3 : 2) scan_out_kernel(ChunkAr
       }
       d[0] += __shfl_xor_sync(0xffffffffu, d[0], 1);
       if (!(lane & 1)) diag[(c >> 5) * C + l0 + (lane >> 1)] = d[0];
+    }
+    if (KIND != 2) {
+#pragma unroll
+      for (int i = 0; i < SB; ++i) {
+        qs[(l0 + i) * LD + c] = qx[i] * tq[l0 + i];
+        ks[(l0 + i) * LD + c] = kx[i] * tk[l0 + i];
+      }
+      continue;
     }
     float f = 1.f;
 #pragma unroll
@@ -351,6 +397,7 @@ __global__ void __launch_bounds__(128, DK == 64 ? 3 : 2) scan_out_kernel(ChunkAr
     halves[2 * s * DK + c] = f;
     deep |= !(f >= kSafe && f <= 1.f / kSafe);
   }
+  if (KIND != 2 && tid < 2 * NS) deep = !(thalf[tid] >= (double)kSafe && thalf[tid] <= 1.0 / kSafe);
   asm volatile("cp.async.wait_all;" ::: "memory");
   auto bonus_of = [&](int t) {
     float d = 0.f;
@@ -376,7 +423,7 @@ __global__ void __launch_bounds__(128, DK == 64 ? 3 : 2) scan_out_kernel(ChunkAr
     __syncthreads();
     for (int i = tid; i < C * DK; i += 128) {
       const int t = i / DK, c = i % DK;
-      ss[t * DK + c] = !(t < n && c < a.dk) ? 1.f : KIND == 2 ? expf(a.decay[(t0 + t) * a.ldd + (int64_t)h * a.dk + c]) : table[t];
+      ss[t * DK + c] = !(t < n && c < a.dk) ? 1.f : KIND == 2 ? expf(a.decay[(t0 + t) * a.ldd + (int64_t)h * a.dk + c]) : (float)table[t];
     }
     __syncthreads();
     if (tid < nj) {
@@ -403,24 +450,28 @@ __global__ void __launch_bounds__(128, DK == 64 ? 3 : 2) scan_out_kernel(ChunkAr
     return;
   }
   // factors between middles, and from the chunk's start to the middles
-  for (int c = tid; c < DK; c += 128) {
-    float h1[NS], h2[NS];
-#pragma unroll
-    for (int s = 0; s < NS; ++s) { h1[s] = halves[2 * s * DK + c]; h2[s] = halves[(2 * s + 1) * DK + c]; }
-    float run = 1.f;
+  auto between = [&](auto h1, auto h2, auto&& put) {      // put(pair or 6 + s, factor)
+    auto run = h1(0) * 0 + 1;
 #pragma unroll
     for (int s = 0; s < NS; ++s) {
-      mids[(6 + s) * DK + c] = run * h1[s];
-      run *= h1[s] * h2[s];
-      float back = h1[s];
+      put(6 + s, run * h1(s));
+      run *= h1(s) * h2(s);
+      auto back = h1(s);
 #pragma unroll
       for (int p = NS - 2; p >= 0; --p) {
         if (p >= s) continue;
-        back *= h2[p];
-        mids[(s * (s - 1) / 2 + p) * DK + c] = back;
-        back *= h1[p];
+        back *= h2(p);
+        put(s * (s - 1) / 2 + p, back);
+        back *= h1(p);
       }
     }
+  };
+  for (int c = tid; c < DK; c += 128) {
+    if (KIND == 2)
+      between([&](int s) { return halves[2 * s * DK + c]; }, [&](int s) { return halves[(2 * s + 1) * DK + c]; },
+              [&](int x, float f) { mids[x * DK + c] = f; });
+    else
+      between([&](int s) { return thalf[2 * s]; }, [&](int s) { return thalf[2 * s + 1]; }, [&](int x, double f) { mids[x * DK + c] = (float)f; });
   }
   // the values, held in registers until the keys' place is free
   const int cg = tid & 15, tg = tid >> 4;
@@ -437,38 +488,52 @@ __global__ void __launch_bounds__(128, DK == 64 ? 3 : 2) scan_out_kernel(ChunkAr
     sp = blk - sb * (sb + 1) / 2;
     si = sb * SB + (w & 3);            // tokens si + 4 m, keys sj + 2 m: neighbouring lanes read neighbouring rows
     sj = sp * SB + (w >> 2);
-    uint64_t acc[4][8];
 #pragma unroll
     for (int i = 0; i < 4; ++i)
 #pragma unroll
-      for (int j = 0; j < 8; ++j) acc[i][j] = 0;
+      for (int j = 0; j < 8; ++j) sc[i][j] = 0.f;
     const float* mid = mids + (sb * (sb - 1) / 2 + sp) * DK;
+    // partial sums of 16 channels: the rounding of a score, and with it the result's, is that of the token-serial form
 #pragma unroll 1
-    for (int c = 0; c < DK; c += 4) {
-      ulonglong2 f;
-      f.x = f.y = pack(1.f, 1.f);
-      if (sb != sp) f = lds2(mid + c);
-      ulonglong2 q4[4];
+    for (int cc = 0; cc < DK; cc += 16) {
+      uint64_t acc[4][8];
 #pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        q4[i] = lds2(qs + (si + 4 * i) * LD + c);
-        q4[i].x = pmul(q4[i].x, f.x);
-        q4[i].y = pmul(q4[i].y, f.y);
+      for (int i = 0; i < 4; ++i)
+#pragma unroll
+        for (int j = 0; j < 8; ++j) acc[i][j] = 0;
+#pragma unroll 1
+      for (int c = cc; c < cc + 16; c += 4) {
+        ulonglong2 f;
+        f.x = f.y = pack(1.f, 1.f);
+        if (sb != sp) f = lds2(mid + c);
+        ulonglong2 q4[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          q4[i] = lds2(qs + (si + 4 * i) * LD + c);
+          q4[i].x = pmul(q4[i].x, f.x);
+          q4[i].y = pmul(q4[i].y, f.y);
+        }
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+          const ulonglong2 k4 = lds2(ks + (sj + 2 * j) * LD + c);
+#pragma unroll
+          for (int i = 0; i < 4; ++i) acc[i][j] = pfma(q4[i].y, k4.y, pfma(q4[i].x, k4.x, acc[i][j]));
+        }
       }
 #pragma unroll
-      for (int j = 0; j < 8; ++j) {
-        const ulonglong2 k4 = lds2(ks + (sj + 2 * j) * LD + c);
+      for (int i = 0; i < 4; ++i)
 #pragma unroll
-        for (int i = 0; i < 4; ++i) acc[i][j] = pfma(q4[i].y, k4.y, pfma(q4[i].x, k4.x, acc[i][j]));
-      }
+        for (int j = 0; j < 8; ++j) {
+          const float2 p = unpack(acc[i][j]);
+          sc[i][j] += p.x + p.y;
+        }
     }
 #pragma unroll
     for (int i = 0; i < 4; ++i)
 #pragma unroll
       for (int j = 0; j < 8; ++j) {
-        const float2 p = unpack(acc[i][j]);
         const int ti = si + 4 * i, tj = sj + 2 * j;
-        float x = p.x + p.y;
+        float x = sc[i][j];
         if (tj > ti) x = 0.f;
         else if (BEFORE && tj == ti) x = bonus_of(ti);
         sc[i][j] = x;
@@ -493,14 +558,19 @@ __global__ void __launch_bounds__(128, DK == 64 ? 3 : 2) scan_out_kernel(ChunkAr
   __syncthreads();
   // ---- o = q S: pairs along the key rows
   float o[8][4];
-  {
+#pragma unroll
+  for (int m = 0; m < 8; ++m)
+#pragma unroll
+    for (int j = 0; j < 4; ++j) o[m][j] = 0.f;
+#pragma unroll 1
+  for (int cc = 0; cc < DK; cc += 32) {      // partial sums of 32 channels
     uint64_t acc[8][4];
 #pragma unroll
     for (int m = 0; m < 8; ++m)
 #pragma unroll
       for (int j = 0; j < 4; ++j) acc[m][j] = 0;
 #pragma unroll 1
-    for (int c = 0; c < DK; c += 4) {
+    for (int c = cc; c < cc + 32; c += 4) {
       ulonglong2 s4[4];
 #pragma unroll
       for (int j = 0; j < 4; ++j) s4[j] = lds2(ss + (cg + 16 * j) * LD + c);
@@ -516,12 +586,17 @@ __global__ void __launch_bounds__(128, DK == 64 ? 3 : 2) scan_out_kernel(ChunkAr
 #pragma unroll
       for (int j = 0; j < 4; ++j) {
         const float2 p = unpack(acc[m][j]);
-        o[m][j] = p.x + p.y;
+        o[m][j] += p.x + p.y;
       }
   }
   // ---- o += scores v: rows of sub-blocks s and later see the keys of sub-block s
 #pragma unroll
   for (int s = 0; s < NS; ++s) {
+    float part[8][4];
+#pragma unroll
+    for (int m = 0; m < 8; ++m)
+#pragma unroll
+      for (int j = 0; j < 4; ++j) part[m][j] = 0.f;
 #pragma unroll 1
     for (int t = s * SB; t < (s + 1) * SB; t += 4) {
       float v4[4][4];
@@ -534,9 +609,13 @@ __global__ void __launch_bounds__(128, DK == 64 ? 3 : 2) scan_out_kernel(ChunkAr
         const float4 w = *reinterpret_cast<const float4*>(as + (tg + 8 * m) * LA + t);
 #pragma unroll
         for (int j = 0; j < 4; ++j)
-          o[m][j] = fmaf(w.w, v4[3][j], fmaf(w.z, v4[2][j], fmaf(w.y, v4[1][j], fmaf(w.x, v4[0][j], o[m][j]))));
+          part[m][j] = fmaf(w.w, v4[3][j], fmaf(w.z, v4[2][j], fmaf(w.y, v4[1][j], fmaf(w.x, v4[0][j], part[m][j]))));
       }
     }
+#pragma unroll
+    for (int m = 2 * s; m < 8; ++m)
+#pragma unroll
+      for (int j = 0; j < 4; ++j) o[m][j] += part[m][j];
   }
 #pragma unroll
   for (int m = 0; m < 8; ++m) {
@@ -551,13 +630,13 @@ __global__ void __launch_bounds__(128, DK == 64 ? 3 : 2) scan_out_kernel(ChunkAr
 template <int DK, int KIND, bool BEFORE>
 int launch_chunks(const ChunkArgs& a, int B, int nch, cudaStream_t stream) {
   const dim3 grid(nch, a.H * a.nslices, B);
-  constexpr int s1 = (C * DK + C * JT + NS * DK + C) * 4, s3 = OutSmem<DK>::FLOATS * 4;
+  constexpr int s1 = (C * DK + C * JT + NS * DK + 2 * C) * 4, s3 = OutSmem<DK>::FLOATS * 4;
   static PerDeviceSmem g1, g3;
   LLMSS_CHECK_CUDA(g1.ensure(scan_state_kernel<DK, KIND>, s1));
   LLMSS_CHECK_CUDA(g3.ensure(scan_out_kernel<DK, KIND, BEFORE>, s3));
   scan_state_kernel<DK, KIND><<<grid, DK, s1, stream>>>(a);
   const int plane = a.H * a.dv * a.dk;
-  scan_carry_kernel<<<dim3((plane + 511) / 512, B), 256, 0, stream>>>(a);
+  scan_carry_kernel<KIND != 2><<<dim3((plane + 511) / 512, B), 256, 0, stream>>>(a);
   scan_out_kernel<DK, KIND, BEFORE><<<grid, 128, s3, stream>>>(a);
   LLMSS_CHECK_CUDA(cudaGetLastError());
   return 0;
@@ -567,7 +646,7 @@ int launch_chunks(const ChunkArgs& a, int B, int nch, cudaStream_t stream) {
 
 // Floats of scratch for T packed tokens of B sequences.
 LLMSS_API int64_t llmss_linear_scan_chunked_floats(int T, int B, int H, int dk, int dv) {
-  return ((int64_t)T / C + B) * H * (int64_t)dk * (dv + 1);
+  return ((int64_t)T / C + B) * H * ((int64_t)dk * (dv + 1) + 1);
 }
 
 // llmss_linear_scan over chunks of 64 tokens (see the head of this file): dk a multiple of 4 up to 128, the state and the scratch on
@@ -581,10 +660,11 @@ LLMSS_API int llmss_linear_scan_chunked(const float* q, int64_t ldq, const float
   LLMSS_REQUIRE(decay_kind >= 0 && decay_kind <= 2 && scratch != nullptr, "linear_scan_chunked: decay kind %d", decay_kind);
   LLMSS_REQUIRE((((uintptr_t)state | (uintptr_t)scratch) & 15) == 0, "linear_scan_chunked: state / scratch off the 16-byte lines");
   if (B <= 0 || max_q <= 0) return 0;
-  ChunkArgs a{q, ldq, k, ldk, v, ldv, decay, ldd, bonus, vscale, ldvs, out, state, cu_q, seq_lens, slots, nullptr, nullptr, heads, heads / qk_heads,
+  ChunkArgs a{q, ldq, k, ldk, v, ldv, decay, ldd, bonus, vscale, ldvs, out, state, cu_q, seq_lens, slots, nullptr, nullptr, nullptr, heads, heads / qk_heads,
               dk, dv, (dv + JT - 1) / JT};
   a.chunks = scratch;
   a.decays = scratch + ((int64_t)T / C + B) * heads * (int64_t)dk * dv;
+  a.decay_rest = a.decays + ((int64_t)T / C + B) * heads * dk;
   const int nch = (max_q + C - 1) / C;
   LLMSS_REQUIRE((int64_t)heads * a.nslices <= 65535 && B <= 65535 && (int64_t)heads * dv * dk < (1ll << 30), "linear_scan_chunked: grid too large");
 #define LLMSS_LC(DK, KIND)                                                                      \
