@@ -13,6 +13,10 @@
 // 64 x 64 output tile per CTA, 16-deep k slices through shared memory, 4 x 4 outputs per thread.
 #include "common.cuh"
 
+LLMSS_API int llmss_gemm_heads(const void* x, int64_t ldx, int64_t sxh, const void* w, int64_t ldw, int64_t swh, const float* scale, int64_t lds,
+                               int64_t ssh, int64_t ssn, void* out, int64_t ldo, int64_t soh, int M, int N, int K, int H, int dtype, int out_f32,
+                               cudaStream_t stream);
+
 namespace {
 
 constexpr int BM = 64, BN = 64, BK = 16, NT = 256;
@@ -267,6 +271,11 @@ LLMSS_API int llmss_bgemm_simt_ex(const void* x, int64_t ldx, int64_t sxh, const
   // 16-bit operands without bias / activation (the per-head products) take the tensor-core form; the 32-bit accumulators
   // are the same, so both forms agree to rounding of the summation order
   const bool mma_ok = dtype != LLMSS_F32 && bias == nullptr && act == LLMSS_ACT_NONE && (M + 127) / 128 <= 65535;
+  // prompts, weights with the contraction index contiguous, whole 16-byte vectors: tensor-memory tiles (csrc/gemm_tcgen05.cu) of 256
+  // tokens; up to 128 tokens the warp-level form fills more blocks, between 129 and 400 the two are equal (15 us with the launch)
+  if (mma_ok && M > 128 && swk == 1 && K % 8 == 0 && (ldx | sxh | swn | swh) % 8 == 0 && ldx > 0 && sxh > 0 && swh > 0 &&
+      (((uintptr_t)x | (uintptr_t)w) & 15) == 0)
+    return llmss_gemm_heads(x, ldx, sxh, w, swn, swh, row_scale, lds, ssh, ssn, out, ldo, soh, M, N, K, H, dtype, out_f32, stream);
   if (mma_ok && dtype == LLMSS_BF16) return launch_bg_mma<__nv_bfloat16>(a, out_f32, stream);
   if (mma_ok && dtype == LLMSS_F16) return launch_bg_mma<__half>(a, out_f32, stream);
   if (dtype == LLMSS_F32) return launch_bg<float>(a, 1, stream);

@@ -230,6 +230,10 @@ int llmss_moe_scatter_rows(const void* h, int64_t ldh, const int* inv, int top, 
  * with K, ldx, ldw and w_group_stride multiples of 8 */
 int llmss_gemm_grouped(const void* x, int64_t ldx, const void* w, int64_t ldw, int64_t w_group_stride, const int* table, int E, void* out,
                        int64_t ldo, int P, int N, int K, int dtype, int out_f32, int act, int gated, llmss_stream_t stream);
+/* per-head products out(t, h, n) = scale(t, h, n) * sum_k x[t * ldx + h * sxh + k] * w[h * swh + n * ldw + k]; llmss_bgemm_simt_ex takes it where it pays */
+int llmss_gemm_heads(const void* x, int64_t ldx, int64_t sxh, const void* w, int64_t ldw, int64_t swh, const float* scale, int64_t lds,
+                     int64_t ssh, int64_t ssn, void* out, int64_t ldo, int64_t soh, int M, int N, int K, int H, int dtype, int out_f32,
+                     llmss_stream_t stream);
 int llmss_moe_combine(const float* y, const int* inv, const float* wts, float* out, int64_t ldo, int T, int W, int top,
                       llmss_stream_t stream);
 int llmss_moe_scale(void* a, int64_t lda, const float* dense, int T, int E, int F, int dtype, llmss_stream_t stream);

@@ -145,3 +145,27 @@ def test_linear_scan_over_chunks(kind, dk, dv, heads, qk_heads, before, deep):
     for s, S in zip(slots[:-1], ends):
         assert _rel(state[s].reshape(heads, dv, dk).transpose(1, 2), S) < 2e-6
     assert torch.equal(state[3], before_state[3])        # a slot that no sequence names
+
+
+@pytest.mark.parametrize("T,H,k,n,xs,form", [(129, 3, 128, 128, None, None), (300, 5, 64, 192, 72, "row"), (513, 2, 192, 128, 256, "elem"), (257, 16, 40, 24, None, "f32"),
+                                             (2000, 33, 128, 136, None, "row")])
+@pytest.mark.parametrize("dt", [torch.bfloat16, torch.float16])
+def test_per_head_products_at_prompt_sizes(T, H, k, n, xs, form, dt):
+    """Tokens, features and contraction off the tile sizes, heads as column ranges of wider rows, results between other columns, the
+    factor per token and head or per element.  Bound: one rounding to 16 bits of 32-bit sums (2^-8 / 2^-11 of a value), 1e-6 in 32-bit."""
+    torch.manual_seed(T)
+    xs = xs or k
+    x = torch.randn(T, H * xs, device="cuda").to(dt)
+    w = (torch.randn(H, n, k, device="cuda") * k ** -0.5).to(dt)
+    row = torch.rand(T, H + 1, device="cuda")[:, 1:] if form == "row" else None
+    elem = torch.rand(T, H * n, device="cuda") if form == "elem" else None
+    out = torch.zeros(T, H * (n + 8), device="cuda", dtype=F32 if form == "f32" else dt)
+    ops.heads_matmul(x, w, H, k, n, False, row_scale=row, x_head_stride=xs, elem_scale=elem, out=out, out_head_stride=n + 8)
+    want = torch.einsum("thk,hnk->thn", x.view(T, H, xs)[:, :, :k].double(), w.double())
+    if row is not None:
+        want = want * row.double()[:, :, None]
+    if elem is not None:
+        want = want * elem.double().view(T, H, n)
+    got = out.view(T, H, n + 8)
+    assert _rel(got[:, :, :n], want.cpu()) < (1e-6 if form == "f32" else 2.0 ** -8 if dt == torch.bfloat16 else 2.0 ** -11)
+    assert not got[:, :, n:].any()
