@@ -229,66 +229,71 @@ template <typename TO> __device__ __forceinline__ void store4(TO* p, float a, fl
   *reinterpret_cast<V4*>(p) = o;
 }
 
-template <int kMaxTaps, int CH, typename TO>
+// TAPS and ACT (-1: decided per element) are compile-time: the window is a register rename and the branch-free body lets the next rows'
+// loads run ahead of the activation.
+template <int TAPS, int ACT, int CH, typename TO>
 __global__ void __launch_bounds__(128) causal_conv4_kernel(const float* __restrict__ u, int64_t ldu, const float* __restrict__ w,
-                                                           const float* __restrict__ bias, TO* __restrict__ out, int C, int taps,
-                                                           int act, const int* __restrict__ cu_q, const int* __restrict__ seq_lens,
+                                                           const float* __restrict__ bias, TO* __restrict__ out, int C, int act,
+                                                           const int* __restrict__ cu_q, const int* __restrict__ seq_lens,
                                                            const int* __restrict__ slots, float* __restrict__ state) {
   const Seq s = seq_of(cu_q, seq_lens, slots, blockIdx.x);
   const int c = (blockIdx.y * 128 + threadIdx.x) * 4;
-  if (c >= C) return;
-  const int hist = taps - 1;
-  float wt[kMaxTaps][4];
-  float4 win[kMaxTaps], old[kMaxTaps];
+  if (c >= C || (int)blockIdx.z * CH >= s.ql) return;
+  constexpr int HIST = TAPS - 1, N = HIST > 0 ? HIST : 1;
+  float wt[TAPS][4];
+  float4 win[N], old[N];
   const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
-  for (int i = 0; i < kMaxTaps; ++i) {
+  for (int i = 0; i < TAPS; ++i)
 #pragma unroll
-    for (int e = 0; e < 4; ++e) wt[i][e] = i < taps ? w[(int64_t)(c + e) * taps + i] : 0.f;
-    old[i] = zero;
-  }
+    for (int e = 0; e < 4; ++e) wt[i][e] = w[(int64_t)(c + e) * TAPS + i];
+#pragma unroll
+  for (int i = 0; i < N; ++i) old[i] = zero;
   const float4 bv = bias != nullptr ? *reinterpret_cast<const float4*>(bias + c) : zero;
-  float* st = state != nullptr && s.slot >= 0 ? state + ((int64_t)s.slot * hist) * C + c : nullptr;
+  float* st = state != nullptr && s.slot >= 0 ? state + ((int64_t)s.slot * HIST) * C + c : nullptr;
+  auto activate = [&](float x) { return ACT == LLMSS_ACT_NONE ? x : ACT == LLMSS_ACT_SILU ? x / (1.0f + expf(-x)) : act_exact(x, act); };
   for (int z = blockIdx.z; z * CH < s.ql; z += gridDim.z) {
     const int j0 = z * CH, j1 = min(s.ql, j0 + CH);
     if (z == 0 && st != nullptr && s.ctx > 0) {
 #pragma unroll
-      for (int i = 0; i < kMaxTaps; ++i) if (i < hist) old[i] = *reinterpret_cast<const float4*>(st + (int64_t)i * C);
-    }
-#pragma unroll
-    for (int i = 0; i < kMaxTaps; ++i) {
-      const int jj = j0 - hist + i;
-      win[i] = i >= hist ? zero : (jj >= 0 ? *reinterpret_cast<const float4*>(u + (int64_t)(s.q0 + jj) * ldu + c) : old[i]);
+      for (int i = 0; i < HIST; ++i) old[i] = *reinterpret_cast<const float4*>(st + (int64_t)i * C);
     }
     const float* up = u + (int64_t)(s.q0 + j0) * ldu + c;
     TO* op = out + (int64_t)(s.q0 + j0) * C + c;
-#pragma unroll 4
-    for (int j = j0; j < j1; ++j, up += ldu, op += C) {
-      const float4 cur = *reinterpret_cast<const float4*>(up);
-      float4 acc = bv;
 #pragma unroll
-      for (int i = 0; i < kMaxTaps; ++i) {
-        if (i < taps) {
-          const float4 v = i < hist ? win[i] : cur;
+    for (int i = 0; i < HIST; ++i)
+      win[i] = j0 - HIST + i >= 0 ? *reinterpret_cast<const float4*>(up + (int64_t)(i - HIST) * ldu) : old[i];
+    // blocks of 8 rows: their loads first (rows past the chunk re-read its last row), then the sums
+#pragma unroll 1
+    for (int j = j0; j < j1; j += 8, up += 8 * ldu, op += (int64_t)8 * C) {
+      float4 cur[8];
+#pragma unroll
+      for (int x = 0; x < 8; ++x) cur[x] = *reinterpret_cast<const float4*>(up + (int64_t)min(x, j1 - 1 - j) * ldu);
+#pragma unroll
+      for (int x = 0; x < 8; ++x) {
+        float4 acc = bv;
+#pragma unroll
+        for (int i = 0; i < TAPS; ++i) {
+          const int back = HIST - i;             // this tap's input lies `back` rows before row x
+          const float4 v = x >= back ? cur[x >= back ? x - back : 0] : win[x < back ? HIST - back + x : 0];
           acc.x = fmaf(wt[i][0], v.x, acc.x); acc.y = fmaf(wt[i][1], v.y, acc.y);
           acc.z = fmaf(wt[i][2], v.z, acc.z); acc.w = fmaf(wt[i][3], v.w, acc.w);
         }
+        if (j + x < j1) store4<TO>(op + (int64_t)x * C, activate(acc.x), activate(acc.y), activate(acc.z), activate(acc.w));
       }
 #pragma unroll
-      for (int i = 0; i < kMaxTaps - 1; ++i) win[i] = i + 1 < hist ? win[i + 1] : cur;
-      store4<TO>(op, act_exact(acc.x, act), act_exact(acc.y, act), act_exact(acc.z, act), act_exact(acc.w, act));
+      for (int i = 0; i < HIST; ++i) win[i] = cur[8 - HIST + i];      // (only read again while whole blocks follow)
     }
     if (z == 0 && st != nullptr) {
-      // new tail: inputs ql - hist .. ql - 1; those before this step's first row come from the old tail
+      // new tail: inputs ql - HIST .. ql - 1; those before this step's first row come from the old tail
 #pragma unroll
-      for (int i = 0; i < kMaxTaps; ++i) {
-        if (i >= hist) continue;
-        const int jj = s.ql - hist + i;
+      for (int i = 0; i < HIST; ++i) {
+        const int jj = s.ql - HIST + i;
         float4 v = zero;
         if (jj >= 0) v = *reinterpret_cast<const float4*>(u + (int64_t)(s.q0 + jj) * ldu + c);
         else {
 #pragma unroll
-          for (int k = 0; k < kMaxTaps; ++k) if (k == i + s.ql) v = old[k];
+          for (int k = 0; k < HIST; ++k) if (k == i + s.ql) v = old[k];
         }
         *reinterpret_cast<float4*>(st + (int64_t)i * C) = v;
       }
@@ -931,6 +936,77 @@ __global__ void __launch_bounds__(256) gated_rmsnorm_kernel(GnArgs a, T* __restr
   }
 }
 
+// The same with a group's channels in the registers of L lanes (16 or 32) as V 16-byte pieces each: every input is read once, and the
+// gate's and the weight's loads are in flight behind the sum of squares.  A warp takes 32 / L neighbouring (row, group) pairs.
+template <typename T, int L, int V>
+__global__ void __launch_bounds__(256) gated_rmsnorm_vec_kernel(GnArgs a, T* __restrict__ out, int64_t pairs) {
+  const int lane = threadIdx.x & 31, l = lane % L;
+  const int64_t pair = (int64_t)blockIdx.x * (256 / L) + threadIdx.x / L;
+  const bool live = pair < pairs;
+  const int64_t p = live ? pair : pairs - 1, t = p / a.groups;
+  constexpr int GS = 4 * L * V;
+  const int c0 = (int)(p % a.groups) * GS + l * 4;
+  float4 v[V], g[V];
+  const float4 one = make_float4(1.f, 1.f, 1.f, 1.f);
+#pragma unroll
+  for (int i = 0; i < V; ++i) v[i] = *reinterpret_cast<const float4*>(a.o + t * a.ldo + c0 + i * 4 * L);
+#pragma unroll
+  for (int i = 0; i < V; ++i) g[i] = a.gate != nullptr ? *reinterpret_cast<const float4*>(a.gate + t * a.ldg + c0 + i * 4 * L) : one;
+  if (a.skip_x != nullptr) {
+    const int hs = a.C / a.H;         // a multiple of 4: a piece lies in one head
+#pragma unroll
+    for (int i = 0; i < V; ++i) {
+      const float4 x = *reinterpret_cast<const float4*>(a.skip_x + t * a.ldx + c0 + i * 4 * L);
+      const float d = a.skip_d[(c0 + i * 4 * L) / hs];
+      v[i] = make_float4(fmaf(d, x.x, v[i].x), fmaf(d, x.y, v[i].y), fmaf(d, x.z, v[i].z), fmaf(d, x.w, v[i].w));
+    }
+  }
+  if (a.gate != nullptr) {
+#pragma unroll
+    for (int i = 0; i < V; ++i) {
+      g[i] = make_float4(gate_fn(g[i].x, a.gate_act), gate_fn(g[i].y, a.gate_act), gate_fn(g[i].z, a.gate_act), gate_fn(g[i].w, a.gate_act));
+      if (a.gate_first) v[i] = make_float4(v[i].x * g[i].x, v[i].y * g[i].y, v[i].z * g[i].z, v[i].w * g[i].w);
+    }
+  }
+  float ss = 0.f;
+#pragma unroll
+  for (int i = 0; i < V; ++i) ss = fmaf(v[i].x, v[i].x, fmaf(v[i].y, v[i].y, fmaf(v[i].z, v[i].z, fmaf(v[i].w, v[i].w, ss))));
+#pragma unroll
+  for (int o = L / 2; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
+  const float r = rsqrtf(ss / GS + a.eps);
+  if (!live) return;
+#pragma unroll
+  for (int i = 0; i < V; ++i) {
+    const int c = c0 + i * 4 * L;
+    float4 y = make_float4(v[i].x * r, v[i].y * r, v[i].z * r, v[i].w * r);
+    if (a.weight != nullptr) {
+      const float4 w = *reinterpret_cast<const float4*>(a.weight + c);
+      y = make_float4(y.x * w.x, y.y * w.y, y.z * w.z, y.w * w.w);
+    }
+    if (a.gate != nullptr && !a.gate_first) y = make_float4(y.x * g[i].x, y.y * g[i].y, y.z * g[i].z, y.w * g[i].w);
+    store4<T>(out + t * a.C + c, y.x, y.y, y.z, y.w);
+  }
+}
+
+// groups of 64, 128, 256, 512 or 1024 channels on 16-byte lines; false: the general kernel
+template <typename T>
+bool launch_gn_vec(const GnArgs& a, T* out, int T_, cudaStream_t stream) {
+  const int gs = a.C / a.groups;
+  const uintptr_t all = (uintptr_t)a.o | (uintptr_t)a.gate | (uintptr_t)a.weight | (uintptr_t)a.skip_x | (uintptr_t)out;
+  if ((all & 15) || a.ldo % 4 || (a.gate != nullptr && a.ldg % 4) || (a.skip_x != nullptr && (a.ldx % 4 || a.C / a.H % 4))) return false;
+  const int64_t pairs = (int64_t)T_ * a.groups;
+#define LLMSS_GN(L, V) gated_rmsnorm_vec_kernel<T, L, V><<<(unsigned)((pairs + 256 / L - 1) / (256 / L)), 256, 0, stream>>>(a, out, pairs)
+  if (pairs > 0x7fffffffll) return false;
+  if (gs == 64) LLMSS_GN(16, 1);
+  else if (gs == 128) LLMSS_GN(32, 1);
+  else if (gs == 256) LLMSS_GN(32, 2);
+  else if (gs == 512) LLMSS_GN(32, 4);
+  else if (gs == 1024) LLMSS_GN(32, 8);
+  else return false;
+#undef LLMSS_GN
+  return true;
+}
+
 int grid_for(int64_t n) {
   const int64_t b = (n + 255) / 256;
   return (int)(b < 148 * 8 ? b : 148 * 8);
@@ -993,7 +1069,20 @@ static int causal_conv_launch(const float* u, int64_t ldu, const float* w, const
       ((((uintptr_t)u) | ((uintptr_t)out) | ((uintptr_t)bias) | ((uintptr_t)state)) & 15) == 0) {
     // (a null bias or state is aligned; the state's rows are C floats apart)
     const dim3 grid4(B, (C / 4 + 127) / 128, max(1, min((max_q + 15) / 16, 128)));
-    causal_conv4_kernel<4, 16, TO><<<grid4, 128, 0, stream>>>(u, ldu, w, bias, out, C, taps, act, cu_q, seq_lens, slots, state);
+#define LLMSS_CONV4(TAPS)                                                                                                             \
+  do {                                                                                                                              \
+    if (act == LLMSS_ACT_SILU)                                                                                                      \
+      causal_conv4_kernel<TAPS, LLMSS_ACT_SILU, 16, TO><<<grid4, 128, 0, stream>>>(u, ldu, w, bias, out, C, act, cu_q, seq_lens, slots, state); \
+    else if (act == LLMSS_ACT_NONE)                                                                                                 \
+      causal_conv4_kernel<TAPS, LLMSS_ACT_NONE, 16, TO><<<grid4, 128, 0, stream>>>(u, ldu, w, bias, out, C, act, cu_q, seq_lens, slots, state); \
+    else                                                                                                                            \
+      causal_conv4_kernel<TAPS, -1, 16, TO><<<grid4, 128, 0, stream>>>(u, ldu, w, bias, out, C, act, cu_q, seq_lens, slots, state);       \
+  } while (0)
+    if (taps == 1) LLMSS_CONV4(1);
+    else if (taps == 2) LLMSS_CONV4(2);
+    else if (taps == 3) LLMSS_CONV4(3);
+    else LLMSS_CONV4(4);
+#undef LLMSS_CONV4
     LLMSS_CHECK_CUDA(cudaGetLastError());
     return 0;
   }
@@ -1157,7 +1246,9 @@ LLMSS_API int llmss_gated_rmsnorm(const float* o, int64_t ldo, const float* gate
   GnArgs a;
   a.o = o; a.ldo = ldo; a.gate = gate; a.ldg = ldg; a.weight = weight; a.skip_x = skip_x; a.ldx = ldx; a.skip_d = skip_d;
   a.C = C; a.groups = groups; a.H = H > 0 ? H : 1; a.gate_act = gate_act; a.gate_first = gate_first; a.eps = eps;
-  LLMSS_BY_DTYPE(dtype, (gated_rmsnorm_kernel<T><<<T_, 256, 0, stream>>>(a, (T*)out)));
+  bool done = false;
+  LLMSS_BY_DTYPE(dtype, (done = launch_gn_vec<T>(a, (T*)out, T_, stream)));
+  if (!done) LLMSS_BY_DTYPE(dtype, (gated_rmsnorm_kernel<T><<<T_, 256, 0, stream>>>(a, (T*)out)));
   LLMSS_CHECK_CUDA(cudaGetLastError());
   return 0;
 }

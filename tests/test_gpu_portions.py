@@ -169,3 +169,54 @@ def test_per_head_products_at_prompt_sizes(T, H, k, n, xs, form, dt):
     got = out.view(T, H, n + 8)
     assert _rel(got[:, :, :n], want.cpu()) < (1e-6 if form == "f32" else 2.0 ** -8 if dt == torch.bfloat16 else 2.0 ** -11)
     assert not got[:, :, n:].any()
+
+
+@pytest.mark.parametrize("C,groups,act,first,skip", [(256, 4, 1, False, False), (128, 1, 2, False, True), (512, 2, 1, True, True), (1024, 1, 0, False, False),
+                                                     (3072, 3, 1, True, False), (96, 1, 1, False, False), (512, 1, None, False, False)])
+@pytest.mark.parametrize("T", [1, 37])
+@pytest.mark.parametrize("off", [0, 1])
+def test_gated_norm_groups(C, groups, act, first, skip, T, off):
+    """Groups that a warp (or half of one) holds in registers, odd group sizes, columns off the 16-byte lines (``off``).
+    Bound: 32-bit arithmetic, 2e-6 of the norm."""
+    torch.manual_seed(C + T)
+    wide = lambda: torch.randn(T, C + 8, device="cuda")[:, off:off + C]
+    o, gate, w, x = wide(), wide(), torch.rand(C, device="cuda") + 0.5, wide()
+    d = torch.randn(4, device="cuda")
+    got = ops.gated_rmsnorm(o, gate if act is not None else None, act or 0, w, groups, 1e-6, first, skip_x=x if skip else None,
+                            skip_d=d if skip else None)
+    y = o.double()
+    if skip:
+        y = y + (x.double().reshape(T, 4, C // 4) * d.double()[None, :, None]).reshape(T, C)
+    g = 1.0
+    if act is not None:
+        g = {0: lambda z: z, 1: torch.nn.functional.silu, 2: torch.sigmoid}[act](gate.double())
+    if first:
+        y = y * g
+    y = y.reshape(T, groups, -1)
+    y = (y * torch.rsqrt(y.square().mean(-1, keepdim=True) + 1e-6)).reshape(T, C) * w.double()
+    assert _rel(got, (y if first else y * g).cpu()) < 2e-6
+
+
+@pytest.mark.parametrize("taps", [1, 2, 3, 4])
+@pytest.mark.parametrize("act", [ops.ACT_NONE, ops.ACT_SILU, ops.ACT_GELU_ERF])
+def test_convolution_rows(taps, act):
+    """Portions around the blocks of 8 and the chunks of 16 rows, shorter than the taps, with and without a tail, an inert row.
+    Bound: 32-bit arithmetic, 2e-6 of the norm; tails are copies."""
+    torch.manual_seed(taps)
+    lens, ctxs, slots, C = [1, 8, 15, 17, 40, 2, 5], [3, 0, 5, 0, 9, 1, 4], [0, 3, 1, 2, 6, 4, -1], 132
+    T = sum(lens)
+    u, w, b = torch.randn(T, C + 4, device="cuda")[:, :C], torch.randn(C, taps, device="cuda"), torch.randn(C, device="cuda")
+    state = torch.randn(7, max(1, taps - 1), C, device="cuda") if taps > 1 else None
+    old = state.clone() if taps > 1 else None
+    got = ops.causal_conv(u, w, b, act, _batch(lens, ctxs, slots), state)
+    at = 0
+    for n, c, s in zip(lens, ctxs, slots):
+        if s >= 0:
+            hist = (old[s] if c else torch.zeros_like(old[s])) if taps > 1 else u[:0]
+            full = torch.cat([hist, u[at:at + n]]).double()
+            y = sum(full[j:j + n] * w[:, j].double() for j in range(taps)) + b.double()
+            y = {ops.ACT_NONE: lambda z: z, ops.ACT_SILU: torch.nn.functional.silu, ops.ACT_GELU_ERF: torch.nn.functional.gelu}[act](y)
+            assert _rel(got[at:at + n], y.cpu()) < 2e-6, (n, c)
+            if taps > 1:
+                assert torch.equal(state[s], full[-(taps - 1):].float())
+        at += n
