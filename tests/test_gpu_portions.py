@@ -220,3 +220,23 @@ def test_convolution_rows(taps, act):
             if taps > 1:
                 assert torch.equal(state[s], full[-(taps - 1):].float())
         at += n
+
+
+@pytest.mark.parametrize("H", [256, 1600, 2048, 2056, 4096, 5120, 8192])
+@pytest.mark.parametrize("kind", [ops.NORM_LAYER, ops.NORM_RMS])
+@pytest.mark.parametrize("extra", [0, 1, 2])
+def test_norm_rows_at_prompt_sizes(H, kind, extra):
+    """Rows off the warp's and the block's multiples, with a residual and a second addend.  The same rounding points as the oracle:
+    bound of one bf16 rounding of the result, 2^-8 of a value, and of the stored sum exactly."""
+    from llmss_b200.ops import reference as R
+
+    torch.manual_seed(H)
+    M, dt = 601, torch.bfloat16
+    x, r, x2 = (torch.randn(M, H, device="cuda").to(dt) for _ in range(3))
+    w, b = (torch.randn(H, device="cuda").to(dt) for _ in range(2))
+    got, res = ops.norm_residual(x, r if extra else None, w, b if kind == ops.NORM_LAYER else None, 1e-5, kind, x2=x2 if extra == 2 else None)
+    total = x.float() + (x2.float() if extra == 2 else 0) + (r.float() if extra else 0)
+    total = total.to(dt)
+    assert torch.equal(res, total)
+    want, _ = R.norm_residual(total.double().cpu(), None, w.cpu(), b.cpu() if kind == ops.NORM_LAYER else None, 1e-5, kind, out_dtype=F32)
+    assert _rel(got, want.double()) < 2.0 ** -8
