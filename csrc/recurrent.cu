@@ -564,6 +564,99 @@ __global__ void __launch_bounds__(SCAN_THREADS) linear_scan_kernel(ScanArgs a) {
   }
 }
 
+// The same recurrence for decode steps (a token per sequence): the state is read and written once and nothing is shared between
+// threads, so the bound is the memory system and the form is a stream.  L lanes take one value column's key rows, 4 each; a thread
+// has 8 columns' 16-byte pieces in flight at once (loads in order: behind a branch each would wait for the one before).  64
+// sequences, 16 heads of 128 x 128 (134 MB) on B200: 29.9 us with 8 x 8 register tiles, 25.9 us.  (A batch that holds more
+// than a token of a sequence after all is walked token by token.)
+template <bool READ_BEFORE, int KIND, int L>
+__global__ void __launch_bounds__(128) linear_scan_step_kernel(ScanArgs a) {
+  constexpr int V = 8, CPV = 32 / L;             // columns per thread, columns side by side in a warp
+  const Seq s = seq_of(a.cu_q, a.seq_lens, a.slots, blockIdx.x);
+  const int lane = threadIdx.x & 31, g = lane % L, i0 = g * 4;
+  const int first = (blockIdx.z * (blockDim.x >> 5) + (threadIdx.x >> 5)) * (V * CPV), j0 = first + lane / L;
+  if (s.ql == 0 || first >= a.dv) return;        // whole warps
+  const int h = blockIdx.y, dk = a.dk, dv = a.dv, hq = h / a.rep;
+  const bool rows = i0 < dk;
+  float* sp = a.state + ((int64_t)s.slot * a.H + h) * dv * dk + (rows ? i0 : 0);
+  float S[V][4];
+  if (s.ctx > 0) {
+#pragma unroll
+    for (int c = 0; c < V; ++c)
+      asm volatile("ld.global.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(S[c][0]), "=f"(S[c][1]), "=f"(S[c][2]), "=f"(S[c][3])
+                   : "l"(sp + (int64_t)min(j0 + c * CPV, dv - 1) * dk));
+  }
+  const bool zero = !(rows && s.ctx > 0);
+#pragma unroll
+  for (int c = 0; c < V; ++c)
+#pragma unroll
+    for (int r = 0; r < 4; ++r) S[c][r] = zero ? 0.f : S[c][r];
+  const float* bon = (READ_BEFORE && a.bonus != nullptr) ? a.bonus + (int64_t)h * dk : nullptr;
+  for (int t = s.q0; t < s.q0 + s.ql; ++t) {
+    const float* qp = a.q + t * a.ldq + (int64_t)hq * dk;
+    const float* kp = a.k + t * a.ldk + (int64_t)hq * dk;
+    const float* dpp = KIND == 2 ? a.decay + t * a.ldd + (int64_t)h * dk : nullptr;
+    const float* vp = a.v + t * a.ldv + (int64_t)h * dv;
+    const bool vec = ((reinterpret_cast<uintptr_t>(qp) | reinterpret_cast<uintptr_t>(kp) | reinterpret_cast<uintptr_t>(dpp) |
+                       reinterpret_cast<uintptr_t>(bon)) & 15) == 0;
+    float vv[V], acc[V];
+#pragma unroll
+    for (int c = 0; c < V; ++c) vv[c] = vp[min(j0 + c * CPV, dv - 1)];
+    const float4 q4 = ld4(qp, i0, dk, vec), k4 = ld4(kp, i0, dk, vec);
+    const float qq[4] = {q4.x, q4.y, q4.z, q4.w}, kk[4] = {k4.x, k4.y, k4.z, k4.w};
+    const float at = KIND == 0 ? a.decay[h] : KIND == 1 ? expf(a.decay[t * a.ldd + h]) : 0.f;
+    float dd[4] = {at, at, at, at};
+    if (KIND == 2) {
+      const float4 x = ld4(dpp, i0, dk, vec);
+      dd[0] = expf(x.x); dd[1] = expf(x.y); dd[2] = expf(x.z); dd[3] = expf(x.w);
+    }
+    float quk = 0.f;
+    if (READ_BEFORE && bon != nullptr) {
+      const float4 u = ld4(bon, i0, dk, vec);
+      quk = fmaf(qq[3], u.w * kk[3], fmaf(qq[2], u.z * kk[2], fmaf(qq[1], u.y * kk[1], qq[0] * (u.x * kk[0]))));
+    }
+    const float sc = a.vscale != nullptr ? a.vscale[t * a.ldvs + h] : 1.f;
+#pragma unroll
+    for (int c = 0; c < V; ++c) {
+      vv[c] *= sc;
+      acc[c] = 0.f;
+#pragma unroll
+      for (int r = 0; r < 4; ++r) {
+        if (READ_BEFORE) acc[c] = fmaf(qq[r], S[c][r], acc[c]);
+        S[c][r] = fmaf(dd[r], S[c][r], kk[r] * vv[c]);
+        if (!READ_BEFORE) acc[c] = fmaf(qq[r], S[c][r], acc[c]);
+      }
+      if (READ_BEFORE) acc[c] = fmaf(vv[c], quk, acc[c]);       // the current token's bonus term
+    }
+    // reduce-scatter over 8 lanes (lane g ends with column g), then over the rest of the column's lanes
+    float b4[4], b2[2];
+    const bool hi4 = g & 4, hi2 = g & 2, hi1 = g & 1;
+#pragma unroll
+    for (int c = 0; c < 4; ++c) b4[c] = (hi4 ? acc[c + 4] : acc[c]) + __shfl_xor_sync(0xffffffffu, hi4 ? acc[c] : acc[c + 4], 4);
+#pragma unroll
+    for (int c = 0; c < 2; ++c) b2[c] = (hi2 ? b4[c + 2] : b4[c]) + __shfl_xor_sync(0xffffffffu, hi2 ? b4[c] : b4[c + 2], 2);
+    float o = (hi1 ? b2[1] : b2[0]) + __shfl_xor_sync(0xffffffffu, hi1 ? b2[0] : b2[1], 1);
+#pragma unroll
+    for (int m = 8; m < L; m *= 2) o += __shfl_xor_sync(0xffffffffu, o, m);
+    const int j = j0 + (g & 7) * CPV;
+    if (g < 8 && j < dv) a.out[(int64_t)t * a.H * dv + (int64_t)h * dv + j] = o;
+  }
+#pragma unroll
+  for (int c = 0; c < V; ++c)
+    if (rows && j0 + c * CPV < dv) *reinterpret_cast<float4*>(sp + (int64_t)(j0 + c * CPV) * dk) = make_float4(S[c][0], S[c][1], S[c][2], S[c][3]);
+}
+
+template <bool READ_BEFORE, int KIND>
+void launch_scan_step(const ScanArgs& a, int B, cudaStream_t stream) {
+  const int lanes = a.dk <= 32 ? 8 : a.dk <= 64 ? 16 : 32, per_warp = 8 * (32 / lanes), warps = (a.dv + per_warp - 1) / per_warp;
+  // four warps a block; single warps where that leaves fewer than four blocks per SM
+  const int w = (int64_t)B * a.H * ((warps + 3) / 4) < 4 * 148 ? 1 : 4;
+  const dim3 grid(B, a.H, (warps + w - 1) / w);
+  if (lanes == 8) linear_scan_step_kernel<READ_BEFORE, KIND, 8><<<grid, 32 * w, 0, stream>>>(a);
+  else if (lanes == 16) linear_scan_step_kernel<READ_BEFORE, KIND, 16><<<grid, 32 * w, 0, stream>>>(a);
+  else linear_scan_step_kernel<READ_BEFORE, KIND, 32><<<grid, 32 * w, 0, stream>>>(a);
+}
+
 // The same recurrence with a two-dimensional register tile: a thread owns 8 key rows x 8 value columns of the state, so the
 // 8 + 8 (+ 8 + 8) staged values it reads per token feed 64 state elements (the column-per-thread form above reads one
 // staged value per element and is bound by shared-memory wavefronts).  RG row groups of 8 (8 for key sizes up to 64, 16 up
@@ -1154,6 +1247,16 @@ LLMSS_API int llmss_linear_scan(const float* q, int64_t ldq, const float* k, int
   a.old_copy = scratch;
   a.chunk_state = scratch != nullptr ? scratch + (int64_t)B * heads * dv * dk : nullptr;
   a.chunk_decay = scratch != nullptr ? a.chunk_state + (int64_t)B * a.nch * heads * dv * dk : nullptr;
+  // decode steps; other key sizes and states off the 16-byte lines keep the general forms below
+  if (max_q == 1 && chunk == 0 && dk <= 128 && dk % 4 == 0 && (reinterpret_cast<uintptr_t>(state) & 15) == 0 && heads <= 65535 && dv <= 8 * 65535) {
+    if (read_before) {
+      if (decay_kind == 0) launch_scan_step<true, 0>(a, B, stream); else if (decay_kind == 1) launch_scan_step<true, 1>(a, B, stream); else launch_scan_step<true, 2>(a, B, stream);
+    } else {
+      if (decay_kind == 0) launch_scan_step<false, 0>(a, B, stream); else if (decay_kind == 1) launch_scan_step<false, 1>(a, B, stream); else launch_scan_step<false, 2>(a, B, stream);
+    }
+    LLMSS_CHECK_CUDA(cudaGetLastError());
+    return 0;
+  }
   if (dk > 32 && dk <= 128) {
     // 8 x 8 register tiles: RG row groups of 8 key rows, value columns in groups of 8
     const int rg = dk <= 64 ? 8 : 16;

@@ -240,3 +240,41 @@ def test_norm_rows_at_prompt_sizes(H, kind, extra):
     assert torch.equal(res, total)
     want, _ = R.norm_residual(total.double().cpu(), None, w.cpu(), b.cpu() if kind == ops.NORM_LAYER else None, 1e-5, kind, out_dtype=F32)
     assert _rel(got, want.double()) < 2.0 ** -8
+
+
+@pytest.mark.parametrize("kind,dk,dv,heads,qk_heads,before", [
+    (2, 64, 64, 2, 2, True), (0, 128, 128, 16, 16, False), (1, 128, 64, 4, 2, False), (2, 4, 1, 3, 3, False), (2, 36, 70, 2, 2, True),
+    (1, 100, 130, 2, 1, True), (0, 32, 33, 2, 2, False), (2, 128, 7, 64, 64, True)])
+def test_linear_scan_one_token(kind, dk, dv, heads, qk_heads, before):
+    """A token per sequence: columns off a warp's and a block's multiples, key sizes that leave lanes idle, few and many blocks, fresh
+    and running states (a fresh one holds NaN before), an inert sequence, strides off the 16-byte lines.  Bound: 32-bit sums, 2e-6."""
+    torch.manual_seed(dk * 7 + dv)
+    ctxs, slots = [5, 0, 9, 64, 3, 1], [4, 0, 2, 5, 1, -1]
+    lens = [1] * len(ctxs)
+    T = len(lens)
+    wide = lambda n: torch.randn(T, n + 3, device="cuda")[:, 1:n + 1]
+    q, k, v = wide(qk_heads * dk), wide(qk_heads * dk), wide(heads * dv)
+    bonus = torch.randn(heads, dk, device="cuda") * 0.5 if before else None
+    scale = torch.rand(T, heads, device="cuda") + 0.5 if kind == 1 else None
+    if kind == 0:
+        dec = torch.rand(heads, device="cuda") * 0.5 + 0.5
+        a = dec.double().cpu().view(1, heads, 1).expand(T, heads, dk)
+    else:
+        dec = -torch.exp(wide(heads if kind == 1 else heads * dk) - 1.0)
+        a = torch.exp(dec.double().cpu()).view(T, heads, -1).expand(T, heads, dk)
+    state = torch.randn(6, heads, dk, dv, device="cuda")
+    state[0] = float("nan")
+    S0 = [state[s].reshape(heads, dv, dk).transpose(1, 2).double().cpu() if c and s >= 0 else torch.zeros(heads, dk, dv, dtype=F64)
+          for s, c in zip(slots, ctxs)]
+    rep = heads // qk_heads
+    d = lambda x, n, w: x.double().cpu().reshape(T, n, w)
+    vv = d(v, heads, dv) * (scale.double().cpu()[:, :, None] if scale is not None else 1.0)
+    want, ends = _scan64(d(q, qk_heads, dk).repeat_interleave(rep, 1), d(k, qk_heads, dk).repeat_interleave(rep, 1), vv, a,
+                         bonus.double().cpu() if before else None, before, lens, S0)
+    untouched = state[3].clone()
+    got = ops.linear_scan(q, k, v, dec, kind, _batch(lens, ctxs, slots), state, heads, qk_heads, dk, dv, bonus=bonus, v_scale=scale,
+                          read_before=before)
+    assert _rel(got[:T - 1], want.reshape(T, -1)[:T - 1]) < 2e-6
+    for s, S in zip(slots[:-1], ends):
+        assert _rel(state[s].reshape(heads, dv, dk).transpose(1, 2), S) < 2e-6
+    assert torch.equal(state[3], untouched)        # a slot that no sequence names
