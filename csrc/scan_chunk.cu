@@ -16,6 +16,9 @@
 // where one does more runs token by token (a column per thread).  Kernel 1 needs no reciprocals: its factors are suffix products.
 // Decays that are one number per token or head are multiplied out in 64 bits, once per chunk: with a constant decay every rounding has
 // the same sign, and the powers' error, not the sums', would be the result's (3.5e-7 of the norm against 7e-8 token by token).
+// What is left of the error is the rounding of the 32-bit sums, twice (scores, then outputs) where the token-serial form has one:
+// against 64 bits 1.0e-7 of the norm (9.3e-8 token by token) for 64 x 64 with a bonus, 128 x 128 per channel 6.8e-8 (5.1e-8), constant
+// decay 6.8e-8 (7.6e-8), 128 x 64 per token 1.08e-7 (9.6e-8).  Factors carried as pairs of numbers change none of these.
 //
 // B200, 8 prompts of 1024 tokens, against the two passes of the token-serial form: 32 heads of 64 x 64, decay per channel and bonus
 // 618 -> 376 us (99 + 36 + 221, ncu: 44 % of the multiply-add pipe, shared memory 37 to 57 % of its bandwidth); 16 heads of 128 x 128, per

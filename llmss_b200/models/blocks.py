@@ -200,7 +200,7 @@ class RoutedExperts:
     spends experts / top times the needed FLOPs, which is nothing while the step is bound by the weight bytes (decode,
     short portions; it is also free of host synchronisation, so it can sit in a captured decode graph).  Prompts long
     enough to give every expert ``LLMSS_MOE_GROUPED_MIN_ROWS`` rows on average run the grouped form: pairs sorted by
-    expert on the device, one pair of tensor-core GEMMs per expert over its contiguous rows, 32-bit weighted sum per
+    expert on the device, one tensor-core GEMM per projection over all experts' contiguous rows, 32-bit weighted sum per
     token.  ``LLMSS_MOE_DENSE_MIN_TOKENS`` moves the gather / dense switch."""
 
     def __init__(self, experts: int, top: int, groups: int, keep: int, route_scale: float, ff: int, act: int = ACT_RELU2,
