@@ -1448,6 +1448,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_consta
           }
           if (fast) store_chunk_full<T, CH>(a, v, n, m0 + cg0 * 8, lane, bval);
           else store_chunk<T, CH>(a, v, rv, n, m0 + cg0 * 8, lane, bval, m_end);
+          __syncwarp();          // lanes past N rejoin: the next load from tensor memory is the whole warp's
         }
       } else {
         // ---- split-K: park the partial accumulator in shared memory: [(cg*2 + half)][feature] float4, conflict-free
@@ -1654,25 +1655,27 @@ gemm_heads_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_const
           __syncwarp();
           if (lane == 0) mbar_arrive(&tempty_bar[as]);
         }
-        if (n >= a.N) continue;
-        float v[32];
+        if (n < a.N) {
+          float v[32];
 #pragma unroll
-        for (int j = 0; j < 32; ++j) v[j] = __uint_as_float(q[j]) * (sp != nullptr ? sc[j] : 1.f);
-        const int64_t at = (int64_t)m * a.ldo + h * a.soh + n;
-        if (a.out_f32) {
-          float* o = reinterpret_cast<float*>(a.out) + at;
+          for (int j = 0; j < 32; ++j) v[j] = __uint_as_float(q[j]) * (sp != nullptr ? sc[j] : 1.f);
+          const int64_t at = (int64_t)m * a.ldo + h * a.soh + n;
+          if (a.out_f32) {
+            float* o = reinterpret_cast<float*>(a.out) + at;
 #pragma unroll
-          for (int j = 0; j < 32; ++j, o += a.ldo) if (j < rows) *o = v[j];
-        } else {
-          T* o = reinterpret_cast<T*>(a.out) + at;
-          if (rows >= 32) {
-#pragma unroll
-            for (int j = 0; j < 32; ++j, o += a.ldo) *o = from_f32<T>(v[j]);
+            for (int j = 0; j < 32; ++j, o += a.ldo) if (j < rows) *o = v[j];
           } else {
+            T* o = reinterpret_cast<T*>(a.out) + at;
+            if (rows >= 32) {
 #pragma unroll
-            for (int j = 0; j < 32; ++j, o += a.ldo) if (j < rows) *o = from_f32<T>(v[j]);
+              for (int j = 0; j < 32; ++j, o += a.ldo) *o = from_f32<T>(v[j]);
+            } else {
+#pragma unroll
+              for (int j = 0; j < 32; ++j, o += a.ldo) if (j < rows) *o = from_f32<T>(v[j]);
+            }
           }
         }
+        __syncwarp();            // lanes past N rejoin: the next load from tensor memory is the whole warp's
       }
       if (++as == 2) { as = 0; aphase ^= 1; }
     }

@@ -148,11 +148,12 @@ def test_linear_scan_over_chunks(kind, dk, dv, heads, qk_heads, before, deep):
 
 
 @pytest.mark.parametrize("T,H,k,n,xs,form", [(129, 3, 128, 128, None, None), (300, 5, 64, 192, 72, "row"), (513, 2, 192, 128, 256, "elem"), (257, 16, 40, 24, None, "f32"),
-                                             (2000, 33, 128, 136, None, "row")])
+                                             (2000, 33, 128, 136, None, "row"), (130, 2, 8, 40, None, "row"), (385, 3, 72, 8, 80, "f32")])
 @pytest.mark.parametrize("dt", [torch.bfloat16, torch.float16])
 def test_per_head_products_at_prompt_sizes(T, H, k, n, xs, form, dt):
-    """Tokens, features and contraction off the tile sizes, heads as column ranges of wider rows, results between other columns, the
-    factor per token and head or per element.  Bound: one rounding to 16 bits of 32-bit sums (2^-8 / 2^-11 of a value), 1e-6 in 32-bit."""
+    """Tokens, features and contraction off the tile sizes, features that end inside a warp's 32 (the other lanes only take part in the
+    loads from tensor memory), heads as column ranges of wider rows, results between other columns, the factor per token and head or per
+    element.  Bound: one rounding to 16 bits of 32-bit sums (2^-8 / 2^-11 of a value), 1e-6 in 32-bit."""
     torch.manual_seed(T)
     xs = xs or k
     x = torch.randn(T, H * xs, device="cuda").to(dt)
