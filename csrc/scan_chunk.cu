@@ -10,10 +10,14 @@
 // Everything is 32-bit on the multiply-add pipe (two numbers per instruction where both operands lie in memory order): a 3-term
 // split on the tensor cores would run at 158 against 126 multiply-adds per clock and SM and round its sums differently.
 //
-// Decays without overflow: a sub-block of 16 tokens takes its middle as reference, q_i gets F(i) and k_j gets 1 / F(j) with F the
-// decay from the middle (products of at most 8 factors, one division); between sub-blocks the factor from middle to middle is at
-// most 1.  F and 1 / F stay finite while half a sub-block decays by no more than 2^-100 (or grows by 2^100) in any channel; a chunk
-// where one does more runs token by token (a column per thread).  Kernel 1 needs no reciprocals: its factors are suffix products.
+// Decays without overflow or underflow: a sub-block of 16 tokens takes its middle as reference, q_i gets F(i) and k_j gets 1 / F(j) with
+// F the decay from the middle (products of at most 8 factors, one division).  Between sub-blocks no factor is formed that could be below
+// what it cancels: the query is first multiplied by its sub-block's first half (what 1 / F may have put in, which leaves the decay from
+// the sub-block's start), the key by its sub-block's second half (the decay to its end), and only then the whole sub-blocks that lie
+// between.  One factor from middle to middle would be a product of two halves, zero in 32 bits for decays of e^-6 per token, where the pair
+// of tokens at the border has weight 1.  Half a sub-block may decay to 2^-80 or grow to 2^15 in any channel: scaled numbers then stay
+// normal for q and k down to 2^-46; a chunk where one does more, or where a scaled number leaves the range, runs token by token (a column
+// per thread).  Kernel 1 needs no reciprocals: its factors are suffix products.
 // Decays that are one number per token or head are multiplied out in 64 bits, once per chunk: with a constant decay every rounding has
 // the same sign, and the powers' error, not the sums', would be the result's (3.5e-7 of the norm against 7e-8 token by token).
 // What is left of the error is the rounding of the 32-bit sums, twice (scores, then outputs) where the token-serial form has one:
@@ -29,7 +33,8 @@
 namespace {
 
 constexpr int C = 64, SB = 16, NS = C / SB, JT = 64;     // chunk, sub-block, value columns per block
-constexpr float kSafe = 7.888609e-31f;                   // 2^-100
+constexpr float kLow = 0x1p-80f, kHigh = 0x1p15f;        // decay or growth of half a sub-block that the products take
+constexpr float kBig = 0x1p120f;                         // scaled numbers above this: token by token
 
 struct ChunkArgs {
   const float* q; int64_t ldq;
@@ -102,7 +107,7 @@ __device__ __forceinline__ void load_rows(const float* p, int64_t ld, int l0, in
     p += l0 + i + 1 < n ? ld : 0;
   }
 }
-// 1 / x by one Newton-Raphson step on the approximate reciprocal; x lies in 2^-100 .. 2^100 wherever the result is used
+// 1 / x by one Newton-Raphson step on the approximate reciprocal; x lies in 2^-80 .. 2^15 wherever the result is used
 __device__ __forceinline__ float recip(float x) {
   float y;
   asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
@@ -294,7 +299,7 @@ __global__ void __launch_bounds__(256) scan_carry_kernel(ChunkArgs a) {
 template <int DK> struct OutSmem {
   static constexpr int LD = DK + 4, LA = C + 4;
   static constexpr int Q = C * LD, S = JT * LD, KA = (C * LD > C * LA + C * JT) ? C * LD : C * LA + C * JT;
-  static constexpr int FLOATS = Q + KA + S + 2 * NS * DK + 10 * DK + (DK / 32 + 4) * C + 2 * 2 * NS;
+  static constexpr int FLOATS = Q + KA + S + 2 * NS * DK + 7 * DK + (DK / 32 + 4) * C + 2 * 2 * NS;
 };
 
 template <int DK, int KIND, bool BEFORE>
@@ -308,8 +313,9 @@ __global__ void __launch_bounds__(128, DK == 64 ? 3 : 2) scan_out_kernel(ChunkAr
   float* vs = ks + C * LA;
   float* ss = ks + M::KA;               // [JT][LD] start state, columns as rows
   float* halves = ss + M::S;            // [NS][2][DK] decay of the first and second half of a sub-block
-  float* mids = halves + 2 * NS * DK;   // [10][DK]: middle of s' to middle of s (pairs (1,0) (2,0) (2,1) (3,0) (3,1) (3,2)), start to middle of s
-  float* diag = mids + 10 * DK;         // [DK / 32][C] bonus products, a part per 32 channels
+  float* between = halves + 2 * NS * DK;   // [4][DK]: ones, decay of sub-block 1, of 2, of both
+  float* before = between + 4 * DK;     // [3][DK]: decay of the chunk in front of sub-blocks 1, 2, 3
+  float* diag = before + 3 * DK;        // [DK / 32][C] bonus products, a part per 32 channels
   double* table = reinterpret_cast<double*>(diag + (DK / 32) * C);   // [C] (kinds 0 and 1)
   double* thalf = table + C;            // [NS][2]
   float* tq = reinterpret_cast<float*>(thalf + 2 * NS);              // [C] factors on q and, [C], on k
@@ -344,7 +350,8 @@ __global__ void __launch_bounds__(128, DK == 64 ? 3 : 2) scan_out_kernel(ChunkAr
     else
       *reinterpret_cast<float4*>(ss + j * LD + c) = make_float4(0.f, 0.f, 0.f, 0.f);
   }
-  bool deep = false;                    // some half sub-block decays by more than 2^-100
+  bool deep = false;                    // out of the products' range
+  float big = 0.f;
 #pragma unroll 1
   for (int task = tid; task < NS * DK; task += 128) {
     const int c = task % DK, cc = min(c, a.dk - 1), s = task / DK, l0 = s * SB;
@@ -374,33 +381,40 @@ __global__ void __launch_bounds__(128, DK == 64 ? 3 : 2) scan_out_kernel(ChunkAr
     if (KIND != 2) {
 #pragma unroll
       for (int i = 0; i < SB; ++i) {
-        qs[(l0 + i) * LD + c] = qx[i] * tq[l0 + i];
-        ks[(l0 + i) * LD + c] = kx[i] * tk[l0 + i];
+        const float y = qx[i] * tq[l0 + i], z = kx[i] * tk[l0 + i];
+        qs[(l0 + i) * LD + c] = y;
+        ks[(l0 + i) * LD + c] = z;
+        big = fmaxf(big, fmaxf(fabsf(y), fabsf(z)));
       }
       continue;
     }
     float f = 1.f;
 #pragma unroll
     for (int i = SB / 2; i < SB; ++i) {
-      const float before = f;
+      const float front = f;
       f *= x[i];
-      qs[(l0 + i) * LD + c] = qx[i] * (BEFORE ? before : f);
-      ks[(l0 + i) * LD + c] = kx[i] * recip(f);
+      const float y = qx[i] * (BEFORE ? front : f), z = kx[i] * recip(f);
+      qs[(l0 + i) * LD + c] = y;
+      ks[(l0 + i) * LD + c] = z;
+      big = fmaxf(big, fmaxf(fabsf(y), fabsf(z)));
     }
     halves[(2 * s + 1) * DK + c] = f;
-    deep |= !(f >= kSafe && f <= 1.f / kSafe);
+    deep |= !(f >= kLow && f <= kHigh);
     f = 1.f;
 #pragma unroll
     for (int i = SB / 2 - 1; i >= 0; --i) {
       const float after = f;
       f *= x[i];
-      qs[(l0 + i) * LD + c] = qx[i] * recip(BEFORE ? f : after);
-      ks[(l0 + i) * LD + c] = kx[i] * after;
+      const float y = qx[i] * recip(BEFORE ? f : after), z = kx[i] * after;
+      qs[(l0 + i) * LD + c] = y;
+      ks[(l0 + i) * LD + c] = z;
+      big = fmaxf(big, fmaxf(fabsf(y), fabsf(z)));
     }
     halves[2 * s * DK + c] = f;
-    deep |= !(f >= kSafe && f <= 1.f / kSafe);
+    deep |= !(f >= kLow && f <= kHigh);
   }
-  if (KIND != 2 && tid < 2 * NS) deep = !(thalf[tid] >= (double)kSafe && thalf[tid] <= 1.0 / kSafe);
+  if (KIND != 2 && tid < 2 * NS) deep = !(thalf[tid] >= (double)kLow && thalf[tid] <= (double)kHigh);
+  deep |= big > kBig;
   asm volatile("cp.async.wait_all;" ::: "memory");
   auto bonus_of = [&](int t) {
     float d = 0.f;
@@ -452,36 +466,31 @@ __global__ void __launch_bounds__(128, DK == 64 ? 3 : 2) scan_out_kernel(ChunkAr
     }
     return;
   }
-  // factors between middles, and from the chunk's start to the middles
-  auto between = [&](auto h1, auto h2, auto&& put) {      // put(pair or 6 + s, factor)
-    auto run = h1(0) * 0 + 1;
-#pragma unroll
-    for (int s = 0; s < NS; ++s) {
-      put(6 + s, run * h1(s));
-      run *= h1(s) * h2(s);
-      auto back = h1(s);
-#pragma unroll
-      for (int p = NS - 2; p >= 0; --p) {
-        if (p >= s) continue;
-        back *= h2(p);
-        put(s * (s - 1) / 2 + p, back);
-        back *= h1(p);
-      }
-    }
-  };
+  // factors of whole sub-blocks
   for (int c = tid; c < DK; c += 128) {
-    if (KIND == 2)
-      between([&](int s) { return halves[2 * s * DK + c]; }, [&](int s) { return halves[(2 * s + 1) * DK + c]; },
-              [&](int x, float f) { mids[x * DK + c] = f; });
-    else
-      between([&](int s) { return thalf[2 * s]; }, [&](int s) { return thalf[2 * s + 1]; }, [&](int x, double f) { mids[x * DK + c] = (float)f; });
+    if (KIND == 2) {
+      float w[NS - 1];
+#pragma unroll
+      for (int x = 0; x < NS - 1; ++x) w[x] = halves[2 * x * DK + c] * halves[(2 * x + 1) * DK + c];
+      between[c] = 1.f; between[DK + c] = w[1]; between[2 * DK + c] = w[2]; between[3 * DK + c] = w[1] * w[2];
+      before[c] = w[0]; before[DK + c] = w[0] * w[1]; before[2 * DK + c] = w[0] * w[1] * w[2];
+    } else {
+      double w[NS - 1];
+#pragma unroll
+      for (int x = 0; x < NS - 1; ++x) w[x] = thalf[2 * x] * thalf[2 * x + 1];
+      between[c] = 1.f; between[DK + c] = (float)w[1]; between[2 * DK + c] = (float)w[2]; between[3 * DK + c] = (float)(w[1] * w[2]);
+      before[c] = (float)w[0]; before[DK + c] = (float)(w[0] * w[1]); before[2 * DK + c] = (float)(w[0] * w[1] * w[2]);
+#pragma unroll
+      for (int x = 0; x < 2 * NS; ++x) halves[x * DK + c] = (float)thalf[x];
+    }
   }
   // the values, held in registers until the keys' place is free
   const int cg = tid & 15, tg = tid >> 4;
   float vr[C * JT / 128];
   load_values<128, C>(a, t0, 0, n, h, j0, nj, vr);
   __syncthreads();
-  // ---- scores: 80 tiles of 4 x 8 (eight per 16 x 16 block of the lower triangle), 20 lanes of every warp
+  // ---- scores: 80 tiles of 4 x 8 (eight per 16 x 16 block of the lower triangle), 20 lanes of every warp.  Off the diagonal a query is
+  // brought to its sub-block's start and a key to its sub-block's end before they meet: factors of at most what each carries
   float sc[4][8];
   int si = 0, sj = 0, sb = 0, sp = 0;
   const bool scorer = lane < 20;
@@ -495,7 +504,9 @@ __global__ void __launch_bounds__(128, DK == 64 ? 3 : 2) scan_out_kernel(ChunkAr
     for (int i = 0; i < 4; ++i)
 #pragma unroll
       for (int j = 0; j < 8; ++j) sc[i][j] = 0.f;
-    const float* mid = mids + (sb * (sb - 1) / 2 + sp) * DK;
+    const float* fq = sb == sp ? between : halves + 2 * sb * DK;
+    const float* fk = sb == sp ? between : halves + (2 * sp + 1) * DK;
+    const float* fb = between + (sb == 2 ? 1 : sp == 1 ? 2 : 3) * DK;          // read where a sub-block lies between
     // partial sums of 16 channels: the rounding of a score, and with it the result's, is that of the token-serial form
 #pragma unroll 1
     for (int cc = 0; cc < DK; cc += 16) {
@@ -506,9 +517,7 @@ __global__ void __launch_bounds__(128, DK == 64 ? 3 : 2) scan_out_kernel(ChunkAr
         for (int j = 0; j < 8; ++j) acc[i][j] = 0;
 #pragma unroll 1
       for (int c = cc; c < cc + 16; c += 4) {
-        ulonglong2 f;
-        f.x = f.y = pack(1.f, 1.f);
-        if (sb != sp) f = lds2(mid + c);
+        const ulonglong2 f = lds2(fq + c), g = lds2(fk + c);
         ulonglong2 q4[4];
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
@@ -516,9 +525,19 @@ __global__ void __launch_bounds__(128, DK == 64 ? 3 : 2) scan_out_kernel(ChunkAr
           q4[i].x = pmul(q4[i].x, f.x);
           q4[i].y = pmul(q4[i].y, f.y);
         }
+        if (sb > sp + 1) {
+          const ulonglong2 b = lds2(fb + c);
+#pragma unroll
+          for (int i = 0; i < 4; ++i) {
+            q4[i].x = pmul(q4[i].x, b.x);
+            q4[i].y = pmul(q4[i].y, b.y);
+          }
+        }
 #pragma unroll
         for (int j = 0; j < 8; ++j) {
-          const ulonglong2 k4 = lds2(ks + (sj + 2 * j) * LD + c);
+          ulonglong2 k4 = lds2(ks + (sj + 2 * j) * LD + c);
+          k4.x = pmul(k4.x, g.x);
+          k4.y = pmul(k4.y, g.y);
 #pragma unroll
           for (int i = 0; i < 4; ++i) acc[i][j] = pfma(q4[i].y, k4.y, pfma(q4[i].x, k4.x, acc[i][j]));
         }
@@ -553,10 +572,16 @@ __global__ void __launch_bounds__(128, DK == 64 ? 3 : 2) scan_out_kernel(ChunkAr
 #pragma unroll
   for (int i = 0; i < C * JT / 128; ++i) vs[tid + i * 128] = vr[i];
   for (int i = tid; i < C * (DK / 4); i += 128) {
-    const int t = i / (DK / 4), c = (i % (DK / 4)) * 4;
+    const int t = i / (DK / 4), c = (i % (DK / 4)) * 4, s = t / SB;
     float4* p = reinterpret_cast<float4*>(qs + t * LD + c);
-    const float4 f = *reinterpret_cast<const float4*>(mids + (6 + t / SB) * DK + c), x = *p;
-    *p = make_float4(x.x * f.x, x.y * f.y, x.z * f.z, x.w * f.w);
+    const float4 f = *reinterpret_cast<const float4*>(halves + 2 * s * DK + c);
+    float4 x = *p;
+    x = make_float4(x.x * f.x, x.y * f.y, x.z * f.z, x.w * f.w);
+    if (s > 0) {
+      const float4 b = *reinterpret_cast<const float4*>(before + (s - 1) * DK + c);
+      x = make_float4(x.x * b.x, x.y * b.y, x.z * b.z, x.w * b.w);
+    }
+    *p = x;
   }
   __syncthreads();
   // ---- o = q S: pairs along the key rows

@@ -147,6 +147,59 @@ def test_linear_scan_over_chunks(kind, dk, dv, heads, qk_heads, before, deep):
     assert torch.equal(state[3], before_state[3])        # a slot that no sequence names
 
 
+def _scan_case(seed, kind, dk, dv, heads, lens, before, decay):
+    """Inputs of a recurrence over fresh sequences and its float64 results; decay(shape) gives the log decays."""
+    torch.manual_seed(seed)
+    T = sum(lens)
+    q, k, v = (torch.randn(T, heads * n, device="cuda") for n in (dk, dk, dv))
+    logs = decay((heads,) if kind == 0 else (T, heads) if kind == 1 else (T, heads * dk))
+    dec = torch.exp(logs) if kind == 0 else logs
+    factors = dec.double().cpu() if kind == 0 else torch.exp(dec.double().cpu())
+    a = factors.view(1, heads, 1).expand(T, heads, dk) if kind == 0 else factors.view(T, heads, -1).expand(T, heads, dk)
+    bonus = torch.randn(heads, dk, device="cuda") * 0.5 if before else None
+
+    def want():
+        d = lambda x, w: x.double().cpu().reshape(T, heads, w)
+        return _scan64(d(q, dk), d(k, dk), d(v, dv), a, bonus.double().cpu() if before else None, before, lens,
+                       [torch.zeros(heads, dk, dv, dtype=F64)] * len(lens))
+
+    def run():
+        state = torch.zeros(len(lens), heads, dk, dv, device="cuda")
+        out = ops.linear_scan(q, k, v, dec, kind, _batch(lens, [0] * len(lens), list(range(len(lens)))), state, heads, heads, dk, dv, bonus=bonus,
+                              read_before=before)
+        return out, state.reshape(len(lens), heads, dv, dk).transpose(2, 3)
+
+    return (q, k, v, dec, bonus), want, run
+
+
+@pytest.mark.parametrize("kind", [0, 1, 2])
+@pytest.mark.parametrize("before", [False, True])
+@pytest.mark.parametrize("dk", [64, 128])
+@pytest.mark.parametrize("log", [-4.0, -5.0, -6.0, -6.8, -7.0, -8.0, -8.6, -9.0, "one", "near"])
+def test_linear_scan_strong_decays(kind, before, dk, log):
+    """Decays that leave little of a state after a few tokens, all of them or one channel in 64 (one head in two): on both sides of what
+    the products take, and around it.  The rows at sub-block starts are looked at one by one: what they see of the sub-block before
+    them has full weight.  Bound: 32-bit sums, 2e-6 of the norm."""
+    def decay(shape):
+        if log == "one":
+            x = torch.full(shape, -0.4, device="cuda")
+            x[..., 1::64 if kind == 2 else 2] = -7.0
+            return x
+        if log == "near":
+            return -torch.exp(torch.randn(shape, device="cuda") * 0.2 + 1.9)
+        return torch.full(shape, log, device="cuda")
+
+    lens = [200, 130]
+    _, want, run = _scan_case(dk + kind, kind, dk, 40, 2, lens, before, decay)
+    (w, ends), (got, state) = want(), run()
+    w = w.reshape(got.shape)
+    assert _rel(got, w) < 2e-6
+    rows = [at + t for at, n in zip((0, 200), lens) for t in range(16 if before else 0, n, 16)]
+    err = (got.double().cpu() - w)[rows].norm(dim=1) / w[rows].norm(dim=1)
+    assert float(err.max()) < 2e-6
+    assert _rel(state, torch.stack(ends)) < 2e-6
+
+
 @pytest.mark.parametrize("T,H,k,n,xs,form", [(129, 3, 128, 128, None, None), (300, 5, 64, 192, 72, "row"), (513, 2, 192, 128, 256, "elem"), (257, 16, 40, 24, None, "f32"),
                                              (2000, 33, 128, 136, None, "row"), (130, 2, 8, 40, None, "row"), (385, 3, 72, 8, 80, "f32")])
 @pytest.mark.parametrize("dt", [torch.bfloat16, torch.float16])
