@@ -16,8 +16,8 @@
 // the sub-block's start), the key by its sub-block's second half (the decay to its end), and only then the whole sub-blocks that lie
 // between.  One factor from middle to middle would be a product of two halves, zero in 32 bits for decays of e^-6 per token, where the pair
 // of tokens at the border has weight 1.  Half a sub-block may decay to 2^-80 or grow to 2^15 in any channel: scaled numbers then stay
-// normal for q and k down to 2^-46; a chunk where one does more, or where a scaled number leaves the range, runs token by token (a column
-// per thread).  Kernel 1 needs no reciprocals: its factors are suffix products.
+// normal for q and k down to 2^-46; a chunk where one does more, where a scaled number leaves the range or a value is not finite (the masked half of the scores x values is a sum of zeros times values:
+// a bad one would reach the tokens before it), runs token by token (a column per thread).  Kernel 1 needs no reciprocals: its factors are suffix products.
 // Decays that are one number per token or head are multiplied out in 64 bits, once per chunk: with a constant decay every rounding has
 // the same sign, and the powers' error, not the sums', would be the result's (3.5e-7 of the norm against 7e-8 token by token).
 // What is left of the error is the rounding of the 32-bit sums, twice (scores, then outputs) where the token-serial form has one:
@@ -34,7 +34,7 @@ namespace {
 
 constexpr int C = 64, SB = 16, NS = C / SB, JT = 64;     // chunk, sub-block, value columns per block
 constexpr float kLow = 0x1p-80f, kHigh = 0x1p15f;        // decay or growth of half a sub-block that the products take
-constexpr float kBig = 0x1p120f;                         // scaled numbers above this: token by token
+constexpr float kBig = 0x1p120f;                         // scaled numbers or values above this (or no numbers): token by token
 
 struct ChunkArgs {
   const float* q; int64_t ldq;
@@ -415,6 +415,10 @@ __global__ void __launch_bounds__(128, DK == 64 ? 3 : 2) scan_out_kernel(ChunkAr
   }
   if (KIND != 2 && tid < 2 * NS) deep = !(thalf[tid] >= (double)kLow && thalf[tid] <= (double)kHigh);
   deep |= big > kBig;
+  float vr[C * JT / 128];               // the values, held in registers until the keys' place is free
+  load_values<128, C>(a, t0, 0, n, h, j0, nj, vr);
+#pragma unroll
+  for (int i = 0; i < C * JT / 128; ++i) deep |= !(fabsf(vr[i]) < kBig);      // (in a product 0 x infinity would reach earlier tokens)
   asm volatile("cp.async.wait_all;" ::: "memory");
   auto bonus_of = [&](int t) {
     float d = 0.f;
@@ -484,10 +488,7 @@ __global__ void __launch_bounds__(128, DK == 64 ? 3 : 2) scan_out_kernel(ChunkAr
       for (int x = 0; x < 2 * NS; ++x) halves[x * DK + c] = (float)thalf[x];
     }
   }
-  // the values, held in registers until the keys' place is free
   const int cg = tid & 15, tg = tid >> 4;
-  float vr[C * JT / 128];
-  load_values<128, C>(a, t0, 0, n, h, j0, nj, vr);
   __syncthreads();
   // ---- scores: 80 tiles of 4 x 8 (eight per 16 x 16 block of the lower triangle), 20 lanes of every warp.  Off the diagonal a query is
   // brought to its sub-block's start and a key to its sub-block's end before they meet: factors of at most what each carries

@@ -200,6 +200,20 @@ def test_linear_scan_strong_decays(kind, before, dk, log):
     assert _rel(state, torch.stack(ends)) < 2e-6
 
 
+@pytest.mark.parametrize("kind,dk,before", [(2, 64, True), (2, 128, False), (1, 128, False), (0, 64, False)])
+@pytest.mark.parametrize("bad", [float("nan"), float("inf")])
+def test_linear_scan_keeps_a_bad_value_behind_its_token(kind, dk, before, bad):
+    """A value that is no number, or infinite, in the middle of a sub-block: earlier tokens and other columns are as without it."""
+    (q, k, v, dec, bonus), want, run = _scan_case(3, kind, dk, 40, 2, [200], before, lambda s: -torch.rand(s, device="cuda") * 0.5)
+    w = want()[0]
+    v[77, 5] = bad
+    got = run()[0].reshape(200, 2, 40)
+    assert _rel(got[:77], w[:77]) < 2e-6
+    assert not torch.isfinite(got[78:, 0, 5]).any()
+    got[:, 0, 5], w[:, 0, 5] = 0.0, 0.0
+    assert _rel(got, w) < 2e-6
+
+
 @pytest.mark.parametrize("T,H,k,n,xs,form", [(129, 3, 128, 128, None, None), (300, 5, 64, 192, 72, "row"), (513, 2, 192, 128, 256, "elem"), (257, 16, 40, 24, None, "f32"),
                                              (2000, 33, 128, 136, None, "row"), (130, 2, 8, 40, None, "row"), (385, 3, 72, 8, 80, "f32")])
 @pytest.mark.parametrize("dt", [torch.bfloat16, torch.float16])
