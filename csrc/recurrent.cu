@@ -355,6 +355,7 @@ struct ScanArgs {
   // [B][nch][H][dk] decay products
   float* old_copy; float* chunk_state; float* chunk_decay;
   int chunk, nch, nslices;
+  int most;            // sequences of more tokens are left alone
 };
 
 __device__ __forceinline__ float4 ld4(const float* p, int i, int n, bool vec) {   // p[i .. i+3], zeros beyond n
@@ -377,7 +378,7 @@ __global__ void __launch_bounds__(SCAN_THREADS) linear_scan_kernel(ScanArgs a) {
   constexpr int STRIP = KPT + 4;        // floats between staged strips: different banks for the strips of one warp
   extern __shared__ __align__(16) float sm[];
   const Seq s = seq_of(a.cu_q, a.seq_lens, a.slots, blockIdx.x);
-  if (s.ql == 0) return;
+  if (s.ql == 0 || s.ql > a.most) return;
   const int h = blockIdx.y;
   const int slice = MODE == 0 ? blockIdx.z : blockIdx.z % a.nslices, ch = MODE == 0 ? 0 : blockIdx.z / a.nslices;
   const int j0 = slice * a.dvt;
@@ -575,7 +576,7 @@ __global__ void __launch_bounds__(128) linear_scan_step_kernel(ScanArgs a) {
   const Seq s = seq_of(a.cu_q, a.seq_lens, a.slots, blockIdx.x);
   const int lane = threadIdx.x & 31, g = lane % L, i0 = g * 4;
   const int first = (blockIdx.z * (blockDim.x >> 5) + (threadIdx.x >> 5)) * (V * CPV), j0 = first + lane / L;
-  if (s.ql == 0 || first >= a.dv) return;        // whole warps
+  if (s.ql == 0 || s.ql > a.most || first >= a.dv) return;        // whole warps
   const int h = blockIdx.y, dk = a.dk, dv = a.dv, hq = h / a.rep;
   const bool rows = i0 < dk;
   float* sp = a.state + ((int64_t)s.slot * a.H + h) * dv * dk + (rows ? i0 : 0);
@@ -668,7 +669,7 @@ template <bool READ_BEFORE, int KIND, int MODE, int RG>
 __global__ void __launch_bounds__(128) linear_scan_tile_kernel(ScanArgs a) {
   extern __shared__ __align__(16) float sm[];
   const Seq s = seq_of(a.cu_q, a.seq_lens, a.slots, blockIdx.x);
-  if (s.ql == 0) return;
+  if (s.ql == 0 || s.ql > a.most) return;
   const int h = blockIdx.y;
   const int slice = MODE == 0 ? blockIdx.z : blockIdx.z % a.nslices, ch = MODE == 0 ? 0 : blockIdx.z / a.nslices;
   const int j0 = slice * a.dvt;
@@ -1228,11 +1229,12 @@ LLMSS_API int64_t llmss_linear_scan_scratch_floats(int B, int heads, int dk, int
 
 // chunk > 0 (and scratch of llmss_linear_scan_scratch_floats floats): two passes over chunks of that many tokens (a
 // multiple of 16) -- for prompt rounds whose sequences are long and few; chunk = 0: one pass.
-LLMSS_API int llmss_linear_scan(const float* q, int64_t ldq, const float* k, int64_t ldk, const float* v, int64_t ldv,
-                                const float* decay, int64_t ldd, int decay_kind, const float* bonus, const float* vscale,
-                                int64_t ldvs, float* out, float* state, const int* cu_q, const int* seq_lens, const int* slots,
-                                int B, int heads, int qk_heads, int dk, int dv, int read_before, float* scratch, int chunk,
-                                int max_q, cudaStream_t stream) {
+// most: sequences of more tokens than that are left alone (llmss_linear_scan_chunked_from takes them).
+LLMSS_API int llmss_linear_scan_upto(const float* q, int64_t ldq, const float* k, int64_t ldk, const float* v, int64_t ldv,
+                                     const float* decay, int64_t ldd, int decay_kind, const float* bonus, const float* vscale,
+                                     int64_t ldvs, float* out, float* state, const int* cu_q, const int* seq_lens, const int* slots,
+                                     int B, int heads, int qk_heads, int dk, int dv, int read_before, float* scratch, int chunk,
+                                     int max_q, int most, cudaStream_t stream) {
   LLMSS_REQUIRE(heads > 0 && qk_heads > 0 && heads % qk_heads == 0, "linear_scan: %d heads over %d q/k heads", heads, qk_heads);
   LLMSS_REQUIRE(dk > 0 && dk <= 1024, "linear_scan: key size %d (at most 1024)", dk);
   LLMSS_REQUIRE(decay_kind >= 0 && decay_kind <= 2, "linear_scan: decay kind %d", decay_kind);
@@ -1242,6 +1244,7 @@ LLMSS_API int llmss_linear_scan(const float* q, int64_t ldq, const float* k, int
   a.q = q; a.ldq = ldq; a.k = k; a.ldk = ldk; a.v = v; a.ldv = ldv; a.decay = decay; a.ldd = ldd; a.bonus = bonus;
   a.vscale = vscale; a.ldvs = ldvs; a.out = out; a.state = state; a.cu_q = cu_q; a.seq_lens = seq_lens; a.slots = slots;
   a.H = heads; a.rep = heads / qk_heads; a.dk = dk; a.dv = dv;
+  a.most = most;
   a.chunk = chunk;
   a.nch = chunk > 0 ? (max_q + chunk - 1) / chunk : 1;
   a.old_copy = scratch;
@@ -1338,6 +1341,15 @@ LLMSS_API int llmss_linear_scan(const float* q, int64_t ldq, const float* k, int
 #undef LLMSS_SCAN2
   LLMSS_CHECK_CUDA(cudaGetLastError());
   return 0;
+}
+
+LLMSS_API int llmss_linear_scan(const float* q, int64_t ldq, const float* k, int64_t ldk, const float* v, int64_t ldv,
+                                const float* decay, int64_t ldd, int decay_kind, const float* bonus, const float* vscale,
+                                int64_t ldvs, float* out, float* state, const int* cu_q, const int* seq_lens, const int* slots,
+                                int B, int heads, int qk_heads, int dk, int dv, int read_before, float* scratch, int chunk,
+                                int max_q, cudaStream_t stream) {
+  return llmss_linear_scan_upto(q, ldq, k, ldk, v, ldv, decay, ldd, decay_kind, bonus, vscale, ldvs, out, state, cu_q, seq_lens, slots, B, heads,
+                                qk_heads, dk, dv, read_before, scratch, chunk, max_q, 0x7fffffff, stream);
 }
 
 LLMSS_API int llmss_gated_rmsnorm(const float* o, int64_t ldo, const float* gate, int64_t ldg, int gate_act, const float* weight,

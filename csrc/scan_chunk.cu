@@ -50,6 +50,7 @@ struct ChunkArgs {
   float* decays;                       // [chunk slots][H][dk]
   float* decay_rest;                   // [chunk slots][H]: what rounding D_c to 32 bits left (kinds 0 and 1)
   int H, rep, dk, dv, nslices;
+  int least;                           // sequences of fewer tokens are left alone
 };
 
 // rows and chunk slots of sequence b; the slots of all sequences take T / 64 + B places: cu_q[b] / 64 + b is the first of b's
@@ -63,7 +64,7 @@ __device__ __forceinline__ Rows rows_of(const ChunkArgs& a, int b) {
   r.ctx = a.seq_lens[b] - r.ql;
   r.slot = a.slots[b];
   r.first = r.q0 / C + b;
-  if (r.slot < 0 || r.ctx < 0) r.ql = 0;
+  if (r.slot < 0 || r.ctx < 0 || r.ql < a.least) r.ql = 0;
   return r;
 }
 
@@ -679,18 +680,20 @@ LLMSS_API int64_t llmss_linear_scan_chunked_floats(int T, int B, int H, int dk, 
 }
 
 // llmss_linear_scan over chunks of 64 tokens (see the head of this file): dk a multiple of 4 up to 128, the state and the scratch on
-// 16-byte lines; any strides, value size and sequence lengths.
-LLMSS_API int llmss_linear_scan_chunked(const float* q, int64_t ldq, const float* k, int64_t ldk, const float* v, int64_t ldv, const float* decay,
-                                        int64_t ldd, int decay_kind, const float* bonus, const float* vscale, int64_t ldvs, float* out,
-                                        float* state, const int* cu_q, const int* seq_lens, const int* slots, int B, int T, int max_q, int heads,
-                                        int qk_heads, int dk, int dv, int read_before, float* scratch, cudaStream_t stream) {
+// 16-byte lines; any strides, value size and sequence lengths.  least: sequences of fewer tokens are left alone (a token alone costs a
+// whole chunk here; llmss_linear_scan_upto takes them).
+LLMSS_API int llmss_linear_scan_chunked_from(const float* q, int64_t ldq, const float* k, int64_t ldk, const float* v, int64_t ldv,
+                                             const float* decay, int64_t ldd, int decay_kind, const float* bonus, const float* vscale, int64_t ldvs,
+                                             float* out, float* state, const int* cu_q, const int* seq_lens, const int* slots, int B, int T,
+                                             int max_q, int heads, int qk_heads, int dk, int dv, int read_before, float* scratch, int least,
+                                             cudaStream_t stream) {
   LLMSS_REQUIRE(heads > 0 && qk_heads > 0 && heads % qk_heads == 0, "linear_scan_chunked: %d heads over %d query/key heads", heads, qk_heads);
   LLMSS_REQUIRE(dk > 0 && dk % 4 == 0 && dk <= 128 && dv > 0, "linear_scan_chunked: key size %d (a multiple of 4 up to 128), value size %d", dk, dv);
   LLMSS_REQUIRE(decay_kind >= 0 && decay_kind <= 2 && scratch != nullptr, "linear_scan_chunked: decay kind %d", decay_kind);
   LLMSS_REQUIRE((((uintptr_t)state | (uintptr_t)scratch) & 15) == 0, "linear_scan_chunked: state / scratch off the 16-byte lines");
   if (B <= 0 || max_q <= 0) return 0;
   ChunkArgs a{q, ldq, k, ldk, v, ldv, decay, ldd, bonus, vscale, ldvs, out, state, cu_q, seq_lens, slots, nullptr, nullptr, nullptr, heads, heads / qk_heads,
-              dk, dv, (dv + JT - 1) / JT};
+              dk, dv, (dv + JT - 1) / JT, least};
   a.chunks = scratch;
   a.decays = scratch + ((int64_t)T / C + B) * heads * (int64_t)dk * dv;
   a.decay_rest = a.decays + ((int64_t)T / C + B) * heads * dk;
@@ -707,4 +710,12 @@ LLMSS_API int llmss_linear_scan_chunked(const float* q, int64_t ldq, const float
   if (decay_kind == 1) LLMSS_LC(128, 1);
   LLMSS_LC(128, 2);
 #undef LLMSS_LC
+}
+
+LLMSS_API int llmss_linear_scan_chunked(const float* q, int64_t ldq, const float* k, int64_t ldk, const float* v, int64_t ldv, const float* decay,
+                                        int64_t ldd, int decay_kind, const float* bonus, const float* vscale, int64_t ldvs, float* out,
+                                        float* state, const int* cu_q, const int* seq_lens, const int* slots, int B, int T, int max_q, int heads,
+                                        int qk_heads, int dk, int dv, int read_before, float* scratch, cudaStream_t stream) {
+  return llmss_linear_scan_chunked_from(q, ldq, k, ldk, v, ldv, decay, ldd, decay_kind, bonus, vscale, ldvs, out, state, cu_q, seq_lens, slots, B, T,
+                                        max_q, heads, qk_heads, dk, dv, read_before, scratch, 0, stream);
 }

@@ -307,6 +307,11 @@ int llmss_linear_scan(const float* q, int64_t ldq, const float* k, int64_t ldk, 
                       int64_t ldd, int decay_kind, const float* bonus, const float* vscale, int64_t ldvs, float* out, float* state,
                       const int* cu_q, const int* seq_lens, const int* slots, int B, int heads, int qk_heads, int dk, int dv,
                       int read_before, float* scratch, int chunk, int max_q, llmss_stream_t stream);
+/* the same for sequences of at most `most` tokens; longer ones are left alone */
+int llmss_linear_scan_upto(const float* q, int64_t ldq, const float* k, int64_t ldk, const float* v, int64_t ldv, const float* decay,
+                           int64_t ldd, int decay_kind, const float* bonus, const float* vscale, int64_t ldvs, float* out, float* state,
+                           const int* cu_q, const int* seq_lens, const int* slots, int B, int heads, int qk_heads, int dk, int dv,
+                           int read_before, float* scratch, int chunk, int max_q, int most, llmss_stream_t stream);
 /* portions of 64 tokens and more as products over 64-token chunks: dk a multiple of 4 up to 128; T = rows of q / k / v (>= cu_q[B]);
  * scratch: llmss_linear_scan_chunked_floats numbers; state and scratch 16-byte aligned */
 int64_t llmss_linear_scan_chunked_floats(int T, int B, int heads, int dk, int dv);
@@ -314,6 +319,11 @@ int llmss_linear_scan_chunked(const float* q, int64_t ldq, const float* k, int64
                               int64_t ldd, int decay_kind, const float* bonus, const float* vscale, int64_t ldvs, float* out, float* state,
                               const int* cu_q, const int* seq_lens, const int* slots, int B, int T, int max_q, int heads, int qk_heads, int dk,
                               int dv, int read_before, float* scratch, llmss_stream_t stream);
+/* the same for sequences of at least `least` tokens; shorter ones are left alone */
+int llmss_linear_scan_chunked_from(const float* q, int64_t ldq, const float* k, int64_t ldk, const float* v, int64_t ldv, const float* decay,
+                                   int64_t ldd, int decay_kind, const float* bonus, const float* vscale, int64_t ldvs, float* out,
+                                   float* state, const int* cu_q, const int* seq_lens, const int* slots, int B, int T, int max_q, int heads,
+                                   int qk_heads, int dk, int dv, int read_before, float* scratch, int least, llmss_stream_t stream);
 /* tcgen05 decode attention with a score bias per head and key distance; x[t, h * dv + c] *= sigmoid(gate[t, h]) */
 int llmss_attn_decode_tc_bias(const void* q, int64_t ldq, const void* k_cache, const void* v_cache, const int* block_tables,
                               int max_blocks, const int* seq_lens, void* out, int64_t ldo, float* scratch, int B, int hq, int hkv,

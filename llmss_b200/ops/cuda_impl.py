@@ -7,6 +7,7 @@ a per-device arena allocated once.
 from __future__ import annotations
 
 import ctypes as C
+import math
 import os
 from typing import Optional
 
@@ -769,10 +770,37 @@ def ssm_dt(dt_raw, dt_bias, a_log):
 
 _SCAN_CHUNK = int(os.environ.get("LLMSS_SCAN_CHUNK", "128"))          # tokens per chunk of the two-pass recurrence
 _SCAN_CHUNK_MIN = int(os.environ.get("LLMSS_SCAN_CHUNK_MIN", "256"))   # portions from this length on run in two passes
-# Portions from this length on run as products over chunks of 64 tokens.  Products / token by token on B200, us: 8 x 128 tokens 90 / 127
-# (32 heads of 64 x 64, decay per channel), 117 / 246 (16 of 128 x 128, per channel), 117 / 134 (constant decay), 116 / 130 (32 of
-# 128 x 64, decay per token); 8 x 64 tokens 94 / 77, 80 / 140, 86 / 80, 82 / 77.
+# Batches whose longest portion has this many tokens may run as products over chunks of 64 tokens (_scan_floor decides)
 _SCAN_TILES_MIN = int(os.environ.get("LLMSS_SCAN_TILES_MIN", "96"))
+
+
+def _scan_floor(T: int, B: int, max_q: int, heads: int, dk: int, dv: int, kind: int) -> Optional[int]:
+    """Of how many tokens a sequence has to be to run as products over chunks; shorter ones of the batch run token by token beside
+    them.  0: all sequences over chunks, None: the whole batch token by token.
+
+    Token by token a batch takes the longer of its chain (0.6 us a token, 0.85 where few blocks run narrow ones; with a decay per channel and
+    keys of more than 64 0.75 and 1.8) and its arithmetic (0.035 us a token and 131072 state elements in one pass, 0.065 in the two passes that
+    portions of 256 tokens take, whose chain is twice a chunk of theirs).  Over chunks it takes 35 us and 2.6 us a chunk, and a lone token is
+    a chunk too; short sequences beside them cost a launch and their states' way.  The lengths other than the longest are on the device:
+    estimated by their mean, and below 128 taken to hold short ones.  Measured on B200, us, all token by token / all over chunks / as decided
+    here, 32 heads of 64 x 64 with a decay per channel (16 of 128 x 128 likewise): 8 x 1024 tokens 585 / 396 / 396 (954 / 704 / 704), 512 + 63 x 1
+    176 / 239 / 93 (215 / 427 / 149), 1024 + 31 x 16 200 / 176 / 109 (236 / 287 / 206), 512 + 63 x 33 258 / 254 / 182 (348 / 442 / 299), 64 x 96
+    251 / 423 / 251 (429 / 757 / 429), 96 + 63 x 1 56 / 210 / 56 (72 / 379 / 72)."""
+    if (max_q < _SCAN_TILES_MIN or dk % 4 or dk > 128 or heads * -(-dv // 64) > 65535 or B > 65535 or heads * dk * dv >= 1 << 30):
+        return None
+    size = heads * dk * dv / 131072
+    two_passes = max_q >= _SCAN_CHUNK_MIN
+    many = B * heads * -(-dv // (128 if dk <= 64 else 64)) * (-(-max_q // _SCAN_CHUNK) if two_passes else 1) >= 4 * 148
+    step = (0.75 if many else 1.8) if kind == 2 and dk > 64 else 0.6 if many else 0.85
+    serial_us = max(2 * step * _SCAN_CHUNK, 0.065 * size * T) if two_passes else max(step * max_q, 0.035 * size * T)
+    others = T - max_q
+    mean = others / (B - 1) if B > 1 else 0.0
+    short = B > 1 and mean < 128 and T - (B - 1) * max_q < 64            # (the shortest has at least T - (B - 1) max_q tokens)
+    chunks = -(-max_q // 64) + (0 if mean < 64 else (B - 1) * math.ceil(mean / 64))
+    tiles_us = 35 + 2.6 * size * chunks
+    if short:
+        tiles_us += 15 + 0.21 * size * B + (0.0 if mean >= 64 else max(step * mean, 0.035 * size * others))
+    return None if serial_us <= tiles_us else 64 if short else 0
 
 
 def linear_scan(q, k, v, decay, decay_kind, batch, state, heads, qk_heads, dk, dv, bonus=None, v_scale=None, read_before=False):
@@ -783,26 +811,27 @@ def linear_scan(q, k, v, decay, decay_kind, batch, state, heads, qk_heads, dk, d
     assert decay.dtype == torch.float32 and state.dtype == torch.float32 and state.is_contiguous()
     out = torch.empty(T, heads * dv, dtype=torch.float32, device=v.device)
     cu, sl, ss, B, mq = _bq(batch)
-    if (mq >= _SCAN_TILES_MIN and dk % 4 == 0 and dk <= 128 and state.data_ptr() % 16 == 0 and heads * -(-dv // 64) <= 65535 and B <= 65535
-            and not torch.cuda.is_current_stream_capturing()):
+    inputs = (_ptr(q), ldq, _ptr(k), ldk, _ptr(v), ldv, _ptr(decay), decay.stride(0) if decay.dim() == 2 else 0, decay_kind, _ptr(bonus),
+              _ptr(v_scale), v_scale.stride(0) if v_scale is not None else 0, _ptr(out), _ptr(state), cu, sl, ss, B)
+    before = 1 if read_before else 0
+    floor = _scan_floor(T, B, mq, heads, dk, dv, decay_kind)
+    if floor is not None and state.data_ptr() % 16 == 0 and not torch.cuda.is_current_stream_capturing():
         # portions: products of tiles over chunks of 64 tokens (csrc/scan_chunk.cu)
         scratch = torch.empty(lib.llmss_linear_scan_chunked_floats(T, B, heads, dk, dv), dtype=torch.float32, device=v.device)
-        rc = lib.llmss_linear_scan_chunked(_ptr(q), ldq, _ptr(k), ldk, _ptr(v), ldv, _ptr(decay), decay.stride(0) if decay.dim() == 2 else 0,
-                                           decay_kind, _ptr(bonus), _ptr(v_scale), v_scale.stride(0) if v_scale is not None else 0, _ptr(out),
-                                           _ptr(state), cu, sl, ss, B, T, mq, heads, qk_heads, dk, dv, 1 if read_before else 0, _ptr(scratch),
-                                           _stream())
-        _lib.check(rc, "llmss_linear_scan_chunked")
+        rc = lib.llmss_linear_scan_chunked_from(*inputs, T, mq, heads, qk_heads, dk, dv, before, _ptr(scratch), floor, _stream())
+        _lib.check(rc, "llmss_linear_scan_chunked_from")
         _count(3)
+        if floor:
+            rc = lib.llmss_linear_scan_upto(*inputs, heads, qk_heads, dk, dv, before, None, 0, floor - 1, floor - 1, _stream())
+            _lib.check(rc, "llmss_linear_scan_upto")
+            _count()
         return out
     # long portions of few sequences: two passes over chunks, every chunk a block (a recurrence is a chain per token)
     chunk, scratch = 0, None
     if mq >= _SCAN_CHUNK_MIN and not torch.cuda.is_current_stream_capturing():
         chunk = _SCAN_CHUNK
         scratch = torch.empty(lib.llmss_linear_scan_scratch_floats(B, heads, dk, dv, mq, chunk), dtype=torch.float32, device=v.device)
-    rc = lib.llmss_linear_scan(_ptr(q), ldq, _ptr(k), ldk, _ptr(v), ldv, _ptr(decay), decay.stride(0) if decay.dim() == 2 else 0,
-                               decay_kind, _ptr(bonus), _ptr(v_scale), v_scale.stride(0) if v_scale is not None else 0, _ptr(out),
-                               _ptr(state), cu, sl, ss, B, heads, qk_heads, dk, dv, 1 if read_before else 0, _ptr(scratch), chunk, mq,
-                               _stream())
+    rc = lib.llmss_linear_scan(*inputs, heads, qk_heads, dk, dv, before, _ptr(scratch), chunk, mq, _stream())
     _lib.check(rc, "llmss_linear_scan")
     _count(2 if chunk else 1)
     return out

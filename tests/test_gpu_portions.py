@@ -214,6 +214,37 @@ def test_linear_scan_keeps_a_bad_value_behind_its_token(kind, dk, before, bad):
     assert _rel(got, w) < 2e-6
 
 
+@pytest.mark.parametrize("kind,dk,before", [(2, 64, True), (2, 128, False), (1, 128, False), (0, 20, False)])
+@pytest.mark.parametrize("floor", [None, 0, 64])
+def test_linear_scan_long_and_short_portions_together(kind, dk, before, floor, monkeypatch):
+    """A batch of whole chunks, of lengths around a chunk and of single tokens, every way that the rule can send it: all token by token,
+    all over chunks, and split at 64 tokens.  Fresh sequences; every state is written once.  Bound: 32-bit sums, 2e-6 of the norm."""
+    from llmss_b200.ops import cuda_impl as cu
+
+    monkeypatch.setattr(cu, "_scan_floor", lambda *a: floor)
+    lens = [1, 130, 1, 63, 64, 65, 2, 1, 200, 16, 1]
+    _, want, run = _scan_case(dk, kind, dk, 24, 2, lens, before, lambda s: -torch.exp(torch.randn(s, device="cuda") - 1.0))
+    (w, ends), (got, state) = want(), run()
+    assert _rel(got, w.reshape(got.shape)) < 2e-6
+    for i, S in enumerate(ends):
+        assert _rel(state[i], S) < 2e-6, lens[i]
+
+
+@pytest.mark.parametrize("kind,dk,before", [(2, 64, True), (2, 128, False), (1, 128, False), (0, 64, False)])
+def test_linear_scan_portions_agree_across_the_rule(kind, dk, before):
+    """The same 192 tokens in portions of 96 and 96, 95 and 97, and whole: equal to rounding, 2e-6 of the norm."""
+    (q, k, v, dec, bonus), want, _ = _scan_case(9, kind, dk, 24, 2, [192], before, lambda s: -torch.rand(s, device="cuda"))
+    w = want()[0].reshape(192, -1)
+    for cut in (96, 95, 192):
+        state, outs = torch.zeros(1, 2, dk, 24, device="cuda"), []
+        for lo, hi in ((0, cut), (cut, 192)):
+            if hi > lo:
+                part = [x[lo:hi] for x in (q, k, v)]
+                outs.append(ops.linear_scan(*part, dec if kind == 0 else dec[lo:hi], kind, _batch([hi - lo], [lo], [0]), state, 2, 2, dk, 24,
+                                            bonus=bonus, read_before=before))
+        assert _rel(torch.cat(outs), w) < 2e-6, cut
+
+
 @pytest.mark.parametrize("T,H,k,n,xs,form", [(129, 3, 128, 128, None, None), (300, 5, 64, 192, 72, "row"), (513, 2, 192, 128, 256, "elem"), (257, 16, 40, 24, None, "f32"),
                                              (2000, 33, 128, 136, None, "row"), (130, 2, 8, 40, None, "row"), (385, 3, 72, 8, 80, "f32")])
 @pytest.mark.parametrize("dt", [torch.bfloat16, torch.float16])
