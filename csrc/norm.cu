@@ -109,8 +109,9 @@ __device__ __forceinline__ uint4 ld_in_order(const void* p) {
 
 // The same at prompt sizes: WPR warps per row (8 16-byte vectors per lane: rows up to 2048 numbers per warp), four warps a block.  A
 // block per row spends its time in barriers and in the tail of its few loads: here a lane has all of its loads in flight at once
-// and a row of up to 2048 numbers needs no barrier.  4004 x 2048, three inputs and two outputs (82 MB) on B200: 21.3 us
-// with a block per row, 16.8 us.
+// and a row of up to 2048 numbers needs no barrier.  The sums are those of the block-per-row kernel, in its order (a warp stands for
+// NP of its eight warps): a row's result does not depend on how many rows the batch has.  4004 x 2048, three inputs and two outputs (82 MB)
+// on B200: 21.3 us with a block per row, 16.8 us (sums in an order of their own took as long).
 template <typename T, int WPR>
 __global__ void __launch_bounds__(128) norm_rows_kernel(
     const T* __restrict__ x, const T* __restrict__ x2, const T* residual_in, T* residual_out,
@@ -118,8 +119,8 @@ __global__ void __launch_bounds__(128) norm_rows_kernel(
     int64_t ldx2, int64_t ldr, int64_t ldo, float eps, int kind) {
   pdl_launch_dependents();
   pdl_wait();
-  constexpr int V = 8;
-  __shared__ float red[2][4];
+  constexpr int V = 8, NP = V / WPR;      // a lane's vectors i, i + NP, ... are those of one thread of the block-per-row kernel
+  __shared__ float red[2][4 / WPR][8];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, part = warp % WPR;
   const int row = blockIdx.x * (4 / WPR) + warp / WPR;
   const int nvec = row < M ? H >> 3 : 0, c0 = part * 32 + lane;      // (past the last row nothing is read or written)
@@ -137,7 +138,9 @@ __global__ void __launch_bounds__(128) norm_rows_kernel(
   if (residual_in != nullptr) fetch(rr, residual_in + r0 * ldr);
   if (x2 != nullptr) fetch(ry, x2 + r0 * ldx2);
   float v[V][8];
-  float sum = 0.f;
+  float sums[NP];
+#pragma unroll
+  for (int m = 0; m < NP; ++m) sums[m] = 0.f;
 #pragma unroll
   for (int i = 0; i < V; ++i) {
     const int c = c0 + i * 32 * WPR;
@@ -158,30 +161,47 @@ __global__ void __launch_bounds__(128) norm_rows_kernel(
       if (c < nvec) *reinterpret_cast<uint4*>(residual_out + row * ldr + c * 8) = r;
       unpack8<T>(r, v[i]);      // the normalisation sees the value as stored
     }
+    if (c < nvec) {
 #pragma unroll
-    for (int j = 0; j < 8; ++j) sum += c >= nvec ? 0.f : kind == LLMSS_NORM_RMS ? v[i][j] * v[i][j] : v[i][j];
+      for (int j = 0; j < 8; ++j) sums[i % NP] += (kind == LLMSS_NORM_RMS) ? v[i][j] * v[i][j] : v[i][j];
+    }
   }
-  auto over_row = [&](float s, int slot) {
-    s = warp_sum(s);
-    if (WPR == 1) return s;
-    if (lane == 0) red[slot][warp] = s;
-    __syncthreads();
-    float t = 0.f;
+  // One number per virtual warp: the exchanges that leave NP sums in lane groups pair lanes as warp_sum does (16, 8, 4, 2, 1 apart), and
+  // the eight warps' numbers meet as block_sum pairs them (4, 2, 1 apart)
+  auto over_row = [&](float (&s)[NP], int slot) {
+    int o = 16;
 #pragma unroll
-    for (int i = 0; i < WPR; ++i) t += red[slot][warp - part + i];
-    return t;
+    for (int w = NP / 2; w > 0; w >>= 1, o >>= 1) {
+      const bool hi = lane & o;
+#pragma unroll
+      for (int m = 0; m < w; ++m) s[m] = (hi ? s[m + w] : s[m]) + __shfl_xor_sync(0xffffffffu, hi ? s[m] : s[m + w], o);
+    }
+    float t = s[0];                     // of virtual warp part + WPR * (lane * NP / 32)
+#pragma unroll
+    for (; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+    if (WPR == 1) {
+#pragma unroll
+      for (int b = 16; b > 2; b >>= 1) t += __shfl_xor_sync(0xffffffffu, t, b);
+      return t;
+    }
+    if (lane % (32 / NP) == 0) red[slot][warp / WPR][part + WPR * (lane * NP / 32)] = t;
+    __syncthreads();
+    const float* r = red[slot][warp / WPR];
+    return ((r[0] + r[4]) + (r[2] + r[6])) + ((r[1] + r[5]) + (r[3] + r[7]));
   };
   float mean = 0.f, rstd;
   if (kind == LLMSS_NORM_RMS) {
-    rstd = rsqrtf(over_row(sum, 0) / (float)H + eps);
+    rstd = rsqrtf(over_row(sums, 0) / (float)H + eps);
   } else {
-    mean = over_row(sum, 0) / (float)H;
-    float sq = 0.f;
+    mean = over_row(sums, 0) / (float)H;
+    float sq[NP];
+#pragma unroll
+    for (int m = 0; m < NP; ++m) sq[m] = 0.f;
 #pragma unroll
     for (int i = 0; i < V; ++i) {
       if (c0 + i * 32 * WPR >= nvec) continue;
 #pragma unroll
-      for (int j = 0; j < 8; ++j) { const float d = v[i][j] - mean; sq += d * d; }
+      for (int j = 0; j < 8; ++j) { const float d = v[i][j] - mean; sq[i % NP] += d * d; }
     }
     rstd = rsqrtf(over_row(sq, 1) / (float)H + eps);
   }

@@ -341,6 +341,24 @@ def test_norm_rows_at_prompt_sizes(H, kind, extra):
     assert _rel(got, want.double()) < 2.0 ** -8
 
 
+@pytest.mark.parametrize("H", [8, 256, 1600, 2048, 2056, 4096, 4104, 5120, 8192])
+@pytest.mark.parametrize("kind", [ops.NORM_LAYER, ops.NORM_RMS])
+@pytest.mark.parametrize("dt", [torch.bfloat16, torch.float16])
+def test_a_norm_row_is_the_same_in_any_batch(H, kind, dt):
+    """Prompt sizes and a block per row sum in the same order: equal bits."""
+    torch.manual_seed(H)
+    M = 603
+    x, r, x2 = (torch.randn(M, H, device="cuda").to(dt) for _ in range(3))
+    w, b = (torch.randn(H, device="cuda").to(dt) for _ in range(2))
+    b = b if kind == ops.NORM_LAYER else None
+    whole = ops.norm_residual(x, r, w, b, 1e-5, kind, x2=x2)
+    for lo in range(0, M, 201):
+        rows = slice(lo, lo + 201)
+        part = ops.norm_residual(x[rows], r[rows], w, b, 1e-5, kind, x2=x2[rows])
+        for a, c in zip(whole, part):
+            assert torch.equal(a[rows], c)
+
+
 @pytest.mark.parametrize("kind,dk,dv,heads,qk_heads,before", [
     (2, 64, 64, 2, 2, True), (0, 128, 128, 16, 16, False), (1, 128, 64, 4, 2, False), (2, 4, 1, 3, 3, False), (2, 36, 70, 2, 2, True),
     (1, 100, 130, 2, 1, True), (0, 32, 33, 2, 2, False), (2, 128, 7, 64, 64, True)])
