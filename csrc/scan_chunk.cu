@@ -7,8 +7,9 @@
 //   1. scan_state_kernel   U_c = sum_j (prod_(t > j) a_t * k_j) v_j^T and the chunk's decay D_c, every chunk a block;
 //   2. scan_carry_kernel   S_(c+1) = D_c S_c + U_c along a sequence's chunks, an element per thread; U_c is replaced by S_c;
 //   3. scan_out_kernel     o = (decayed q) S_c + tril((decayed q) (decayed k)^T) v, every chunk a block.
-// Everything is 32-bit on the multiply-add pipe (two numbers per instruction where both operands lie in memory order): a 3-term
-// split on the tensor cores would run at 158 against 126 multiply-adds per clock and SM and round its sums differently.
+// Operands, states and results are 32-bit numbers.  Products over channels and over a chunk's keys run on the multiply-add pipe, two numbers
+// per instruction where both operands lie in memory order (a 3-term split on the tensor cores would run at 158 against 126 multiply-adds per
+// clock and SM); scores x values sum in 64 bits on its tensor form (62 multiply-adds per clock and SM).
 //
 // Decays without overflow or underflow: a sub-block of 16 tokens takes its middle as reference, q_i gets F(i) and k_j gets 1 / F(j) with
 // F the decay from the middle (products of at most 8 factors, one division).  Between sub-blocks no factor is formed that could be below
@@ -16,18 +17,24 @@
 // the sub-block's start), the key by its sub-block's second half (the decay to its end), and only then the whole sub-blocks that lie
 // between.  One factor from middle to middle would be a product of two halves, zero in 32 bits for decays of e^-6 per token, where the pair
 // of tokens at the border has weight 1.  Half a sub-block may decay to 2^-80 or grow to 2^15 in any channel: scaled numbers then stay
-// normal for q and k down to 2^-46; a chunk where one does more, where a scaled number leaves the range or a value is not finite (the masked half of the scores x values is a sum of zeros times values:
-// a bad one would reach the tokens before it), runs token by token (a column per thread).  Kernel 1 needs no reciprocals: its factors are suffix products.
-// Decays that are one number per token or head are multiplied out in 64 bits, once per chunk: with a constant decay every rounding has
-// the same sign, and the powers' error, not the sums', would be the result's (3.5e-7 of the norm against 7e-8 token by token).
-// What is left of the error is the rounding of the 32-bit sums, twice (scores, then outputs) where the token-serial form has one:
-// against 64 bits 1.0e-7 of the norm (9.3e-8 token by token) for 64 x 64 with a bonus, 128 x 128 per channel 6.8e-8 (5.1e-8), constant
-// decay 6.8e-8 (7.6e-8), 128 x 64 per token 1.08e-7 (9.6e-8).  Factors carried as pairs of numbers change none of these.
+// normal for q and k down to 2^-46.  A chunk runs token by token (a column per thread) where a half does more, where a scaled number
+// leaves the range, or where a value is not finite (the masked half of scores x values is zeros times values: a bad one would reach
+// the tokens before it).  Kernel 1 needs no reciprocals: its factors are suffix products.
+//
+// Rounding.  Two sums stand behind an output (scores, then outputs) where the token-serial form has one, and a chain of products behind a
+// decay.  So that the result is not further from 64 bits than token by token:
+//   - decays that are one number per token or head are multiplied out in 64 bits, once per chunk (with a constant decay every rounding has
+//     the same sign); a key's decay to the chunk's end, per channel, is carried as a pair of numbers;
+//   - a score is the sum of parts of 8 channels with the roundings of the additions carried along;
+//   - scores x values, the chain of up to 64 additions to a result of full size, sum in 64 bits and are rounded once.
+// Against 64 bits, of the norm (token by token in brackets): 64 x 64 with a bonus 9.0e-8 (9.4e-8), 128 x 128 per channel 4.7e-8 (5.0e-8),
+// one decay per head 1.3e-7 (1.7e-7), 128 x 64 per token 8.2e-8 (9.8e-8); decays near 1 per channel 2.3e-7 (2.4e-7).  With 32-bit sums
+// throughout the first two were 1.0e-7 and 6.9e-8.
 //
 // B200, 8 prompts of 1024 tokens, against the two passes of the token-serial form: 32 heads of 64 x 64, decay per channel and bonus
-// 618 -> 376 us (99 + 36 + 221, ncu: 44 % of the multiply-add pipe, shared memory 37 to 57 % of its bandwidth); 16 heads of 128 x 128, per
-// channel 979 -> 643 us, constant decay 846 -> 616 us; 32 heads of 128 x 64, decay per token 830 -> 612 us.  Kernel 3 is bound by shared
-// memory: a tile of 8 x 4 per thread reads 12 16-byte pieces for 64 packed multiply-adds, and every piece takes 4 clocks of the SM.
+// 585 -> 415 us (101 + 37 + 287 under ncu, where the issue slots are half full and shared memory's path 39 %; with 32-bit sums throughout 385);
+// 16 heads of 128 x 128, per channel 954 -> 728 us, constant decay 821 -> 630 us; 32 heads of 128 x 64, decay per token 810 -> 620 us.
+// Kernel 3 is bound by its phases between barriers, at two or three blocks per SM.  With every chunk token by token: 696, 1522, 1231, 1222 us.
 #include "common.cuh"
 
 namespace {
@@ -78,6 +85,16 @@ __device__ __forceinline__ uint64_t pmul(uint64_t x, uint64_t y) {
   asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(x), "l"(y));
   return d;
 }
+__device__ __forceinline__ uint64_t padd(uint64_t x, uint64_t y) {
+  uint64_t d;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(x), "l"(y));
+  return d;
+}
+__device__ __forceinline__ uint64_t psub(uint64_t x, uint64_t y) {
+  uint64_t d;
+  asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(x), "l"(y));
+  return d;
+}
 __device__ __forceinline__ uint64_t pack(float lo, float hi) {
   uint64_t d;
   asm("mov.b64 %0, {%1, %2};" : "=l"(d) : "f"(lo), "f"(hi));
@@ -107,6 +124,10 @@ __device__ __forceinline__ void load_rows(const float* p, int64_t ld, int l0, in
     x[i] = ld_f32(p);
     p += l0 + i + 1 < n ? ld : 0;
   }
+}
+// c[8 x 8] += a[8 x 4] b[4 x 8] in 64 bits: lane l holds a(l / 4, l % 4), b(l % 4, l / 4) and c(l / 4, 2 (l % 4) + {0, 1})
+__device__ __forceinline__ void mma_f64(double (&c)[2], double a, double b) {
+  asm("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};" : "+d"(c[0]), "+d"(c[1]) : "d"(a), "d"(b));
 }
 // 1 / x by one Newton-Raphson step on the approximate reciprocal; x lies in 2^-80 .. 2^15 wherever the result is used
 __device__ __forceinline__ float recip(float x) {
@@ -163,11 +184,10 @@ __device__ __forceinline__ double product(const double* table, int lo, int hi) {
 template <int DK, int KIND>
 __global__ void __launch_bounds__(DK, DK == 64 ? 7 : 4) scan_state_kernel(ChunkArgs a) {
   extern __shared__ __align__(16) float sm[];
-  float* ks = sm;                      // [C][DK] keys times the decay behind them, inside the sub-block
+  float* ks = sm;                      // [C][DK] keys times the decay behind them, to the chunk's end
   float* vs = ks + C * DK;             // [C][JT]
-  float* ds = vs + C * JT;             // [NS][DK] decay of a sub-block (kind 2)
-  float* behind = ds;                  // [C] decay behind a token, to the chunk's end (kinds 0 and 1)
-  double* table = reinterpret_cast<double*>(ds + NS * DK);         // [C]
+  float* behind = vs + C * JT;         // [C] decay behind a token, to the chunk's end (kinds 0 and 1)
+  double* table = reinterpret_cast<double*>(behind + C);           // [C]
   const Rows r = rows_of(a, blockIdx.z);
   const int t_lo = blockIdx.x * C;
   if (t_lo >= r.ql) return;
@@ -175,6 +195,7 @@ __global__ void __launch_bounds__(DK, DK == 64 ? 7 : 4) scan_state_kernel(ChunkA
   const int j0 = slice * JT, nj = min(JT, a.dv - j0);
   const int64_t t0 = r.q0 + t_lo;
   const int hq = h / a.rep;
+  float decay = 1.f;                   // of the chunk, this thread's channel
   if (KIND != 2) {
     fill_table<KIND>(a, table, t0, n, h);
     if (threadIdx.x < C) behind[threadIdx.x] = (float)product(table, threadIdx.x + 1, C);
@@ -185,19 +206,24 @@ __global__ void __launch_bounds__(DK, DK == 64 ? 7 : 4) scan_state_kernel(ChunkA
     const bool in = c < a.dk;
     const float* kp = a.k + t0 * a.ldk + (int64_t)hq * a.dk + cc;
     const float* dp = KIND == 2 ? a.decay + t0 * a.ldd + (int64_t)h * a.dk + cc : nullptr;
+    // last sub-block first.  decay + lo: the product of the factors behind a token, with what its roundings left (a key's weight, and the
+    // chunk's decay, have one rounding and not up to 64)
+    float lo = 0.f;
 #pragma unroll 1
-    for (int s = 0; s < NS; ++s) {
+    for (int s = NS - 1; s >= 0; --s) {
       float kx[SB], x[SB], vr[C * JT / DK / NS];
       load_rows(kp, a.ldk, s * SB, n, kx);
       if (KIND == 2) load_factors(dp, a.ldd, s * SB, n, in, x);
       load_values<DK, SB>(a, t0, s * SB, n, h, j0, nj, vr);
-      float p = 1.f;
 #pragma unroll
       for (int i = SB - 1; i >= 0; --i) {
-        ks[(s * SB + i) * DK + c] = in && s * SB + i < n ? kx[i] * (KIND == 2 ? p : behind[s * SB + i]) : 0.f;
-        if (KIND == 2) p *= x[i];
+        ks[(s * SB + i) * DK + c] = !(in && s * SB + i < n) ? 0.f : KIND == 2 ? fmaf(kx[i], decay, kx[i] * lo) : kx[i] * behind[s * SB + i];
+        if (KIND == 2) {
+          const float y = decay * x[i];
+          lo = fmaf(lo, x[i], fmaf(decay, x[i], -y));
+          decay = y;
+        }
       }
-      if (KIND == 2) ds[s * DK + c] = p;
 #pragma unroll
       for (int i = 0; i < C * JT / DK / NS; ++i) vs[s * SB * JT + threadIdx.x + i * DK] = vr[i];
     }
@@ -211,27 +237,15 @@ __global__ void __launch_bounds__(DK, DK == 64 ? 7 : 4) scan_state_kernel(ChunkA
   for (int p = 0; p < 4; ++p)
 #pragma unroll
     for (int j = 0; j < 8; ++j) acc[p][j] = 0;
-#pragma unroll 1
-  for (int s = 0; s < NS; ++s) {
-    if (KIND == 2 && s > 0) {
-      const ulonglong2 d0 = lds2(ds + s * DK + i0), d1 = lds2(ds + s * DK + i1);
-#pragma unroll
-      for (int j = 0; j < 8; ++j) {
-        acc[0][j] = pmul(acc[0][j], d0.x); acc[1][j] = pmul(acc[1][j], d0.y);
-        acc[2][j] = pmul(acc[2][j], d1.x); acc[3][j] = pmul(acc[3][j], d1.y);
-      }
-    }
 #pragma unroll 2
-    for (int i = 0; i < SB; ++i) {
-      const int t = s * SB + i;
-      const ulonglong2 k0 = lds2(ks + t * DK + i0), k1 = lds2(ks + t * DK + i1);
-      const float4 x = *reinterpret_cast<const float4*>(vs + t * JT + c0), y = *reinterpret_cast<const float4*>(vs + t * JT + c1);
-      const uint64_t vv[8] = {pack(x.x, x.x), pack(x.y, x.y), pack(x.z, x.z), pack(x.w, x.w), pack(y.x, y.x), pack(y.y, y.y), pack(y.z, y.z), pack(y.w, y.w)};
+  for (int t = 0; t < C; ++t) {
+    const ulonglong2 k0 = lds2(ks + t * DK + i0), k1 = lds2(ks + t * DK + i1);
+    const float4 x = *reinterpret_cast<const float4*>(vs + t * JT + c0), y = *reinterpret_cast<const float4*>(vs + t * JT + c1);
+    const uint64_t vv[8] = {pack(x.x, x.x), pack(x.y, x.y), pack(x.z, x.z), pack(x.w, x.w), pack(y.x, y.x), pack(y.y, y.y), pack(y.z, y.z), pack(y.w, y.w)};
 #pragma unroll
-      for (int j = 0; j < 8; ++j) {
-        acc[0][j] = pfma(k0.x, vv[j], acc[0][j]); acc[1][j] = pfma(k0.y, vv[j], acc[1][j]);
-        acc[2][j] = pfma(k1.x, vv[j], acc[2][j]); acc[3][j] = pfma(k1.y, vv[j], acc[3][j]);
-      }
+    for (int j = 0; j < 8; ++j) {
+      acc[0][j] = pfma(k0.x, vv[j], acc[0][j]); acc[1][j] = pfma(k0.y, vv[j], acc[1][j]);
+      acc[2][j] = pfma(k1.x, vv[j], acc[2][j]); acc[3][j] = pfma(k1.y, vv[j], acc[3][j]);
     }
   }
   const int64_t at = (int64_t)(r.first + blockIdx.x) * a.H + h;
@@ -245,16 +259,12 @@ __global__ void __launch_bounds__(DK, DK == 64 ? 7 : 4) scan_state_kernel(ChunkA
     if (i1 < a.dk) *reinterpret_cast<float4*>(u + i1) = make_float4(p2.x, p2.y, p3.x, p3.y);
   }
   if (slice == 0 && (int)threadIdx.x < a.dk) {
-    float p = 1.f;
-    if (KIND == 2) {
-#pragma unroll
-      for (int s = 0; s < NS; ++s) p *= ds[s * DK + threadIdx.x];
-    } else {
+    if (KIND != 2) {
       const double all = product(table, 0, C);
-      p = (float)all;
-      if (threadIdx.x == 0) a.decay_rest[at] = (float)(all - (double)p);
+      decay = (float)all;
+      if (threadIdx.x == 0) a.decay_rest[at] = (float)(all - (double)decay);
     }
-    a.decays[at * a.dk + threadIdx.x] = p;
+    a.decays[at * a.dk + threadIdx.x] = decay;
   }
 }
 
@@ -301,6 +311,7 @@ template <int DK> struct OutSmem {
   static constexpr int LD = DK + 4, LA = C + 4;
   static constexpr int Q = C * LD, S = JT * LD, KA = (C * LD > C * LA + C * JT) ? C * LD : C * LA + C * JT;
   static constexpr int FLOATS = Q + KA + S + 2 * NS * DK + 7 * DK + (DK / 32 + 4) * C + 2 * 2 * NS;
+  static_assert(C * LA <= Q && LA >= JT, "the outputs pass through the queries' place");
 };
 
 template <int DK, int KIND, bool BEFORE>
@@ -415,11 +426,22 @@ __global__ void __launch_bounds__(128, DK == 64 ? 3 : 2) scan_out_kernel(ChunkAr
     deep |= !(f >= kLow && f <= kHigh);
   }
   if (KIND != 2 && tid < 2 * NS) deep = !(thalf[tid] >= (double)kLow && thalf[tid] <= (double)kHigh);
-  deep |= big > kBig;
-  float vr[C * JT / 128];               // the values, held in registers until the keys' place is free
+  // the values: to shared memory where their place is free, otherwise held in registers until the keys are done with it.  Columns are
+  // swizzled by the token (the eight columns x four tokens that a product reads lie in different banks)
+  float vr[C * JT / 128];
   load_values<128, C>(a, t0, 0, n, h, j0, nj, vr);
 #pragma unroll
   for (int i = 0; i < C * JT / 128; ++i) deep |= !(fabsf(vr[i]) < kBig);      // (in a product 0 x infinity would reach earlier tokens)
+  deep |= big > kBig;
+  auto put_values = [&]() {
+#pragma unroll
+    for (int i = 0; i < C * JT / 128; ++i) {
+      const int t = (tid + i * 128) / JT, j = tid % JT;
+      vs[t * JT + (j ^ (8 * (t & 3)))] = vr[i];
+    }
+  };
+  constexpr bool kValuesNow = C * LA >= C * LD;
+  if (kValuesNow) put_values();
   asm volatile("cp.async.wait_all;" ::: "memory");
   auto bonus_of = [&](int t) {
     float d = 0.f;
@@ -452,21 +474,24 @@ __global__ void __launch_bounds__(128, DK == 64 ? 3 : 2) scan_out_kernel(ChunkAr
       for (int t = 0; t < n; ++t) {
         float v = a.v[(t0 + t) * a.ldv + (int64_t)h * a.dv + j0 + tid];
         if (a.vscale != nullptr) v *= a.vscale[(t0 + t) * a.ldvs + h];
-        float o0 = 0.f, o1 = 0.f;
+        float sums[8], o = 0.f;           // chains of 8 channels, added pairwise: sums[l] is what 2^l of them left
 #pragma unroll
         for (int c = 0; c < DK; c += 4) {
           const float4 q4 = *reinterpret_cast<const float4*>(qs + t * DK + c), k4 = *reinterpret_cast<const float4*>(ks + t * DK + c),
                        x4 = *reinterpret_cast<const float4*>(ss + t * DK + c);
-          if (BEFORE) {
-            o0 = fmaf(q4.x, col[c], o0); o1 = fmaf(q4.y, col[c + 1], o1); o0 = fmaf(q4.z, col[c + 2], o0); o1 = fmaf(q4.w, col[c + 3], o1);
-          }
+          if ((c & 4) == 0) o = 0.f;
+          if (BEFORE) o = fmaf(q4.w, col[c + 3], fmaf(q4.z, col[c + 2], fmaf(q4.y, col[c + 1], fmaf(q4.x, col[c], o))));
           col[c] = fmaf(x4.x, col[c], k4.x * v); col[c + 1] = fmaf(x4.y, col[c + 1], k4.y * v);
           col[c + 2] = fmaf(x4.z, col[c + 2], k4.z * v); col[c + 3] = fmaf(x4.w, col[c + 3], k4.w * v);
-          if (!BEFORE) {
-            o0 = fmaf(q4.x, col[c], o0); o1 = fmaf(q4.y, col[c + 1], o1); o0 = fmaf(q4.z, col[c + 2], o0); o1 = fmaf(q4.w, col[c + 3], o1);
+          if (!BEFORE) o = fmaf(q4.w, col[c + 3], fmaf(q4.z, col[c + 2], fmaf(q4.y, col[c + 1], fmaf(q4.x, col[c], o))));
+          if (c & 4) {
+            int l = 0;
+#pragma unroll
+            for (int g = c / 8; g & 1; g >>= 1) o += sums[l++];
+            sums[l] = o;
           }
         }
-        op[t * ldo + tid] = BEFORE ? fmaf(bonus_of(t), v, o0 + o1) : o0 + o1;
+        op[t * ldo + tid] = BEFORE ? fmaf(bonus_of(t), v, o) : o;
       }
     }
     return;
@@ -489,11 +514,10 @@ __global__ void __launch_bounds__(128, DK == 64 ? 3 : 2) scan_out_kernel(ChunkAr
       for (int x = 0; x < 2 * NS; ++x) halves[x * DK + c] = (float)thalf[x];
     }
   }
-  const int cg = tid & 15, tg = tid >> 4;
   __syncthreads();
   // ---- scores: 80 tiles of 4 x 8 (eight per 16 x 16 block of the lower triangle), 20 lanes of every warp.  Off the diagonal a query is
   // brought to its sub-block's start and a key to its sub-block's end before they meet: factors of at most what each carries
-  float sc[4][8];
+  uint64_t sc[4][4];                   // two neighbouring keys' scores per number
   int si = 0, sj = 0, sb = 0, sp = 0;
   const bool scorer = lane < 20;
   if (scorer) {
@@ -502,23 +526,25 @@ __global__ void __launch_bounds__(128, DK == 64 ? 3 : 2) scan_out_kernel(ChunkAr
     sp = blk - sb * (sb + 1) / 2;
     si = sb * SB + (w & 3);            // tokens si + 4 m, keys sj + 2 m: neighbouring lanes read neighbouring rows
     sj = sp * SB + (w >> 2);
-#pragma unroll
-    for (int i = 0; i < 4; ++i)
-#pragma unroll
-      for (int j = 0; j < 8; ++j) sc[i][j] = 0.f;
     const float* fq = sb == sp ? between : halves + 2 * sb * DK;
     const float* fk = sb == sp ? between : halves + (2 * sp + 1) * DK;
     const float* fb = between + (sb == 2 ? 1 : sp == 1 ? 2 : 3) * DK;          // read where a sub-block lies between
-    // partial sums of 16 channels: the rounding of a score, and with it the result's, is that of the token-serial form
+    // sums of 8 channels, added with the roundings of the additions carried along: a score is rounded like one number, and the output
+    // (a second sum) not further from 64 bits than token by token
+    uint64_t lost[4][4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+      for (int j = 0; j < 4; ++j) sc[i][j] = lost[i][j] = 0;
 #pragma unroll 1
-    for (int cc = 0; cc < DK; cc += 16) {
+    for (int cc = 0; cc < DK; cc += 8) {
       uint64_t acc[4][8];
 #pragma unroll
       for (int i = 0; i < 4; ++i)
 #pragma unroll
         for (int j = 0; j < 8; ++j) acc[i][j] = 0;
-#pragma unroll 1
-      for (int c = cc; c < cc + 16; c += 4) {
+#pragma unroll
+      for (int c = cc; c < cc + 8; c += 4) {
         const ulonglong2 f = lds2(fq + c), g = lds2(fk + c);
         ulonglong2 q4[4];
 #pragma unroll
@@ -547,32 +573,34 @@ __global__ void __launch_bounds__(128, DK == 64 ? 3 : 2) scan_out_kernel(ChunkAr
 #pragma unroll
       for (int i = 0; i < 4; ++i)
 #pragma unroll
-        for (int j = 0; j < 8; ++j) {
-          const float2 p = unpack(acc[i][j]);
-          sc[i][j] += p.x + p.y;
+        for (int j = 0; j < 4; ++j) {
+          const float2 p0 = unpack(acc[i][2 * j]), p1 = unpack(acc[i][2 * j + 1]);
+          const uint64_t y = padd(pack(p0.x + p0.y, p1.x + p1.y), lost[i][j]), t = padd(sc[i][j], y);
+          lost[i][j] = psub(y, psub(t, sc[i][j]));
+          sc[i][j] = t;
         }
     }
 #pragma unroll
     for (int i = 0; i < 4; ++i)
 #pragma unroll
-      for (int j = 0; j < 8; ++j) {
-        const int ti = si + 4 * i, tj = sj + 2 * j;
-        float x = sc[i][j];
-        if (tj > ti) x = 0.f;
-        else if (BEFORE && tj == ti) x = bonus_of(ti);
-        sc[i][j] = x;
-      }
+      for (int j = 0; j < 4; ++j) sc[i][j] = padd(sc[i][j], lost[i][j]);
   }
   __syncthreads();
-  // ---- scores over the keys, values behind them, q from its sub-block's middle to the chunk's start
+  // ---- scores over the keys, q from its sub-block's middle to the chunk's start
   if (scorer) {
 #pragma unroll
     for (int i = 0; i < 4; ++i)
 #pragma unroll
-      for (int j = 0; j < 8; ++j) as[(si + 4 * i) * LA + sj + 2 * j] = sc[i][j];
+      for (int j = 0; j < 8; ++j) {
+        const int ti = si + 4 * i, tj = sj + 2 * j;
+        const float2 pair = unpack(sc[i][j / 2]);
+        float x = j & 1 ? pair.y : pair.x;
+        if (tj > ti) x = 0.f;
+        else if (BEFORE && tj == ti) x = bonus_of(ti);
+        as[ti * LA + tj] = x;
+      }
   }
-#pragma unroll
-  for (int i = 0; i < C * JT / 128; ++i) vs[tid + i * 128] = vr[i];
+  if (!kValuesNow) put_values();
   for (int i = tid; i < C * (DK / 4); i += 128) {
     const int t = i / (DK / 4), c = (i % (DK / 4)) * 4, s = t / SB;
     float4* p = reinterpret_cast<float4*>(qs + t * LD + c);
@@ -587,6 +615,7 @@ __global__ void __launch_bounds__(128, DK == 64 ? 3 : 2) scan_out_kernel(ChunkAr
   }
   __syncthreads();
   // ---- o = q S: pairs along the key rows
+  const int cg = tid & 15, tg = tid >> 4;
   float o[8][4];
 #pragma unroll
   for (int m = 0; m < 8; ++m)
@@ -619,48 +648,62 @@ __global__ void __launch_bounds__(128, DK == 64 ? 3 : 2) scan_out_kernel(ChunkAr
         o[m][j] += p.x + p.y;
       }
   }
-  // ---- o += scores v: rows of sub-blocks s and later see the keys of sub-block s
+  // ---- o += scores v in 64-bit products of 8 x 8 x 4 (scores and values are 32-bit numbers, only the sums are wider: a chain of up to
+  // 64 additions to a result of full size would cost more than the serial form's whole error).  Warp w takes the token tiles w and 7 - w,
+  // together 18 steps of 4 keys; the sums so far change hands through the queries' place
+  __syncthreads();
 #pragma unroll
-  for (int s = 0; s < NS; ++s) {
-    float part[8][4];
+  for (int m = 0; m < 8; ++m)
 #pragma unroll
-    for (int m = 0; m < 8; ++m)
+    for (int j = 0; j < 4; ++j) qs[(tg + 8 * m) * LA + cg + 16 * j] = o[m][j];
+  __syncthreads();
+  const int lr = lane >> 2, lk = lane & 3;
+  double acc[2][8][2];
 #pragma unroll
-      for (int j = 0; j < 4; ++j) part[m][j] = 0.f;
-#pragma unroll 1
-    for (int t = s * SB; t < (s + 1) * SB; t += 4) {
-      float v4[4][4];
+  for (int x = 0; x < 2; ++x) {
+    const float* p = qs + (8 * (x == 0 ? 7 - warp : warp) + lr) * LA + 2 * lk;
 #pragma unroll
-      for (int x = 0; x < 4; ++x)
-#pragma unroll
-        for (int j = 0; j < 4; ++j) v4[x][j] = vs[(t + x) * JT + cg + 16 * j];
-#pragma unroll
-      for (int m = 2 * s; m < 8; ++m) {
-        const float4 w = *reinterpret_cast<const float4*>(as + (tg + 8 * m) * LA + t);
-#pragma unroll
-        for (int j = 0; j < 4; ++j)
-          part[m][j] = fmaf(w.w, v4[3][j], fmaf(w.z, v4[2][j], fmaf(w.y, v4[1][j], fmaf(w.x, v4[0][j], part[m][j]))));
-      }
+    for (int y = 0; y < 8; ++y) {
+      const float2 v = *reinterpret_cast<const float2*>(p + 8 * y);
+      acc[x][y][0] = v.x;
+      acc[x][y][1] = v.y;
     }
+  }
+  const float* a0 = as + (8 * (7 - warp) + lr) * LA + lk;
+  const float* a1 = as + (8 * warp + lr) * LA + lk;
+  const float* vp = vs + lk * JT + lr;
+#pragma unroll 2
+  for (int t = 0; t < 8 * (8 - warp); t += 4) {
+    double b[8];
 #pragma unroll
-    for (int m = 2 * s; m < 8; ++m)
+    for (int y = 0; y < 8; ++y) b[y] = vp[t * JT + ((8 * y) ^ (8 * lk))];
+    const double w0 = a0[t];
 #pragma unroll
-      for (int j = 0; j < 4; ++j) o[m][j] += part[m][j];
+    for (int y = 0; y < 8; ++y) mma_f64(acc[0][y], w0, b[y]);
+    if (t < 8 * (warp + 1)) {
+      const double w1 = a1[t];
+#pragma unroll
+      for (int y = 0; y < 8; ++y) mma_f64(acc[1][y], w1, b[y]);
+    }
   }
 #pragma unroll
-  for (int m = 0; m < 8; ++m) {
-    const int t = tg + 8 * m;
+  for (int x = 0; x < 2; ++x) {
+    const int t = 8 * (x == 0 ? 7 - warp : warp) + lr;
     if (t >= n) continue;
 #pragma unroll
-    for (int j = 0; j < 4; ++j)
-      if (cg + 16 * j < nj) op[t * ldo + cg + 16 * j] = o[m][j];
+    for (int y = 0; y < 8; ++y)
+#pragma unroll
+      for (int e = 0; e < 2; ++e) {
+        const int j = 8 * y + 2 * lk + e;
+        if (j < nj) op[t * ldo + j] = (float)acc[x][y][e];
+      }
   }
 }
 
 template <int DK, int KIND, bool BEFORE>
 int launch_chunks(const ChunkArgs& a, int B, int nch, cudaStream_t stream) {
   const dim3 grid(nch, a.H * a.nslices, B);
-  constexpr int s1 = (C * DK + C * JT + NS * DK + 2 * C) * 4, s3 = OutSmem<DK>::FLOATS * 4;
+  constexpr int s1 = (C * DK + C * JT + 3 * C) * 4, s3 = OutSmem<DK>::FLOATS * 4;
   static PerDeviceSmem g1, g3;
   LLMSS_CHECK_CUDA(g1.ensure(scan_state_kernel<DK, KIND>, s1));
   LLMSS_CHECK_CUDA(g3.ensure(scan_out_kernel<DK, KIND, BEFORE>, s3));

@@ -783,9 +783,9 @@ def _scan_floor(T: int, B: int, max_q: int, heads: int, dk: int, dv: int, kind: 
     portions of 256 tokens take, whose chain is twice a chunk of theirs).  Over chunks it takes 35 us and 2.6 us a chunk, and a lone token is
     a chunk too; short sequences beside them cost a launch and their states' way.  The lengths other than the longest are on the device:
     estimated by their mean, and below 128 taken to hold short ones.  Measured on B200, us, all token by token / all over chunks / as decided
-    here, 32 heads of 64 x 64 with a decay per channel (16 of 128 x 128 likewise): 8 x 1024 tokens 585 / 396 / 396 (954 / 704 / 704), 512 + 63 x 1
-    176 / 239 / 93 (215 / 427 / 149), 1024 + 31 x 16 200 / 176 / 109 (236 / 287 / 206), 512 + 63 x 33 258 / 254 / 182 (348 / 442 / 299), 64 x 96
-    251 / 423 / 251 (429 / 757 / 429), 96 + 63 x 1 56 / 210 / 56 (72 / 379 / 72)."""
+    here, 32 heads of 64 x 64 with a decay per channel (16 of 128 x 128 likewise): 8 x 1024 tokens 585 / 415 / 415 (954 / 728 / 728), 512 + 63 x 1
+    176 / 255 / 93 (215 / 465 / 148), 1024 + 31 x 16 200 / 188 / 110 (236 / 315 / 207), 512 + 63 x 33 258 / 275 / 182 (348 / 484 / 298), 64 x 96
+    251 / 461 / 251 (429 / 834 / 429), 96 + 63 x 1 56 / 226 / 57 (72 / 410 / 72)."""
     if (max_q < _SCAN_TILES_MIN or dk % 4 or dk > 128 or heads * -(-dv // 64) > 65535 or B > 65535 or heads * dk * dv >= 1 << 30):
         return None
     size = heads * dk * dv / 131072
