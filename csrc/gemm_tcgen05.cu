@@ -272,8 +272,7 @@ __device__ __forceinline__ void store_chunk(const GemmArgs& a, const float (&v)[
 }
 
 // Plain flavour (bias / residual only), all CH*8 token rows and the feature in range: one pointer walked by the row
-// stride, no per-element predicate or address arithmetic -- ~4 instructions per output instead of ~25 (the generic
-// path above made the epilogue of a 128 x 256 tile instruction-bound: 11 us, ncu source page of gemm_pair_kernel).
+// stride, no per-element predicate or address arithmetic (with the generic path above the epilogue of a 128 x 256 tile took 11 us).
 template <typename T, int CH>
 __device__ __forceinline__ void store_chunk_plain_full(const GemmArgs& a, const float (&v)[CH][8], int n, int mb0, float bval) {
   T* o = reinterpret_cast<T*>(a.out) + (int64_t)mb0 * a.ldo + n;
@@ -1447,8 +1446,10 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_consta
             if (lane == 0) mbar_arrive_remote(tempty_leader + (uint32_t)(as * 8));
           }
           if (fast) store_chunk_full<T, CH>(a, v, n, m0 + cg0 * 8, lane, bval);
-          else store_chunk<T, CH>(a, v, rv, n, m0 + cg0 * 8, lane, bval, m_end);
-          __syncwarp();          // lanes past N rejoin: the next load from tensor memory is the whole warp's
+          else {
+            store_chunk<T, CH>(a, v, rv, n, m0 + cg0 * 8, lane, bval, m_end);
+            __syncwarp();        // lanes past N rejoin: the next load from tensor memory is the whole warp's
+          }
         }
       } else {
         // ---- split-K: park the partial accumulator in shared memory: [(cg*2 + half)][feature] float4, conflict-free
