@@ -58,6 +58,8 @@ _ARENAS = {}
 
 
 def arena(device) -> _Arena:
+    if type(device) is not torch.device:       # a name or an index (a torch.device, the usual case, is not made again)
+        device = torch.device(device)
     key = device.index or 0
     a = _ARENAS.get(key)
     if a is None:

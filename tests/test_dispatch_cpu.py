@@ -1,5 +1,6 @@
-"""Rules that choose a kernel, on the CPU: they look at sizes only."""
+"""Host-side rules of the CUDA path, on the CPU: which kernel a call takes by its sizes, and which arena by its device."""
 import pytest
+import torch
 
 from llmss_b200.ops import cuda_impl as cu
 
@@ -25,3 +26,13 @@ def test_a_batch_without_a_floor_has_no_short_sequences_or_many_long_ones(lens, 
     T, B = sum(lens), len(lens)
     if cu._scan_floor(T, B, max(lens), 32, 64, 64, kind) == 0:
         assert min(lens) >= 64 or (T - max(lens)) / (B - 1) >= 128
+
+
+@pytest.mark.parametrize("device", [torch.device("cuda", 1), "cuda:1", 1])
+def test_arena_by_device_name_or_index(device, monkeypatch):
+    """One arena per GPU, however the device is given."""
+    monkeypatch.setattr(cu, "_ARENAS", {})
+    monkeypatch.setattr(cu, "_Arena", lambda d: object())
+    assert cu.arena(device) is cu.arena(torch.device("cuda", 1))
+    assert cu.arena(torch.device("cuda", 0)) is not cu.arena(device)
+    assert cu.arena("cuda") is cu.arena(torch.device("cuda:0"))
