@@ -27,8 +27,8 @@ def _rel(got, want):
                                                        (100, 70, 2, 2, True), (200, 40, 1, 1, False), (300, 10, 1, 1, True)])
 @pytest.mark.parametrize("copies", [1, 40])
 def test_delta_portions(dk, dv, heads, qk_heads, unit, copies):
-    """Portions around the 16-token stages, states carried over; ``copies`` > 1 has enough columns in flight for 64 key rows per
-    thread.  Bound: 32-bit sums, 3e-6 of the norm."""
+    """Portions around the 16-token stages, states carried over, key sizes that take 1 to 16 lanes to a column pair; ``copies`` = 40: more
+    blocks than the GPU holds at once, over as many state slots.  Bound: 32-bit sums, 3e-6 of the norm."""
     torch.manual_seed(dk + dv)
     lens, ctxs = [16, 1, 33, 47][:4 if copies == 1 else 2] * copies, [0, 3, 8, 0][:4 if copies == 1 else 2] * copies
     slots, T = list(range(len(lens))), sum(lens)
@@ -64,7 +64,9 @@ def test_delta_portions(dk, dv, heads, qk_heads, unit, copies):
                                                     (1024, 64, 256, 8, 32, True, False), (700, 64, 3, 3, 264, False, False), (1, 64, 8, 2, 64, False, False)])
 def test_experts_sorted_on_the_device(T, W, E, top, F, gated, skew):
     """Groups of no rows, of less and of more than a token tile, features off the 256-feature pairs, hidden sizes off the 64-column
-    k-blocks, down matrices as a view of wider rows, a sum onto another result.  Bound: bf16 operands and hidden rows, 1e-2."""
+    k-blocks, down matrices as a view of wider rows, a sum onto another result.  Every (token, expert) pair alone, with weight 1, row by row,
+    so that a pair lost or misplaced at a group's edge is an error of the whole row; then all of them as weighted.  Bound: hidden
+    rows rounded to bf16, 1e-2."""
     from llmss_b200.ops import cuda_impl as cu
 
     torch.manual_seed(T + E)
@@ -77,14 +79,43 @@ def test_experts_sorted_on_the_device(T, W, E, top, F, gated, skew):
     ids, wts = ops.moe_route(z, E, top, 1, 1, 1.0)
     base = torch.randn(T, W, device="cuda")
     assert cu.moe_groups_on_device(h, up, down, gated)
-    got = cu.moe_experts_grouped(h, ids, wts, up, down, ops.ACT_SILU, gated, base=base.clone())
-    want = base.double()
+    pairs = torch.empty(T, top, W, device="cuda", dtype=F64)
     for e in range(E):
         t, j = torch.nonzero(ids == e, as_tuple=True)
         x = h[t].double() @ up[e].double().t()
         x = torch.nn.functional.silu(x[:, 0::2]) * x[:, 1::2] if gated else torch.nn.functional.silu(x)
-        want.index_add_(0, t, wts[t, j].double()[:, None] * (x @ down[:, e * F:(e + 1) * F].double().t()))
-    assert _rel(got, want.cpu()) < 1e-2
+        pairs[t, j] = x @ down[:, e * F:(e + 1) * F].double().t()
+    for j in range(top):
+        one = torch.zeros_like(wts)
+        one[:, j] = 1.0
+        got = cu.moe_experts_grouped(h, ids, one, up, down, ops.ACT_SILU, gated)
+        assert float(((got.double() - pairs[:, j]).norm(dim=1) / pairs[:, j].norm(dim=1)).max()) < 1e-2
+    got = cu.moe_experts_grouped(h, ids, wts, up, down, ops.ACT_SILU, gated, base=base.clone())
+    want = (wts.double()[:, :, None] * pairs).sum(1)
+    assert _rel(got.double() - base.double(), want.cpu()) < 1e-2
+
+
+@pytest.mark.parametrize("T,top,E,skew", [(1, 2, 8, False), (300, 4, 16, False), (513, 1, 5, True), (1024, 8, 256, False), (1025, 3, 3, False), (4096, 2, 200, True)])
+def test_pairs_sorted_by_expert(T, top, E, skew):
+    """Places, row ranges and tile counts against a stable sort: single blocks and several, experts without pairs, a partial last block."""
+    from llmss_b200.ops import _lib
+    from llmss_b200.ops import cuda_impl as cu
+
+    torch.manual_seed(T)
+    P = T * top
+    ids = torch.randint(0, E, (T, top), device="cuda", dtype=torch.int32)
+    if skew:
+        ids[torch.rand(T, top, device="cuda") < 0.9] = E // 2
+    hist, table, inv = (torch.full((n,), -1, dtype=torch.int32, device="cuda") for n in (-(-P // 1024) * E, 2 * (E + 1), P))
+    _lib.check(_lib.load().llmss_moe_group(cu._ptr(ids), P, E, cu._ptr(hist), cu._ptr(table), cu._ptr(inv), cu._stream()), "llmss_moe_group")
+    counts = torch.bincount(ids.flatten().cpu(), minlength=E)
+    order = torch.sort(ids.flatten().cpu(), stable=True).indices
+    want = torch.empty(P, dtype=torch.long)
+    want[order] = torch.arange(P)
+    assert torch.equal(inv.cpu().long(), want)
+    zero = torch.zeros(1, dtype=torch.long)
+    assert torch.equal(table[:E + 1].cpu().long(), torch.cat([zero, counts.cumsum(0)]))
+    assert torch.equal(table[E + 1:].cpu().long(), torch.cat([zero, ((counts + 255) // 256).cumsum(0)]))
 
 
 def _scan64(q, k, v, a, bonus, before, lens, S0):
@@ -109,7 +140,7 @@ def _scan64(q, k, v, a, bonus, before, lens, S0):
     (1, 64, 16, 2, 2, False, 2)])
 def test_linear_scan_over_chunks(kind, dk, dv, heads, qk_heads, before, deep):
     """Portions that end inside, at and behind a chunk, with and without a state, in packed order and with an inert sequence; strides
-    off the 16-byte lines; ``deep``: decays past 2^-100 within half a sub-block (1), growth (2) -- the token-by-token form of a chunk.
+    off the 16-byte lines; ``deep``: decays past 2^-80 within half a sub-block (1), growth (2) -- the token-by-token form of a chunk.
     Bound: 32-bit sums, 2e-6 of the norm."""
     torch.manual_seed(dk * 7 + dv)
     lens, ctxs, slots = [64, 1, 130, 65, 200, 3], [0, 5, 7, 0, 64, 9], [4, 0, 2, 5, 1, -1]
