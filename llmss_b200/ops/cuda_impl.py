@@ -784,10 +784,12 @@ def _scan_floor(T: int, B: int, max_q: int, heads: int, dk: int, dv: int, kind: 
     keys of more than 64 0.75 and 1.8) and its arithmetic (0.035 us a token and 131072 state elements in one pass, 0.065 in the two passes that
     portions of 256 tokens take, whose chain is twice a chunk of theirs).  Over chunks it takes 35 us and 2.6 us a chunk, and a lone token is
     a chunk too; short sequences beside them cost a launch and their states' way.  The lengths other than the longest are on the device:
-    estimated by their mean, and below 128 taken to hold short ones.  Measured on B200, us, all token by token / all over chunks / as decided
+    estimated by their mean; below 128, and among 16 sequences and more, they are taken to hold short ones.  Measured on B200, us, all token
+    by token / all over chunks / as decided
     here, 32 heads of 64 x 64 with a decay per channel (16 of 128 x 128 likewise): 8 x 1024 tokens 585 / 415 / 415 (954 / 728 / 728), 512 + 63 x 1
     176 / 255 / 93 (215 / 465 / 148), 1024 + 31 x 16 200 / 188 / 110 (236 / 315 / 207), 512 + 63 x 33 258 / 275 / 182 (348 / 484 / 298), 64 x 96
-    251 / 461 / 251 (429 / 834 / 429), 96 + 63 x 1 56 / 226 / 57 (72 / 410 / 72)."""
+    251 / 461 / 251 (429 / 834 / 429), 96 + 63 x 1 56 / 226 / 57 (72 / 410 / 72), 63 of 1 .. 64 or 590 747 / 660 / 595 (1049 / 1150 / 1026).
+    Over 112 random batches of four flavours the decided form took 0.79 of the token-serial time on average, none more than it."""
     if (max_q < _SCAN_TILES_MIN or dk % 4 or dk > 128 or heads * -(-dv // 64) > 65535 or B > 65535 or heads * dk * dv >= 1 << 30):
         return None
     size = heads * dk * dv / 131072
@@ -797,7 +799,7 @@ def _scan_floor(T: int, B: int, max_q: int, heads: int, dk: int, dv: int, kind: 
     serial_us = max(2 * step * _SCAN_CHUNK, 0.065 * size * T) if two_passes else max(step * max_q, 0.035 * size * T)
     others = T - max_q
     mean = others / (B - 1) if B > 1 else 0.0
-    short = B > 1 and mean < 128 and T - (B - 1) * max_q < 64            # (the shortest has at least T - (B - 1) max_q tokens)
+    short = B > 1 and (mean < 128 or B >= 16) and T - (B - 1) * max_q < 64       # (the shortest has at least T - (B - 1) max_q tokens)
     chunks = -(-max_q // 64) + (0 if mean < 64 else (B - 1) * math.ceil(mean / 64))
     tiles_us = 35 + 2.6 * size * chunks
     if short:
