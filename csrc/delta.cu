@@ -10,30 +10,19 @@
 // per token (decay, write strength, the norms 1 / sqrt(sum x^2 + eps), k . q) lie beside them.  The state lies in memory
 // column-major per head ([dv][dk]).
 //
+// Long portions go over chunks of 32 tokens on the tensor cores where that is faster (delta_chunk.cu); this file's portions are the others.
+//
 // A batch of single tokens (decode) runs the row-split form instead (delta_step_kernel): one warp per value column, lanes over
 // the key rows, so that every state access is one contiguous column (512 bytes at dk = 128) -- a decode step is bound by
 // reading and writing the states once.
 // Everything is 32-bit with full-precision exponentials.
 #include "common.cuh"
+#include "delta.cuh"
 
 namespace {
 
 constexpr int DTCH = 16;
-
-struct DeltaArgs {
-  const float* q; int64_t ldq;
-  const float* k; int64_t ldk;
-  const float* v; int64_t ldv;
-  const float* log_decay; int64_t ldg;   // [T, H]
-  const float* beta; int64_t ldb;        // [T, H]
-  float* out;                            // [T, H * dv]
-  float* state;                          // [slots, H, dv, dk]
-  const int* cu_q; const int* seq_lens; const int* slots;
-  int H, rep, dk, dv, dvt;
-  float unit_eps, q_scale;
-  int unit, beta_sigmoid;
-  int vec16;       // q / k / v rows, the key size and the value slices allow 16-byte copies
-};
+constexpr int kChunkLeast = 32;        // shorter sequences of a batch that goes over chunks stay here: a block over chunks takes 9 us to start and end
 
 __device__ __forceinline__ void cp_async_4(float* dst, const float* src) {
   asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(smem_u32(dst)), "l"(src) : "memory");
@@ -86,7 +75,7 @@ __global__ void __launch_bounds__(256) delta_scan_kernel(DeltaArgs a) {
   extern __shared__ __align__(16) float sm[];
   const int b = blockIdx.x;
   const int q0 = a.cu_q[b], ql = a.cu_q[b + 1] - q0, ctx = a.seq_lens[b] - ql, slot = a.slots[b];
-  if (slot < 0 || ctx < 0 || ql <= 0) return;
+  if (slot < 0 || ctx < 0 || ql < a.least || ql >= a.below) return;
   const int h = blockIdx.y, hk = h / a.rep;
   const int j0 = blockIdx.z * a.dvt, nj = min(a.dvt, a.dv - j0);
   const int dk = a.dk, nthr = blockDim.x;
@@ -354,38 +343,24 @@ __global__ void __launch_bounds__(STEP_WARPS * 32) delta_step_kernel(DeltaArgs a
 
 }  // namespace
 
-// q, k [T, qk_heads * dk] (value head h reads q / k head h / (heads / qk_heads)); v [T, heads * dv]; log_decay, beta [T, heads];
-// out [T, heads * dv]; state [slots, heads, dv, dk].  unit_eps >= 0: q and k become x / sqrt(sum x^2 + unit_eps) per head first.
-LLMSS_API int llmss_delta_scan(const float* q, int64_t ldq, const float* k, int64_t ldk, const float* v, int64_t ldv,
-                               const float* log_decay, int64_t ldg, const float* beta, int64_t ldb, float* out, float* state,
-                               const int* cu_q, const int* seq_lens, const int* slots, int B, int max_q, int heads, int qk_heads, int dk,
-                               int dv, float unit_eps, float q_scale, int beta_sigmoid, cudaStream_t stream) {
-  LLMSS_REQUIRE(heads > 0 && qk_heads > 0 && heads % qk_heads == 0, "delta_scan: %d value heads over %d query/key heads", heads, qk_heads);
-  LLMSS_REQUIRE(dk > 0 && dk <= 1024 && dv > 0, "delta_scan: key size %d (at most 1024), value size %d", dk, dv);
-  if (B <= 0) return 0;
-  DeltaArgs a;
+namespace {
+
+bool delta_args(DeltaArgs& a, const float* q, int64_t ldq, const float* k, int64_t ldk, const float* v, int64_t ldv, const float* log_decay,
+                int64_t ldg, const float* beta, int64_t ldb, float* out, float* state, const int* cu_q, const int* seq_lens, const int* slots,
+                int heads, int qk_heads, int dk, int dv, float unit_eps, float q_scale, int beta_sigmoid) {
+  if (heads <= 0 || qk_heads <= 0 || heads % qk_heads != 0 || dk <= 0 || dk > 1024 || dv <= 0) return false;
+  memset(&a, 0, sizeof(a));
   a.q = q; a.ldq = ldq; a.k = k; a.ldk = ldk; a.v = v; a.ldv = ldv; a.log_decay = log_decay; a.ldg = ldg; a.beta = beta; a.ldb = ldb;
   a.out = out; a.state = state; a.cu_q = cu_q; a.seq_lens = seq_lens; a.slots = slots;
   a.H = heads; a.rep = heads / qk_heads; a.dk = dk; a.dv = dv;
   a.unit = unit_eps >= 0.f ? 1 : 0; a.unit_eps = unit_eps >= 0.f ? unit_eps : 0.f; a.q_scale = q_scale; a.beta_sigmoid = beta_sigmoid;
-  if (max_q <= 1 && dk <= 256) {
-    // every sequence brings one token: one warp per value column, lanes over the key rows
-    a.dvt = 0;
-    const int per_pass = STEP_WARPS * STEP_COLS;
-    int groups = 1;
-    while ((int64_t)B * heads * groups < 1024 && groups * per_pass < dv) groups *= 2;
-    int cols = (dv + groups - 1) / groups;
-    cols = ((cols + per_pass - 1) / per_pass) * per_pass;
-    const dim3 sgrid(B, heads, (dv + cols - 1) / cols);
-    LLMSS_REQUIRE(sgrid.y <= 65535 && sgrid.z <= 65535, "delta_scan: grid too large");
-    const int kl = (dk + 31) / 32;
-    if (kl <= 1) delta_step_kernel<1><<<sgrid, STEP_WARPS * 32, 0, stream>>>(a, cols);
-    else if (kl <= 2) delta_step_kernel<2><<<sgrid, STEP_WARPS * 32, 0, stream>>>(a, cols);
-    else if (kl <= 4) delta_step_kernel<4><<<sgrid, STEP_WARPS * 32, 0, stream>>>(a, cols);
-    else delta_step_kernel<8><<<sgrid, STEP_WARPS * 32, 0, stream>>>(a, cols);
-    LLMSS_CHECK_CUDA(cudaGetLastError());
-    return 0;
-  }
+  a.least = 1; a.below = 0x7fffffff;
+  return true;
+}
+
+// token by token: sequences of a.least .. a.below - 1 tokens
+int delta_portions(DeltaArgs a, int B, cudaStream_t stream) {
+  const int dk = a.dk, dv = a.dv;
   // up to 32 key rows per thread, R lanes (a power of two) to a column pair
   const int kpt = dk <= 8 ? 8 : (dk <= 16 ? 16 : 32);
   int R = 1;
@@ -394,10 +369,10 @@ LLMSS_API int llmss_delta_scan(const float* q, int64_t ldq, const float* k, int6
   const int most = R <= 4 ? 64 : 256;       // long keys: a stage of q and k is shared by more columns
   threads = threads > most ? most : threads;
   a.dvt = threads / R * 2;
-  const dim3 grid(B, heads, (dv + a.dvt - 1) / a.dvt);
+  const dim3 grid(B, a.H, (dv + a.dvt - 1) / a.dvt);
   LLMSS_REQUIRE(grid.y <= 65535 && grid.z <= 65535, "delta_scan: grid too large");
-  a.vec16 = (dk % 4 == 0 && dv % 4 == 0 && a.dvt % 4 == 0 && ldq % 4 == 0 && ldk % 4 == 0 && ldv % 4 == 0 &&
-             (((uintptr_t)q | (uintptr_t)k | (uintptr_t)v) & 15) == 0) ? 1 : 0;
+  a.vec16 = (dk % 4 == 0 && dv % 4 == 0 && a.dvt % 4 == 0 && a.ldq % 4 == 0 && a.ldk % 4 == 0 && a.ldv % 4 == 0 &&
+             (((uintptr_t)a.q | (uintptr_t)a.k | (uintptr_t)a.v) & 15) == 0) ? 1 : 0;
   const size_t smem = 2 * sizeof(float) * ((size_t)2 * DTCH * R * (kpt + 4) + (size_t)DTCH * a.dvt + 8 * DTCH);
 #define LLMSS_DS(K, RR)                                                                     \
   do {                                                                                      \
@@ -416,4 +391,62 @@ LLMSS_API int llmss_delta_scan(const float* q, int64_t ldq, const float* k, int6
 #undef LLMSS_DS
   LLMSS_CHECK_CUDA(cudaGetLastError());
   return 0;
+}
+
+}  // namespace
+
+// q, k [T, qk_heads * dk] (value head h reads q / k head h / (heads / qk_heads)); v [T, heads * dv]; log_decay, beta [T, heads];
+// out [T, heads * dv]; state [slots, heads, dv, dk].  unit_eps >= 0: q and k become x / sqrt(sum x^2 + unit_eps) per head first.
+LLMSS_API int llmss_delta_scan(const float* q, int64_t ldq, const float* k, int64_t ldk, const float* v, int64_t ldv,
+                               const float* log_decay, int64_t ldg, const float* beta, int64_t ldb, float* out, float* state,
+                               const int* cu_q, const int* seq_lens, const int* slots, int B, int max_q, int heads, int qk_heads, int dk,
+                               int dv, float unit_eps, float q_scale, int beta_sigmoid, cudaStream_t stream) {
+  LLMSS_REQUIRE(heads > 0 && qk_heads > 0 && heads % qk_heads == 0, "delta_scan: %d value heads over %d query/key heads", heads, qk_heads);
+  LLMSS_REQUIRE(dk > 0 && dk <= 1024 && dv > 0, "delta_scan: key size %d (at most 1024), value size %d", dk, dv);
+  if (B <= 0) return 0;
+  DeltaArgs a;
+  delta_args(a, q, ldq, k, ldk, v, ldv, log_decay, ldg, beta, ldb, out, state, cu_q, seq_lens, slots, heads, qk_heads, dk, dv, unit_eps, q_scale, beta_sigmoid);
+  if (max_q <= 1 && dk <= 256) {
+    // every sequence brings one token: one warp per value column, lanes over the key rows
+    a.dvt = 0;
+    const int per_pass = STEP_WARPS * STEP_COLS;
+    int groups = 1;
+    while ((int64_t)B * heads * groups < 1024 && groups * per_pass < dv) groups *= 2;
+    int cols = (dv + groups - 1) / groups;
+    cols = ((cols + per_pass - 1) / per_pass) * per_pass;
+    const dim3 sgrid(B, heads, (dv + cols - 1) / cols);
+    LLMSS_REQUIRE(sgrid.y <= 65535 && sgrid.z <= 65535, "delta_scan: grid too large");
+    const int kl = (dk + 31) / 32;
+    if (kl <= 1) delta_step_kernel<1><<<sgrid, STEP_WARPS * 32, 0, stream>>>(a, cols);
+    else if (kl <= 2) delta_step_kernel<2><<<sgrid, STEP_WARPS * 32, 0, stream>>>(a, cols);
+    else if (kl <= 4) delta_step_kernel<4><<<sgrid, STEP_WARPS * 32, 0, stream>>>(a, cols);
+    else delta_step_kernel<8><<<sgrid, STEP_WARPS * 32, 0, stream>>>(a, cols);
+    LLMSS_CHECK_CUDA(cudaGetLastError());
+    return 0;
+  }
+  return delta_portions(a, B, stream);
+}
+
+// Sequences of at least 32 tokens over chunks (delta_chunk.cu), shorter ones beside them token by token.  T: rows of the batch; scratch:
+// llmss_delta_scan_chunked_bytes bytes.  Key sizes up to 128 that are multiples of 4; q, k (rows too), state and scratch on 16-byte lines.
+LLMSS_API int64_t llmss_delta_scan_chunked_bytes(int T, int B, int heads) { return ((int64_t)T / 32 + B) * heads * LLMSS_DELTA_PREPARED; }
+LLMSS_API int llmss_delta_scan_chunked(const float* q, int64_t ldq, const float* k, int64_t ldk, const float* v, int64_t ldv,
+                               const float* log_decay, int64_t ldg, const float* beta, int64_t ldb, float* out, float* state,
+                               const int* cu_q, const int* seq_lens, const int* slots, int B, int max_q, int heads, int qk_heads, int dk,
+                               int dv, float unit_eps, float q_scale, int beta_sigmoid, void* scratch, cudaStream_t stream) {
+  DeltaArgs a;
+  LLMSS_REQUIRE(delta_args(a, q, ldq, k, ldk, v, ldv, log_decay, ldg, beta, ldb, out, state, cu_q, seq_lens, slots, heads, qk_heads, dk, dv, unit_eps, q_scale, beta_sigmoid),
+                "delta_scan_chunked: %d value heads over %d query/key heads, sizes %d, %d", heads, qk_heads, dk, dv);
+  LLMSS_REQUIRE(dk <= 128 && dk % 4 == 0 && ldq % 4 == 0 && ldk % 4 == 0 &&
+                    (((uintptr_t)q | (uintptr_t)k | (uintptr_t)state | (uintptr_t)scratch) & 15) == 0,
+                "delta_scan_chunked: key size %d (at most 128, a multiple of 4), rows of q and k on 16-byte lines", dk);
+  LLMSS_REQUIRE(B <= 65535 && heads <= 65535 && (dv + 127) / 128 <= 65535, "delta_scan_chunked: grid too large");
+  if (B <= 0) return 0;
+  a.prepared = static_cast<uint8_t*>(scratch);
+  a.least = kChunkLeast;
+  const int rc = delta_chunk_launch(a, B, max_q, stream);
+  if (rc != 0 || B == 1) return rc;
+  a.least = 1;
+  a.below = kChunkLeast;
+  return delta_portions(a, B, stream);
 }

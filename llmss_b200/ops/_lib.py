@@ -166,6 +166,10 @@ _SIGS = {
     "llmss_delta_scan": (c_int, [c_void_p, c_int64, c_void_p, c_int64, c_void_p, c_int64, c_void_p, c_int64, c_void_p, c_int64, c_void_p,
                                  c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_float, c_float, c_int,
                                  c_void_p]),
+    "llmss_delta_scan_chunked_bytes": (c_int64, [c_int, c_int, c_int]),
+    "llmss_delta_scan_chunked": (c_int, [c_void_p, c_int64, c_void_p, c_int64, c_void_p, c_int64, c_void_p, c_int64, c_void_p, c_int64, c_void_p,
+                                 c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_float, c_float, c_int,
+                                 c_void_p, c_void_p]),
     "llmss_moe_route_ex": (c_int, [c_void_p, c_int64, c_int, c_int, c_int, c_int, c_int, c_float, c_int, c_void_p, c_int, c_int, c_void_p,
                                    c_void_p, c_void_p, c_void_p]),
     "llmss_attention_sink": (c_int, [c_void_p, c_int64, c_void_p, c_void_p, c_void_p, c_int, c_int, c_void_p, c_void_p, c_void_p,

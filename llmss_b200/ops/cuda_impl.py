@@ -884,6 +884,20 @@ def hyper_residual(xs, y=None, mix=None, w_out=None, w_in=None, norm_w=None, eps
     return out
 
 
+def _delta_over_chunks(T, B, max_q, heads, dk, dv):
+    """Whether the gated delta rule goes over chunks of 32 tokens (csrc/delta_chunk.cu) or token by token: the smaller of two estimates in
+    us.  Over chunks a block carries one (sequence, head, 128 columns) through its chunks at 6 us each, one block per SM, 9 us to start and end a block, 13 us for
+    the launches, and the chunks' own part costs 0.55 ns per token and head; token by token the longest portion's chain takes 0.4 us a token, and a full GPU
+    3.2e12 state elements a second.  Measured (chunks / tokens): 16 heads of 128 x 128, prompts of 576 .. 1472: 362 / 907, 8 x 1024: 280 / 635,
+    8 x 64: 39 / 47, 8 x 48: 38 / 37, 32 x 48: 103 / 114, one of 64: 33 / 31, one of 1500: 266 / 604; 32 heads of 64 x 64, 8 x 1024: 610 / 381.
+    Counts that a graph's capture fixes decide, nothing on the device."""
+    if max_q < 32 or dk > 128 or dk % 4 or B > 65535 or heads > 65535:
+        return False
+    blocks = B * heads * -(-dv // 128)
+    chunks = max(6.0 * -(-max_q // 32), -(-blocks // 148) * (6.0 * -(-T // (32 * B)) + 9.0) - 9.0) + 22.0 + 0.55e-3 * T * heads
+    return chunks < max(0.4 * max_q, T * heads * dk * dv / 3.2e6) + 5.0
+
+
 def delta_scan(q, k, v, log_decay, beta, batch, state, heads, qk_heads, dk, dv, unit_eps=None, q_scale=1.0, beta_sigmoid=False):
     lib = _lib.load()
     T, _, ldv = _f32rows(v)
@@ -894,10 +908,13 @@ def delta_scan(q, k, v, log_decay, beta, batch, state, heads, qk_heads, dk, dv, 
     assert state.dtype == torch.float32 and state.is_contiguous() and state[0].numel() == heads * dk * dv
     out = torch.empty(T, heads * dv, dtype=torch.float32, device=v.device)
     cu, sl, ss, B, mq = _bq(batch)
-    rc = lib.llmss_delta_scan(_ptr(q), ldq, _ptr(k), ldk, _ptr(v), ldv, _ptr(log_decay), ldg, _ptr(beta), ldb, _ptr(out), _ptr(state),
-                              cu, sl, ss, B, mq, heads, qk_heads, dk, dv, -1.0 if unit_eps is None else float(unit_eps), float(q_scale),
-                              1 if beta_sigmoid else 0, _stream())
-    _lib.check(rc, "llmss_delta_scan")
+    args = (_ptr(q), ldq, _ptr(k), ldk, _ptr(v), ldv, _ptr(log_decay), ldg, _ptr(beta), ldb, _ptr(out), _ptr(state),
+            cu, sl, ss, B, mq, heads, qk_heads, dk, dv, -1.0 if unit_eps is None else float(unit_eps), float(q_scale), 1 if beta_sigmoid else 0)
+    if _delta_over_chunks(T, B, mq, heads, dk, dv) and ldq % 4 == 0 and ldk % 4 == 0 and (args[0] | args[2] | args[11]) % 16 == 0:
+        scratch = torch.empty(lib.llmss_delta_scan_chunked_bytes(T, B, heads), dtype=torch.uint8, device=v.device)
+        _lib.check(lib.llmss_delta_scan_chunked(*args, _ptr(scratch), _stream()), "llmss_delta_scan_chunked")
+    else:
+        _lib.check(lib.llmss_delta_scan(*args, _stream()), "llmss_delta_scan")
     _count()
     return out
 

@@ -60,6 +60,102 @@ def test_delta_portions(dk, dv, heads, qk_heads, unit, copies):
     assert _rel(state.reshape(len(lens), heads, dv, dk).transpose(2, 3), torch.stack(ends)) < 3e-6
 
 
+def _delta64(q, k, v, g, beta, S0, lens, ctxs, heads, qk_heads, dk, dv, unit):
+    rep, T = heads // qk_heads, sum(lens)
+    qf, kf = (x.double().cpu().reshape(T, qk_heads, dk) for x in (q, k))
+    if unit:
+        qf, kf = (x * torch.rsqrt(x.square().sum(-1, keepdim=True) + 1e-6) for x in (qf, kf))
+    qf, kf, vf = (qf * 0.25).repeat_interleave(rep, 1), kf.repeat_interleave(rep, 1), v.double().cpu().reshape(T, heads, dv)
+    a, beta = torch.exp(g.double().cpu()), torch.sigmoid(beta.double().cpu())
+    out, ends, at = torch.zeros_like(vf), [], 0
+    for i, n in enumerate(lens):
+        S = S0[i].clone() if ctxs[i] else torch.zeros(heads, dk, dv, dtype=F64)
+        for t in range(at, at + n):
+            S = S * a[t][:, None, None]
+            u = beta[t][:, None] * (vf[t] - torch.einsum("hkv,hk->hv", S, kf[t]))
+            S = S + kf[t][:, :, None] * u[:, None, :]
+            out[t] = torch.einsum("hkv,hk->hv", S, qf[t])
+        ends.append(S)
+        at += n
+    return out, torch.stack(ends)
+
+
+def _delta_inputs(lens, heads, qk_heads, dk, dv, unit, wide=0):
+    T = sum(lens)
+    rows = [torch.randn(T, n + wide, device="cuda")[:, wide:] for n in (qk_heads * dk, qk_heads * dk, heads * dv)]
+    if not unit:        # keys of norm 1 keep the rule stable
+        rows[1] = torch.nn.functional.normalize(rows[1].reshape(T, qk_heads, dk), dim=-1).reshape(T, -1)
+    return rows, torch.randn(T, heads, device="cuda"), torch.randn(len(lens), heads, dk, dv, device="cuda") * 0.1
+
+
+@pytest.mark.parametrize("dk,dv,heads,qk_heads,unit", [(128, 128, 2, 1, True), (128, 128, 3, 3, False), (64, 48, 2, 2, True), (100, 200, 6, 2, True), (4, 3, 1, 1, True)])
+@pytest.mark.parametrize("decay", ["mild", "slow", "strong", "one", "above one"])
+def test_delta_over_chunks(dk, dv, heads, qk_heads, unit, decay, monkeypatch):
+    """Portions around the 32-token chunks, shorter ones beside them, states carried over, rows of wider tensors, key heads of one and more value
+    heads; decays that leave nothing of a chunk's start, decays of exactly one, and growing ones (token by token inside their chunks).  Bound:
+    32-bit sums, 1e-6 of the norm (growth over 100 tokens multiplies it)."""
+    from llmss_b200.ops import cuda_impl as cu
+
+    monkeypatch.setattr(cu, "_delta_over_chunks", lambda *a: True)
+    torch.manual_seed(dk + dv)
+    lens, ctxs = [32, 7, 100, 33, 64, 31], [0, 5, 8, 0, 3, 2]
+    (q, k, v), b, S0 = _delta_inputs(lens, heads, qk_heads, dk, dv, unit, wide=4)
+    u = torch.rand(sum(lens), heads, device="cuda")
+    g = {"mild": -0.3 * u, "slow": -0.01 * u, "strong": -3.0 - 9.0 * u, "one": 0.0 * u, "above one": 0.6 * u - 0.25}[decay]
+    state = S0.transpose(2, 3).contiguous().view(len(lens), heads, dk, dv)
+    want, ends = _delta64(q, k, v, g, b, S0.double().cpu(), lens, ctxs, heads, qk_heads, dk, dv, unit)
+    got = ops.delta_scan(q, k, v, g, b, _batch(lens, ctxs, range(len(lens))), state, heads, qk_heads, dk, dv, unit_eps=1e-6 if unit else None,
+                         q_scale=0.25, beta_sigmoid=True)
+    bound = 1e-5 if decay == "above one" else 1e-6
+    assert _rel(got, want.reshape(sum(lens), -1)) < bound
+    assert _rel(state.reshape(len(lens), heads, dv, dk).transpose(2, 3), ends) < bound
+
+
+@pytest.mark.parametrize("where", ["value", "key", "strength", "decay", "state", "huge value"])
+def test_delta_over_chunks_bad_numbers(where, monkeypatch):
+    """A value that is no number, or too large to scale, reaches what it reaches token by token: later tokens of its column (value, state) or of
+    its head (key, strength, decay), never an earlier token or another head."""
+    from llmss_b200.ops import cuda_impl as cu
+
+    monkeypatch.setattr(cu, "_delta_over_chunks", lambda *a: True)
+    torch.manual_seed(5)
+    lens, heads, d = [100], 2, 128
+    (q, k, v), b, S0 = _delta_inputs(lens, heads, 2, d, d, True)
+    g, at, state = -0.3 * torch.rand(100, heads, device="cuda"), 45, S0.transpose(2, 3).contiguous().view(1, heads, d, d)
+    clean_state = state.clone()
+    call = lambda s: ops.delta_scan(q, k, v, g, b, _batch(lens, [3], [0]), s, heads, 2, d, d, unit_eps=1e-6, q_scale=0.25, beta_sigmoid=True).view(100, heads, d)
+    clean = call(clean_state)
+    bad = float("nan")
+    if where == "value":
+        v[at, d + 7] = bad
+    elif where == "huge value":
+        v[at, d + 7] = 1e35
+    elif where == "key":
+        k[at, d + 7] = bad
+    elif where == "strength":
+        b[at, 1] = bad
+    elif where == "decay":
+        g[at, 1] = bad
+    else:
+        state.view(1, heads, d, d)[0, 1, 7, 3] = bad
+    got = call(state)
+    assert torch.equal(got[:, 0], clean[:, 0]) and torch.equal(state[:, 0], clean_state[:, 0])
+    from_ = 0 if where == "state" else at
+    if where != "state":        # (the chunk of the bad number is computed token by token: other sums, the same bound)
+        assert torch.equal(got[:32, 1], clean[:32, 1])
+        assert _rel(got[32:at, 1], clean[32:at, 1].double().cpu()) < 1e-6
+    if where in ("value", "state"):
+        assert got[from_ + 1:, 1, 7].isnan().all()
+        others = [i for i in range(d) if i != 7]
+        assert _rel(got[:, 1, others], clean[:, 1, others].double().cpu()) < 1e-6
+    elif where == "huge value":
+        (S64,) = (S0.double().cpu(),)
+        want, _ = _delta64(q, k, v, g, b, S64, lens, [3], heads, 2, d, d, True)
+        assert _rel(got, want) < 1e-6
+    else:
+        assert got[at + 1:, 1].isnan().all()
+
+
 @pytest.mark.parametrize("T,W,E,top,F,gated,skew", [(300, 128, 16, 4, 64, False, False), (1500, 256, 8, 2, 136, True, False), (513, 72, 5, 1, 40, False, True),
                                                     (1024, 64, 256, 8, 32, True, False), (700, 64, 3, 3, 264, False, False), (1, 64, 8, 2, 64, False, False)])
 def test_experts_sorted_on_the_device(T, W, E, top, F, gated, skew):
