@@ -229,11 +229,23 @@ __device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, uint32_t parity) {
       : "memory");
   return ok != 0;
 }
-__device__ __forceinline__ void mbar_wait(uint64_t* bar, uint32_t parity, int tag = 0) {
-  SpinGuard g;
-  while (!mbar_try_wait(bar, parity)) {
-    if (!g.ok()) spin_timeout_trap("mbarrier wait", tag, (int)parity);
+// The loop of a wait stands outside of the kernels: a warp that finds its phase completed goes on after 45 clocks (150 beside eight busy warps) where
+// the loop in place took 56 (150 to 285), and one that waits goes on 83 clocks after the arrival (270) and not 137 (441).
+static __device__ __noinline__ void mbar_wait_loop(uint32_t bar, uint32_t parity, int tag) {
+  const uint64_t t0 = globaltimer_ns();
+  for (;;) {
+    uint32_t n = 0, ok;
+    do {
+      asm volatile(
+          "{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}"
+          : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
+    } while (!ok && ++n < 16384);
+    if (ok) return;
+    if (globaltimer_ns() - t0 > LLMSS_SPIN_TIMEOUT_NS) spin_timeout_trap("mbarrier wait", tag, (int)parity);
   }
+}
+__device__ __forceinline__ void mbar_wait(uint64_t* bar, uint32_t parity, int tag = 0) {
+  if (!mbar_try_wait(bar, parity)) mbar_wait_loop(smem_u32(bar), parity, tag);
 }
 
 // One lane of a converged warp.  Issuing tcgen05 / TMA instructions under this predicate (instead of a

@@ -142,8 +142,7 @@ __global__ void __launch_bounds__(kThreads, 1) delta_chunk_kernel(DeltaArgs a) {
   const int h = blockIdx.y, hk = h / a.rep, dk = a.dk;
   const int j0 = blockIdx.z * VL, nj = min(VL, a.dv - j0);
   const int nch = (ql + C - 1) / C;
-  Patience quit;
-  quit.quit = &sm.quit;
+  int* quit = &sm.quit;
 
   if (warp == 15) {
     tmem_alloc(&sm.tmem, 512);

@@ -117,26 +117,23 @@ __device__ __forceinline__ void umma_ss(uint32_t d, uint32_t a_lo, uint32_t b_lo
                "tcgen05.mma.cta_group::1.kind::f16 [%0], a, b, %3, p;\n\t}" ::"r"(d), "r"(a_lo), "r"(b_lo), "r"(id), "r"(acc), "r"(kDescHi) : "memory");
 }
 
-// Waits a bounded number of attempts.  A warp whose wait runs out waits for nothing any more (`patience` is its own) and says so; the results are
-// marked at the end.  Written out as a loop of two instructions: with a loop around mbar_try_wait a wait for what has long arrived took 145 clocks
-// and not 55 to 110, and a chunk of these kernels has a dozen of them in its chain.
-struct Patience {
-  uint32_t left = 1u << 22;
-  int* quit;
-};
-__device__ __forceinline__ void wait_bar(uint64_t* bar, uint32_t parity, Patience& w) {
-  uint32_t n;
-  asm volatile(
-      "{\n\t.reg .pred p, q;\n\tmov.u32 %0, 0;\n\t"
-      "WAIT:\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t@p bra DONE;\n\t"
-      "add.u32 %0, %0, 1;\n\tsetp.lt.u32 q, %0, %3;\n\t@q bra WAIT;\n\tDONE:\n\t}"
-      : "=&r"(n)
-      : "r"(smem_u32(bar)), "r"(parity & 1), "r"(w.left)
-      : "memory");
-  if (n >= w.left) {
-    *w.quit = 1;
-    w.left = 1;
+// mbar_wait for kernels that end by themselves: a wait of more than LLMSS_SPIN_TIMEOUT_NS sets *quit (shared memory), and waits that find it set
+// end; the results are marked then
+static __device__ __noinline__ void wait_bar_loop(uint32_t bar, uint32_t parity, volatile int* quit) {
+  const uint64_t t0 = globaltimer_ns();
+  for (;;) {
+    uint32_t n = 0, ok;
+    do {
+      asm volatile(
+          "{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}"
+          : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
+    } while (!ok && ++n < 4096);
+    if (ok || *quit) return;
+    if (globaltimer_ns() - t0 > LLMSS_SPIN_TIMEOUT_NS) *quit = 1;
   }
+}
+__device__ __forceinline__ void wait_bar(uint64_t* bar, uint32_t parity, int* quit) {
+  if (!mbar_try_wait(bar, parity & 1)) wait_bar_loop(smem_u32(bar), parity & 1, quit);
 }
 // arrival of a warp whose lanes have written shared memory or read or written tensor memory
 __device__ __forceinline__ void arrive_warp(uint64_t* bar) {
