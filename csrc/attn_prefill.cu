@@ -6,10 +6,11 @@
 // materialises S^2 data:
 //
 //   one CTA = 128 queries of one (sequence, q head); it walks the causal range of KV tiles.
-//   warp 0      TMA producer: Q once, then K_j / V_j tiles (2-stage ring), 128B-swizzled
+//   warp 0      TMA producer: Q once, then K_j / V_j tiles (2-stage rings, keys a tile ahead of values), 128B-swizzled
 //   warp 1      issues  S_j = Q K_j^T  (A,B K-major) -> TMEM [128 x BN] fp32, double-buffered: S runs up
-//               to two tiles ahead of the softmax (gated only by "softmax has copied S out of TMEM")
-//   warp 6      issues  O += P_j V_j   (B = V, MN-major) -> TMEM [128 x D] fp32, as soon as P_j is published
+//               to two tiles ahead of the softmax (D = 256: gated only by "softmax has copied S out of TMEM"), and with P in
+//               tensor memory (D <= 128) also the other product: P_j V_j and, over P_j, S_{j+2} back to back
+//   warp 6      D = 256: issues  O += P_j V_j   (B = V, MN-major) -> TMEM [128 x D] fp32, as soon as P_j is published
 //   warps 2-5   one thread per query row: tcgen05.ld its S row, scale + causal mask, online softmax in
 //               fp32 (no shuffles: the row is thread-private), write P_j (bf16/fp16) into one of two
 //               shared-memory buffers in the UMMA K-major swizzled layout.  The running max is lazy: it
@@ -28,6 +29,13 @@
 // row (again TMA's fill: the box starts at a shifted column), so ONE MMA per tile forms the scores of both maps from one
 // read of K and V.  The epilogue hands the second map's rows over through shared memory, subtracts, divides by the root mean
 // square over the head and stores the 16-bit result: the two maps' outputs never leave the SM.
+//
+// What bounds it (D = 128, 8 prompts of 576 .. 1472 tokens, 32 heads): neither the products (the tensor pipe is about half busy; with a quarter of
+// them the kernel takes 106 us instead of 118) nor the exponentials (without them 110), but the hand-overs of a 64-key tile between warps, each 100
+// to 300 clocks beside busy warps, and the 4000 clocks before a CTA's first tile.  One issuing warp instead of two that wait for one
+// another, descriptors of two additions, keys copied a tile ahead and the copies started before tensor memory is there: 119 -> 113 us
+// (under the power cap 138 -> 131).  Tried and slower: 128-key tiles with one S buffer (135 -> 152), two teams of softmax warps on
+// alternate tiles (141 -> 157), the heaviest query tiles of all heads first (120 -> 133: keys and values leave L2).
 #include "common.cuh"
 
 #include <cuda.h>
@@ -44,7 +52,6 @@
 namespace {
 
 constexpr int BM = 128;  // queries per CTA
-constexpr int kThreads = 224;
 
 // D = 256: one fat CTA per SM (64-key tiles, P double-buffered).  D = 128 / 64: 64-key tiles and ONE P buffer
 // shrink the CTA to <= 112 KB of shared memory and 256 TMEM columns, so TWO CTAs share an SM: eight softmax
@@ -61,6 +68,7 @@ struct PCfg {
   // too, for free; the QK of tile j+2 then has to wait for PV_j instead of for "S_j is in registers".
   static constexpr bool P_TMEM = (D < 256) && (LLMSS_PREFILL_P_TMEM != 0);
   static constexpr int P_BUFS = P_TMEM ? 0 : ((D >= 256) ? 2 : 1);
+  static constexpr int THREADS = P_TMEM ? 192 : 224;          // one warp issues both products where P lies in tensor memory
   static constexpr int MIN_CTAS = (D >= 256) ? 1 : 2;        // CTAs per SM the launch bounds ask for
   static constexpr int FMA_EXP_EVERY = (D >= 256) ? 0 : LLMSS_PREFILL_FMA_EXP_EVERY;  // every n-th PAIR computes one of its two exps on the FMA pipe (0 = none)
   static constexpr int Q_BYTES = BM * D * 2;
@@ -153,15 +161,18 @@ __device__ __forceinline__ float ex2_fma(float x) {
   return __int_as_float(__float_as_int(p) + (n << 23));
 }
 
-// D[tmem] (+)= A[tmem] * B[smem desc]: the A operand (M x 16, 16-bit, two K elements per 32-bit column, row m in
-// lane m) is read from tensor memory.
-__device__ __forceinline__ void umma_f16_ts(uint32_t tmem_d, uint32_t tmem_a, uint64_t desc_b, uint32_t idesc, uint32_t accumulate) {
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}" ::"r"(tmem_d),
-      "r"(tmem_a), "l"(desc_b), "r"(idesc), "r"(accumulate)
-      : "memory");
+// Products from the descriptors' lower words (the upper word is the same for all tiles of 128-byte swizzled rows): two additions a product for the
+// warp that issues them, where descriptors put together per product took it 100 clocks beside eight softmax warps.
+constexpr uint32_t kDescHi = 0x40004040u;
+__device__ __forceinline__ uint32_t desc_lo(uint32_t addr, uint32_t lbo = 16) { return ((addr & 0x3FFFFu) >> 4) | ((lbo >> 4) << 16); }
+__device__ __forceinline__ void umma_ss_lo(uint32_t d, uint32_t a_lo, uint32_t b_lo, uint32_t id, uint32_t acc) {
+  asm volatile("{\n\t.reg .pred p;\n\t.reg .b64 a, b;\n\tsetp.ne.b32 p, %4, 0;\n\tmov.b64 a, {%1, %5};\n\tmov.b64 b, {%2, %5};\n\t"
+               "tcgen05.mma.cta_group::1.kind::f16 [%0], a, b, %3, p;\n\t}" ::"r"(d), "r"(a_lo), "r"(b_lo), "r"(id), "r"(acc), "r"(kDescHi) : "memory");
+}
+// the A operand (M x 16, 16-bit, two K elements per 32-bit column, row m in lane m) from tensor memory
+__device__ __forceinline__ void umma_ts_lo(uint32_t d, uint32_t a, uint32_t b_lo, uint32_t id, uint32_t acc) {
+  asm volatile("{\n\t.reg .pred p;\n\t.reg .b64 b;\n\tsetp.ne.b32 p, %4, 0;\n\tmov.b64 b, {%2, %5};\n\t"
+               "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], b, %3, p;\n\t}" ::"r"(d), "r"(a), "r"(b_lo), "r"(id), "r"(acc), "r"(kDescHi) : "memory");
 }
 
 template <typename T>
@@ -182,7 +193,7 @@ __device__ __forceinline__ uint32_t pack2(float a, float b) {
 //                chunk, addressed through the block table), which already holds this step's keys (rope_kv_write
 //                runs first).  Query i of a sequence sits at position ctx + i, ctx = seq_len - q_len.
 template <typename T, int D, bool PAGED, bool BIAS = false, int MAPS = 0>
-__global__ void __launch_bounds__(kThreads, PCfg<D>::MIN_CTAS)
+__global__ void __launch_bounds__(PCfg<D>::THREADS, PCfg<D>::MIN_CTAS)
 attn_prefill_kernel(const __grid_constant__ CUtensorMap tmap, const __grid_constant__ CUtensorMap tmap_k,
                     const __grid_constant__ CUtensorMap tmap_v, const __grid_constant__ PArgs a) {
   using C = PCfg<D>;
@@ -217,23 +228,6 @@ attn_prefill_kernel(const __grid_constant__ CUtensorMap tmap, const __grid_const
   const int seq = blockIdx.z, head = blockIdx.y;
   pdl_launch_dependents();
   pdl_wait();
-  const int seq_start = a.cu_seqlens[seq];
-  const int len = a.cu_seqlens[seq + 1] - seq_start;
-  // heaviest (longest causal range) query tiles are scheduled first
-  const int q0 = (gridDim.x - 1 - blockIdx.x) * QT;  // first query (position within the sequence) of this CTA
-  if (q0 >= len) return;           // uniform for the whole CTA
-  const int kvh = head / (a.hq / a.hkv);
-  const int ctx = PAGED ? a.seq_lens[seq] - len : 0;   // tokens already in the cache before this step's queries
-  const int kv_end = min(ctx + len, ctx + q0 + QT);     // causal: keys [0, kv_end)
-  // window: the walk takes tiles 0 .. n_first - 1 (kept first tokens), then t_first .. (the first row's window on)
-  int t_first = 0, n_first = 0;
-  if constexpr (SPAN) {
-    t_first = first_visible(ctx + q0, a.window, a.chunk) / BN;
-    n_first = min((a.keep + BN - 1) / BN, t_first);
-  }
-  const int n_tiles = (kv_end + BN - 1) / BN - t_first + n_first;
-  auto key_tile = [&](int j) { return SPAN ? (j < n_first ? j : j - n_first + t_first) : j; };
-
   if (warp == 0 && lane == 0) {
     tma_prefetch_desc(&tmap);
     if (PAGED) {
@@ -255,14 +249,34 @@ attn_prefill_kernel(const __grid_constant__ CUtensorMap tmap, const __grid_const
     }
     fence_mbar_init();
   }
+  __syncwarp();
+  const int seq_start = a.cu_seqlens[seq];
+  const int len = a.cu_seqlens[seq + 1] - seq_start;
+  // heaviest (longest causal range) query tiles are scheduled first
+  const int q0 = (gridDim.x - 1 - blockIdx.x) * QT;  // first query (position within the sequence) of this CTA
+  if (q0 >= len) return;           // uniform for the whole CTA
+  const int kvh = head / (a.hq / a.hkv);
+  const int ctx = PAGED ? a.seq_lens[seq] - len : 0;   // tokens already in the cache before this step's queries
+  const int kv_end = min(ctx + len, ctx + q0 + QT);     // causal: keys [0, kv_end)
+  // window: the walk takes tiles 0 .. n_first - 1 (kept first tokens), then t_first .. (the first row's window on)
+  int t_first = 0, n_first = 0;
+  if constexpr (SPAN) {
+    t_first = first_visible(ctx + q0, a.window, a.chunk) / BN;
+    n_first = min((a.keep + BN - 1) / BN, t_first);
+  }
+  const int n_tiles = (kv_end + BN - 1) / BN - t_first + n_first;
+  auto key_tile = [&](int j) { return SPAN ? (j < n_first ? j : j - n_first + t_first) : j; };
+
   if (warp == 1) {
     tmem_alloc(tmem_slot, C::TMEM_COLS);
     tmem_relinquish();
   }
+  // the copying warp has set the barriers up itself and needs no tensor memory: it only announces them
   tcgen05_fence_before();
-  __syncthreads();
+  if (warp == 0) asm volatile("bar.arrive 15, %0;" ::"n"(C::THREADS) : "memory");
+  else asm volatile("bar.sync 15, %0;" ::"n"(C::THREADS) : "memory");
   tcgen05_fence_after();
-  const uint32_t tmem_base = *tmem_slot;
+  const uint32_t tmem_base = warp == 0 ? 0 : *tmem_slot;
   const uint32_t tS = tmem_base, tO = tmem_base + 2 * BN;  // S buffer b lives at tS + b * BN
 
   if (warp == 0) {
@@ -295,13 +309,14 @@ attn_prefill_kernel(const __grid_constant__ CUtensorMap tmap, const __grid_const
                         seq_start + q0 + h * BN, pol);
       }
       __syncwarp();
-      int stage = 0;
-      uint32_t phase = 0;
-      for (int j = 0; j < n_tiles; ++j) {
+      // keys run one tile ahead of values: S_{j+1} is formed while P_j is, and a value tile's place is free only behind P V
+      static_assert(C::KV_STAGES == 2, "stages by the tile's last bit");
+      auto keys = [&](int j) {
         const int row = seq_start + j * BN;
-        mbar_wait(&bar_kempty[stage], phase ^ 1, 50);
+        (void)row;
+        mbar_wait(&bar_kempty[j & 1], ((j >> 1) & 1) ^ 1, 50);
         if (elect_one()) {
-          mbar_arrive_expect_tx(&bar_kfull[stage], k_tx);
+          mbar_arrive_expect_tx(&bar_kfull[j & 1], k_tx);
           if constexpr (PAGED) {
             // BN / page boxes per 64-column chunk; 8-row multiples keep the 128B-swizzle pattern contiguous
             const int* bt = a.block_tables + (int64_t)seq * a.max_blocks;
@@ -310,18 +325,22 @@ attn_prefill_kernel(const __grid_constant__ CUtensorMap tmap, const __grid_const
               const int crow = (bt[bi] * a.hkv + kvh) * a.page;
 #pragma unroll
               for (int c = 0; c < DSUB; ++c)
-                if (!SPAN || c * 64 < a.dkp) tma_load_2d(sK + stage * C::K_BYTES + c * (BN * 128) + pg * a.page * 128, &tmap_k, &bar_kfull[stage], c * 64, crow, pol);
+                if (!SPAN || c * 64 < a.dkp) tma_load_2d(sK + (j & 1) * C::K_BYTES + c * (BN * 128) + pg * a.page * 128, &tmap_k, &bar_kfull[j & 1], c * 64, crow, pol);
             }
           } else {
 #pragma unroll
             for (int c = 0; c < DSUB; ++c)
-              tma_load_2d(sK + stage * C::K_BYTES + c * (BN * 128), &tmap, &bar_kfull[stage], a.k_col + kvh * D + c * 64, row, pol);
+              tma_load_2d(sK + (j & 1) * C::K_BYTES + c * (BN * 128), &tmap, &bar_kfull[j & 1], a.k_col + kvh * D + c * 64, row, pol);
           }
         }
         __syncwarp();
-        mbar_wait(&bar_vempty[stage], phase ^ 1, 51);
+      };
+      auto values = [&](int j) {
+        const int row = seq_start + j * BN;
+        (void)row;
+        mbar_wait(&bar_vempty[j & 1], ((j >> 1) & 1) ^ 1, 51);
         if (elect_one()) {
-          mbar_arrive_expect_tx(&bar_vfull[stage], v_tx);
+          mbar_arrive_expect_tx(&bar_vfull[j & 1], v_tx);
           if constexpr (PAGED) {
             const int* bt = a.block_tables + (int64_t)seq * a.max_blocks;
             for (int pg = 0; pg < BN / a.page; ++pg) {
@@ -329,19 +348,68 @@ attn_prefill_kernel(const __grid_constant__ CUtensorMap tmap, const __grid_const
               const int crow = (bt[bi] * a.hkv + kvh) * a.page;
 #pragma unroll
               for (int c = 0; c < DSUB; ++c)
-                if (!SPAN || c * 64 < a.dv) tma_load_2d(sV + stage * C::V_BYTES + c * (BN * 128) + pg * a.page * 128, &tmap_v, &bar_vfull[stage], c * 64, crow, pol);
+                if (!SPAN || c * 64 < a.dv) tma_load_2d(sV + (j & 1) * C::V_BYTES + c * (BN * 128) + pg * a.page * 128, &tmap_v, &bar_vfull[j & 1], c * 64, crow, pol);
             }
           } else {
 #pragma unroll
             for (int c = 0; c < DSUB; ++c)
-              tma_load_2d(sV + stage * C::V_BYTES + c * (BN * 128), &tmap, &bar_vfull[stage], a.v_col + kvh * D + c * 64, row, pol);
+              tma_load_2d(sV + (j & 1) * C::V_BYTES + c * (BN * 128), &tmap, &bar_vfull[j & 1], a.v_col + kvh * D + c * 64, row, pol);
           }
         }
         __syncwarp();
-        if (++stage == C::KV_STAGES) { stage = 0; phase ^= 1; }
+      };
+      keys(0);
+      for (int j = 0; j < n_tiles; ++j) {
+        if (j + 1 < n_tiles) keys(j + 1);
+        values(j);
       }
     }
-  } else if (warp == 1) {
+  } else if (C::P_TMEM && warp == 1) {
+    // ===================== both products from one warp (whole warp runs the loop, one elected lane issues) =================
+    // S_{j+2} goes over P_j: issued behind PV_j by the same thread it runs behind it, and no barrier stands between the two
+    const int fmt = a.dtype == LLMSS_BF16 ? 1 : 0;
+    const uint32_t idesc_s = idesc_f16(fmt, BM, BN, 0);  // S = Q K^T : both operands K-major
+    const uint32_t idesc_o = idesc_f16(fmt, BM, SPAN ? (a.dv + 15) / 16 * 16 : D, 1);   // O += P V  : B (= V) is MN-major
+    const uint32_t q_lo = desc_lo(smem_u32(sQ)), k_base = desc_lo(smem_u32(sK)), v_base = desc_lo(smem_u32(sV), BN * 128);
+    auto scores = [&](int j) {
+      tcgen05_fence_after();
+      const uint32_t k_lo = k_base + (j & 1) * (C::K_BYTES / 16), d = tS + (j & 1) * BN;
+      if (elect_one()) {
+#pragma unroll
+        for (int c = 0; c < DSUB; ++c)
+#pragma unroll
+          for (int k = 0; k < 4; ++k)
+            if (!SPAN || c * 64 + k * 16 < a.dkp)
+              umma_ss_lo(d, q_lo + (c * (BM * 128) + k * 32) / 16, k_lo + (c * (BN * 128) + k * 32) / 16, idesc_s, (c | k) ? 1u : 0u);
+        umma_commit(&bar_s[j & 1]);
+        umma_commit(&bar_kempty[j & 1]);
+      }
+      __syncwarp();
+    };
+    mbar_wait(bar_q, 0, 60);
+    for (int j = 0; j < min(n_tiles, 2); ++j) {
+      mbar_wait(&bar_kfull[j], 0, 61);
+      scores(j);
+    }
+    for (int j = 0; j < n_tiles; ++j) {
+      mbar_wait(&bar_vfull[j & 1], (j >> 1) & 1, 63);
+      mbar_wait(&bar_p[j & 1], (j >> 1) & 1, 62);
+      tcgen05_fence_after();
+      const uint32_t v_lo = v_base + (j & 1) * (C::V_BYTES / 16), p = tS + (j & 1) * BN;
+      if (elect_one()) {
+#pragma unroll
+        for (int k = 0; k < BN / 16; ++k)      // 16 keys = 8 packed columns per step, P_j sits at the start of S buffer j & 1
+          umma_ts_lo(tO, p + k * 8, v_lo + k * 128, idesc_o, (j > 0 || k > 0) ? 1u : 0u);
+        umma_commit(&bar_o[j & 1]);
+        umma_commit(&bar_vempty[j & 1]);
+      }
+      __syncwarp();
+      if (j + 2 < n_tiles) {
+        mbar_wait(&bar_kfull[j & 1], ((j + 2) >> 1) & 1, 61);
+        scores(j + 2);
+      }
+    }
+  } else if (!C::P_TMEM && warp == 1) {
     // ===================== QK issuer (whole warp runs the loop, one elected lane issues) =================
     const int fmt = a.dtype == LLMSS_BF16 ? 1 : 0;
     const uint32_t idesc_s = idesc_f16(fmt, BM, BN, 0);  // S = Q K^T : both operands K-major
@@ -350,11 +418,7 @@ attn_prefill_kernel(const __grid_constant__ CUtensorMap tmap, const __grid_const
     int stage = 0;
     uint32_t phase = 0;
     for (int j = 0; j < n_tiles; ++j) {
-      if constexpr (C::P_TMEM) {
-        if (j >= 2) mbar_wait(&bar_o[j & 1], ((j >> 1) & 1) ^ 1, 64);    // PV_{j-2} has read P_{j-2} out of this S buffer
-      } else {
-        if (j >= 2) mbar_wait(&bar_sfree[j & 1], ((j >> 1) & 1) ^ 1, 64);  // softmax_{j-2} has left this S buffer
-      }
+      if (j >= 2) mbar_wait(&bar_sfree[j & 1], ((j >> 1) & 1) ^ 1, 64);  // softmax_{j-2} has left this S buffer
       mbar_wait(&bar_kfull[stage], phase, 61);
       tcgen05_fence_after();
       const uint32_t k_addr = k_base + stage * C::K_BYTES;
@@ -371,7 +435,7 @@ attn_prefill_kernel(const __grid_constant__ CUtensorMap tmap, const __grid_const
       __syncwarp();
       if (++stage == C::KV_STAGES) { stage = 0; phase ^= 1; }
     }
-  } else if (warp == 6) {
+  } else if (!C::P_TMEM && warp == 6) {
     // ===================== PV issuer =====================
     const int fmt = a.dtype == LLMSS_BF16 ? 1 : 0;
     const uint32_t idesc_o = idesc_f16(fmt, BM, SPAN ? (a.dv + 15) / 16 * 16 : D, 1);   // O += P V  : B (= V) is MN-major
@@ -388,22 +452,17 @@ attn_prefill_kernel(const __grid_constant__ CUtensorMap tmap, const __grid_const
 #pragma unroll
         for (int c = 0; c < NSUB; ++c)
 #pragma unroll
-          for (int k = 0; k < 4; ++k) {
-            if constexpr (C::P_TMEM)   // 16 keys = 8 packed columns per step, P_j sits at the start of S buffer j & 1
-              umma_f16_ts(tO, tS + (j & 1) * BN + (c * 4 + k) * 8, umma_desc_mn_sw128(v_addr + (c * 64 + k * 16) * 128, BN * 128),
-                          idesc_o, (j > 0 || c > 0 || k > 0) ? 1u : 0u);
-            else
-              umma_f16_ss(tO, umma_desc_k_sw128(pj + c * (BM * 128) + k * 32),
-                          umma_desc_mn_sw128(v_addr + (c * 64 + k * 16) * 128, BN * 128), idesc_o,
-                          (j > 0 || c > 0 || k > 0) ? 1u : 0u);
-          }
+          for (int k = 0; k < 4; ++k)
+            umma_f16_ss(tO, umma_desc_k_sw128(pj + c * (BM * 128) + k * 32),
+                        umma_desc_mn_sw128(v_addr + (c * 64 + k * 16) * 128, BN * 128), idesc_o,
+                        (j > 0 || c > 0 || k > 0) ? 1u : 0u);
         umma_commit(&bar_o[j & 1]);
         umma_commit(&bar_vempty[stage]);
       }
       __syncwarp();
       if (++stage == C::KV_STAGES) { stage = 0; phase ^= 1; }
     }
-  } else if (warp < 6) {
+  } else if (warp >= 2 && warp < 6) {
     // ===================== softmax / correction / epilogue: one thread per query row =====================
     const int quarter = warp & 3;
     const int row = quarter * 32 + lane;         // query row within the tile == TMEM lane
@@ -433,9 +492,11 @@ attn_prefill_kernel(const __grid_constant__ CUtensorMap tmap, const __grid_const
 #pragma unroll
           for (int i = 0; i < 32; ++i) sc[c * 32 + i] = __uint_as_float(r[c][i]);
       }
-      tcgen05_fence_before();
-      __syncwarp();
-      if (lane == 0) mbar_arrive(&bar_sfree[j & 1]);  // S_j is in registers: the buffer can take QK_{j+2}
+      if constexpr (!C::P_TMEM) {
+        tcgen05_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&bar_sfree[j & 1]);  // S_j is in registers: the buffer can take QK_{j+2}
+      }
       if (BIAS && a.bias != nullptr) {
         const float* bt = a.bias + (int64_t)head * a.n_dist;
         const int dmax = a.n_dist - 1, d0 = qpos - kbase;   // distance from this row to the tile's first key
@@ -536,7 +597,7 @@ attn_prefill_kernel(const __grid_constant__ CUtensorMap tmap, const __grid_const
       }
       l_run = l_run * alpha + l_tile;
       tcgen05_fence_before();
-      fence_proxy_async_smem();  // generic-proxy writes of P must be visible to the tensor-core (async) proxy
+      if constexpr (!C::P_TMEM) fence_proxy_async_smem();  // generic-proxy writes of P must be visible to the tensor-core (async) proxy
       __syncwarp();
       if (lane == 0) mbar_arrive(&bar_p[j & 1]);
     }
@@ -644,7 +705,7 @@ int launch_prefill(const CUtensorMap& tm, const CUtensorMap& tk, const CUtensorM
   auto kern = attn_prefill_kernel<T, D, PAGED, BIAS>;
   LLMSS_CHECK_CUDA(configured.ensure(kern, C::SMEM_BYTES));
   dim3 grid((max_seqlen + BM - 1) / BM, a.hq, num_seqs);
-  LLMSS_CHECK_CUDA(launch_pdl(kern, grid, dim3(kThreads), (size_t)C::SMEM_BYTES, stream, tm, tk, tv, a));
+  LLMSS_CHECK_CUDA(launch_pdl(kern, grid, dim3(C::THREADS), (size_t)C::SMEM_BYTES, stream, tm, tk, tv, a));
   return 0;
 }
 
@@ -658,7 +719,7 @@ int launch_span(const CUtensorMap& tm, const CUtensorMap& tk, const CUtensorMap&
   constexpr int QT = MAPS == 2 ? BM / 2 : BM;
   dim3 grid((max_q + QT - 1) / QT, a.hq, num_seqs);
   LLMSS_REQUIRE(grid.y <= 65535 && grid.z <= 65535, "attn_prefill_span: grid too large");
-  LLMSS_CHECK_CUDA(launch_pdl(kern, grid, dim3(kThreads), (size_t)C::SMEM_BYTES, stream, tm, tk, tv, a));
+  LLMSS_CHECK_CUDA(launch_pdl(kern, grid, dim3(C::THREADS), (size_t)C::SMEM_BYTES, stream, tm, tk, tv, a));
   return 0;
 }
 
