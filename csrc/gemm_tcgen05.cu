@@ -1535,7 +1535,9 @@ PFN_encodeTiled get_encode() {
 // Few k-blocks per tile, so the work is moving x in and out once; persistent CTAs keep the next tiles' loads (4 stages of 64
 // columns) and the previous tile's stores in flight around the products.  A tile is 128 features of a head x 256 tokens, heads
 // fastest (the rows of x and out that run together are neighbours).  Both operands are 3-D tensor maps [K, rows, heads]: a head's
-// last k-block and feature tile are zero-filled at its own edge.
+// last k-block and feature tile are zero-filled at its own edge.  A factor per token and head comes by one load a lane and exchanges: 8192 tokens of
+// 32 heads 58 -> 46 us, 2048 21 -> 17 (a load per token and warp stood in front of every 32 stores; without factors 31 and 14).  Tokens as
+// lanes, with 16-byte stores that lie a row apart, were slower without factors (31 -> 41 us).
 // Against warp-level MMAs on k slices staged by hand (bf16, B200): 8192 tokens, 32 heads of 128 x 128 127 -> 33 us (134 MB: 21 at the copy
 // rate), 16 heads 65 -> 23, 128 -> 192 features 113 -> 32; 2048 tokens, 32 heads 36 -> 16; up to 400 tokens both are under the launch.
 // ======================================================================================
@@ -1638,15 +1640,24 @@ gemm_heads_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_const
       const int n = tn * BM + f, m0 = tm * BN;
       const uint32_t t_addr = tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(as * BN);
       const float* sp = a.scale != nullptr ? a.scale + (int64_t)m0 * a.lds + h * a.ssh + (n < a.N ? n : 0) * a.ssn : nullptr;
+      // a factor per token and head (the usual one): a lane loads one of 32 tokens', a chunk ahead, and the warp exchanges them
+      const bool each = sp != nullptr && a.ssn != 0;
+      auto factor = [&](int cg) { return m0 + cg * 8 + lane < a.M ? __ldg(sp + (int64_t)(cg * 8 + lane) * a.lds) : 0.f; };
+      float next = sp != nullptr && !each ? factor(0) : 0.f;
       mbar_wait(&tfull_bar[as], aphase, 73);
       tcgen05_fence_after();
 #pragma unroll 1
       for (int cg0 = 0; cg0 < NG; cg0 += 4) {
         const int m = m0 + cg0 * 8, rows = a.M - m;      // valid token rows of this chunk (may be <= 0 or >= 32)
         float sc[32];
-        if (sp != nullptr) {
+        if (each) {
 #pragma unroll
           for (int j = 0; j < 32; ++j) sc[j] = j < rows ? __ldg(sp + (int64_t)(cg0 * 8 + j) * a.lds) : 0.f;
+        } else if (sp != nullptr) {
+          const float mine = next;
+          if (cg0 + 4 < NG) next = factor(cg0 + 4);
+#pragma unroll
+          for (int j = 0; j < 32; ++j) sc[j] = __shfl_sync(0xffffffffu, mine, j);
         }
         uint32_t q[32];
         tmem_ld_32x32b_x32(t_addr + cg0 * 8, q);
