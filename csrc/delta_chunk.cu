@@ -541,11 +541,15 @@ __global__ void __launch_bounds__(kThreads, 1) delta_chunk_kernel(DeltaArgs a) {
 
 // ---- first launch: 128 threads, a block per (chunk, key head, sequence)
 struct PrepSmem {
-  float k[C][KD + 4], q[C][KD + 4], g[2 * C][C + 4];         // rows of k and q; scores of both with the keys
+  union {
+    float k[C][KD + 4];                                      // rows of k;
+    float L[2][C * (C + 4)];                                 // once the scores are there: L of two heads
+  };
+  float q[C][KD + 4], g[2 * C][C + 4];                       // rows of q; scores of both with the keys
   float kf[C], qf[C], ks[C], qs[C];                          // norm factors, scales
-  float L[2][C * (C + 4)], bad[2];
+  float bad[2];
 };
-__global__ void __launch_bounds__(128) delta_prep_kernel(DeltaArgs a) {
+__global__ void __launch_bounds__(128, 5) delta_prep_kernel(DeltaArgs a) {
   extern __shared__ __align__(16) uint8_t smem_raw[];
   PrepSmem& sm = *reinterpret_cast<PrepSmem*>(smem_raw);
   const int b = blockIdx.z, hk = blockIdx.y, c = blockIdx.x;

@@ -889,13 +889,17 @@ def _delta_over_chunks(T, B, max_q, heads, dk, dv):
     us.  Over chunks a block carries one (sequence, head, 128 columns) through its chunks at 6 us each, one block per SM, 9 us to start and end a block, 13 us for
     the launches, and the chunks' own part costs 0.55 ns per token and head; token by token the longest portion's chain takes 0.4 us a token, and a full GPU
     3.2e12 state elements a second.  Measured (chunks / tokens): 16 heads of 128 x 128, prompts of 576 .. 1472: 362 / 907, 8 x 1024: 280 / 635,
-    8 x 64: 39 / 47, 8 x 48: 38 / 37, 32 x 48: 103 / 114, one of 64: 33 / 31, one of 1500: 266 / 604; 32 heads of 64 x 64, 8 x 1024: 610 / 381.
+    8 x 64: 39 / 47, 8 x 48: 38 / 37, 32 x 48: 103 / 114, one of 64: 33 / 31, one of 1500: 266 / 604; 32 heads of 64 x 64, 8 x 1024: 610 / 381;
+    32 heads of 128 x 128, 23 portions of 16 .. 46: 148 / 126, 31 of 20 .. 56: 197 / 192, 7 of 52: 64 / 75.
     Counts that a graph's capture fixes decide, nothing on the device."""
     if max_q < 32 or dk > 128 or dk % 4 or B > 65535 or heads > 65535:
         return False
     blocks = B * heads * -(-dv // 128)
+    arithmetic = T * heads * dk * dv / 3.2e6
     chunks = max(6.0 * -(-max_q // 32), -(-blocks // 148) * (6.0 * -(-T // (32 * B)) + 9.0) - 9.0) + 22.0 + 0.55e-3 * T * heads
-    return chunks < max(0.4 * max_q, T * heads * dk * dv / 3.2e6) + 5.0
+    if T < 48 * B:          # some of the portions are below a chunk, and run token by token behind the others
+        chunks += 0.5 * arithmetic
+    return chunks < max(0.4 * max_q, arithmetic) + 5.0
 
 
 def delta_scan(q, k, v, log_decay, beta, batch, state, heads, qk_heads, dk, dv, unit_eps=None, q_scale=1.0, beta_sigmoid=False):
