@@ -374,7 +374,7 @@ int64_t llmss_delta_scan_chunked_bytes(int T, int B, int heads);
 int llmss_delta_scan_chunked(const float* q, int64_t ldq, const float* k, int64_t ldk, const float* v, int64_t ldv, const float* log_decay,
                      int64_t ldg, const float* beta, int64_t ldb, float* out, float* state, const int* cu_q, const int* seq_lens,
                      const int* slots, int B, int max_q, int heads, int qk_heads, int dk, int dv, float unit_eps, float q_scale,
-                     int beta_sigmoid, llmss_stream_t stream);
+                     int beta_sigmoid, void* scratch, llmss_stream_t stream);
 
 /* ---- rotation by a frequency table, sandwich norms, gated linear recurrence inputs (csrc/rotary.cu) and the general forms they
  * use elsewhere.  freq: n_pairs 64-bit frequencies (the first 2 n_pairs channels of a head rotate, the rest pass); mag multiplies
