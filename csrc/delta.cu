@@ -444,9 +444,11 @@ LLMSS_API int llmss_delta_scan_chunked(const float* q, int64_t ldq, const float*
   if (B <= 0) return 0;
   a.prepared = static_cast<uint8_t*>(scratch);
   a.least = kChunkLeast;
-  const int rc = delta_chunk_launch(a, B, max_q, stream);
-  if (rc != 0 || B == 1) return rc;
-  a.least = 1;
+  if (max_q >= kChunkLeast) {
+    const int rc = delta_chunk_launch(a, B, max_q, stream);
+    if (rc != 0) return rc;
+  }
+  a.least = 1;      // (lengths lie on the device: also behind a single sequence)
   a.below = kChunkLeast;
   return delta_portions(a, B, stream);
 }

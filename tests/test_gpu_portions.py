@@ -111,6 +111,24 @@ def test_delta_over_chunks(dk, dv, heads, qk_heads, unit, decay, monkeypatch):
     assert _rel(state.reshape(len(lens), heads, dv, dk).transpose(2, 3), ends) < bound
 
 
+@pytest.mark.parametrize("n,max_q", [(1, 1), (7, 7), (31, 31), (31, 64), (32, 32), (7, 0)])
+def test_delta_over_chunks_of_one_sequence(n, max_q):
+    """The C entry, one sequence of any length: a short one runs token by token, whatever bound on the lengths the caller names."""
+    from llmss_b200.ops import _lib, cuda_impl as cu
+
+    torch.manual_seed(n)
+    heads, d = 2, 64
+    (q, k, v), b, S0 = _delta_inputs([n], heads, heads, d, d, True)
+    g, batch = -0.3 * torch.rand(n, heads, device="cuda"), _batch([n], [3], [0])
+    state, out = S0.transpose(2, 3).contiguous(), torch.full((n, heads * d), float("nan"), device="cuda")
+    want, ends = _delta64(q, k, v, g, b, S0.double().cpu(), [n], [3], heads, heads, d, d, True)
+    lib, p = _lib.load(), cu._ptr
+    scratch = torch.empty(lib.llmss_delta_scan_chunked_bytes(n, 1, heads), dtype=torch.uint8, device="cuda")
+    _lib.check(lib.llmss_delta_scan_chunked(p(q), q.stride(0), p(k), k.stride(0), p(v), v.stride(0), p(g), heads, p(b), heads, p(out), p(state), p(batch.cu_q),
+                                            p(batch.seq_lens), p(batch.state_slots), 1, max_q, heads, heads, d, d, 1e-6, 0.25, 1, p(scratch), cu._stream()), "chunked")
+    assert _rel(out, want.reshape(n, -1)) < 1e-6 and _rel(state.transpose(2, 3), ends) < 1e-6
+
+
 @pytest.mark.parametrize("where", ["value", "key", "strength", "decay", "state", "huge value"])
 def test_delta_over_chunks_bad_numbers(where, monkeypatch):
     """A value that is no number, or too large to scale, reaches what it reaches token by token: later tokens of its column (value, state) or of
