@@ -74,10 +74,17 @@ __global__ void __launch_bounds__(256) delta_scan_kernel(DeltaArgs a) {
   constexpr int STRIP = KPT + 4, row = R * STRIP, COLS = 2;
   extern __shared__ __align__(16) float sm[];
   const int b = blockIdx.x;
-  const int q0 = a.cu_q[b], ql = a.cu_q[b + 1] - q0, ctx = a.seq_lens[b] - ql, slot = a.slots[b];
-  if (slot < 0 || ctx < 0 || ql < a.least || ql >= a.below) return;
-  const int h = blockIdx.y, hk = h / a.rep;
-  const int j0 = blockIdx.z * a.dvt, nj = min(a.dvt, a.dv - j0);
+  int q0 = a.cu_q[b], ql = a.cu_q[b + 1] - q0, ctx = a.seq_lens[b] - ql;
+  const int slot = a.slots[b], h = blockIdx.y, hk = h / a.rep, j0 = blockIdx.z * a.dvt, nj = min(a.dvt, a.dv - j0);
+  if (slot < 0 || ctx < 0 || ql <= 0) return;
+  if (a.prepared != nullptr && ql >= a.least) {          // what the launch over chunks has left of this sequence (a slice lies in one of its blocks)
+    const uint8_t* first = a.prepared + ((int64_t)(q0 / kDeltaChunk + b) * a.H + h) * LLMSS_DELTA_PREPARED;
+    const int done = reinterpret_cast<const int*>(first + kDeltaDoneAt)[j0 / kDeltaCols];
+    if (done >= ql) return;
+    q0 += done;
+    ql -= done;
+    ctx += done;
+  }
   const int dk = a.dk, nthr = blockDim.x;
   const int r = threadIdx.x % R, c0 = threadIdx.x / R * COLS;          // key strip, first column (inside the slice)
   const int i0 = r * KPT;
@@ -354,11 +361,10 @@ bool delta_args(DeltaArgs& a, const float* q, int64_t ldq, const float* k, int64
   a.out = out; a.state = state; a.cu_q = cu_q; a.seq_lens = seq_lens; a.slots = slots;
   a.H = heads; a.rep = heads / qk_heads; a.dk = dk; a.dv = dv;
   a.unit = unit_eps >= 0.f ? 1 : 0; a.unit_eps = unit_eps >= 0.f ? unit_eps : 0.f; a.q_scale = q_scale; a.beta_sigmoid = beta_sigmoid;
-  a.least = 1; a.below = 0x7fffffff;
   return true;
 }
 
-// token by token: sequences of a.least .. a.below - 1 tokens
+// token by token: all sequences, or what a launch over chunks has left of them
 int delta_portions(DeltaArgs a, int B, cudaStream_t stream) {
   const int dk = a.dk, dv = a.dv;
   // up to 32 key rows per thread, R lanes (a power of two) to a column pair
@@ -368,7 +374,7 @@ int delta_portions(DeltaArgs a, int B, cudaStream_t stream) {
   int threads = (((dv + 1) / 2 * R + 31) / 32) * 32;
   const int most = R <= 4 ? 64 : 256;       // long keys: a stage of q and k is shared by more columns
   threads = threads > most ? most : threads;
-  a.dvt = threads / R * 2;
+  a.dvt = threads / R * 2;                  // (key sizes up to 128: 16 to 128, so that a slice lies within 128 columns)
   const dim3 grid(B, a.H, (dv + a.dvt - 1) / a.dvt);
   LLMSS_REQUIRE(grid.y <= 65535 && grid.z <= 65535, "delta_scan: grid too large");
   a.vec16 = (dk % 4 == 0 && dv % 4 == 0 && a.dvt % 4 == 0 && a.ldq % 4 == 0 && a.ldk % 4 == 0 && a.ldv % 4 == 0 &&
@@ -442,13 +448,12 @@ LLMSS_API int llmss_delta_scan_chunked(const float* q, int64_t ldq, const float*
                 "delta_scan_chunked: key size %d (at most 128, a multiple of 4), rows of q and k on 16-byte lines", dk);
   LLMSS_REQUIRE(B <= 65535 && heads <= 65535 && (dv + 127) / 128 <= 65535, "delta_scan_chunked: grid too large");
   if (B <= 0) return 0;
-  a.prepared = static_cast<uint8_t*>(scratch);
-  a.least = kChunkLeast;
-  if (max_q >= kChunkLeast) {
+  // (lengths lie on the device: the token-by-token launch always follows, also behind a single sequence)
+  if (max_q >= kChunkLeast && dv <= kDeltaDone * kDeltaCols) {
+    a.prepared = static_cast<uint8_t*>(scratch);
+    a.least = kChunkLeast;
     const int rc = delta_chunk_launch(a, B, max_q, stream);
     if (rc != 0) return rc;
   }
-  a.least = 1;      // (lengths lie on the device: also behind a single sequence)
-  a.below = kChunkLeast;
   return delta_portions(a, B, stream);
 }

@@ -17,8 +17,15 @@ struct DeltaArgs {
   float unit_eps, q_scale;
   int unit, beta_sigmoid;
   int vec16;       // q / k / v rows, the key size and the value slices allow 16-byte copies
-  uint8_t* prepared;                     // [T / 32 + sequences][H] x LLMSS_DELTA_PREPARED, on a 16-byte line
-  int least, below;      // sequences of least .. below - 1 tokens are this launch's
+  // Over chunks: [T / 32 + sequences][H] x LLMSS_DELTA_PREPARED, on a 16-byte line (else null).  A sequence of `least` tokens and more goes over chunks until
+  // a chunk that its products cannot take; the record of its first chunk then says how many tokens are done, per 128 value columns, and
+  // the token-by-token launch takes the others.
+  uint8_t* prepared;
+  int least;
 };
 
+constexpr int kDeltaChunk = 32, kDeltaCols = 128, kDeltaDone = 29;       // tokens of a chunk, value columns of a block over chunks, blocks that a record has room for
+
 int delta_chunk_launch(const DeltaArgs& a, int B, int max_q, cudaStream_t stream);
+// where in a record the tokens done lie: behind the tiles and the numbers per token
+constexpr int kDeltaDoneAt = LLMSS_DELTA_PREPARED - 4 * kDeltaDone;

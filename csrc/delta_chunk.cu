@@ -21,11 +21,14 @@
 // Rounding.  Operands are rows scaled and cut into three 16-bit numbers (split16.cuh); their sums are exact in one accumulator, close to it in
 // the other, and meet in one 32-bit addition.  (The state has two parts only: an error of 2^-24 of a column's largest number, once per chunk.)  The
 // state itself is a 32-bit number in a register, rounded once per chunk where it was rounded once per token.  Log decays sum in 64 bits.
-// A chunk that the products cannot take (decays that grow by more than e^0.25 a token, values that are not finite or beyond 2^100, entries
-// of T beyond 2^20) runs token by token in the state's warps, so that a value that is no number reaches what it reaches token by token.
+// At a chunk that the products cannot take (decays that grow by more than e^0.25 a token or shrink by more than e^(-2^20), values that are not finite or
+// beyond 2^100, entries of T of 4 and more) a block ends: it leaves the state in front of it, and delta_scan_kernel, launched behind, takes the sequence's
+// other tokens, so that a value that is no number reaches what it reaches token by token.  (Such chunks token by token in this kernel took 114 us
+// each, one after another: 8 prompts of 576 .. 1472 tokens whose decays grow 910 us token by token, 5267 so, 1005 now; a batch takes no longer than
+// its chunks in front of such ones and their sequences' other tokens, one launch after the other.)
 //
-// B200, 16 heads of 128 x 128, against token by token: 8 prompts of 576 .. 1472 tokens 907 -> 362 us (72 + 288 for the two launches), 8 of 1024
-// 635 -> 280, one of 1500 604 -> 268, 8 of 64 47 -> 39.  Against 64 bits, of the norm (token by token in brackets): outputs 1.1e-7 (1.2e-7), states
+// B200, 16 heads of 128 x 128, against token by token: 8 prompts of 576 .. 1472 tokens 910 -> 336 us, 8 of 1024
+// 640 -> 270, one of 1500 610 -> 239, 8 of 64 50 -> 40.  Against 64 bits, of the norm (token by token in brackets): outputs 1.1e-7 (1.2e-7), states
 // 8.3e-8 (1.1e-7); decays near 1 1.5e-7 (2.6e-7) and 1.3e-7 (3.4e-7).  The second launch is bound by its chain, about 9500 clocks a chunk: products with
 // the state 1700, R 1000, T R 500, U 1000, the update's product 1300, the state 2700, half of each the arithmetic of splitting (24 clocks of a
 // scheduler for two numbers) and the rest six hand-overs of 300 to 400 clocks.  With scores and T in the same launch (no first launch) a chunk took
@@ -38,7 +41,7 @@ namespace {
 
 using namespace split16;
 
-constexpr int C = 32, KD = 128, VL = 128;            // tokens of a chunk, key rows, value columns of a block
+constexpr int C = kDeltaChunk, KD = 128, VL = kDeltaCols;            // tokens of a chunk, key rows, value columns of a block
 constexpr int kWarps = 16, kThreads = kWarps * 32;
 constexpr int SUB = 2 * C * 128;                     // 64 key rows (columns of the tile) of [k; q], 16-bit, 128-byte rows
 constexpr int SLICE = 2 * SUB, KQ = 3 * SLICE;       // one of h / l / m; a stage
@@ -55,26 +58,27 @@ struct __align__(16) Scalars {      // of a chunk and head, per token
   float gq[C];                      // decay since the chunk's start * scale of q
   float gend[C];                    // decay to the chunk's end * scale of k, of `most`
   float as[C];                      // scales of the rows of the outputs' weights
-  float fk[C], fq[C];               // norm factors alone
   float all, most;                  // decay of the chunk; a power of two
   int bad;                          // not for the products
-  int pad[29];
+  int pad[64];
+  int done[kDeltaDone];             // (of a sequence's first chunk) tokens that the second launch has done, per 128 value columns
 };
 struct __align__(16) Prepared {     // what the first launch leaves, and the second copies
   uint8_t tri[TRIS];                // [h, l, m][32 rows][T: 64 bytes, the outputs' weights: 64 bytes]
   Scalars sc;
 };
 static_assert(sizeof(Prepared) == LLMSS_DELTA_PREPARED && sizeof(Prepared) % 1024 == 0, "tiles stay on their swizzle period");
+static_assert(sizeof(Scalars) == 1024 && kDeltaDoneAt % 4 == 0, "the tokens done end a record");
 struct Bars {
   uint64_t kq_full[STAGES], kq_empty[STAGES], ops_full[4];
   uint64_t s_full, p, pq_read, r_full, tr, u1_full, u2_full, s2, o2;
 };
 struct __align__(16) Smem {
   float o[C][VL];                   // decayed products of the state in front of the chunk with the queries
-  float s_scale[VL], u1_scale[VL], u2_scale[2][VL], smax[2][VL], ex[2][2][VL];
+  float s_scale[VL], u1_scale[VL], u2_scale[2][VL], smax[2][VL];
   Bars bar;
   int solve_bad[2], state_bad[2], skip[2];
-  int quit;
+  int quit, stop;                   // a wait ran out; a chunk is left to the launch behind
   uint32_t tmem;
 };
 constexpr int kSmemBytes = 1024 + STAGES * KQ + 4 * (int)sizeof(Prepared) + (int)sizeof(Smem);
@@ -163,7 +167,7 @@ __global__ void __launch_bounds__(kThreads, 1) delta_chunk_kernel(DeltaArgs a) {
       mbar_init(&bar.u2_full, 4);
       mbar_init(&bar.s2, 2);
       mbar_init(&bar.o2, 1);
-      sm.quit = 0;
+      sm.quit = sm.stop = 0;
       fence_mbar_init();
     }
   }
@@ -190,6 +194,10 @@ __global__ void __launch_bounds__(kThreads, 1) delta_chunk_kernel(DeltaArgs a) {
         for (int i = 0; i < C; i += 2) x[i / 2] = pack(i < rows ? f[i] : 0.f, i + 1 < rows ? f[i + 1] : 0.f);
       }
       wait_bar(&bar.ops_full[c & 3], c >> 2, quit);
+      if (c > 0) {
+        wait_bar(&bar.s2, c - 1, quit);
+        if (sm.skip[(c - 1) & 1]) break;
+      }
       wait_bar(&bar.p, c, quit);
       tcgen05_fence_after();
       const pair_t ss = both(-sm.s_scale[v]);
@@ -269,10 +277,10 @@ __global__ void __launch_bounds__(kThreads, 1) delta_chunk_kernel(DeltaArgs a) {
     float ss = 0.f, mx[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
     for (int i = 0; i < 32; ++i) mx[i & 3] = max_abs(mx[i & 3], S[i]);
-    bool bad = false;
+    int c = 0;
     // parts of the state in front of chunk c; then that chunk
 #pragma unroll 1
-    for (int c = 0;; ++c) {
+    for (;; ++c) {
       if (c < nch) {
         const float mine = max_abs(max_abs(mx[0], mx[1], mx[2]), mx[3], 0.f);
         sm.smax[part][v] = mine;
@@ -301,7 +309,7 @@ __global__ void __launch_bounds__(kThreads, 1) delta_chunk_kernel(DeltaArgs a) {
       }
       if (c > 0) {
         // outputs of the chunk before (everything read before the first store: the compiler cannot tell `out` from shared memory)
-        const int p = c - 1, n = v < nj && !bad ? min(C, ql - p * C) - part * 16 : 0;
+        const int p = c - 1, n = v < nj ? min(C, ql - p * C) - part * 16 : 0;
         const Scalars& sc = prep[p & 3].sc;
         pair_t o[8];
         get_sums3(row + tO + part * 16, o);
@@ -341,62 +349,23 @@ __global__ void __launch_bounds__(kThreads, 1) delta_chunk_kernel(DeltaArgs a) {
       }
       wait_bar(&bar.s2, c, quit);
       tcgen05_fence_after();
-      bad = sm.skip[c & 1];
-      if (!bad) {
-        const pair_t us = both(sm.u1_scale[v]);
-        mx[0] = mx[1] = mx[2] = mx[3] = 0.f;
+      if (sm.skip[c & 1]) break;
+      const pair_t us = both(sm.u1_scale[v]);
+      mx[0] = mx[1] = mx[2] = mx[3] = 0.f;
 #pragma unroll
-        for (int i = 0; i < 4; ++i) {
-          pair_t p[8];
-          get_sums(row + tXS + part * 64 + i * 16, row + tYS + part * 64 + i * 16, p);
+      for (int i = 0; i < 4; ++i) {
+        pair_t p[8];
+        get_sums(row + tXS + part * 64 + i * 16, row + tYS + part * 64 + i * 16, p);
 #pragma unroll
-          for (int e = 0; e < 8; ++e) {
-            S[i * 8 + e] = pfma(all, S[i * 8 + e], pmul(us, p[e]));
-            mx[e & 3] = max_abs(mx[e & 3], S[i * 8 + e]);
-          }
+        for (int e = 0; e < 8; ++e) {
+          S[i * 8 + e] = pfma(all, S[i * 8 + e], pmul(us, p[e]));
+          mx[e & 3] = max_abs(mx[e & 3], S[i * 8 + e]);
         }
-      } else {
-        // token by token; the two threads of a column meet in shared memory
-        float* op = a.out + (int64_t)(q0 + c * C) * ldo + (int64_t)h * a.dv + j0 + v;
-        const int n = min(C, ql - c * C);
-        int turn = 0;
-        auto total = [&](float x) {
-          sm.ex[turn][part][v] = x;
-          meet();
-          const float y = sm.ex[turn][0][v] + sm.ex[turn][1][v];
-          turn ^= 1;
-          return y;
-        };
-#pragma unroll 1
-        for (int i = 0; i < n; ++i) {
-          const int64_t t = q0 + c * C + i;
-          const float* kp = a.k + t * a.ldk + (int64_t)hk * dk + part * 64;
-          const float* qp = a.q + t * a.ldq + (int64_t)hk * dk + part * 64;
-          const float g = expf(a.log_decay[t * a.ldg + h]), xb = a.beta[t * a.ldb + h], be = a.beta_sigmoid ? 1.f / (1.f + expf(-xb)) : xb;
-          const float fk = sc.fk[i], fq = sc.fq[i], val = v < nj ? a.v[t * a.ldv + (int64_t)h * a.dv + j0 + v] : 0.f;
-          pair_t d = 0;
-#pragma unroll
-          for (int e = 0; e < 32; ++e)
-            if (part * 64 + 2 * e < dk) d = pfma(S[e], *reinterpret_cast<const pair_t*>(kp + 2 * e), d);
-          const float2 ds = unpack(d);
-          const float w = (be * val - be * g * fk * total(ds.x + ds.y)) * fk;
-          pair_t y = 0;
-#pragma unroll
-          for (int e = 0; e < 32; ++e)
-            if (part * 64 + 2 * e < dk) {
-              S[e] = pfma(both(g), S[e], pmul(*reinterpret_cast<const pair_t*>(kp + 2 * e), both(w)));
-              y = pfma(S[e], *reinterpret_cast<const pair_t*>(qp + 2 * e), y);
-            }
-          const float2 ys = unpack(y);
-          const float out = total(ys.x + ys.y) * fq;
-          if (part == 0 && v < nj) op[i * ldo] = out;
-        }
-        meet();
-        mx[0] = mx[1] = mx[2] = mx[3] = 0.f;
-#pragma unroll
-        for (int i = 0; i < 32; ++i) mx[i & 3] = max_abs(mx[i & 3], S[i]);
       }
     }
+    // the state in front of chunk c, and what is left of the sequence
+    if (threadIdx.x == 128)
+      reinterpret_cast<Prepared*>(a.prepared)[(int64_t)(q0 / C + b) * a.H + h].sc.done[blockIdx.z] = c < nch ? c * C : ql;
     if (sm.quit) {
       if (threadIdx.x == 128) printf("[llmss_b200] delta_chunk: a wait ran out (block %d,%d,%d)\n", b, h, (int)blockIdx.z);
 #pragma unroll
@@ -437,6 +406,7 @@ __global__ void __launch_bounds__(kThreads, 1) delta_chunk_kernel(DeltaArgs a) {
       for (int o = 4; o > 0; o >>= 1) mx = max_abs(mx, __shfl_xor_sync(0xffffffffu, mx, o), 0.f);
       const Scale s = scale_of(mx);
       if (c >= STAGES) wait_bar(&bar.kq_empty[stage], c / STAGES - 1, quit);
+      if (*(volatile int*)&sm.stop) break;
       uint8_t* to = sKQ + stage * KQ + ((at & 8) ? C * 128 : 0) + i * 128 + ((l8 & 1) << 3);
 #pragma unroll
       for (int m = 0; m < 4; ++m) {
@@ -515,13 +485,19 @@ __global__ void __launch_bounds__(kThreads, 1) delta_chunk_kernel(DeltaArgs a) {
         }
         umma_commit(&bar.s2);
         sm.skip[st] = bad;
+        if (bad) *(volatile int*)&sm.stop = 1;
         mbar_arrive(&bar.s2);
+        if (bad) mbar_arrive(&bar.kq_empty[c % STAGES]);       // nothing reads these rows any more: their warps go on and find `stop`
       }
       __syncwarp();
+      if (bad) {
+        for (int f = c + 1; f < min(nch, c + 3); ++f) wait_bar(&bar.ops_full[f & 3], f >> 2, quit);      // copies in flight
+        break;
+      }
       wait_bar(&bar.u2_full, c, quit);
       tcgen05_fence_after();
       if (elect_one()) {
-        if (!bad) by_triangle(tmem + tO, tmem + tU2, tmem + tU2 + 32, desc_lo(tr) + 4);
+        by_triangle(tmem + tO, tmem + tU2, tmem + tU2 + 32, desc_lo(tr) + 4);
         umma_commit(&bar.o2);
         umma_commit(&bar.kq_empty[c % STAGES]);
       }
@@ -665,7 +641,6 @@ __global__ void __launch_bounds__(128, 5) delta_prep_kernel(DeltaArgs a) {
       no |= __any_sync(0xffffffffu, s.huge);
       out.sc.as[lane] = s.s;
       out.sc.gq[lane] = since * sm.qs[lane];
-      out.sc.fq[lane] = sm.qf[lane];
       uint8_t* to = out.tri + lane * 128;
 #pragma unroll
       for (int j = 0; j < C; j += 8) {
@@ -688,7 +663,6 @@ __global__ void __launch_bounds__(128, 5) delta_prep_kernel(DeltaArgs a) {
       out.sc.be[lane] = be;
       out.sc.bk[lane] = be * ks * since;
       out.sc.gend[lane] = end * s.inv * 0x1p-12f;
-      out.sc.fk[lane] = sm.kf[lane];
       if (lane == 31) {
         out.sc.all = since;
         out.sc.most = s.s * 0x1p12f;

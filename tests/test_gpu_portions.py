@@ -129,6 +129,52 @@ def test_delta_over_chunks_of_one_sequence(n, max_q):
     assert _rel(out, want.reshape(n, -1)) < 1e-6 and _rel(state.transpose(2, 3), ends) < 1e-6
 
 
+@pytest.mark.parametrize("dk,dv,heads,qk_heads", [(128, 128, 4, 2), (20, 300, 2, 2), (64, 70, 2, 1)])
+@pytest.mark.parametrize("tokens", [[0], [40, 99], [32 + 107, 99 + 3], [107 + 63, 107 + 64 + 32]])
+def test_delta_over_chunks_until_a_chunk_that_grows(dk, dv, heads, qk_heads, tokens, monkeypatch):
+    """One token with a growing decay in the first, a middle or the last chunk of some sequences and one head: what is left of those runs token by
+    token behind, from the state in front of the chunk, and nothing else changes.  Bound: 32-bit sums, 1e-6 of the norm."""
+    from llmss_b200.ops import cuda_impl as cu
+
+    monkeypatch.setattr(cu, "_delta_over_chunks", lambda *a: True)
+    torch.manual_seed(dk + dv)
+    lens, ctxs, slots = [100, 7, 64, 33], [0, 5, 8, 2], [2, 0, 3, 1]
+    (q, k, v), b, S0 = _delta_inputs(lens, heads, qk_heads, dk, dv, True)
+    g = -0.3 * torch.rand(sum(lens), heads, device="cuda")
+    g[tokens, 1] = 0.3
+    state = torch.empty(len(lens), heads, dk, dv, device="cuda")
+    state.view(len(lens), heads, dv, dk)[slots] = S0.transpose(2, 3)
+    want, ends = _delta64(q, k, v, g, b, S0.double().cpu(), lens, ctxs, heads, qk_heads, dk, dv, True)
+    got = ops.delta_scan(q, k, v, g, b, _batch(lens, ctxs, slots), state, heads, qk_heads, dk, dv, unit_eps=1e-6, q_scale=0.25, beta_sigmoid=True)
+    assert _rel(got, want.reshape(sum(lens), -1)) < 1e-6
+    assert _rel(state.view(len(lens), heads, dv, dk)[slots].transpose(2, 3), ends) < 1e-6
+
+
+def test_delta_over_chunks_costs_no_more_where_it_cannot_be_used(monkeypatch):
+    """Decays that grow in every chunk: one pass over the portions token by token and what the chunks' launches take to notice (token by token in
+    the chunks' own kernel it was 5.8 times as long)."""
+    from llmss_b200.ops import cuda_impl as cu
+
+    torch.manual_seed(1)
+    lens, heads, d = [512] * 4, 8, 128
+    (q, k, v), b, S0 = _delta_inputs(lens, heads, 4, d, d, True)
+    g, state, batch = 0.26 + 0.04 * torch.rand(sum(lens), heads, device="cuda"), S0, _batch(lens, [0] * 4, range(4))
+
+    def best(form):
+        monkeypatch.setattr(cu, "_delta_over_chunks", lambda *a: form)
+        times = []
+        for _ in range(8):
+            at = [torch.cuda.Event(enable_timing=True) for _ in range(2)]
+            at[0].record()
+            ops.delta_scan(q, k, v, g, b, batch, state, heads, 4, d, d, unit_eps=1e-6, q_scale=0.25, beta_sigmoid=True)
+            at[1].record()
+            torch.cuda.synchronize()
+            times.append(at[0].elapsed_time(at[1]))
+        return min(times[2:])
+
+    assert best(True) < 1.6 * best(False)
+
+
 @pytest.mark.parametrize("where", ["value", "key", "strength", "decay", "state", "huge value"])
 def test_delta_over_chunks_bad_numbers(where, monkeypatch):
     """A value that is no number, or too large to scale, reaches what it reaches token by token: later tokens of its column (value, state) or of
