@@ -363,15 +363,15 @@ __global__ void __launch_bounds__(kThreads, 1) delta_chunk_kernel(DeltaArgs a) {
         }
       }
     }
-    // the state in front of chunk c, and what is left of the sequence
-    if (threadIdx.x == 128)
-      reinterpret_cast<Prepared*>(a.prepared)[(int64_t)(q0 / C + b) * a.H + h].sc.done[blockIdx.z] = c < nch ? c * C : ql;
-    if (sm.quit) {
-      if (threadIdx.x == 128) printf("[llmss_b200] delta_chunk: a wait ran out (block %d,%d,%d)\n", b, h, (int)blockIdx.z);
-#pragma unroll
-      for (int i = 0; i < 32; ++i) S[i] = ~0ull;
+    // The state in front of chunk c, and what is left of the sequence.  Where a wait ran out that is all of it: the state in memory is still the one in
+    // front of the sequence, and the launch behind writes every output again.  (One answer for all of these warps.)
+    uint32_t ran_out = *(volatile int*)&sm.quit;
+    asm volatile("{\n\t.reg .pred p, q;\n\tsetp.ne.u32 p, %0, 0;\n\tbar.red.or.pred q, 5, 256, p;\n\tselp.u32 %0, 1, 0, q;\n\t}" : "+r"(ran_out)::"memory");
+    if (threadIdx.x == 128) {
+      if (ran_out) printf("[llmss_b200] delta_chunk: a wait ran out, token by token instead (block %d,%d,%d)\n", b, h, (int)blockIdx.z);
+      reinterpret_cast<Prepared*>(a.prepared)[(int64_t)(q0 / C + b) * a.H + h].sc.done[blockIdx.z] = ran_out ? 0 : c < nch ? c * C : ql;
     }
-    if (v < nj) {
+    if (v < nj && !ran_out) {
 #pragma unroll
       for (int i = 0; i < 32; i += 2) {
         const float2 x = unpack(S[i]), y = unpack(S[i + 1]);

@@ -118,7 +118,7 @@ __device__ __forceinline__ void umma_ss(uint32_t d, uint32_t a_lo, uint32_t b_lo
 }
 
 // mbar_wait for kernels that end by themselves: a wait of more than LLMSS_SPIN_TIMEOUT_NS sets *quit (shared memory), and waits that find it set
-// end; the results are marked then
+// end.  What the block has computed since is worth nothing: the kernel leaves its state as it was and its work to another one
 static __device__ __noinline__ void wait_bar_loop(uint32_t bar, uint32_t parity, volatile int* quit) {
   const uint64_t t0 = globaltimer_ns();
   for (;;) {
