@@ -21,11 +21,11 @@ struct DeltaArgs {
   // a chunk that its products cannot take; the record of its first chunk then says how many tokens are done, per 128 value columns, and
   // the token-by-token launch takes the others.
   uint8_t* prepared;
-  int least;
+  int least, chunks;     // (chunks: the most that are prepared of one sequence)
 };
 
 constexpr int kDeltaChunk = 32, kDeltaCols = 128, kDeltaDone = 29;       // tokens of a chunk, value columns of a block over chunks, blocks that a record has room for
 
-int delta_chunk_launch(const DeltaArgs& a, int B, int max_q, cudaStream_t stream);
+int delta_chunk_launch(DeltaArgs a, int B, int max_q, cudaStream_t stream);
 // where in a record the tokens done lie: behind the tiles and the numbers per token
 constexpr int kDeltaDoneAt = LLMSS_DELTA_PREPARED - 4 * kDeltaDone;

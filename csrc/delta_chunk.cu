@@ -145,7 +145,7 @@ __global__ void __launch_bounds__(kThreads, 1) delta_chunk_kernel(DeltaArgs a) {
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int h = blockIdx.y, hk = h / a.rep, dk = a.dk;
   const int j0 = blockIdx.z * VL, nj = min(VL, a.dv - j0);
-  const int nch = (ql + C - 1) / C;
+  const int nch = min((ql + C - 1) / C, a.chunks);
   int* quit = &sm.quit;
 
   if (warp == 15) {
@@ -369,7 +369,7 @@ __global__ void __launch_bounds__(kThreads, 1) delta_chunk_kernel(DeltaArgs a) {
     asm volatile("{\n\t.reg .pred p, q;\n\tsetp.ne.u32 p, %0, 0;\n\tbar.red.or.pred q, 5, 256, p;\n\tselp.u32 %0, 1, 0, q;\n\t}" : "+r"(ran_out)::"memory");
     if (threadIdx.x == 128) {
       if (ran_out) printf("[llmss_b200] delta_chunk: a wait ran out, token by token instead (block %d,%d,%d)\n", b, h, (int)blockIdx.z);
-      reinterpret_cast<Prepared*>(a.prepared)[(int64_t)(q0 / C + b) * a.H + h].sc.done[blockIdx.z] = ran_out ? 0 : c < nch ? c * C : ql;
+      reinterpret_cast<Prepared*>(a.prepared)[(int64_t)(q0 / C + b) * a.H + h].sc.done[blockIdx.z] = ran_out ? 0 : min(c * C, ql);
     }
     if (v < nj && !ran_out) {
 #pragma unroll
@@ -715,11 +715,12 @@ __global__ void __launch_bounds__(128, 5) delta_prep_kernel(DeltaArgs a) {
 }  // namespace
 
 // sequences of at least a.least tokens; the caller has checked the sizes (dk <= 128, multiple of 4, 16-byte rows)
-int delta_chunk_launch(const DeltaArgs& a, int B, int max_q, cudaStream_t stream) {
+int delta_chunk_launch(DeltaArgs a, int B, int max_q, cudaStream_t stream) {
+  a.chunks = (max_q + C - 1) / C;
   static PerDeviceSmem granted, granted_prep;
   LLMSS_CHECK_CUDA(granted_prep.ensure(delta_prep_kernel, (int)sizeof(PrepSmem)));
   LLMSS_CHECK_CUDA(granted.ensure(delta_chunk_kernel, kSmemBytes));
-  delta_prep_kernel<<<dim3((max_q + C - 1) / C, a.H / a.rep, B), 128, sizeof(PrepSmem), stream>>>(a);
+  delta_prep_kernel<<<dim3(a.chunks, a.H / a.rep, B), 128, sizeof(PrepSmem), stream>>>(a);
   LLMSS_CHECK_CUDA(cudaGetLastError());
   delta_chunk_kernel<<<dim3(B, a.H, (a.dv + VL - 1) / VL), kThreads, kSmemBytes, stream>>>(a);
   LLMSS_CHECK_CUDA(cudaGetLastError());

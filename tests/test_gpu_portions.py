@@ -111,9 +111,10 @@ def test_delta_over_chunks(dk, dv, heads, qk_heads, unit, decay, monkeypatch):
     assert _rel(state.reshape(len(lens), heads, dv, dk).transpose(2, 3), ends) < bound
 
 
-@pytest.mark.parametrize("n,max_q", [(1, 1), (7, 7), (31, 31), (31, 64), (32, 32), (7, 0)])
+@pytest.mark.parametrize("n,max_q", [(1, 1), (7, 7), (31, 31), (31, 64), (32, 32), (7, 0), (100, 64), (100, 40)])
 def test_delta_over_chunks_of_one_sequence(n, max_q):
-    """The C entry, one sequence of any length: a short one runs token by token, whatever bound on the lengths the caller names."""
+    """The C entry, one sequence of any length: a short one runs token by token, and ``max_q`` is a hint on the lengths: tokens
+    beyond it run token by token."""
     from llmss_b200.ops import _lib, cuda_impl as cu
 
     torch.manual_seed(n)
