@@ -433,12 +433,16 @@ __global__ void __launch_bounds__(kThreads, 1) delta_chunk_kernel(DeltaArgs a) {
       }
       __syncwarp();
     };
-    // a row of U or R (three parts, 32 tokens) times a triangle, whose parts are stacked: h [h | l | m], l [h | l] one run further, m h two
+    // a row of U or R (three parts, 32 tokens) times a triangle: h h | h l, l h | h m, l l, m h, an accumulator each.  (Products onto one accumulator are
+    // all of one shape: only those are sure to be added one after the other.)
     auto by_triangle = [&](uint32_t d, uint32_t at, uint32_t at3, uint32_t lo) {
 #pragma unroll
       for (int x = 0; x < 3; ++x)
 #pragma unroll
-        for (int k = 0; k < 2; ++k) umma_ts(d + x * C, (x == 2 ? at3 : at + x * 16) + k * 8, lo + k * 2, idesc((3 - x) * C, 0), x > 0 || k > 0);
+        for (int y = 0; y < 3 - x; ++y)
+#pragma unroll
+          for (int k = 0; k < 2; ++k)
+            umma_ts(d + (x + y) * C, (x == 2 ? at3 : at + x * 16) + k * 8, lo + y * (TRI / 16) + k * 2, idesc(C, 0), x > 0 || k > 0);
     };
     for (int c = 0; c < min(nch, 3); ++c) fetch(c);
     for (int c = 0; c < nch; ++c) {
