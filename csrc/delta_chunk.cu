@@ -19,7 +19,7 @@
 // The products that wait for the state (S_0^T k -> R -> T R -> S) are the chain; the others lie in its gaps.
 //
 // Rounding.  Operands are rows scaled and cut into three 16-bit numbers (split16.cuh); their sums are exact in one accumulator, close to it in
-// the other, and meet in one 32-bit addition.  (The state has two parts only: an error of 2^-24 of a column's largest number, once per chunk.)  The
+// the other, and meet in one 32-bit addition.  (With two parts of the state an entry 2^-10 of its column's largest entered the products with 14 bits.)  The
 // state itself is a 32-bit number in a register, rounded once per chunk where it was rounded once per token.  Log decays sum in 64 bits.
 // At a chunk that the products cannot take (decays that grow by more than e^0.25 a token or shrink by more than e^(-2^20), values that are not finite or
 // beyond 2^100, entries of T of 4 and more) a block ends: it leaves the state in front of it, and delta_scan_kernel, launched behind, takes the sequence's
@@ -50,8 +50,9 @@ constexpr int TRI = C * 128, TRIS = 3 * TRI;         // a part of [T | outputs' 
 constexpr float kTScale = 0x1p-10f;                  // entries of T, below 4
 
 // tensor memory, columns: products with the state [0, 128) and R over those with k; T R (three runs); over them the state's update [0, 256);
-// outputs (three runs); the state's parts and, once both products with the state are done, U's
-constexpr int tXP = 0, tYP = 64, tU = 128, tR = 0, tR3 = 64, tXS = 0, tYS = 128, tO = 256, tSH = 384, tSL = 448, tU1 = 384, tU2 = 432;
+// outputs (three runs); the state's parts (the last one, of two runs, over the update that its own thread has read) and, once both products with the
+// state are done, U's
+constexpr int tXP = 0, tYP = 64, tU = 128, tR = 0, tR3 = 64, tXS = 0, tYS = 128, tO = 256, tSH = 384, tSL = 448, tSM = 128, tU1 = 384, tU2 = 432;
 
 struct __align__(16) Scalars {      // of a chunk and head, per token
   float be[C], bk[C];               // strength; strength * decay since the chunk's start * scale of k
@@ -291,9 +292,10 @@ __global__ void __launch_bounds__(kThreads, 1) delta_chunk_kernel(DeltaArgs a) {
         if (part == 0) sm.s_scale[v] = s.s;
 #pragma unroll
         for (int i = 0; i < 2; ++i) {
-          uint32_t hi[16], lo[16];
+          uint32_t hi[16], lo[16], mi[16];
 #pragma unroll
-          for (int e = 0; e < 16; ++e) split2(pmul(S[i * 16 + e], both(s.inv)), hi[e], lo[e]);
+          for (int e = 0; e < 16; ++e) split3(pmul(S[i * 16 + e], both(s.inv)), hi[e], lo[e], mi[e]);
+          tmem_st16(row + tSM + part * 64 + i * 16, mi);
           if (i == 0) {
             if (c > 0) wait_bar(&bar.o2, c - 1, quit);         // U's parts, in the same place, have been read
             tcgen05_fence_after();
@@ -452,14 +454,15 @@ __global__ void __launch_bounds__(kThreads, 1) delta_chunk_kernel(DeltaArgs a) {
       wait_bar(&bar.ops_full[c & 3], c >> 2, quit);
       wait_bar(&bar.s_full, c, quit);
       tcgen05_fence_after();
-      if (elect_one()) {        // the state times [k; q]: h h, h l, l h, l l, h m
+      if (elect_one()) {        // the state times [k; q]
         const uint32_t lo = desc_lo(base);
 #pragma unroll 1
-        for (int x = 0; x < 5; ++x) {
-          const uint32_t at = tmem + (((kFirst >> (2 * x)) & 3) ? tSL : tSH), lb = lo + ((kSecond >> (2 * x)) & 3) * (SLICE / 16);
+        for (int x = 0; x < 6; ++x) {
+          const uint32_t first = (kFirst >> (2 * x)) & 3, lb = lo + ((kSecond >> (2 * x)) & 3) * (SLICE / 16);
+          const uint32_t at = tmem + (first == 0 ? tSH : first == 1 ? tSL : tSM), skip = first == 2 ? 32 : 0;
           const uint32_t d = tmem + (x == 0 ? tXP : tYP);
 #pragma unroll
-          for (int k = 0; k < 8; ++k) umma_ts(d, at + k * 8, lb + (k >> 2) * (SUB / 16) + (k & 3) * 2, idesc(2 * C, 0), x > 1 || k > 0);
+          for (int k = 0; k < 8; ++k) umma_ts(d, at + k * 8 + (k >> 2) * skip, lb + (k >> 2) * (SUB / 16) + (k & 3) * 2, idesc(2 * C, 0), x > 1 || k > 0);
         }
         umma_commit(&bar.p);
         mbar_arrive(&bar.p);

@@ -86,13 +86,6 @@ __device__ __forceinline__ void split3(pair_t y, uint32_t& h, uint32_t& l, uint3
   l = half2_bits(b);
   m = half2_bits(psub(r, b));
 }
-// h and l alone: to 2^-24 of the scale
-__device__ __forceinline__ void split2(pair_t y, uint32_t& h, uint32_t& l) {
-  const pair_t a = psub(padd(y, kGrid1), kGrid1);
-  h = half2_bits(a);
-  l = half2_bits(psub(y, a));
-}
-
 // ---- the instructions around tensor memory that these products use
 __device__ __forceinline__ void tmem_st16(uint32_t addr, const uint32_t (&r)[16]) {
   asm volatile("tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16};" ::"r"(addr),

@@ -176,6 +176,29 @@ def test_delta_over_chunks_costs_no_more_where_it_cannot_be_used(monkeypatch):
     assert best(True) < 1.6 * best(False)
 
 
+def _delta_worst(got, want, dims):
+    """Largest error of a part (a token of a head, a column, ..) over the norm of that part."""
+    return float(((got.double().cpu() - want).norm(dim=dims) / want.norm(dim=dims).clamp_min(1e-300)).max())
+
+
+def test_delta_over_chunks_channels_of_unequal_size(monkeypatch):
+    """Key channels between 2^-6 and 2^6, queries the other way round: small entries of the state meet large ones of the queries.  Bound: 2^-24 a term,
+    64 of them: 4e-6 of each token and head (token by token 5e-7; a state of two 16-bit parts: 8e-5)."""
+    from llmss_b200.ops import cuda_impl as cu
+
+    monkeypatch.setattr(cu, "_delta_over_chunks", lambda *a: True)
+    torch.manual_seed(3)
+    n, heads, d = 160, 2, 128
+    (q, k, v), b, S0 = _delta_inputs([n], heads, heads, d, d, True)
+    size = torch.exp2(torch.rand(d, device="cuda") * 12 - 6)
+    k.view(n, heads, d).mul_(size), q.view(n, heads, d).div_(size)
+    g, state = -0.3 * torch.rand(n, heads, device="cuda"), S0.transpose(2, 3).contiguous()
+    want, ends = _delta64(q, k, v, g, b, S0.double().cpu(), [n], [0], heads, heads, d, d, True)
+    got = ops.delta_scan(q, k, v, g, b, _batch([n], [0], [0]), state, heads, heads, d, d, unit_eps=1e-6, q_scale=0.25, beta_sigmoid=True).view(n, heads, d)
+    assert _delta_worst(got, want, 2) < 4e-6
+    assert _delta_worst(state.transpose(2, 3), ends, 3) < 4e-6          # each key row of the state
+
+
 @pytest.mark.parametrize("where", ["value", "key", "strength", "decay", "state", "huge value"])
 def test_delta_over_chunks_bad_numbers(where, monkeypatch):
     """A value that is no number, or too large to scale, reaches what it reaches token by token: later tokens of its column (value, state) or of
