@@ -19,19 +19,23 @@
 // The products that wait for the state (S_0^T k -> R -> T R -> S) are the chain; the others lie in its gaps.
 //
 // Rounding.  Operands are rows scaled and cut into three 16-bit numbers (split16.cuh); their sums are exact in one accumulator, close to it in
-// the other, and meet in one 32-bit addition.  (With two parts of the state an entry 2^-10 of its column's largest entered the products with 14 bits.)  The
-// state itself is a 32-bit number in a register, rounded once per chunk where it was rounded once per token.  Log decays sum in 64 bits.
+// the other, and meet in one 32-bit addition.  A row's parts carry 2^-34 of its largest number: entries down to 2^-11 of it have the bits of a 32-bit number,
+// smaller ones fewer.  That is no loss while the larger ones are in the same sums; where they are not (tokens that a decay has parted, keys of other
+// channels, a large value behind the token), `spread` and the count over the state notice.  (With two parts of the state an entry 2^-10 of its column's
+// largest entered the products with 14 bits.)  The state itself is a 32-bit number in a register, rounded once per chunk where it was rounded once per
+// token.  Log decays sum in 64 bits.
 // At a chunk that the products cannot take (decays that grow by more than e^0.25 a token or shrink by more than e^(-2^20), values that are not finite or
-// beyond 2^100, entries of T of 4 and more) a block ends: it leaves the state in front of it, and delta_scan_kernel, launched behind, takes the sequence's
+// beyond 2^100, entries of T of 4 and more, numbers that differ by more than the parts carry) a block ends: it leaves the state in front of it, and delta_scan_kernel, launched behind, takes the sequence's
 // other tokens, so that a value that is no number reaches what it reaches token by token.  (Such chunks token by token in this kernel took 114 us
 // each, one after another: 8 prompts of 576 .. 1472 tokens whose decays grow 910 us token by token, 5267 so, 1005 now; a batch takes no longer than
 // its chunks in front of such ones and their sequences' other tokens, one launch after the other.)
 //
-// B200, 16 heads of 128 x 128, against token by token: 8 prompts of 576 .. 1472 tokens 910 -> 336 us, 8 of 1024
-// 640 -> 270, one of 1500 610 -> 239, 8 of 64 50 -> 40.  Against 64 bits, of the norm (token by token in brackets): outputs 1.1e-7 (1.2e-7), states
-// 8.3e-8 (1.1e-7); decays near 1 1.5e-7 (2.6e-7) and 1.3e-7 (3.4e-7).  The second launch is bound by its chain, about 9500 clocks a chunk: products with
-// the state 1700, R 1000, T R 500, U 1000, the update's product 1300, the state 2700, half of each the arithmetic of splitting (24 clocks of a
-// scheduler for two numbers) and the rest six hand-overs of 300 to 400 clocks.  With scores and T in the same launch (no first launch) a chunk took
+// B200, 16 heads of 128 x 128, against token by token: 8 prompts of 576 .. 1472 tokens 910 -> 344 us (68 + 273 for the two launches, 3 for the one behind),
+// 8 of 1024 640 -> 286, one of 1500 610 -> 288, 8 of 64 50 -> 41; without the three tests of the numbers' size 336, 268, 264 and 40.  Against 64 bits, of the
+// norm (token by token in brackets): outputs 1.3e-7 (1.5e-7), states 7.9e-8 (1.1e-7); decays near 1 1.3e-7 (2.7e-7) and 1.1e-7 (2.5e-7); worst token 2.3e-7
+// (2.7e-7), worst column 1.7e-7 (1.9e-7).  The second launch is bound by its chain, 5.9 us or about 11 000 clocks a chunk: products with
+// the state 2000, R 1000, T R 500, U 1000, the update's product 1300, the state 3200, half of each the arithmetic of splitting (24 clocks of a
+// scheduler for two numbers) and the rest six hand-overs of 300 to 400 clocks each, part of these figures.  With scores and T in the same launch (no first launch) a chunk took
 // 13000 clocks, the scores' products taking shared memory's path from the other warps; with 16 warps for the state 13000 against 11000.  Straight-line
 // code of 200 KB, before its loops were rolled, took 24000.
 #include "delta.cuh"
@@ -59,9 +63,10 @@ struct __align__(16) Scalars {      // of a chunk and head, per token
   float gq[C];                      // decay since the chunk's start * scale of q
   float gend[C];                    // decay to the chunk's end * scale of k, of `most`
   float as[C];                      // scales of the rows of the outputs' weights
-  float all, most;                  // decay of the chunk; a power of two
+  float decay[C];                   // of a token; 0 in a chunk of sparse keys (see spread)
+  float all, most, low;             // decay of the chunk; a power of two; the smallest decay since its start
   int bad;                          // not for the products
-  int pad[64];
+  int pad[31];
   int done[kDeltaDone];             // (of a sequence's first chunk) tokens that the second launch has done, per 128 value columns
 };
 struct __align__(16) Prepared {     // what the first launch leaves, and the second copies
@@ -72,13 +77,13 @@ static_assert(sizeof(Prepared) == LLMSS_DELTA_PREPARED && sizeof(Prepared) % 102
 static_assert(sizeof(Scalars) == 1024 && kDeltaDoneAt % 4 == 0, "the tokens done end a record");
 struct Bars {
   uint64_t kq_full[STAGES], kq_empty[STAGES], ops_full[4];
-  uint64_t s_full, p, pq_read, r_full, tr, u1_full, u2_full, s2, o2;
+  uint64_t s_full, p, pq_read, r_full, tr, u1_full, u2_full, s2, o2, verdict;
 };
 struct __align__(16) Smem {
   float o[C][VL];                   // decayed products of the state in front of the chunk with the queries
   float s_scale[VL], u1_scale[VL], u2_scale[2][VL], smax[2][VL];
   Bars bar;
-  int solve_bad[2], state_bad[2], skip[2];
+  int solve_bad[2], state_bad[2];   // 1 + the last chunk of this parity whose values, or the state in front of it, are not for the products
   int quit, stop;                   // a wait ran out; a chunk is left to the launch behind
   uint32_t tmem;
 };
@@ -133,6 +138,34 @@ __device__ __forceinline__ void lds_pairs(const float* p, pair_t& x, pair_t& y) 
   y = v.y;
 }
 
+// Whether the tokens of a chunk differ by more than a column's parts carry.  What the tokens up to one have written to the column, decayed, and the state in
+// front of the chunk give the size n of that token's numbers; where n is below 2^-11 to 2^-12 of the column's largest (us: a column's numbers are scaled to
+// 2^11 .. 2^12), fewer than 24 bits of them are left.  One such number is chance (1 in 1400 of normal ones that stand alone); a token that is small
+// in all 32 columns of the warp, or five tokens of a column, are not.  s: scale of the column's state.  The same answer for the whole warp.
+// The state has the like (in its warps): 8 of a thread's 64 key rows below 2^-11 to 2^-12 of the column's largest, 3 once keys were sparse.
+// Earlier forms: in front of T R in the chain 343 -> 349 us, the state's count beside U 352.
+__device__ __forceinline__ bool spread(const pair_t (&y)[C / 2], const Scalars& sc, float s, float us) {
+  float n = s > 0x1p-98f ? s * 0x1p11f : 0.f;
+  if (__all_sync(0xffffffffu, n * sc.low >= us)) return false;          // the usual case: the state alone is not small at any token
+  const float most = __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(us)));
+  uint32_t small = 0, some = 0;
+  int few = 0;
+#pragma unroll
+  for (int i = 0; i < C; i += 4) {
+    const float4 f = *reinterpret_cast<const float4*>(sc.decay + i);
+    const float2 p = unpack(y[i / 2]), q = unpack(y[i / 2 + 1]);
+    const float by[4] = {f.x, f.y, f.z, f.w}, x[4] = {p.x, p.y, q.x, q.y};
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      n = fmaxf(n * by[e], fabsf(x[e]) * us);
+      if (n < most) small |= 1u << (i + e);
+      if (n > 0.f) some |= 1u << (i + e);
+      few += n > 0.f && n < us;
+    }
+  }
+  return (__reduce_and_sync(0xffffffffu, small) & __reduce_or_sync(0xffffffffu, some)) != 0 || __any_sync(0xffffffffu, few >= 5);
+}
+
 __global__ void __launch_bounds__(kThreads, 1) delta_chunk_kernel(DeltaArgs a) {
   extern __shared__ uint8_t smem_raw[];
   const int b = blockIdx.x;
@@ -168,6 +201,7 @@ __global__ void __launch_bounds__(kThreads, 1) delta_chunk_kernel(DeltaArgs a) {
       mbar_init(&bar.u2_full, 4);
       mbar_init(&bar.s2, 2);
       mbar_init(&bar.o2, 1);
+      mbar_init(&bar.verdict, 4);
       sm.quit = sm.stop = 0;
       fence_mbar_init();
     }
@@ -176,6 +210,8 @@ __global__ void __launch_bounds__(kThreads, 1) delta_chunk_kernel(DeltaArgs a) {
   __syncthreads();
   tcgen05_fence_after();
   const uint32_t tmem = sm.tmem;
+  // behind the waits for its verdict and for s2 or pq_read: whether chunk c is not for the products
+  auto bad = [&](int c) { return prep[c & 3].sc.bad || sm.solve_bad[c & 1] == c + 1 || sm.state_bad[c & 1] == c + 1; };
 
   if (warp < 4) {
     // ---- R and U: one value column per thread
@@ -197,7 +233,8 @@ __global__ void __launch_bounds__(kThreads, 1) delta_chunk_kernel(DeltaArgs a) {
       wait_bar(&bar.ops_full[c & 3], c >> 2, quit);
       if (c > 0) {
         wait_bar(&bar.s2, c - 1, quit);
-        if (sm.skip[(c - 1) & 1]) break;
+        wait_bar(&bar.verdict, c - 1, quit);
+        if (bad(c - 1)) break;
       }
       wait_bar(&bar.p, c, quit);
       tcgen05_fence_after();
@@ -259,6 +296,9 @@ __global__ void __launch_bounds__(kThreads, 1) delta_chunk_kernel(DeltaArgs a) {
       arrive_warp(&bar.u1_full);
       put_row(row + tU2, row + tU2 + 32, x);
       arrive_warp(&bar.u2_full);
+      if (spread(x, sc, sm.s_scale[v], us) && lane == 0) sm.solve_bad[st] = c + 1;
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&bar.verdict);
     }
   } else if (warp < 12) {
     // ---- the state: a value column and 64 key rows per thread; tokens 16 part .. 16 part + 15 of the outputs
@@ -276,6 +316,7 @@ __global__ void __launch_bounds__(kThreads, 1) delta_chunk_kernel(DeltaArgs a) {
     auto meet = [&] { asm volatile("bar.sync %0, 64;" ::"r"(1 + quarter) : "memory"); };       // the two warps of 32 columns
     const int64_t ldo = (int64_t)a.H * a.dv;
     float ss = 0.f, mx[4] = {0.f, 0.f, 0.f, 0.f};
+    int most_few = 7;                  // once keys are sparse: 2
 #pragma unroll
     for (int i = 0; i < 32; ++i) mx[i & 3] = max_abs(mx[i & 3], S[i]);
     int c = 0;
@@ -305,6 +346,17 @@ __global__ void __launch_bounds__(kThreads, 1) delta_chunk_kernel(DeltaArgs a) {
         }
         tmem_st_wait();
         arrive_warp(&bar.s_full);
+        // key rows (of 64) whose numbers are below 2^-11 to 2^-12 of the column's largest, and not 0: see spread
+        int few = 0;
+        const uint32_t below = 2 * __float_as_uint(ss) - 1;
+#pragma unroll
+        for (int e = 0; e < 32; ++e) {
+          const float2 x = unpack(S[e]);
+          few += (2 * __float_as_uint(x.x) - 1 < below) + (2 * __float_as_uint(x.y) - 1 < below);
+        }
+        wait_bar(&bar.ops_full[c & 3], c >> 2, quit);
+        if (prep[c & 3].sc.low == 0.f) most_few = 2;
+        if (__any_sync(0xffffffffu, few > most_few) && lane == 0) sm.state_bad[c & 1] = c + 1;
       } else {
         wait_bar(&bar.o2, c - 1, quit);
         tcgen05_fence_after();
@@ -334,7 +386,6 @@ __global__ void __launch_bounds__(kThreads, 1) delta_chunk_kernel(DeltaArgs a) {
       }
       if (c >= nch) break;
       const Scalars& sc = prep[c & 3].sc;
-      wait_bar(&bar.ops_full[c & 3], c >> 2, quit);
       const pair_t all = both(sc.all);
       wait_bar(&bar.p, c, quit);
       tcgen05_fence_after();
@@ -349,10 +400,11 @@ __global__ void __launch_bounds__(kThreads, 1) delta_chunk_kernel(DeltaArgs a) {
           sm.o[part * 16 + 2 * i + 1][v] = y.y * sc.gq[part * 16 + 2 * i + 1];
         }
       }
+      wait_bar(&bar.verdict, c, quit);
+      const pair_t us = both(sm.u1_scale[v]);
       wait_bar(&bar.s2, c, quit);
       tcgen05_fence_after();
-      if (sm.skip[c & 1]) break;
-      const pair_t us = both(sm.u1_scale[v]);
+      if (bad(c)) break;
       mx[0] = mx[1] = mx[2] = mx[3] = 0.f;
 #pragma unroll
       for (int i = 0; i < 4; ++i) {
@@ -448,7 +500,6 @@ __global__ void __launch_bounds__(kThreads, 1) delta_chunk_kernel(DeltaArgs a) {
     };
     for (int c = 0; c < min(nch, 3); ++c) fetch(c);
     for (int c = 0; c < nch; ++c) {
-      const int st = c & 1;
       const uint32_t base = kq + (c % STAGES) * KQ, tr = smem_u32(prep[c & 3].tri);
       wait_bar(&bar.kq_full[c % STAGES], c / STAGES, quit);
       wait_bar(&bar.ops_full[c & 3], c >> 2, quit);
@@ -478,36 +529,39 @@ __global__ void __launch_bounds__(kThreads, 1) delta_chunk_kernel(DeltaArgs a) {
       wait_bar(&bar.pq_read, c, quit);          // (and the outputs of chunk c - 1 have been read)
       wait_bar(&bar.u1_full, c, quit);
       tcgen05_fence_after();
-      const bool bad = prep[c & 3].sc.bad || sm.solve_bad[st] == c + 1 || sm.state_bad[st] == c + 1;
-      if (elect_one()) {
-        if (!bad) {                // U times the keys, whose rows are the tokens
-          const uint32_t lo = desc_lo(base, SUB);
+      if (elect_one()) {          // U times the keys, whose rows are the tokens
+        const uint32_t lo = desc_lo(base, SUB);
 #pragma unroll 1
-          for (int x = 0; x < 6; ++x) {
-            const uint32_t at = tmem + tU1 + ((kFirst >> (2 * x)) & 3) * 16, lb = lo + ((kSecond >> (2 * x)) & 3) * (SLICE / 16);
-            const uint32_t d = tmem + (x == 0 ? tXS : tYS);
-            umma_ts(d, at, lb, idesc(KD, 1), x > 1);
-            umma_ts(d, at + 8, lb + 16 * 128 / 16, idesc(KD, 1), 1);
-          }
+        for (int x = 0; x < 6; ++x) {
+          const uint32_t at = tmem + tU1 + ((kFirst >> (2 * x)) & 3) * 16, lb = lo + ((kSecond >> (2 * x)) & 3) * (SLICE / 16);
+          const uint32_t d = tmem + (x == 0 ? tXS : tYS);
+          umma_ts(d, at, lb, idesc(KD, 1), x > 1);
+          umma_ts(d, at + 8, lb + 16 * 128 / 16, idesc(KD, 1), 1);
         }
         umma_commit(&bar.s2);
-        sm.skip[st] = bad;
-        if (bad) *(volatile int*)&sm.stop = 1;
         mbar_arrive(&bar.s2);
-        if (bad) mbar_arrive(&bar.kq_empty[c % STAGES]);       // nothing reads these rows any more: their warps go on and find `stop`
       }
       __syncwarp();
-      if (bad) {
-        for (int f = c + 1; f < min(nch, c + 3); ++f) wait_bar(&bar.ops_full[f & 3], f >> 2, quit);      // copies in flight
-        break;
-      }
       wait_bar(&bar.u2_full, c, quit);
       tcgen05_fence_after();
       if (elect_one()) {
         by_triangle(tmem + tO, tmem + tU2, tmem + tU2 + 32, desc_lo(tr) + 4);
         umma_commit(&bar.o2);
-        umma_commit(&bar.kq_empty[c % STAGES]);
       }
+      __syncwarp();
+      wait_bar(&bar.verdict, c, quit);
+      if (bad(c)) {
+        wait_bar(&bar.o2, c, quit);
+        // nothing reads the later rows of k and q: their warps get this chunk's place and find `stop`.  (No other phase is completed out of turn: a warp that
+        // still waits for the one before would never see it.)
+        if (lane == 0) {
+          *(volatile int*)&sm.stop = 1;
+          mbar_arrive(&bar.kq_empty[c % STAGES]);
+        }
+        for (int f = c + 1; f < min(nch, c + 3); ++f) wait_bar(&bar.ops_full[f & 3], f >> 2, quit);      // copies in flight
+        break;
+      }
+      if (elect_one()) umma_commit(&bar.kq_empty[c % STAGES]);
       __syncwarp();
       if (c + 3 < nch) fetch(c + 3);        // (over chunk c - 1, whose outputs the state's warps have stored)
     }
@@ -579,6 +633,7 @@ __global__ void __launch_bounds__(128, 5) delta_prep_kernel(DeltaArgs a) {
     }
   }
   bad = __syncthreads_or(bad);
+  int zeros = 0;
   {
     // scores: 4 rows x 4 keys per thread (rows r, r + 16, .. of [k; q], keys j, j + 8, ..), two sums a pair
     const int r = threadIdx.x >> 3, j = threadIdx.x & 7;
@@ -613,9 +668,10 @@ __global__ void __launch_bounds__(128, 5) delta_prep_kernel(DeltaArgs a) {
       for (int y = 0; y < 4; ++y) {
         const float2 s = unpack(all[x][y]);
         sm.g[r + 16 * x][j + 8 * y] = s.x + s.y;
+        if (x < 2) zeros += s.x + s.y == 0.f && r + 16 * x < n && j + 8 * y < n;
       }
   }
-  __syncthreads();
+  const bool sparse = __syncthreads_count(zeros >= 2) >= 32;        // scores of the keys with one another that are exactly 0
   // value heads of the key head, two at a time: even warps L and T, odd warps the outputs' weights; a token per lane
   const bool is_q = warp & 1;
   const int w2 = warp >> 1;
@@ -669,8 +725,13 @@ __global__ void __launch_bounds__(128, 5) delta_prep_kernel(DeltaArgs a) {
       no |= s.huge;
       out.sc.be[lane] = be;
       out.sc.bk[lane] = be * ks * since;
+      out.sc.decay[lane] = sparse ? 0.f : expf(lg);
       out.sc.gend[lane] = end * s.inv * 0x1p-12f;
+      float low = since;
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) low = fminf(low, __shfl_xor_sync(0xffffffffu, low, o));
       if (lane == 31) {
+        out.sc.low = sparse ? 0.f : low;
         out.sc.all = since;
         out.sc.most = s.s * 0x1p12f;
       }

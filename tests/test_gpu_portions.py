@@ -199,6 +199,46 @@ def test_delta_over_chunks_channels_of_unequal_size(monkeypatch):
     assert _delta_worst(state.transpose(2, 3), ends, 3) < 4e-6          # each key row of the state
 
 
+@pytest.mark.parametrize("what", ["1e3", "1e6", "1e12", "1e29", "early 1e12", "forgotten 1e6", "unequal tokens", "forgetful", "sparse keys", "small first token"])
+def test_delta_over_chunks_wide_numbers(what, monkeypatch):
+    """Numbers of very different size in one chunk and column: a large value takes nothing from the tokens in front of it, from other columns, or from
+    tokens behind a decay that has forgotten it; tokens of 2^-12 to 2^12, also where each stands alone (strong decays; keys with one channel each).  Bound: 2^-24 a
+    term, 32 of them: 2e-6 of every token's own norm, tokens behind a value that the rule itself cancels left out."""
+    from llmss_b200.ops import cuda_impl as cu
+
+    monkeypatch.setattr(cu, "_delta_over_chunks", lambda *a: True)
+    torch.manual_seed(4)
+    n, heads, d = 160, 2, 128
+    (q, k, v), b, S0 = _delta_inputs([n], heads, heads, d, d, True)
+    u, at, ctx, last = torch.rand(n, heads, device="cuda"), 77, 3, n
+    g, V = -0.3 * u, v.view(n, heads, d)
+    if what[-1].isdigit():
+        at = 66 if "early" in what else at
+        V[at, 1, 7] = float(what.split()[-1])
+        if "forgotten" in what:
+            g = torch.where(u < 0.2, -40.0, g)
+        else:
+            last = at
+    elif what == "small first token":
+        ctx, V[0] = 0, V[0] * 2.0 ** -20
+    else:
+        V.mul_(torch.exp2(torch.rand(n, 1, 1, device="cuda") * 24 - 12))
+    if what == "forgetful":
+        g = -3.0 - 9.0 * u
+    if what == "sparse keys":
+        i = torch.randint(0, d, (n, heads, 1), device="cuda")
+        k.zero_().view(n, heads, d).scatter_(2, i, 1.0)
+        q.zero_().view(n, heads, d).scatter_(2, i.roll(3, 0), 1.0)
+    state = S0.transpose(2, 3).contiguous()
+    want, ends = _delta64(q, k, v, g, b, S0.double().cpu(), [n], [ctx], heads, heads, d, d, True)
+    got = ops.delta_scan(q, k, v, g, b, _batch([n], [ctx], [0]), state, heads, heads, d, d, unit_eps=1e-6, q_scale=0.25, beta_sigmoid=True).view(n, heads, d)
+    keep = want[:last].norm(dim=(1, 2)) > 0
+    assert _delta_worst(got[:last][keep.cuda()], want[:last][keep], (1, 2)) < 2e-6
+    others = [i for i in range(d) if i != 7]
+    assert _delta_worst(got[..., others], want[..., others], 0) < 1e-6              # each other column over all tokens
+    assert _delta_worst(state.transpose(2, 3)[..., others], ends[..., others], 2) < 1e-6
+
+
 @pytest.mark.parametrize("where", ["value", "key", "strength", "decay", "state", "huge value"])
 def test_delta_over_chunks_bad_numbers(where, monkeypatch):
     """A value that is no number, or too large to scale, reaches what it reaches token by token: later tokens of its column (value, state) or of
