@@ -9,7 +9,7 @@
 //   warp 0      TMA producer: Q once, then K_j / V_j tiles (2-stage rings, keys a tile ahead of values), 128B-swizzled
 //   warp 1      issues  S_j = Q K_j^T  (A,B K-major) -> TMEM [128 x BN] fp32, double-buffered: S runs up
 //               to two tiles ahead of the softmax (D = 256: gated only by "softmax has copied S out of TMEM"), and with P in
-//               tensor memory (D <= 128) also the other product: P_j V_j and, over P_j, S_{j+2} back to back
+//               tensor memory (D <= 128) also the other product: P_j V_j and, once it has read P_j, S_{j+2} over it
 //   warp 6      D = 256: issues  O += P_j V_j   (B = V, MN-major) -> TMEM [128 x D] fp32, as soon as P_j is published
 //   warps 2-5   one thread per query row: tcgen05.ld its S row, scale + causal mask, online softmax in
 //               fp32 (no shuffles: the row is thread-private), write P_j (bf16/fp16) into one of two
@@ -366,7 +366,7 @@ attn_prefill_kernel(const __grid_constant__ CUtensorMap tmap, const __grid_const
     }
   } else if (C::P_TMEM && warp == 1) {
     // ===================== both products from one warp (whole warp runs the loop, one elected lane issues) =================
-    // S_{j+2} goes over P_j: issued behind PV_j by the same thread it runs behind it, and no barrier stands between the two
+    // S_{j+2} goes over P_j: it is issued once PV_j has completed, which the warp that issued PV_j waits for without another warp between
     const int fmt = a.dtype == LLMSS_BF16 ? 1 : 0;
     const uint32_t idesc_s = idesc_f16(fmt, BM, BN, 0);  // S = Q K^T : both operands K-major
     const uint32_t idesc_o = idesc_f16(fmt, BM, SPAN ? (a.dv + 15) / 16 * 16 : D, 1);   // O += P V  : B (= V) is MN-major
@@ -406,6 +406,7 @@ attn_prefill_kernel(const __grid_constant__ CUtensorMap tmap, const __grid_const
       __syncwarp();
       if (j + 2 < n_tiles) {
         mbar_wait(&bar_kfull[j & 1], ((j + 2) >> 1) & 1, 61);
+        mbar_wait(&bar_o[j & 1], (j >> 1) & 1, 64);      // PV_j has read P_j: products of other shapes are not sure to run in the order of issue
         scores(j + 2);
       }
     }
