@@ -884,22 +884,25 @@ def hyper_residual(xs, y=None, mix=None, w_out=None, w_in=None, norm_w=None, eps
     return out
 
 
-def _delta_over_chunks(T, B, max_q, heads, dk, dv):
-    """Whether the gated delta rule goes over chunks of 32 tokens (csrc/delta_chunk.cu) or token by token: the smaller of two estimates in
-    us.  Over chunks a block carries one (sequence, head, 128 columns) through its chunks at 6 us each, one block per SM, 9 us to start and end a block, 13 us for
-    the launches, and the chunks' own part costs 0.55 ns per token and head; token by token the longest portion's chain takes 0.4 us a token, and a full GPU
-    3.2e12 state elements a second.  Measured (chunks / tokens): 16 heads of 128 x 128, prompts of 576 .. 1472: 362 / 907, 8 x 1024: 280 / 635,
-    8 x 64: 39 / 47, 8 x 48: 38 / 37, 32 x 48: 103 / 114, one of 64: 33 / 31, one of 1500: 266 / 604; 32 heads of 64 x 64, 8 x 1024: 610 / 381;
-    32 heads of 128 x 128, 23 portions of 16 .. 46: 148 / 126, 31 of 20 .. 56: 197 / 192, 7 of 52: 64 / 75.
-    Counts that a graph's capture fixes decide, nothing on the device."""
+def _delta_over_chunks(T, B, max_q, heads, qk_heads, dk, dv):
+    """Whether the gated delta rule goes over chunks of 32 tokens (csrc/delta_chunk.cu) or token by token: the smaller of two estimates in us.
+    Over chunks a block carries one (sequence, head, 128 columns) through its chunks at 5.9 us each, one block per SM, 9 us to start and end one more; 24 us are the
+    launches and the first block's; the chunks' own part costs 0.55 ns per token and key head and 0.27 per token and head.  Token by token the longest portion's
+    chain takes 0.4 us a token and a full GPU 3.2e12 state elements a second, the smaller of the two adding a fifth of itself.  Where the mean is below 48
+    tokens some portions may be below a chunk and run token by token behind the others, at most 31 tokens of each.
+    Measured (chunks / tokens): 16 heads of 128 x 128 over 8 key heads, prompts of 576 .. 1472: 344 / 910, 8 x 1024: 286 / 640, 11 of 77 on average: 78 / 99, 12 of 49:
+    86 / 67, 8 x 64: 41 / 50, one of 64: 40 / 34, one of 1500: 288 / 610; 32 over 16, 7 of 52: 63 / 73, 4 of 52: 49 / 56, 23 of 16 .. 46: 149 / 128, 20 of 41: 139 / 143;
+    32 heads of 64 x 64, prompts of 576 .. 1472: 702 / 550, 8 x 1024: 622 / 386, one of 1500: 306 / 554; 16 of 32 x 32, 8 x 1024: 277 / 399.
+    Counts on the host decide, which a graph's capture fixes; nothing on the device.  So the form, and with it the last bits of a sequence's results, may depend on
+    the batch that it comes in."""
     if max_q < 32 or dk > 128 or dk % 4 or B > 65535 or heads > 65535:
         return False
-    blocks = B * heads * -(-dv // 128)
+    waves, chain = -(-B * heads * -(-dv // 128) // 148), 0.4 * max_q
     arithmetic = T * heads * dk * dv / 3.2e6
-    chunks = max(6.0 * -(-max_q // 32), -(-blocks // 148) * (6.0 * -(-T // (32 * B)) + 9.0) - 9.0) + 22.0 + 0.55e-3 * T * heads
-    if T < 48 * B:          # some of the portions are below a chunk, and run token by token behind the others
-        chunks += 0.5 * arithmetic
-    return chunks < max(0.4 * max_q, arithmetic) + 5.0
+    chunks = 5.9 * -(-max_q // 32) + (waves - 1) * (5.9 * (T / (32 * B) + 0.5) + 9.0) + 24.0 + T * (0.55e-3 * qk_heads + 0.27e-3 * heads)
+    if T < 48 * B:
+        chunks += 0.5 * arithmetic * min(T - max_q, 31 * (B - 1)) / T
+    return chunks < max(chain, arithmetic) + 0.2 * min(chain, arithmetic) + 6.0
 
 
 def delta_scan(q, k, v, log_decay, beta, batch, state, heads, qk_heads, dk, dv, unit_eps=None, q_scale=1.0, beta_sigmoid=False):
@@ -914,7 +917,7 @@ def delta_scan(q, k, v, log_decay, beta, batch, state, heads, qk_heads, dk, dv, 
     cu, sl, ss, B, mq = _bq(batch)
     args = (_ptr(q), ldq, _ptr(k), ldk, _ptr(v), ldv, _ptr(log_decay), ldg, _ptr(beta), ldb, _ptr(out), _ptr(state),
             cu, sl, ss, B, mq, heads, qk_heads, dk, dv, -1.0 if unit_eps is None else float(unit_eps), float(q_scale), 1 if beta_sigmoid else 0)
-    if _delta_over_chunks(T, B, mq, heads, dk, dv) and ldq % 4 == 0 and ldk % 4 == 0 and (args[0] | args[2] | args[11]) % 16 == 0:
+    if _delta_over_chunks(T, B, mq, heads, qk_heads, dk, dv) and ldq % 4 == 0 and ldk % 4 == 0 and (args[0] | args[2] | args[11]) % 16 == 0:
         scratch = torch.empty(lib.llmss_delta_scan_chunked_bytes(T, B, heads), dtype=torch.uint8, device=v.device)
         _lib.check(lib.llmss_delta_scan_chunked(*args, _ptr(scratch), _stream()), "llmss_delta_scan_chunked")
     else:
