@@ -176,6 +176,50 @@ def test_delta_over_chunks_costs_no_more_where_it_cannot_be_used(monkeypatch):
     assert best(True) < 1.6 * best(False)
 
 
+def test_delta_over_chunks_in_odd_batches(monkeypatch):
+    """An empty sequence, one without a slot, slots in another order than the batch, scratch that holds other bytes; then the same call captured and
+    replayed from the same state, and with rows off the 16-byte lines (token by token).  Bound: 32-bit sums, 1e-6 of the norm."""
+    from llmss_b200.ops import cuda_impl as cu
+
+    monkeypatch.setattr(cu, "_delta_over_chunks", lambda *a: True)
+    torch.manual_seed(6)
+    lens, ctxs, slots, heads, qk_heads, d = [64, 0, 40, 5, 97], [0, 4, 3, 2, 6], [3, 1, -1, 0, 5], 4, 2, 128
+    T, rows = sum(lens), slice(64, 104)
+    (q, k, v), b, S0 = _delta_inputs(lens, heads, qk_heads, d, d, True)
+    g, batch = -0.3 * torch.rand(T, heads, device="cuda"), _batch(lens, ctxs, slots)
+    start = torch.randn(6, heads, d, d, device="cuda")
+    live = [i for i in range(len(lens)) if slots[i] >= 0 and lens[i]]
+    start[[slots[i] for i in live]] = S0[live].transpose(2, 3)
+    want, ends = _delta64(q, k, v, g, b, S0.double().cpu(), lens, ctxs, heads, qk_heads, d, d, True)
+
+    def check(got, state):
+        got = torch.cat([got[:rows.start], got[rows.stop:]])
+        assert _rel(got, torch.cat([want[:rows.start], want[rows.stop:]]).reshape(got.shape)) < 1e-6
+        assert _rel(state[[slots[i] for i in live]].transpose(2, 3), ends[live]) < 1e-6
+        assert torch.equal(state[[1, 2, 4]], start[[1, 2, 4]])          # nobody's, an empty sequence's
+
+    def call(q, k, state):
+        return ops.delta_scan(q, k, v, g, b, batch, state, heads, qk_heads, d, d, unit_eps=1e-6, q_scale=0.25, beta_sigmoid=True)
+
+    dirty = torch.full((1 << 20,), 255, dtype=torch.uint8, device="cuda")
+    del dirty
+    state = start.clone()
+    eager = call(q, k, state)
+    check(eager, state)
+
+    held, graph = start.clone(), torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        out = call(q, k, held)
+    for _ in range(2):
+        held.copy_(start)
+        graph.replay()
+        assert torch.equal(held, state) and torch.equal(out[:rows.start], eager[:rows.start]) and torch.equal(out[rows.stop:], eager[rows.stop:])
+
+    off = [torch.empty(T, x.shape[1] + 1, device="cuda")[:, 1:].copy_(x) for x in (q, k)]
+    state = start.clone()
+    check(call(*off, state), state)
+
+
 def _delta_worst(got, want, dims):
     """Largest error of a part (a token of a head, a column, ..) over the norm of that part."""
     return float(((got.double().cpu() - want).norm(dim=dims) / want.norm(dim=dims).clamp_min(1e-300)).max())
