@@ -30,8 +30,8 @@
 // each, one after another: 8 prompts of 576 .. 1472 tokens whose decays grow 910 us token by token, 5267 so, 1005 now; a batch takes no longer than
 // its chunks in front of such ones and their sequences' other tokens, one launch after the other.)
 //
-// B200, 16 heads of 128 x 128, against token by token: 8 prompts of 576 .. 1472 tokens 910 -> 344 us (68 + 273 for the two launches, 3 for the one behind),
-// 8 of 1024 640 -> 286, one of 1500 610 -> 288, 8 of 64 50 -> 41; without the three tests of the numbers' size 336, 268, 264 and 40.  Against 64 bits, of the
+// B200, 16 heads of 128 x 128, against token by token: 8 prompts of 576 .. 1472 tokens 910 -> 343 us (68 + 272 for the two launches, 3 for the one behind),
+// 8 of 1024 640 -> 284, one of 1500 610 -> 278, 8 of 64 50 -> 41; without the three tests of the numbers' size 336, 268, 264 and 40.  Against 64 bits, of the
 // norm (token by token in brackets): outputs 1.3e-7 (1.5e-7), states 7.9e-8 (1.1e-7); decays near 1 1.3e-7 (2.7e-7) and 1.1e-7 (2.5e-7); worst token 2.3e-7
 // (2.7e-7), worst column 1.7e-7 (1.9e-7).  The second launch is bound by its chain, 5.9 us or about 11 000 clocks a chunk: products with
 // the state 2000, R 1000, T R 500, U 1000, the update's product 1300, the state 3200, half of each the arithmetic of splitting (24 clocks of a
@@ -64,7 +64,7 @@ struct __align__(16) Scalars {      // of a chunk and head, per token
   float gend[C];                    // decay to the chunk's end * scale of k, of `most`
   float as[C];                      // scales of the rows of the outputs' weights
   float decay[C];                   // of a token; 0 in a chunk of sparse keys (see spread)
-  float all, most, low;             // decay of the chunk; a power of two; the smallest decay since its start
+  float all, most, low;             // decay of the chunk; a power of two; the smallest decay since its start, negative in a chunk of sparse keys
   int bad;                          // not for the products
   int pad[31];
   int done[kDeltaDone];             // (of a sequence's first chunk) tokens that the second launch has done, per 128 value columns
@@ -144,12 +144,11 @@ __device__ __forceinline__ void lds_pairs(const float* p, pair_t& x, pair_t& y) 
 // in all 32 columns of the warp, or five tokens of a column, are not.  s: scale of the column's state.  The same answer for the whole warp.
 // The state has the like (in its warps): 8 of a thread's 64 key rows below 2^-11 to 2^-12 of the column's largest, 3 once keys were sparse.
 // Earlier forms: in front of T R in the chain 343 -> 349 us, the state's count beside U 352.
-__device__ __forceinline__ bool spread(const pair_t (&y)[C / 2], const Scalars& sc, float s, float us) {
+__device__ __forceinline__ bool spread(const pair_t (&y)[C / 2], const Scalars& sc, int tokens, float s, float us) {
   float n = s > 0x1p-98f ? s * 0x1p11f : 0.f;
   if (__all_sync(0xffffffffu, n * sc.low >= us)) return false;          // the usual case: the state alone is not small at any token
   const float most = __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(us)));
-  uint32_t small = 0, some = 0;
-  int few = 0;
+  uint32_t small = 0, some = 0, few = 0;
 #pragma unroll
   for (int i = 0; i < C; i += 4) {
     const float4 f = *reinterpret_cast<const float4*>(sc.decay + i);
@@ -160,10 +159,11 @@ __device__ __forceinline__ bool spread(const pair_t (&y)[C / 2], const Scalars& 
       n = fmaxf(n * by[e], fabsf(x[e]) * us);
       if (n < most) small |= 1u << (i + e);
       if (n > 0.f) some |= 1u << (i + e);
-      few += n > 0.f && n < us;
+      if (n > 0.f && n < us) few |= 1u << (i + e);
     }
   }
-  return (__reduce_and_sync(0xffffffffu, small) & __reduce_or_sync(0xffffffffu, some)) != 0 || __any_sync(0xffffffffu, few >= 5);
+  const uint32_t there = tokens < C ? (1u << tokens) - 1 : ~0u;
+  return (__reduce_and_sync(0xffffffffu, small) & __reduce_or_sync(0xffffffffu, some) & there) != 0 || __any_sync(0xffffffffu, __popc(few & there) >= 5);
 }
 
 __global__ void __launch_bounds__(kThreads, 1) delta_chunk_kernel(DeltaArgs a) {
@@ -296,7 +296,7 @@ __global__ void __launch_bounds__(kThreads, 1) delta_chunk_kernel(DeltaArgs a) {
       arrive_warp(&bar.u1_full);
       put_row(row + tU2, row + tU2 + 32, x);
       arrive_warp(&bar.u2_full);
-      if (spread(x, sc, sm.s_scale[v], us) && lane == 0) sm.solve_bad[st] = c + 1;
+      if (spread(x, sc, n, sm.s_scale[v], us) && lane == 0) sm.solve_bad[st] = c + 1;
       __syncwarp();
       if (lane == 0) mbar_arrive(&bar.verdict);
     }
@@ -355,7 +355,7 @@ __global__ void __launch_bounds__(kThreads, 1) delta_chunk_kernel(DeltaArgs a) {
           few += (2 * __float_as_uint(x.x) - 1 < below) + (2 * __float_as_uint(x.y) - 1 < below);
         }
         wait_bar(&bar.ops_full[c & 3], c >> 2, quit);
-        if (prep[c & 3].sc.low == 0.f) most_few = 2;
+        if (prep[c & 3].sc.low < 0.f) most_few = 2;
         if (__any_sync(0xffffffffu, few > most_few) && lane == 0) sm.state_bad[c & 1] = c + 1;
       } else {
         wait_bar(&bar.o2, c - 1, quit);
@@ -731,7 +731,7 @@ __global__ void __launch_bounds__(128, 5) delta_prep_kernel(DeltaArgs a) {
 #pragma unroll
       for (int o = 16; o > 0; o >>= 1) low = fminf(low, __shfl_xor_sync(0xffffffffu, low, o));
       if (lane == 31) {
-        out.sc.low = sparse ? 0.f : low;
+        out.sc.low = sparse ? -1.f : low;
         out.sc.all = since;
         out.sc.most = s.s * 0x1p12f;
       }

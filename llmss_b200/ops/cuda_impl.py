@@ -890,8 +890,8 @@ def _delta_over_chunks(T, B, max_q, heads, qk_heads, dk, dv):
     launches and the first block's; the chunks' own part costs 0.55 ns per token and key head and 0.27 per token and head.  Token by token the longest portion's
     chain takes 0.4 us a token and a full GPU 3.2e12 state elements a second, the smaller of the two adding a fifth of itself.  Where the mean is below 48
     tokens some portions may be below a chunk and run token by token behind the others, at most 31 tokens of each.
-    Measured (chunks / tokens): 16 heads of 128 x 128 over 8 key heads, prompts of 576 .. 1472: 344 / 910, 8 x 1024: 286 / 640, 11 of 77 on average: 78 / 99, 12 of 49:
-    86 / 67, 8 x 64: 41 / 50, one of 64: 40 / 34, one of 1500: 288 / 610; 32 over 16, 7 of 52: 63 / 73, 4 of 52: 49 / 56, 23 of 16 .. 46: 149 / 128, 20 of 41: 139 / 143;
+    Measured (chunks / tokens): 16 heads of 128 x 128 over 8 key heads, prompts of 576 .. 1472: 343 / 910, 8 x 1024: 284 / 640, 11 of 77 on average: 78 / 99, 12 of 49:
+    86 / 67, 8 x 64: 41 / 50, one of 64: 40 / 34, one of 1500: 278 / 610; 32 over 16, 7 of 52: 63 / 73, 4 of 52: 49 / 56, 23 of 16 .. 46: 149 / 128, 20 of 41: 139 / 143;
     32 heads of 64 x 64, prompts of 576 .. 1472: 702 / 550, 8 x 1024: 622 / 386, one of 1500: 306 / 554; 16 of 32 x 32, 8 x 1024: 277 / 399.
     Counts on the host decide, which a graph's capture fixes; nothing on the device.  So the form, and with it the last bits of a sequence's results, may depend on
     the batch that it comes in."""

@@ -33,7 +33,7 @@ PROMPTS = [576, 640, 777, 900, 1024, 1100, 1300, 1472]
 
 
 @pytest.mark.parametrize("heads,qk_heads,d,lens,chunks,tokens", [
-    (16, 8, 128, PROMPTS, 344, 910), (16, 8, 128, [1024] * 8, 286, 640), (16, 8, 128, [1500], 288, 610), (16, 8, 128, [4096], 794, 1660), (16, 8, 128, [64] * 8, 41, 50),
+    (16, 8, 128, PROMPTS, 343, 910), (16, 8, 128, [1024] * 8, 284, 640), (16, 8, 128, [1500], 278, 610), (16, 8, 128, [4096], 794, 1660), (16, 8, 128, [64] * 8, 41, 50),
     (16, 8, 128, [112] + [73] * 9 + [78], 78, 99), (16, 8, 128, [1000] + [8] * 31, 243, 667), (16, 8, 128, [200, 16] * 8, 102, 181), (32, 16, 128, [72] + [45] * 3, 49, 56),
     (32, 32, 64, [1500], 306, 554), (16, 8, 32, [1024] * 8, 277, 399), (64, 32, 128, [512] * 8, 552, 1082), (4, 4, 128, [1024] * 2, 196, 422),
     (32, 32, 64, PROMPTS, 702, 550), (32, 32, 64, [1024] * 8, 622, 386), (16, 8, 128, [64], 40, 34), (16, 8, 128, [32] * 8, 36, 31), (16, 8, 128, [71] + [47] * 11, 86, 67),

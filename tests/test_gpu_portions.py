@@ -283,6 +283,35 @@ def test_delta_over_chunks_wide_numbers(what, monkeypatch):
     assert _delta_worst(state.transpose(2, 3)[..., others], ends[..., others], 2) < 1e-6
 
 
+@pytest.mark.parametrize("decay,stays", [("mild", True), ("slow", True), ("strong", True), ("resets", True), ("strong, unequal tokens", False), ("growing", False)])
+def test_delta_over_chunks_keeps_ordinary_inputs(decay, stays):
+    """The record of a sequence's first chunk says how many tokens went over chunks: all of them for SiLU inputs under decays of any size, with whole and partial
+    last chunks; not all for tokens of 2^-12 to 2^12 that decays part, and none for decays that grow."""
+    from llmss_b200.ops import _lib, cuda_impl as cu
+
+    torch.manual_seed(8)
+    lens, heads, qk_heads, d = [640, 33, 417, 512, 100, 290], 8, 4, 128
+    T, B = sum(lens), len(lens)
+    q, k, v = (torch.nn.functional.silu(torch.randn(T, n * d, device="cuda")) for n in (qk_heads, qk_heads, heads))
+    if "unequal" in decay:
+        v *= torch.exp2(torch.rand(T, 1, device="cuda") * 24 - 12)
+    u, b = torch.rand(T, heads, device="cuda"), torch.randn(T, heads, device="cuda")
+    g = {"mild": -0.3 * u, "slow": -0.01 * u, "strong": -3.0 - 9.0 * u, "resets": torch.where(u < 0.02, -20.0, -0.1 * u), "growing": 0.3 + 0.0 * u}[decay.split(",")[0]]
+    batch, state, out = _batch(lens, [0] * B, range(B)), torch.empty(B, heads, d, d, device="cuda"), torch.empty(T, heads * d, device="cuda")
+    lib, p = _lib.load(), cu._ptr
+    scratch = torch.empty(lib.llmss_delta_scan_chunked_bytes(T, B, heads), dtype=torch.uint8, device="cuda")
+    _lib.check(lib.llmss_delta_scan_chunked(p(q), q.stride(0), p(k), k.stride(0), p(v), v.stride(0), p(g), heads, p(b), heads, p(out), p(state), p(batch.cu_q),
+                                            p(batch.seq_lens), p(batch.state_slots), B, max(lens), heads, qk_heads, d, d, 1e-6, d ** -0.5, 1, p(scratch), cu._stream()),
+               "chunked")
+    records = scratch.view(-1, heads, 13312)[:, :, 13312 - 4 * 29:13312 - 4 * 28].contiguous().view(torch.int32)[:, :, 0].cpu()
+    firsts = [sum(lens[:i]) // 32 + i for i in range(B)]
+    done = records[firsts]
+    if stays:
+        assert torch.equal(done, torch.tensor(lens, dtype=torch.int32)[:, None].expand(-1, heads))
+    else:
+        assert (done < torch.tensor(lens)[:, None]).any() and (decay != "growing" or not done.any())
+
+
 @pytest.mark.parametrize("where", ["value", "key", "strength", "decay", "state", "huge value"])
 def test_delta_over_chunks_bad_numbers(where, monkeypatch):
     """A value that is no number, or too large to scale, reaches what it reaches token by token: later tokens of its column (value, state) or of
