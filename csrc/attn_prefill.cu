@@ -1,6 +1,6 @@
 // K8 attn_prefill: causal varlen flash-attention forward on the 5th-generation tensor cores.
 //
-// Replaces the reference's prefill attention (SURVEY.md G7/G8/G17: cuBLAS QK^T into a materialised
+// Replaces the reference's prefill attention (cuBLAS QK^T into a materialised
 // [B,h,S,T] fp32 score tensor, where-mask from a [max_pos,max_pos] bool buffer, softmax, cuBLAS PV;
 // gptj_modeling.py:128-169, gpt_bigcode_modeling.py:170-246) with one kernel that never
 // materialises S^2 data:
@@ -34,7 +34,7 @@
 // them the kernel takes 106 us instead of 118) nor the exponentials (without them 110), but the hand-overs of a 64-key tile between warps, each 100
 // to 300 clocks beside busy warps, and the 4000 clocks before a CTA's first tile.  One issuing warp instead of two that wait for one
 // another, descriptors of two additions, keys copied a tile ahead and the copies started before tensor memory is there: 119 -> 113 us
-// (under the power cap 138 -> 131).  Tried and slower: 128-key tiles with one S buffer (135 -> 152), two teams of softmax warps on
+// (under the power cap 138 -> 134); 112 without the wait between P_j V_j and S_{j+2}.  Tried and slower: 128-key tiles with one S buffer (135 -> 152), two teams of softmax warps on
 // alternate tiles (141 -> 157), the heaviest query tiles of all heads first (120 -> 133: keys and values leave L2).
 #include "common.cuh"
 
@@ -161,19 +161,7 @@ __device__ __forceinline__ float ex2_fma(float x) {
   return __int_as_float(__float_as_int(p) + (n << 23));
 }
 
-// Products from the descriptors' lower words (the upper word is the same for all tiles of 128-byte swizzled rows): two additions a product for the
-// warp that issues them, where descriptors put together per product took it 100 clocks beside eight softmax warps.
-constexpr uint32_t kDescHi = 0x40004040u;
-__device__ __forceinline__ uint32_t desc_lo(uint32_t addr, uint32_t lbo = 16) { return ((addr & 0x3FFFFu) >> 4) | ((lbo >> 4) << 16); }
-__device__ __forceinline__ void umma_ss_lo(uint32_t d, uint32_t a_lo, uint32_t b_lo, uint32_t id, uint32_t acc) {
-  asm volatile("{\n\t.reg .pred p;\n\t.reg .b64 a, b;\n\tsetp.ne.b32 p, %4, 0;\n\tmov.b64 a, {%1, %5};\n\tmov.b64 b, {%2, %5};\n\t"
-               "tcgen05.mma.cta_group::1.kind::f16 [%0], a, b, %3, p;\n\t}" ::"r"(d), "r"(a_lo), "r"(b_lo), "r"(id), "r"(acc), "r"(kDescHi) : "memory");
-}
-// the A operand (M x 16, 16-bit, two K elements per 32-bit column, row m in lane m) from tensor memory
-__device__ __forceinline__ void umma_ts_lo(uint32_t d, uint32_t a, uint32_t b_lo, uint32_t id, uint32_t acc) {
-  asm volatile("{\n\t.reg .pred p;\n\t.reg .b64 b;\n\tsetp.ne.b32 p, %4, 0;\n\tmov.b64 b, {%2, %5};\n\t"
-               "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], b, %3, p;\n\t}" ::"r"(d), "r"(a), "r"(b_lo), "r"(id), "r"(acc), "r"(kDescHi) : "memory");
-}
+using namespace umma_lo;
 
 template <typename T>
 __device__ __forceinline__ uint32_t pack2(float a, float b) {
@@ -380,7 +368,7 @@ attn_prefill_kernel(const __grid_constant__ CUtensorMap tmap, const __grid_const
 #pragma unroll
           for (int k = 0; k < 4; ++k)
             if (!SPAN || c * 64 + k * 16 < a.dkp)
-              umma_ss_lo(d, q_lo + (c * (BM * 128) + k * 32) / 16, k_lo + (c * (BN * 128) + k * 32) / 16, idesc_s, (c | k) ? 1u : 0u);
+              umma_ss(d, q_lo + (c * (BM * 128) + k * 32) / 16, k_lo + (c * (BN * 128) + k * 32) / 16, idesc_s, (c | k) ? 1u : 0u);
         umma_commit(&bar_s[j & 1]);
         umma_commit(&bar_kempty[j & 1]);
       }
@@ -399,7 +387,7 @@ attn_prefill_kernel(const __grid_constant__ CUtensorMap tmap, const __grid_const
       if (elect_one()) {
 #pragma unroll
         for (int k = 0; k < BN / 16; ++k)      // 16 keys = 8 packed columns per step, P_j sits at the start of S buffer j & 1
-          umma_ts_lo(tO, p + k * 8, v_lo + k * 128, idesc_o, (j > 0 || k > 0) ? 1u : 0u);
+          umma_ts(tO, p + k * 8, v_lo + k * 128, idesc_o, (j > 0 || k > 0) ? 1u : 0u);
         umma_commit(&bar_o[j & 1]);
         umma_commit(&bar_vempty[j & 1]);
       }

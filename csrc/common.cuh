@@ -4,7 +4,7 @@
 // mbarrier pipelines, TMA (cp.async.bulk.tensor), tcgen05 (alloc / mma / commit / ld),
 // system-scope acquire/release for the NVLink peer-memory protocols, and a bounded-spin
 // watchdog so a lost peer or a broken pipeline traps instead of hanging the GPU
-// (SURVEY.md section 5.3: the reference's only failure detection is the 60 s c10d timeout).
+// (the reference's only failure detection is the 60 s c10d timeout).
 #pragma once
 #include <cuda_runtime.h>
 #include <cuda_fp16.h>
@@ -311,6 +311,68 @@ __device__ __forceinline__ void fmul2(float& d0, float& d1, float a0, float a1, 
   asm("{\n\t.reg .b64 a, b, d;\n\tmov.b64 a, {%2, %3};\n\tmov.b64 b, {%4, %5};\n\tmul.rn.f32x2 d, a, b;\n\tmov.b64 {%0, %1}, d;\n\t}"
       : "=f"(d0), "=f"(d1) : "f"(a0), "f"(a1), "f"(b0), "f"(b1));
 }
+
+// The same on numbers that stay in pairs.
+namespace packed {
+
+using pair_t = uint64_t;
+__device__ __forceinline__ pair_t pfma(pair_t x, pair_t y, pair_t z) {
+  pair_t d;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(x), "l"(y), "l"(z));
+  return d;
+}
+__device__ __forceinline__ pair_t pmul(pair_t x, pair_t y) {
+  pair_t d;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(x), "l"(y));
+  return d;
+}
+__device__ __forceinline__ pair_t padd(pair_t x, pair_t y) {
+  pair_t d;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(x), "l"(y));
+  return d;
+}
+__device__ __forceinline__ pair_t psub(pair_t x, pair_t y) {
+  pair_t d;
+  asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(x), "l"(y));
+  return d;
+}
+__device__ __forceinline__ pair_t pack(float lo, float hi) {
+  pair_t d;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(d) : "f"(lo), "f"(hi));
+  return d;
+}
+__device__ __forceinline__ pair_t pack(uint32_t lo, uint32_t hi) {
+  pair_t d;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(d) : "r"(lo), "r"(hi));
+  return d;
+}
+__device__ __forceinline__ pair_t both(float x) { return pack(x, x); }
+__device__ __forceinline__ float2 unpack(pair_t v) {
+  float2 r;
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
+  return r;
+}
+
+}  // namespace packed
+
+// ---------------------------------------------------------------- products by halves of their descriptors
+// The upper word of a shared-memory descriptor is the same for all tiles of 128-byte swizzled rows, so that a product costs the warp that issues it two
+// additions (descriptors put together per product: 100 clocks beside eight softmax warps).
+namespace umma_lo {
+
+constexpr uint32_t kDescHi = 0x40004040u;
+__device__ __forceinline__ uint32_t desc_lo(uint32_t addr, uint32_t lbo = 16) { return ((addr & 0x3FFFFu) >> 4) | ((lbo >> 4) << 16); }
+// A from tensor memory (M x 16, 16-bit, two K elements per 32-bit column, row m in lane m)
+__device__ __forceinline__ void umma_ts(uint32_t d, uint32_t a, uint32_t b_lo, uint32_t id, uint32_t acc) {
+  asm volatile("{\n\t.reg .pred p;\n\t.reg .b64 b;\n\tsetp.ne.b32 p, %4, 0;\n\tmov.b64 b, {%2, %5};\n\t"
+               "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], b, %3, p;\n\t}" ::"r"(d), "r"(a), "r"(b_lo), "r"(id), "r"(acc), "r"(kDescHi) : "memory");
+}
+__device__ __forceinline__ void umma_ss(uint32_t d, uint32_t a_lo, uint32_t b_lo, uint32_t id, uint32_t acc) {
+  asm volatile("{\n\t.reg .pred p;\n\t.reg .b64 a, b;\n\tsetp.ne.b32 p, %4, 0;\n\tmov.b64 a, {%1, %5};\n\tmov.b64 b, {%2, %5};\n\t"
+               "tcgen05.mma.cta_group::1.kind::f16 [%0], a, b, %3, p;\n\t}" ::"r"(d), "r"(a_lo), "r"(b_lo), "r"(id), "r"(acc), "r"(kDescHi) : "memory");
+}
+
+}  // namespace umma_lo
 
 // ---------------------------------------------------------------- visible keys
 // first key position that query position p sees through a sliding window (0: none) and / or a chunked mask (0: none; p sees its own

@@ -10,12 +10,13 @@
 // per token (decay, write strength, the norms 1 / sqrt(sum x^2 + eps), k . q) lie beside them.  The state lies in memory
 // column-major per head ([dv][dk]).
 //
-// Long portions go over chunks of 32 tokens on the tensor cores where that is faster (delta_chunk.cu); this file's portions are the others.
+// Long portions go over chunks of 32 tokens on the tensor cores where that is faster (delta_chunk.cu); this file's portions are the others, and what a
+// launch over chunks leaves of a sequence.
 //
 // A batch of single tokens (decode) runs the row-split form instead (delta_step_kernel): one warp per value column, lanes over
 // the key rows, so that every state access is one contiguous column (512 bytes at dk = 128) -- a decode step is bound by
 // reading and writing the states once.
-// Everything is 32-bit with full-precision exponentials.
+// Everything here is 32-bit with full-precision exponentials (over chunks: products of 16-bit parts, see delta_chunk.cu on rounding).
 #include "common.cuh"
 #include "delta.cuh"
 
@@ -36,25 +37,10 @@ __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_gr
 
 // Two 32-bit numbers per instruction: half the issue slots of the same arithmetic (148 SMs, 8 warps each: 126 against 116 multiply-adds
 // per clock and SM when nothing else is issued, and the slots left over take the shared-memory loads).
-__device__ __forceinline__ uint64_t fma_pair(uint64_t a, uint64_t b, uint64_t c) {
-  uint64_t d;
-  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
-  return d;
-}
-__device__ __forceinline__ uint64_t mul_pair(uint64_t a, uint64_t b) {
-  uint64_t d;
-  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
-  return d;
-}
-__device__ __forceinline__ uint64_t pair_of(float lo, float hi) {
-  uint64_t d;
-  asm("mov.b64 %0, {%1, %2};" : "=l"(d) : "f"(lo), "f"(hi));
-  return d;
-}
+using namespace packed;
 __device__ __forceinline__ float sum_of_pair(uint64_t v) {
-  float lo, hi;
-  asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v));
-  return lo + hi;
+  const float2 x = unpack(v);
+  return x.x + x.y;
 }
 
 // Portions.  Per token a thread makes two dot products with its rows of the OLD state (S^T k and S^T q) and then writes; the
@@ -107,8 +93,8 @@ __global__ void __launch_bounds__(256) delta_scan_kernel(DeltaArgs a) {
           if (i0 + ii + 3 < dk) t4.w = p[i0 + ii + 3];
         }
       }
-      S[c][ii / 2] = pair_of(t4.x, t4.y);
-      S[c][ii / 2 + 1] = pair_of(t4.z, t4.w);
+      S[c][ii / 2] = pack(t4.x, t4.y);
+      S[c][ii / 2 + 1] = pack(t4.z, t4.w);
     }
   // the strips' padding (beyond dk, and between strips) is read by the arithmetic and never copied into: zero it once
   for (int idx = threadIdx.x; idx < 2 * stage_floats; idx += nthr) sm[idx] = 0.f;
@@ -213,14 +199,14 @@ __global__ void __launch_bounds__(256) delta_scan_kernel(DeltaArgs a) {
         kk[2 * ii] = k4.x;
         kk[2 * ii + 1] = k4.y;
         if (ii == 0) {
-          d0 = mul_pair(S[0][0], k4.x); d1 = mul_pair(S[1][0], k4.x);
-          e0 = mul_pair(S[0][0], q4.x); e1 = mul_pair(S[1][0], q4.x);
+          d0 = pmul(S[0][0], k4.x); d1 = pmul(S[1][0], k4.x);
+          e0 = pmul(S[0][0], q4.x); e1 = pmul(S[1][0], q4.x);
         } else {
-          d0 = fma_pair(S[0][2 * ii], k4.x, d0); d1 = fma_pair(S[1][2 * ii], k4.x, d1);
-          e0 = fma_pair(S[0][2 * ii], q4.x, e0); e1 = fma_pair(S[1][2 * ii], q4.x, e1);
+          d0 = pfma(S[0][2 * ii], k4.x, d0); d1 = pfma(S[1][2 * ii], k4.x, d1);
+          e0 = pfma(S[0][2 * ii], q4.x, e0); e1 = pfma(S[1][2 * ii], q4.x, e1);
         }
-        d0 = fma_pair(S[0][2 * ii + 1], k4.y, d0); d1 = fma_pair(S[1][2 * ii + 1], k4.y, d1);
-        e0 = fma_pair(S[0][2 * ii + 1], q4.y, e0); e1 = fma_pair(S[1][2 * ii + 1], q4.y, e1);
+        d0 = pfma(S[0][2 * ii + 1], k4.y, d0); d1 = pfma(S[1][2 * ii + 1], k4.y, d1);
+        e0 = pfma(S[0][2 * ii + 1], q4.y, e0); e1 = pfma(S[1][2 * ii + 1], q4.y, e1);
       }
       float x0 = sum_of_pair(d0), x1 = sum_of_pair(d1);
 #pragma unroll
@@ -230,11 +216,11 @@ __global__ void __launch_bounds__(256) delta_scan_kernel(DeltaArgs a) {
       }
       const float u0 = fmaf(f.x, v2.x, -f.y * x0), u1 = fmaf(f.x, v2.y, -f.y * x1);
       const float w0 = u0 * f.z, w1 = u1 * f.z;
-      const uint64_t g2 = pair_of(f.w, f.w), p0 = pair_of(w0, w0), p1 = pair_of(w1, w1);
+      const uint64_t g2 = pack(f.w, f.w), p0 = pack(w0, w0), p1 = pack(w1, w1);
 #pragma unroll
       for (int ii = 0; ii < KPT / 2; ++ii) {
-        S[0][ii] = fma_pair(g2, S[0][ii], mul_pair(kk[ii], p0));
-        S[1][ii] = fma_pair(g2, S[1][ii], mul_pair(kk[ii], p1));
+        S[0][ii] = pfma(g2, S[0][ii], pmul(kk[ii], p0));
+        S[1][ii] = pfma(g2, S[1][ii], pmul(kk[ii], p1));
       }
       // S^T q of the old state: the first exchange leaves one column per lane
       const float y0 = sum_of_pair(e0), y1 = sum_of_pair(e1);

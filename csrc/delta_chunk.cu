@@ -6,6 +6,7 @@
 // values of a chunk solve a triangular system, and everything else is products:
 //   R_i = beta_i (v_i - exp(G_i) S_0^T k_i)          L_ij = beta_i w_ij k_i . k_j  (j < i)        U = (1 + L)^-1 R
 //   o_i = exp(G_i) S_0^T q_i + sum_(j <= i) w_ij (q_i . k_j) U_j          S = exp(G_C) S_0 + sum_j w_Cj k_j U_j^T
+// (the chunkwise form of the delta rule of Yang, Wang, Zhang, Shen and Kim, 2024, with the decays of Yang, Kautz and Hatamizadeh, 2024).
 // T = (1 + L)^-1 does not depend on the state; for unit keys, strengths up to 1 and decays up to 1 its entries are at most 1.
 //
 // Two launches.  delta_prep_kernel, a block per chunk and key head: scores, L, T, the outputs' weights and the numbers per token, for every value head;

@@ -3,9 +3,8 @@
 //
 //   out[M, N] = epilogue( x[M, K] @ w[N, K]^T )          (w in HF nn.Linear layout)
 //
-// Replaces the reference's cuBLAS `F.linear` call sites (SURVEY.md G3, G4, G9, G10, G12,
-// G14; layers.py:62,123) and, for row-parallel layers, the separate blocking NCCL
-// all-reduce that follows them (N1; layers.py:175-179).
+// Replaces the reference's cuBLAS `F.linear` call sites (layers.py:62,123) and, for row-parallel layers, the separate blocking NCCL
+// all-reduce that follows them (layers.py:175-179).
 //
 // Design (B200-first, not a cuBLAS clone):
 //  * swap-AB: the *weight* tile is the UMMA A operand (M=128 output features per tile) and
@@ -1640,17 +1639,18 @@ gemm_heads_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_const
       const int n = tn * BM + f, m0 = tm * BN;
       const uint32_t t_addr = tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(as * BN);
       const float* sp = a.scale != nullptr ? a.scale + (int64_t)m0 * a.lds + h * a.ssh + (n < a.N ? n : 0) * a.ssn : nullptr;
-      // a factor per token and head (the usual one): a lane loads one of 32 tokens', a chunk ahead, and the warp exchanges them
-      const bool each = sp != nullptr && a.ssn != 0;
+      // a factor per feature: a load per token.  One per token and head (the usual one): a lane loads one of 32 tokens', a chunk ahead, and the warp
+      // exchanges them
+      const bool by_feature = sp != nullptr && a.ssn != 0;
       auto factor = [&](int cg) { return m0 + cg * 8 + lane < a.M ? __ldg(sp + (int64_t)(cg * 8 + lane) * a.lds) : 0.f; };
-      float next = sp != nullptr && !each ? factor(0) : 0.f;
+      float next = sp != nullptr && !by_feature ? factor(0) : 0.f;
       mbar_wait(&tfull_bar[as], aphase, 73);
       tcgen05_fence_after();
 #pragma unroll 1
       for (int cg0 = 0; cg0 < NG; cg0 += 4) {
         const int m = m0 + cg0 * 8, rows = a.M - m;      // valid token rows of this chunk (may be <= 0 or >= 32)
         float sc[32];
-        if (each) {
+        if (by_feature) {
 #pragma unroll
           for (int j = 0; j < 32; ++j) sc[j] = j < rows ? __ldg(sp + (int64_t)(cg0 * 8 + j) * a.lds) : 0.f;
         } else if (sp != nullptr) {

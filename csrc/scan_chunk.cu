@@ -75,36 +75,7 @@ __device__ __forceinline__ Rows rows_of(const ChunkArgs& a, int b) {
   return r;
 }
 
-__device__ __forceinline__ uint64_t pfma(uint64_t x, uint64_t y, uint64_t z) {
-  uint64_t d;
-  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(x), "l"(y), "l"(z));
-  return d;
-}
-__device__ __forceinline__ uint64_t pmul(uint64_t x, uint64_t y) {
-  uint64_t d;
-  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(x), "l"(y));
-  return d;
-}
-__device__ __forceinline__ uint64_t padd(uint64_t x, uint64_t y) {
-  uint64_t d;
-  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(x), "l"(y));
-  return d;
-}
-__device__ __forceinline__ uint64_t psub(uint64_t x, uint64_t y) {
-  uint64_t d;
-  asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(x), "l"(y));
-  return d;
-}
-__device__ __forceinline__ uint64_t pack(float lo, float hi) {
-  uint64_t d;
-  asm("mov.b64 %0, {%1, %2};" : "=l"(d) : "f"(lo), "f"(hi));
-  return d;
-}
-__device__ __forceinline__ float2 unpack(uint64_t v) {
-  float2 r;
-  asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
-  return r;
-}
+using namespace packed;
 __device__ __forceinline__ ulonglong2 lds2(const float* p) { return *reinterpret_cast<const ulonglong2*>(p); }
 
 // Loads never stand behind a branch: rows past the chunk's end and channels past dk are read from the last valid place and replaced

@@ -1,4 +1,4 @@
-// 32-bit numbers as sums of 16-bit ones for the tensor cores, and arithmetic on pairs of 32-bit numbers (one instruction for two).
+// 32-bit numbers as sums of 16-bit ones for the tensor cores.
 //
 // A row is scaled by a power of two s so that |x / s| < 4096, and cut into h (a multiple of 2), l (a multiple of 2^-10, |l| <= 1) and m (the rest,
 // |m| <= 2^-11), each exact in 16 bits but for the last bits of m (2^-34 of the scale).  Products h h are multiples of 4 below 2^24, so that their sums
@@ -9,43 +9,9 @@
 
 namespace split16 {
 
-using pair_t = uint64_t;
-__device__ __forceinline__ pair_t pfma(pair_t x, pair_t y, pair_t z) {
-  pair_t d;
-  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(x), "l"(y), "l"(z));
-  return d;
-}
-__device__ __forceinline__ pair_t pmul(pair_t x, pair_t y) {
-  pair_t d;
-  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(x), "l"(y));
-  return d;
-}
-__device__ __forceinline__ pair_t padd(pair_t x, pair_t y) {
-  pair_t d;
-  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(x), "l"(y));
-  return d;
-}
-__device__ __forceinline__ pair_t psub(pair_t x, pair_t y) {
-  pair_t d;
-  asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(x), "l"(y));
-  return d;
-}
-__device__ __forceinline__ pair_t pack(float lo, float hi) {
-  pair_t d;
-  asm("mov.b64 %0, {%1, %2};" : "=l"(d) : "f"(lo), "f"(hi));
-  return d;
-}
-__device__ __forceinline__ pair_t pack(uint32_t lo, uint32_t hi) {
-  pair_t d;
-  asm("mov.b64 %0, {%1, %2};" : "=l"(d) : "r"(lo), "r"(hi));
-  return d;
-}
-__device__ __forceinline__ pair_t both(float x) { return pack(x, x); }
-__device__ __forceinline__ float2 unpack(pair_t v) {
-  float2 r;
-  asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
-  return r;
-}
+using namespace packed;
+using namespace umma_lo;
+
 // the largest magnitude of three; a value that is no number stays one
 __device__ __forceinline__ float max_abs(float a, float b, float c) {
   float d;
@@ -97,18 +63,7 @@ __device__ __forceinline__ void tmem_st8(uint32_t addr, const uint32_t (&r)[8]) 
                "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]) : "memory");
 }
 __device__ __forceinline__ void tmem_st_wait() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
-// shared-memory descriptors by halves: the upper one is the same for all tiles of 128-byte swizzled rows
-constexpr uint32_t kDescHi = 0x40004040u;
-__device__ __forceinline__ uint32_t desc_lo(uint32_t addr, uint32_t lbo = 16) { return ((addr & 0x3FFFFu) >> 4) | ((lbo >> 4) << 16); }
 constexpr uint32_t idesc(int N, int mn) { return umma_idesc_f16(0, 128, N) | ((uint32_t)mn << 16); }
-__device__ __forceinline__ void umma_ts(uint32_t d, uint32_t a, uint32_t b_lo, uint32_t id, uint32_t acc) {       // A from tensor memory
-  asm volatile("{\n\t.reg .pred p;\n\t.reg .b64 b;\n\tsetp.ne.b32 p, %4, 0;\n\tmov.b64 b, {%2, %5};\n\t"
-               "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], b, %3, p;\n\t}" ::"r"(d), "r"(a), "r"(b_lo), "r"(id), "r"(acc), "r"(kDescHi) : "memory");
-}
-__device__ __forceinline__ void umma_ss(uint32_t d, uint32_t a_lo, uint32_t b_lo, uint32_t id, uint32_t acc) {
-  asm volatile("{\n\t.reg .pred p;\n\t.reg .b64 a, b;\n\tsetp.ne.b32 p, %4, 0;\n\tmov.b64 a, {%1, %5};\n\tmov.b64 b, {%2, %5};\n\t"
-               "tcgen05.mma.cta_group::1.kind::f16 [%0], a, b, %3, p;\n\t}" ::"r"(d), "r"(a_lo), "r"(b_lo), "r"(id), "r"(acc), "r"(kDescHi) : "memory");
-}
 
 // mbar_wait for kernels that end by themselves: a wait of more than LLMSS_SPIN_TIMEOUT_NS sets *quit (shared memory), and waits that find it set
 // end.  What the block has computed since is worth nothing: the kernel leaves its state as it was and its work to another one
