@@ -1,7 +1,7 @@
 """Baseline tier R2: "the reference's library path at equal shapes" for models the reference cannot load.
 
-The reference registers only `gptj` and `gpt_bigcode` (custom_modeling/__init__.py:4-7), so BASELINE.json's
-Llama-2 7B / 13B and OPT-1.3B configs have no reference model code to run.  What the reference *would* run for
+The reference registers only `gptj` and `gpt_bigcode` (custom_modeling/__init__.py:4-7), so the
+Llama-2 7B / 13B and OPT-1.3B workloads have no reference model code to run.  What the reference *would* run for
 them is its own tensor-parallel layer library, so this file assembles exactly those classes -- imported unmodified
 from baseline/_ref: `TensorParallelEmbedding`, `TensorParallelColumnLinear`, `TensorParallelRowLinear`,
 `TensorParallelHead` (layers.py:79-214), loaded through the reference's `Weights` -- into a decoder that follows

@@ -1,13 +1,12 @@
 """Runs the UNMODIFIED reference package (installed with pip --target baseline/_ref) so that
 bench.py --impl reference measures the reference's own code path on this box.
 
-Install (recorded in DESIGN.md):
+Install (from a read-only checkout of the reference):
     python -m pip install --no-index --no-build-isolation --no-deps --find-links /opt/wheelhouse \
-        --target baseline/_ref /root/reference
+        --target baseline/_ref <reference>
 
 Three in-process shims are needed because the reference pins torch 2.0.1 / transformers 4.30.2 /
-accelerate 0.21.0 and this image has torch 2.11 / transformers 5.5 / no accelerate (SURVEY.md
-section 6.3).  None of them touches the reference's files or its compute path:
+accelerate 0.21.0 and this image has torch 2.11 / transformers 5.5 / no accelerate.  None of them touches the reference's files or its compute path:
   1. a stub `accelerate` module whose `init_empty_weights` is `torch.device("meta")`
      (used only while constructing LayerNorm shells, reference layers.py:6,16,27);
   2. `PreTrainedModel.get_head_mask` (removed in transformers 5) returning `[None] * n`;
@@ -59,7 +58,7 @@ def _install_shims():
 
 def import_reference():
     if not (REF_ROOT / "llmss").is_dir():
-        raise RuntimeError(f"{REF_ROOT}/llmss not found: run the pip --target install described in DESIGN.md")
+        raise RuntimeError(f"{REF_ROOT}/llmss not found: run the pip --target install named at the top of this file")
     _install_shims()
     if str(REF_ROOT) not in sys.path:
         sys.path.insert(0, str(REF_ROOT))

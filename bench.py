@@ -5,9 +5,9 @@
         --master-port P bench.py --gpus N --steps K --warmup W
     python bench.py --impl reference ...  # the UNMODIFIED reference (baseline/_ref), same metric
 
-Metric (BASELINE.json): decode tokens/s, device-timed (CUDA events), max over ranks; plus p50
-TTFT / TPOT.  Config: GPT-J-6B shape (the largest architecture the reference can load
-R1), batch 64, 1024-token synthetic prompts, random-init weights in HF safetensors layout, bf16
+Metric: decode tokens/s, device-timed (CUDA events), max over ranks; plus p50
+TTFT / TPOT.  Config: GPT-J-6B shape (the largest architecture the reference can
+load), batch 64, 1024-token synthetic prompts, random-init weights in HF safetensors layout, bf16
 (ours) / fp16 (reference hard-codes fp16, generate.py:53).  A "step" is one decode step of the
 whole batch = `batch` new tokens.  TP serving splits a fixed batch over N GPUs: strong scaling.
 
@@ -195,7 +195,7 @@ def synthetic_prompts(batch: int, prompt_len: int, vocab: int):
     return torch.randint(10, vocab - 10, (batch, prompt_len), generator=g).tolist()
 
 
-BASELINE_VALUE = None  # the reference publishes no number (BASELINE.md section 1)
+BASELINE_VALUE = None  # the reference publishes no number
 
 
 def bench_config(args, world: int) -> dict:

@@ -1,8 +1,8 @@
 // K9 attn_decode_paged: single-query attention against the paged KV cache, split-KV.
 //
-// Replaces the reference's decode-step attention (SURVEY.md G7/G8: fp32 upcast, cuBLAS
+// Replaces the reference's decode-step attention (fp32 upcast, cuBLAS
 // batched QK^T, where-mask, softmax, cuBLAS PV on a [B,h,1,T] score tensor, plus the
-// G17 mask buffers and the H2D mask copy of quirk Q18).  Decode attention is pure
+// mask buffers and the host-to-device mask copy).  Decode attention is pure
 // KV-bandwidth: every cached byte is read once per step, so the kernel is organised
 // around 16-byte streaming loads (ld.global.nc, no L1 allocation) with 2*U loads in
 // flight per lane, fp32 online softmax, and a split-KV grid so that small batches still

@@ -23,8 +23,8 @@
 // beyond the size arrive as TMA's zero fill), and two query / key maps per head: the key row holds both maps, the
 // query rows come zero-padded to that width, so a group's 2 G rows share one read of K and V; the combine pass subtracts.
 //
-// Replaces SURVEY.md G8 (`baddbmm` + TorchScript softmax + `bmm` on a replicated KV tensor,
-// gpt_bigcode_modeling.py:170-246) and G7 for grouped models.
+// Replaces the grouped attention of the reference (`baddbmm` + TorchScript softmax + `bmm` on a replicated KV tensor,
+// gpt_bigcode_modeling.py:170-246).
 #include "common.cuh"
 
 #include <cuda.h>

@@ -1,7 +1,7 @@
 // comm runtime + K4 collectives over NVLink 5 / NVSwitch peer memory.
 //
 // The reference issues every collective as a separate blocking NCCL launch through c10d
-// (SURVEY.md sections 2.4/2.5; layers.py:125,133,178,213).  Here each rank owns one
+// (layers.py:125,133,178,213).  Here each rank owns one
 // symmetric region (cudaMalloc + CUDA IPC, mapped into every peer once at start-up) and
 // the collectives are plain kernels that store straight into peer memory and synchronise
 // with system-scope release/acquire flags.  No host involvement, fixed addresses ->

@@ -1,7 +1,7 @@
 // K10 embed: token (+ learned position) embedding gather.
 //
 // The reference shards the table over ranks, remaps out-of-shard ids to a zero row and
-// all-reduces [B,S,H] (SURVEY.md G1 + N2; layers.py:182-214; BigCode does it twice,
+// all-reduces [B,S,H] (layers.py:182-214; BigCode does it twice,
 // gpt_bigcode_modeling.py:696-697).  With 180 GB of HBM per GPU the tables (<= 0.8 GB)
 // are simply replicated, which removes 1-2 collectives per forward; the sharded + reduce
 // variant remains available through TensorParallelEmbedding for API parity.

@@ -1,8 +1,7 @@
 // K6 norm_residual: (x [+ x2] [+ residual]) -> new residual, LayerNorm / RMSNorm of it.
 //
-// Replaces the reference's separate ATen add + layer_norm launches (SURVEY.md G2, G13;
-// gptj_modeling.py:296,310,496; gpt_bigcode_modeling.py:367,379,404,407) and provides the
-// capability of the never-instantiated FastLayerNorm wrapper (layers.py:217-256, G18).
+// Replaces the reference's separate ATen add + layer_norm launches (gptj_modeling.py:296,310,496; gpt_bigcode_modeling.py:367,379,404,407) and provides the
+// capability of the never-instantiated FastLayerNorm wrapper (layers.py:217-256).
 // One CTA per row, row held in registers (16-byte vector loads), fp32 statistics,
 // two-pass variance.  Memory-bound: reads x(+res) once, writes normed(+res) once.
 #include "common.cuh"

@@ -1,9 +1,9 @@
 // K7 rope_kv_write: rotary embedding on q and k (in place in the packed QKV activation) and
 // append of k, v into the paged KV cache, one launch.
 //
-// Replaces the reference's ~10 ATen kernels for RoPE (SURVEY.md G5; gptj_modeling.py:26-47,
+// Replaces the reference's ~10 ATen kernels for RoPE (gptj_modeling.py:26-47,
 // 206-224: gather sin/cos by position, rotate_every_two, cat) and the per-step torch.cat
-// KV append (G6; gptj_modeling.py:229-233, gpt_bigcode_modeling.py:288-289), which copies
+// KV append (gptj_modeling.py:229-233, gpt_bigcode_modeling.py:288-289), which copies
 // the whole cache every token.  Styles: GPT-J interleaved pairs on the first rotary_dim
 // dims, NeoX/Llama half rotation, or none (GPT-2 / OPT / BigCode learned positions).
 // cos/sin are evaluated in fp32 from the position (no table, no gather).

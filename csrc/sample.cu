@@ -1,10 +1,10 @@
 // K11 (sampling half): fused greedy / top-p / top-k / temperature sampler over fp32 logits.
 //
-// Replaces the reference's rank-0-only sampling (SURVEY.md G15/G16 + N6: argmax or
+// Replaces the reference's rank-0-only sampling (argmax or
 // softmax + HF warpers + multinomial on rank 0, then a broadcast of the token,
 // generate.py:109-144) with one launch that every rank runs on identical gathered logits
 // and an identical counter-based RNG, so all ranks agree without a collective.  It
-// implements the *intended* warper semantics (quirk Q1: the reference never applies
+// implements the *intended* warper semantics (the reference never applies
 // them): top-p on the raw distribution, then top-k, then temperature, then one draw.
 //
 // One CTA per row.  Passes over the row (L2-resident): max/argmax, sum-exp, a 4-pass

@@ -3,7 +3,7 @@
     torchrun --nproc_per_node N generate.py --pretrained_model_path P --prompts "a" "b" \
         --max_new_tokens 20 [--is_greedy] [--temperature 1.0] [--top_p 0.95] [--top_k 50] [--use_cache]
 
-Differences from the reference (all deliberate, see SURVEY.md section 2.8):
+Differences from the reference (all deliberate):
   * runs at WORLD_SIZE=1 and on CPU (Q2, Q4);                * sampling flags take effect (Q1);
   * `max_position_embeddings` is honoured when `n_positions` is absent (Q5);
   * prompts keep their own lengths -- no pad tokens enter the model (Q6);

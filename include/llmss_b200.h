@@ -5,8 +5,8 @@
  * All launches go to the given stream; nothing here synchronises the device except the
  * symmetric-memory set-up calls.  dtype: 0 = fp16, 1 = bf16, 2 = fp32.
  *
- * Each declaration cites the reference (jongwon-jay-lee/llmss) code it replaces; see
- * SURVEY.md sections 2.5 / 2.6 for the N-number / G-number labels.
+ * Each declaration cites the reference (jongwon-jay-lee/llmss) code it replaces (G: an ATen call
+ * site of its models, N: a collective, K: a kernel of this library).
  */
 #ifndef LLMSS_B200_H_
 #define LLMSS_B200_H_
@@ -38,7 +38,7 @@ int llmss_symm_create(int rank, int nranks, void* const* peer_bases, size_t buf_
 int llmss_symm_destroy(llmss_symm_t* ws);
 int llmss_symm_epoch(llmss_symm_t* ws, uint32_t* out_host);
 
-/* ---- symmetric heap on the CUDA VMM API + NVLS multicast (csrc/vmm.cu; SURVEY section 5.8) ----
+/* ---- symmetric heap on the CUDA VMM API + NVLS multicast (csrc/vmm.cu) ----
  * Each rank: llmss_vmm_padded_size (identical on all ranks) -> llmss_vmm_alloc -> llmss_symm_init_region on
  * llmss_vmm_ptr -> llmss_vmm_export_fd once per peer, descriptor sent with llmss_fdx_send / received with
  * llmss_fdx_recv (abstract Unix datagram sockets, SCM_RIGHTS) -> llmss_vmm_import.  Optional NVLS: rank 0

@@ -1,7 +1,7 @@
 """llmss_b200 -- Blackwell (B200, sm_100a) native tensor-parallel LLM serving.
 
 Capability parity target: jongwon-jay-lee/llmss (reference `src/llmss/`), re-designed
-B200-first.  Layer map (see DESIGN.md):
+B200-first.  Layer map:
 
     serving/   broker (RESP LPUSH/RPOP/LLEN), HTTP producer, consumer, gRPC, scheduler
     engine/    paged KV cache, ModelRunner (prefill + CUDA-graph decode), sampler

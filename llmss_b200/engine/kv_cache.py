@@ -1,6 +1,6 @@
 """Pre-allocated paged KV cache + block allocator.
 
-Replaces the reference's per-step ``torch.cat`` cache growth (SURVEY.md G6: a full O(T) copy
+Replaces the reference's per-step ``torch.cat`` cache growth (a full O(T) copy
 and a fresh allocation per layer per token; gptj_modeling.py:229-233,
 gpt_bigcode_modeling.py:288-289).  Layout per layer: ``[num_blocks, kv_heads_per_rank,
 block_size, head_dim]`` for K and for V, sized once for the 180 GB of HBM3e.

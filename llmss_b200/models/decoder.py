@@ -17,7 +17,7 @@ into *two* GEMMs and *one* all-reduce per layer (the reference does 5 GEMMs + 2 
     attention writes its context over q                      ->  z = y[:, kv_dim:] = [ctx | act(up)]
     w2 = [wo | wdown]       ->  out = all_reduce(z @ w2^T) + b_down
 
-Sharding rules are the reference's (SURVEY.md section 2.7h; weights.py:97-115, layers.py:138-214)
+Sharding rules are the reference's (weights.py:97-115, layers.py:138-214)
 so any unsharded HF safetensors checkpoint loads unchanged.
 """
 from __future__ import annotations

@@ -3,8 +3,8 @@
 Parity families (reference MODEL_REGISTRY, custom_modeling/__init__.py:4-7):
   gptj         gptj_modeling.py:84-95,259-264,281,368-377,520-524
   gpt_bigcode  gpt_bigcode_modeling.py:122-155,316-319,340-343,562-579,793-797  (MQA)
-North-star families the reference cannot load: gpt2, opt, llama.
-Key names follow the HF state dicts (SURVEY.md section 2.7h).
+Families the reference cannot load: gpt2, opt, llama.
+Key names follow the HF state dicts.
 """
 from __future__ import annotations
 

@@ -1,9 +1,9 @@
 """Plain-PyTorch fp32 oracles for every op in ``llmss_b200.ops``.
 
-These are (a) the CPU execution path (BASELINE config 1: generate.py on CPU, TP=1; gloo
+These are (a) the CPU execution path (generate.py on CPU, TP=1; gloo
 multi-process tests) and (b) the numerical reference every CUDA kernel in ``csrc/`` is
 tested against (tests/test_gpu_*.py).  They mirror the math of the reference's ATen call
-sites listed in SURVEY.md section 2.6 (G1-G16), not its code.
+sites, not its code.
 """
 from __future__ import annotations
 
@@ -314,7 +314,7 @@ MAX_CANDIDATES = 1024
 
 def sample(logits, greedy, temperature, top_k, top_p, rng_state, vocab: Optional[int] = None,
            u_shift: float = 0.0) -> torch.Tensor:
-    """Next-token choice per row (G15/G16 with the *intended* semantics).
+    """Next-token choice per row with the *intended* semantics (the reference never applies its warpers to the draw).
 
     Order = the reference's warper list order (generate.py:114-120): top-p on the raw
     distribution, then top-k, then temperature; then one inverse-CDF draw over the

@@ -1,10 +1,10 @@
 """Collective front door used by every layer of the framework.
 
 The reference calls `torch.distributed.all_reduce / all_gather / broadcast` inline at each
-call site (SURVEY.md section 2.5, N1-N10; `layers.py:125,133,178,213`, `generate.py:85,144`).
+call site (`layers.py:125,133,178,213`, `generate.py:85,144`).
 Here every call site goes through a :class:`Communicator`, which picks per message:
 
-  * world_size == 1 / `FakeGroup`         -> no-op (fixes SURVEY Q2)
+  * world_size == 1 / `FakeGroup`         -> no-op (the reference fails there)
   * CUDA + symmetric-memory workspace       -> hand-written one-shot / two-shot P2P kernels
                                               over NVLink / NVSwitch multicast (csrc/comm.cu), CUDA-graph safe
   * otherwise (CPU gloo, or message too big for the workspace) -> torch.distributed

@@ -1,6 +1,6 @@
 """Request broker: a work queue speaking the Redis list protocol the reference uses.
 
-The reference's "pubsub" is two Redis lists used as FIFO queues (SURVEY.md section 2.7c):
+The reference's "pubsub" is two Redis lists used as FIFO queues:
 requests  `LPUSH pqueue <json>` / `LLEN pqueue` + `RPOP pqueue`   (producer_server.py:48, consumer_server.py:79-80)
 responses `LPUSH squeue <json>` / `LLEN squeue` + `RPOP squeue`   (consumer_server.py:172-173, producer_server.py:51-52)
 

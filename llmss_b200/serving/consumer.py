@@ -2,7 +2,7 @@
 continuous batching, pushes responses back.
 
 Parity: reference `poc-server/producer-consumer/consumer_server.py:33-173` (same queue names and
-JSON bodies).  Differences, all deliberate (quirk Q14):
+JSON bodies).  Differences, all deliberate:
   * many requests in flight (continuous batching) instead of batch size 1;
   * rank 0 shares each step's *new requests* with the other TP ranks as ONE fixed-layout int32
     tensor broadcast (no pickled objects, no per-token broadcast -- sampling is replicated);

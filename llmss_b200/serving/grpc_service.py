@@ -1,7 +1,6 @@
 """gRPC front end.
 
-The reference's README advertises gRPC but ships no gRPC code, proto or import (SURVEY.md
-section 0); this defines it.  `grpc_tools` / `protoc` are not available on the target boxes, so the
+The reference's README advertises gRPC but ships no gRPC code, proto or import; this defines it.  `grpc_tools` / `protoc` are not available on the target boxes, so the
 messages are built at run time from a `FileDescriptorProto` (equivalent .proto below) and the
 service is registered with `grpc.method_handlers_generic_handler`.
 
@@ -16,7 +15,7 @@ service is registered with `grpc.method_handlers_generic_handler`.
                     rpc Health(HealthRequest) returns (HealthResponse); }
 
 Like the HTTP producer, the service is a *front end*: it forwards requests through the broker to the
-tensor-parallel consumer and mirrors the HTTP schema (SURVEY.md section 2.7e).
+tensor-parallel consumer and mirrors the HTTP schema.
 """
 from __future__ import annotations
 

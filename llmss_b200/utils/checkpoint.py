@@ -1,7 +1,7 @@
 """Random-init HF-format checkpoints (config.json + *.safetensors) for benches and tests.
 
 There is no network for real checkpoints, so benchmarks use random weights of the named
-architecture written in the ordinary unsharded HF layout (SURVEY.md section 2.7h) -- the same
+architecture written in the ordinary unsharded HF layout -- the same
 files are then loaded by this framework *and* by the unmodified reference through its
 `Weights` class.  Tensors are generated shard by shard on `device` (GPU when available) so a
 6B-parameter checkpoint takes seconds, not minutes.
@@ -17,7 +17,7 @@ import torch
 from safetensors.torch import save_file
 
 PRESETS: Dict[str, dict] = {
-    # GPT-J-6B shape: the largest architecture the reference itself can load (BASELINE.md R1)
+    # GPT-J-6B shape: the largest architecture the reference itself can load
     "gptj-6b": dict(model_type="gptj", architectures=["GPTJForCausalLM"], vocab_size=50400, n_positions=2048,
                     n_embd=4096, n_layer=28, n_head=16, rotary_dim=64, n_inner=None, activation_function="gelu_new",
                     layer_norm_epsilon=1e-5, tie_word_embeddings=False, bos_token_id=50256, eos_token_id=50256),
@@ -51,7 +51,7 @@ PRESETS: Dict[str, dict] = {
                      num_hidden_layers=24, ffn_dim=8192, num_attention_heads=32, max_position_embeddings=2048,
                      do_layer_norm_before=True, word_embed_proj_dim=2048, activation_function="relu",
                      tie_word_embeddings=True),
-    # GPT-2 XL: 25 heads -- not divisible by 2; BASELINE config 2 names it at TP=2 (heads are padded, models/decoder.py)
+    # GPT-2 XL: 25 heads -- not divisible by 2; at TP=2 (heads are padded, models/decoder.py)
     "gpt2-xl": dict(model_type="gpt2", architectures=["GPT2LMHeadModel"], vocab_size=50257, n_positions=1024, n_embd=1600,
                     n_layer=48, n_head=25, activation_function="gelu_new", layer_norm_epsilon=1e-5,
                     tie_word_embeddings=True),

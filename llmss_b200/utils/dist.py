@@ -3,7 +3,7 @@
 Parity: reference `src/llmss/server/models/utils/dist.py:9-77`
 (`initialize_torch_distributed`, `FakeGroup`, `FakeBarrier`).
 
-Differences (deliberate, SURVEY.md Q2/Q4):
+Differences (deliberate):
   * `FakeGroup` here is a *complete* in-process group: besides the c10d duck-typed
     methods of the reference (`allreduce`/`allgather`/`barrier`/`size`/`rank`) it is
     understood by every collective helper in :mod:`llmss_b200.parallel.comm`, so
@@ -50,7 +50,7 @@ class FakeGroup:
 
     def allgather(self, outputs, inputs, *args, **kwargs):
         # torch >= 2.1 passes an extra options argument; accept and ignore it
-        # (the reference's signature breaks there, SURVEY.md section 2.4).
+        # (the reference's signature breaks there).
         for out_list, inp in zip(outputs, inputs):
             for o in out_list:
                 o.data = inp.data

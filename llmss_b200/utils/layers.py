@@ -4,7 +4,7 @@ Parity: reference `src/llmss/server/models/utils/layers.py:12-256` -- `FastLinea
 `get_linear`, `SuperLayer`, `TensorParallelHead`, `TensorParallelColumnLinear`,
 `TensorParallelRowLinear`, `TensorParallelEmbedding`, `LayerNorm.load / load_no_bias`,
 `FastLayerNorm`.  Constructors, `load(config, prefix, weights, bias)` classmethods and the
-sharding rules (SURVEY.md section 2.7h) are the same, so model code written against the
+sharding rules are the same, so model code written against the
 reference's layers keeps working.  What runs underneath is different:
 
   * every matmul is the tcgen05 GEMM (ops.linear) instead of cuBLAS `F.linear`;

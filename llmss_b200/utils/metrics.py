@@ -1,9 +1,9 @@
 """Serving metrics: counters, gauges and latency reservoirs (TTFT / TPOT / step time).
 
 The reference has no observability beyond one wall-clock print that includes model load
-(SURVEY.md section 5.5; generate.py:193-194).  This registry is process-local, lock-protected,
+(generate.py:193-194).  This registry is process-local, lock-protected,
 exports Prometheus text (`render_prometheus`) for the HTTP `/metrics` route, and answers
-quantile queries (`quantile("ttft_seconds", 0.5)`) for BASELINE's p50 TTFT / TPOT.
+quantile queries (`quantile("ttft_seconds", 0.5)`) for p50 TTFT / TPOT.
 """
 from __future__ import annotations
 

@@ -1,4 +1,4 @@
-"""Tracing / profiling hooks (the reference has none: SURVEY.md section 5.1).
+"""Tracing / profiling hooks (the reference has none).
 
 Two switches, both off by default so the hot path pays one attribute test per op:
   * ``LLMSS_NVTX=1``        -- NVTX ranges around every op and every layer (visible in Nsight tools);

@@ -6,10 +6,10 @@ cached handles, whole-tensor reads and lazy per-rank slices along dim 0 / dim 1,
 dtype cast except for int32/int64 payloads, optional aliases.
 
 The on-disk format stays the ordinary *unsharded* HF safetensors checkpoint; every rank
-slices its block at load time (SURVEY.md section 2.7h).  Additions used by the fused
+slices its block at load time.  Additions used by the fused
 per-rank weight layouts of this framework: `get_range` (arbitrary lazy row/col range,
-so a fused `c_attn` is never read whole -- SURVEY Q9) and `ceil` mode for vocab
-sharding (SURVEY Q10: the reference's floor division silently drops `V mod t` rows).
+so a fused `c_attn` is never read whole) and `ceil` mode for vocab
+sharding (the reference's floor division silently drops `V mod t` rows).
 """
 from __future__ import annotations
 

@@ -2,7 +2,7 @@
 
     torchrun --nproc-per-node N --master-addr 127.0.0.1 scripts/bench_gemm_ar.py
 Shapes: the row-parallel GEMMs of GPT-J-6B (fused out_proj+fc_out: N=4096, K=20480/N) and Llama-2 7B/13B
-(o_proj, down_proj) for decode batches M=1..256 (BASELINE config 5).
+(o_proj, down_proj) for decode batches M=1..256.
 """
 import json
 import math

@@ -1,4 +1,4 @@
-"""Long-context numbers (SURVEY 5.7): time to first token and time per output token for 8k / 16k-token prompts.
+"""Long-context numbers: time to first token and time per output token for 8k / 16k-token prompts.
 
     python scripts/bench_long_context.py [--model llama-2-7b] [--json out.json]
 

@@ -1,4 +1,4 @@
-"""Serving benchmark through the real front ends (BASELINE.json configs 3 and 4), one process per GPU.
+"""Serving benchmark through the real front ends (Llama-2 7B and 13B), one process per GPU.
 
     torchrun --nproc-per-node 8 --master-addr 127.0.0.1 scripts/bench_serving.py --model llama-2-13b \
         --frontend pubsub --batch 64 --prompt-len 1024 --gen 256

@@ -11,7 +11,7 @@ def f(x):
 
 
 def main():
-    out = ["# Row-parallel GEMM -> all-reduce (BASELINE.json config 5): every row, losing ones included", "",
+    out = ["# Row-parallel GEMM -> all-reduce (o_proj, down_proj; M = 1..256): every row, losing ones included", "",
            "`scripts/bench_gemm_ar.py` under `torchrun`, one rank per B200: each variant is captured as a CUDA graph of 20",
            "back-to-back launches (weights cycled through a pool larger than L2), timed with CUDA events, max over ranks,",
            "median of 5 replays.  All times in microseconds.  Raw rows: `raw/gemm_ar_tp*.json`.", "",

@@ -205,7 +205,7 @@ def main():
         log(f"graph replay done (epoch now {symm.epoch()})")
 
         # ---- 4b. protocol stress: randomised per-rank arrival skew, alternating kernels / sizes / parities.
-        # (compute-sanitizer's racecheck cannot see inter-GPU races)
+        # (compute-sanitizer's racecheck cannot see inter-GPU races.)
         n_stress = int(sys.argv[sys.argv.index("--stress") + 1]) if "--stress" in sys.argv else 60
         import random
         rnd = random.Random(1234 + rank)
