@@ -1936,8 +1936,8 @@ int pick_cluster_split(int tiles, int kb_total, int bn, int sms, int dtype) {
   }
   if (forced == 1) return 0;
   // Splitting K over a cluster divides the weight stream AND the epilogue (each CTA finishes 1/S of the tile) at the
-  // price of a cluster barrier and a DSMEM exchange.  Measured on the TP=8 per-rank shapes (M = 16..128, K = 512..2560,
-  // scripts/bench_gemm_small.py): the deepest split that leaves two k-blocks per CTA wins everywhere -- 8.2 us vs
+  // price of a cluster barrier and a DSMEM exchange.  Measured on the TP=8 per-rank shapes (M = 16..128, K = 512..2560):
+  // the deepest split that leaves two k-blocks per CTA wins everywhere -- 8.2 us vs
   // 12.0 us for one CTA per tile at M=64, K=512 -- because the epilogue, not the stream, is the long pole.  A "cluster"
   // of one (K of one or two k-blocks) still runs this kernel, so the fused all-reduce epilogues stay available.
   for (int s = 8; s >= 1; --s) {
