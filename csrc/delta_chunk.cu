@@ -143,7 +143,8 @@ __device__ __forceinline__ void lds_pairs(const float* p, pair_t& x, pair_t& y) 
 // front of the chunk give the size n of that token's numbers; where n is below 2^-11 to 2^-12 of the column's largest (us: a column's numbers are scaled to
 // 2^11 .. 2^12), fewer than 24 bits of them are left.  One such number is chance (1 in 1400 of normal ones that stand alone); a token that is small
 // in all 32 columns of the warp, or five tokens of a column, are not.  s: scale of the column's state.  The same answer for the whole warp.
-// The state has the like (in its warps): 8 of a thread's 64 key rows below 2^-11 to 2^-12 of the column's largest, 3 once keys were sparse.
+// The state has the like (in its warps): 8 of a thread's 64 key rows below 2^-11 to 2^-12 of the column's largest, 3 once keys were sparse.  Fewer such rows
+// stay: a query that reads nothing but them gets them to 2^-34 of the column's largest.
 // Earlier forms: in front of T R in the chain 343 -> 349 us, the state's count beside U 352.
 __device__ __forceinline__ bool spread(const pair_t (&y)[C / 2], const Scalars& sc, int tokens, float s, float us) {
   float n = s > 0x1p-98f ? s * 0x1p11f : 0.f;

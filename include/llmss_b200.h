@@ -369,7 +369,8 @@ int llmss_delta_scan(const float* q, int64_t ldq, const float* k, int64_t ldk, c
                      const int* slots, int B, int max_q, int heads, int qk_heads, int dk, int dv, float unit_eps, float q_scale,
                      int beta_sigmoid, llmss_stream_t stream);
 /* the same over chunks of 32 tokens on the tensor cores (sequences of 32 tokens and more; shorter ones token by token): key sizes up to 128 that are
- * multiples of 4; q, k (rows too), state and scratch (llmss_delta_scan_chunked_bytes bytes, T: rows of the batch) 16-byte aligned */
+ * multiples of 4; q, k (rows too), state and scratch (llmss_delta_scan_chunked_bytes bytes, T: rows of the batch) 16-byte aligned; max_q is a hint on the
+ * lengths: tokens beyond it run token by token, and so do those behind numbers and decays that the products cannot take (csrc/delta_chunk.cu) */
 int64_t llmss_delta_scan_chunked_bytes(int T, int B, int heads);
 int llmss_delta_scan_chunked(const float* q, int64_t ldq, const float* k, int64_t ldk, const float* v, int64_t ldv, const float* log_decay,
                      int64_t ldg, const float* beta, int64_t ldb, float* out, float* state, const int* cu_q, const int* seq_lens,
