@@ -292,6 +292,21 @@ __device__ __forceinline__ void tma_load_3d(void* smem_dst, const void* map, uin
       "l"(map), "r"(smem_u32(bar)), "r"(c0), "r"(c1), "r"(c2), "l"(policy)
       : "memory");
 }
+// The same by a CTA of a pair (cta_group::2), whose barrier may lie in the other CTA: `bar` is a shared::cluster address
+__device__ __forceinline__ void tma_load_2d_pair(void* smem_dst, const void* map, uint32_t bar, int c0, int c1, uint64_t policy) {
+  asm volatile(
+      "cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.tile.mbarrier::complete_tx::bytes.L2::cache_hint"
+      " [%0], [%1, {%3, %4}], [%2], %5;" ::"r"(smem_u32(smem_dst)),
+      "l"(map), "r"(bar), "r"(c0), "r"(c1), "l"(policy)
+      : "memory");
+}
+__device__ __forceinline__ void tma_load_3d_pair(void* smem_dst, const void* map, uint32_t bar, int c0, int c1, int c2, uint64_t policy) {
+  asm volatile(
+      "cp.async.bulk.tensor.3d.cta_group::2.shared::cluster.global.tile.mbarrier::complete_tx::bytes.L2::cache_hint"
+      " [%0], [%1, {%3, %4, %5}], [%2], %6;" ::"r"(smem_u32(smem_dst)),
+      "l"(map), "r"(bar), "r"(c0), "r"(c1), "r"(c2), "l"(policy)
+      : "memory");
+}
 
 // ---------------------------------------------------------------- packed arithmetic
 // Packed fp32x2 arithmetic (one issue slot for two numbers): the softmax warps of the prompt-attention kernel are bound by
@@ -370,6 +385,11 @@ __device__ __forceinline__ void umma_ts(uint32_t d, uint32_t a, uint32_t b_lo, u
 __device__ __forceinline__ void umma_ss(uint32_t d, uint32_t a_lo, uint32_t b_lo, uint32_t id, uint32_t acc) {
   asm volatile("{\n\t.reg .pred p;\n\t.reg .b64 a, b;\n\tsetp.ne.b32 p, %4, 0;\n\tmov.b64 a, {%1, %5};\n\tmov.b64 b, {%2, %5};\n\t"
                "tcgen05.mma.cta_group::1.kind::f16 [%0], a, b, %3, p;\n\t}" ::"r"(d), "r"(a_lo), "r"(b_lo), "r"(id), "r"(acc), "r"(kDescHi) : "memory");
+}
+// the pair's form (cta_group::2); issuing it takes a warp about 30 clocks, with both 64-bit descriptors formed in the loop 45
+__device__ __forceinline__ void umma_ss_pair(uint32_t d, uint32_t a_lo, uint32_t b_lo, uint32_t id, uint32_t acc) {
+  asm volatile("{\n\t.reg .pred p;\n\t.reg .b64 a, b;\n\tsetp.ne.b32 p, %4, 0;\n\tmov.b64 a, {%1, %5};\n\tmov.b64 b, {%2, %5};\n\t"
+               "tcgen05.mma.cta_group::2.kind::f16 [%0], a, b, %3, p;\n\t}" ::"r"(d), "r"(a_lo), "r"(b_lo), "r"(id), "r"(acc), "r"(kDescHi) : "memory");
 }
 
 }  // namespace umma_lo
@@ -465,15 +485,6 @@ __device__ __forceinline__ void tmem_relinquish_pair() {
 }
 __device__ __forceinline__ void tmem_dealloc_pair(uint32_t taddr, uint32_t ncols) {  // same warp id in both CTAs
   asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(taddr), "r"(ncols) : "memory");
-}
-__device__ __forceinline__ void umma_f16_ss_pair(uint32_t tmem_d, uint64_t desc_a, uint64_t desc_b, uint32_t idesc,
-                                                 uint32_t accumulate) {
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(tmem_d),
-      "l"(desc_a), "l"(desc_b), "r"(idesc), "r"(accumulate)
-      : "memory");
 }
 // Arrive on the mbarrier at this shared-memory offset in every CTA of `cta_mask` (bit = rank in the cluster) once the
 // MMAs issued so far have completed.

@@ -102,6 +102,8 @@ struct GemmArgs {
   int tm_rot;                  // token-tile rotation: with ag, every rank starts on the tiles of its own shard
   const int* groups;           // grouped pair kernel: [E + 1] first row of every group, then [E + 1] first token tile
   int n_groups;                // E
+  int bn;                      // pair kernel: token columns of a tile, a multiple of 32 up to 256
+  int nacc;                    // pair kernel: accumulators of a tile, each over its own stretch of K (see pair_accumulators)
   unsigned long long* dbg;  // optional per-CTA phase timestamps [grid][8] (globaltimer ns), see llmss_gemm_set_debug
   SymmWs ws;
 };
@@ -1187,7 +1189,7 @@ gemm_cluster_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
 }
 
 // ======================================================================================
-// CTA-pair kernel (tcgen05 cta_group::2) for token dimensions above 128.
+// CTA-pair kernel (tcgen05 cta_group::2): every product of more than 64 tokens, and fewer tokens over many features.
 //
 // With 128-feature tiles every CTA re-reads the whole 256-token activation tile per k-block: 32 KB of activations from
 // L2 for 16 KB of weights, and from M = 256 upwards the L2 -> SM traffic and the bytes a 4-stage ring can keep in
@@ -1196,7 +1198,9 @@ gemm_cluster_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
 // offsets), the even CTA issues `tcgen05.mma.cta_group::2`, the tensor cores of both SMs read both halves of the
 // activation tile, and each CTA's tensor memory receives the accumulator of its own 128 features.  Activation traffic per
 // weight byte halves and the ring holds 6 stages instead of 4 (measured: 313 ns per k-block of 256 x 256 x 64, against
-// ~410 ns for two single-CTA tiles at M = 8192).
+// ~410 ns for two single-CTA tiles at M = 8192).  The token tile is 32 .. 256 columns wide, chosen per launch (pick_pair): fewer tokens, or few feature
+// tiles, take narrower ones, whose k-blocks take as much less time down to 128 columns.  Against tiles of 256 columns only (us): 366 tokens 4096 x 4096
+// 24.5 -> 18, 526 tokens 4096 x 11008 62 -> 45, 827 tokens 2048 x 2048 19.1 -> 12.2, 64 tokens 28672 x 4096 45.1 -> 42 (from the single-CTA kernel).
 //
 // Two schedules, chosen on the host:
 //  * persistent (clusters of 2, S = 1): every pair walks tiles p, p + P, p + 2P, ... with TWO accumulators of 256 columns
@@ -1206,21 +1210,23 @@ gemm_cluster_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
 //    parity h = rank % 2 selects the feature half; the S partial tiles of one parity are reduced out of the peers' shared
 //    memory like in the cluster kernel above (pull mode, CTA order, deterministic), each CTA finishing 1/S of its tile.
 //
-// Protocol: every CTA's TMA warp fills its own ring and arms its own `full` barrier.  The odd CTA's warp 1 forwards
-// each `full` completion to the even CTA's `peer_full` barrier (remote mbarrier arrive); the even CTA's warp 1 waits
-// for both before it issues, and frees the stage in BOTH CTAs with one multicast commit.  Accumulator hand-over: one
+// Protocol: every CTA's TMA warp fills its own ring; the loads of both CTAs report to the even CTA's `full` barrier (cta_group::2), which that CTA
+// arms with the bytes of both.  The even CTA's warp 1 issues, and frees the stage in BOTH CTAs with one multicast commit.  Accumulator hand-over: one
 // multicast commit raises `tfull` in both CTAs; the epilogue warps of both CTAs arrive on the EVEN CTA's `tempty`
 // (8 arrivals: 4 local, 4 remote) when they have drained a buffer.  All loads are plain per-CTA TMA loads of this
 // GPU's own operands.
 // ======================================================================================
 struct PCfg2 {
-  static constexpr int BN = 256;                 // token columns of the pair's accumulator
-  static constexpr int XH = BN / 2;              // token rows each CTA loads
+  static constexpr int BN = 256;                 // most token columns of the pair's accumulator (GemmArgs::bn: those of a launch)
   static constexpr int W_BYTES = BM * BK * 2;
-  static constexpr int X_BYTES = XH * BK * 2;
-  static constexpr int STAGE_BYTES = W_BYTES + X_BYTES;
-  static constexpr int STAGES = 6;               // 192 KB ring; the parked fp32 tile of the split-K schedule (128 KB) reuses it
-  static constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + 1024 /*align*/ + 512 /*barriers*/;
+  static constexpr int RING_BYTES = 192 * 1024;  // the parked fp32 tile of the split-K schedule (up to 128 KB) reuses it
+  static constexpr int MAX_STAGES = 10;
+  static constexpr int SMEM_BYTES = RING_BYTES + 1024 /*align*/ + 512 /*barriers*/;
+  // a stage: 64 columns of 128 weight rows and, in each CTA, of half of the token rows.  Its MMAs take 2 * bn clocks; waiting for it, issuing them and the
+  // commit take 250, its loads' issue as much (one arrival more per stage, both descriptors formed anew and a test beside them made these 480)
+  __host__ __device__ static constexpr int stage_bytes(int bn) { return W_BYTES + bn / 2 * BK * 2; }
+  __host__ __device__ static constexpr int stages(int bn) { return RING_BYTES / stage_bytes(bn) < MAX_STAGES ? RING_BYTES / stage_bytes(bn) : MAX_STAGES; }
+  static_assert((2 * MAX_STAGES + 4) * 8 + 16 <= 512, "barriers");
   static constexpr int MAX_GROUPS = 256, GROUP_BYTES = 2 * (MAX_GROUPS + 1) * 4;   // grouped form: its table, behind the barriers
 };
 
@@ -1236,12 +1242,13 @@ struct GroupWalk {
   const int* rows;               // [E + 1]
   const int* tiles;              // [E + 1] token tiles in front of group e
   int e = 0, ptn;
-  __device__ GroupWalk(const int* table, int E, int pair_tiles_n) : rows(table), tiles(table + E + 1), ptn(pair_tiles_n) {}
+  int bn;                        // rows of a token tile
+  __device__ GroupWalk(const int* table, int E, int pair_tiles_n, int bn_) : rows(table), tiles(table + E + 1), ptn(pair_tiles_n), bn(bn_) {}
   // tile < ptn * tiles[E], called with growing tiles
   __device__ __forceinline__ GroupTile at(int tile) {
     while (tile >= ptn * tiles[e + 1]) ++e;
     const int local = tile - ptn * tiles[e], tm = tiles[e + 1] - tiles[e];
-    return GroupTile{e, local / tm, rows[e] + (local % tm) * PCfg2::BN, rows[e + 1]};
+    return GroupTile{e, local / tm, rows[e] + (local % tm) * bn, rows[e + 1]};
   }
 };
 
@@ -1250,14 +1257,13 @@ __global__ void __launch_bounds__(kNumThreads, 1)
 gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant__ CUtensorMap tmap_x,
                  const __grid_constant__ GemmArgs a) {
   using C = PCfg2;
-  constexpr int BN = C::BN;
+  const int BN = a.bn, NST = C::stages(BN), stage_bytes = C::stage_bytes(BN);
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
-  uint64_t* bars = reinterpret_cast<uint64_t*>(smem + C::STAGES * C::STAGE_BYTES);
-  uint64_t* full_bar = bars;                       // own ring stage landed (TMA transaction bytes)
-  uint64_t* empty_bar = bars + C::STAGES;          // stage consumed (multicast commit of the even CTA)
-  uint64_t* peer_full_bar = bars + 2 * C::STAGES;  // even CTA only: the odd CTA's stage landed
-  uint64_t* tfull_bar = bars + 3 * C::STAGES;      // [2] accumulator complete (multicast commit)
+  uint64_t* bars = reinterpret_cast<uint64_t*>(smem + C::RING_BYTES);
+  uint64_t* full_bar = bars;                       // even CTA's: both CTAs' parts of a stage have landed (TMA transaction bytes)
+  uint64_t* empty_bar = bars + C::MAX_STAGES;      // stage consumed (multicast commit of the even CTA)
+  uint64_t* tfull_bar = bars + 2 * C::MAX_STAGES;  // [2] accumulator complete (multicast commit)
   uint64_t* tempty_bar = tfull_bar + 2;            // [2] even CTA only: accumulator drained by both CTAs' epilogues
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(tempty_bar + 2);
 
@@ -1269,21 +1275,18 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_consta
   int* group_table = reinterpret_cast<int*>(tmem_slot + 4);
   const int n_clusters = (int)gridDim.x / CS, cluster_id = (int)blockIdx.x / CS;   // S > 1: n_clusters == n_tiles
   const int kb0 = (int)(((int64_t)p * a.kb_total) / S), kb1 = (int)(((int64_t)(p + 1) * a.kb_total) / S);
-  constexpr int NG = BN / 8;
-  constexpr int TCOLS = 2 * BN;
-  // bring-up / profiling switch (LLMSS_GEMM_PAIR_DEBUG; results are WRONG unless 0): 2 = no MMAs (load pipeline
-  // alone), 3 = no loads (MMA issue rate alone)
-  const int dbg_mode = a.tm_rot;
+  const int NG = BN / 8;
+  const int stretch = (kb1 - kb0 + a.nacc - 1) / a.nacc, nacc = (kb1 - kb0 + stretch - 1) / stretch;      // k-blocks of an accumulator; those in use
+  constexpr int TCOLS = 2 * C::BN;
   pdl_launch_dependents();
   if (threadIdx.x == 0) LLMSS_STAMP(0);
 
   if (warp == 0 && lane == 0) {
     tma_prefetch_desc(&tmap_w);
     tma_prefetch_desc(&tmap_x);
-    for (int s = 0; s < C::STAGES; ++s) {
+    for (int s = 0; s < NST; ++s) {
       mbar_init(&full_bar[s], 1);
       mbar_init(&empty_bar[s], 1);
-      mbar_init(&peer_full_bar[s], 1);
     }
     for (int s = 0; s < 2; ++s) {
       mbar_init(&tfull_bar[s], 1);
@@ -1307,89 +1310,77 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_consta
     __syncthreads();
     n_tiles = pair_tiles_n * group_table[2 * a.n_groups + 1];
   }
-  GroupWalk walk(group_table, a.n_groups, pair_tiles_n);     // each role walks the tiles on its own
+  GroupWalk walk(group_table, a.n_groups, pair_tiles_n, BN);     // each role walks the tiles on its own
   if (threadIdx.x == 0) LLMSS_STAMP(1);
 
   if (warp == 0) {
     const uint64_t pol_w = l2_policy_evict_first();
     const uint64_t pol_x = l2_policy_evict_last();
+    const uint32_t full_leader = mapa_shared(smem_u32(full_bar), (uint32_t)(r & ~1));
     int stage = 0;
     uint32_t phase = 0;
-    for (int tile = cluster_id; tile < n_tiles && dbg_mode != 3; tile += n_clusters) {
+    for (int tile = cluster_id; tile < n_tiles; tile += n_clusters) {
       // token tile fastest: the pairs running at the same time share ONE weight tile (streamed from HBM once, L2 hits
       // for the others) and sweep the activation, which stays L2-resident across the weight tiles
       int tn, xrow, group = 0;        // tn: this CTA's 128-feature tile (may lie past N: zero-filled, unstored)
       if (GROUPED) {
         const GroupTile t = walk.at(tile);
         tn = t.fn * 2 + h;
-        xrow = t.row0 + h * C::XH;
+        xrow = t.row0 + h * (BN >> 1);
         group = t.e;
       } else {
         tn = (tile / a.tiles_m) * 2 + h;
-        xrow = (tile % a.tiles_m) * BN + (h ^ (a.aligned & 1)) * C::XH;   // a.aligned: bring-up switch for the half order
+        xrow = (tile % a.tiles_m) * BN + h * (BN >> 1);
       }
       for (int kb = kb0; kb < kb1; ++kb) {
         mbar_wait(&empty_bar[stage], phase ^ 1, 60);
-        uint8_t* sw = smem + stage * C::STAGE_BYTES;
+        uint8_t* sw = smem + stage * stage_bytes;
+        const uint32_t bar = full_leader + (uint32_t)(stage * 8);
         if (elect_one()) {
-          mbar_arrive_expect_tx(&full_bar[stage], C::STAGE_BYTES);
-          if (GROUPED) tma_load_3d(sw, &tmap_w, &full_bar[stage], kb * BK, tn * BM, group, pol_w);
-          else tma_load_2d(sw, &tmap_w, &full_bar[stage], kb * BK, tn * BM, pol_w);
-          tma_load_2d(sw + C::W_BYTES, &tmap_x, &full_bar[stage], kb * BK, xrow, pol_x);
+          if (h == 0) mbar_arrive_expect_tx(&full_bar[stage], (uint32_t)(2 * stage_bytes));
+          if (GROUPED) tma_load_3d_pair(sw, &tmap_w, bar, kb * BK, tn * BM, group, pol_w);
+          else tma_load_2d_pair(sw, &tmap_w, bar, kb * BK, tn * BM, pol_w);
+          tma_load_2d_pair(sw + C::W_BYTES, &tmap_x, bar, kb * BK, xrow, pol_x);
         }
         __syncwarp();
-        if (++stage == C::STAGES) { stage = 0; phase ^= 1; }
+        if (++stage == NST) { stage = 0; phase ^= 1; }
       }
     }
-  } else if (warp == 1 && h == 0) {
-    // ---- issuer (even CTA): one MMA of 256 features x 256 tokens x 16 per instruction, over both CTAs' stages
+  } else if (warp == 1) {
+    // ---- issuer (even CTA): one MMA of 256 features x BN tokens x 16 per instruction, over both CTAs' stages
     const uint32_t idesc = umma_idesc_f16(a.dtype == LLMSS_BF16 ? 1 : 0, 2 * BM, BN);
     const uint32_t smem_base = smem_u32(smem);
     const uint16_t pair_mask = (uint16_t)(3u << (r & ~1));
     int stage = 0, as = 0;
     uint32_t phase = 0, aphase = 0;
-    for (int tile = cluster_id; tile < n_tiles; tile += n_clusters) {
+    for (int tile = cluster_id; tile < n_tiles && h == 0; tile += n_clusters) {
       mbar_wait(&tempty_bar[as], aphase ^ 1, 65);   // both CTAs' epilogues have drained this accumulator
       tcgen05_fence_after();
-      const uint32_t d_tmem = tmem_base + (uint32_t)(as * BN);
-      for (int kb = kb0; kb < kb1; ++kb) {
-        if (dbg_mode != 3) {
-          mbar_wait(&full_bar[stage], phase, 61);
-          mbar_wait(&peer_full_bar[stage], phase, 62);
+      const uint32_t d_tile = tmem_base + (uint32_t)(as * C::BN);
+      int kb_acc = kb0;          // first block of the present accumulator's stretch
+      uint32_t d_tmem = d_tile;
+      for (int kb = kb0; kb < kb1; ++kb) {       // (straight-line code: see PCfg2)
+        if (kb - kb_acc == stretch) {
+          kb_acc = kb;
+          d_tmem += (uint32_t)BN;
         }
-        if (lane == 0 && a.dbg != nullptr && a.dbg[(size_t)blockIdx.x * 8 + 3] == 0) LLMSS_STAMP(3);
+        mbar_wait(&full_bar[stage], phase, 61);
         tcgen05_fence_after();
-        const uint32_t sw = smem_base + stage * C::STAGE_BYTES;
-        const uint32_t sx = sw + C::W_BYTES;
+        const uint32_t sw = umma_lo::desc_lo(smem_base + stage * stage_bytes), sx = sw + C::W_BYTES / 16;
         if (elect_one()) {
 #pragma unroll
           for (int k = 0; k < BK / 16; ++k)
-            if (dbg_mode != 2)
-              umma_f16_ss_pair(d_tmem, umma_desc_k_sw128(sw + k * 32), umma_desc_k_sw128(sx + k * 32), idesc,
-                               (kb > kb0 || k > 0) ? 1u : 0u);
+            umma_lo::umma_ss_pair(d_tmem, sw + k * 2, sx + k * 2, idesc, (kb > kb_acc || k > 0) ? 1u : 0u);
           umma_commit_pair(&empty_bar[stage], pair_mask);   // frees this stage in both CTAs
         }
         __syncwarp();
-        if (++stage == C::STAGES) { stage = 0; phase ^= 1; }
+        if (++stage == NST) { stage = 0; phase ^= 1; }
       }
       if (elect_one()) umma_commit_pair(&tfull_bar[as], pair_mask);
       __syncwarp();
       if (++as == 2) { as = 0; aphase ^= 1; }
     }
     if (lane == 0) LLMSS_STAMP(4);
-  } else if (warp == 1) {
-    // ---- forwarder (odd CTA): tell the issuer that this CTA's half of the stage has landed
-    int stage = 0;
-    uint32_t phase = 0;
-    const uint32_t leader = (uint32_t)(r & ~1);
-    for (int tile = cluster_id; tile < n_tiles && dbg_mode != 3; tile += n_clusters) {
-      for (int kb = kb0; kb < kb1; ++kb) {
-        mbar_wait(&full_bar[stage], phase, 63);
-        if (elect_one()) mbar_arrive_remote(mapa_shared(smem_u32(&peer_full_bar[stage]), leader));
-        __syncwarp();
-        if (++stage == C::STAGES) { stage = 0; phase ^= 1; }
-      }
-    }
   } else {
     const int quarter = warp & 3;
     const int f = quarter * 32 + lane;
@@ -1409,7 +1400,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_consta
         m0 = (tile % a.tiles_m) * BN;
       }
       const int n = tn * BM + f;
-      const uint32_t t_addr = tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(as * BN);
+      const uint32_t t_addr = tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(as * C::BN);
       mbar_wait(&tfull_bar[as], aphase, 64);  // all MMAs of the tile retired => its stages of BOTH CTAs have been consumed
       tcgen05_fence_after();
       if (threadIdx.x == 64) LLMSS_STAMP(5);
@@ -1438,6 +1429,15 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_consta
             for (int u = 0; u < CH; ++u)
 #pragma unroll
               for (int j = 0; j < 8; ++j) v[u][j] = __uint_as_float(q[u * 8 + j]);
+#pragma unroll 1
+            for (int x = 1; x < nacc; ++x) {
+              tmem_ld_32x32b_x32(t_addr + x * BN + cg0 * 8, q);
+              tmem_ld_wait();
+#pragma unroll
+              for (int u = 0; u < CH; ++u)
+#pragma unroll
+                for (int j = 0; j < 8; ++j) v[u][j] += __uint_as_float(q[u * 8 + j]);
+            }
           }
           if (cg0 + CH >= NG) {   // accumulator fully read: hand the buffer back before the stores
             tcgen05_fence_before();
@@ -1457,6 +1457,14 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_consta
           uint32_t q[32];
           tmem_ld_32x32b_x32(t_addr + cg0 * 8, q);
           tmem_ld_wait();
+#pragma unroll 1
+          for (int x = 1; x < nacc; ++x) {
+            uint32_t more[32];
+            tmem_ld_32x32b_x32(t_addr + x * BN + cg0 * 8, more);
+            tmem_ld_wait();
+#pragma unroll
+            for (int i = 0; i < 32; ++i) q[i] = __float_as_uint(__uint_as_float(q[i]) + __uint_as_float(more[i]));
+          }
 #pragma unroll
           for (int u = 0; u < 8; ++u)
             staging[((cg0 + (u >> 1)) * 2 + (u & 1)) * BM + f] = make_float4(
@@ -1858,26 +1866,70 @@ int pair_mode() {
   static int env_mode = -1;
   if (env_mode < 0) {
     const char* e = getenv("LLMSS_GEMM_PAIR");
-    env_mode = 8;  // default: automatic (pick_pair_split)
+    env_mode = 8;  // default: automatic (pick_pair)
     if (e != nullptr) env_mode = strcmp(e, "off") == 0 ? 0 : strcmp(e, "auto") == 0 ? 8 : atoi(e);
     if (env_mode != 0 && env_mode != 1 && env_mode != 2 && env_mode != 4 && env_mode != 8) env_mode = 8;
   }
   return env_mode;
 }
-// Pairs per cluster for a plain GEMM with a 256-token tile, 0 = keep the single-CTA kernels.  Deepest split-K that
-// still fits the machine in one wave and leaves every pair at least two k-blocks.
-int pick_pair_split(int M, int N, int kb_total, int sms) {
-  const int mode = pair_mode();
-  if (mode == 0 || M <= 128) return 0;
-  const int pair_tiles = ((N + 2 * BM - 1) / (2 * BM)) * ((M + 255) / 256);
-  if (mode == 1 || mode == 2 || mode == 4) return mode <= kb_total ? mode : 1;
-  // automatic (profiles/bench_gemm_pair.md): persistent pairs from 38 pair tiles upwards (N >= 9728 at M <= 256, every
-  // prefill GEMM); 24..37 pair tiles: two pairs per cluster split K, which fills the machine (4 CTAs per tile) and beat
-  // both the persistent form and the single-CTA kernels on every measured shape; below that the single-CTA cluster
-  // kernel with its deeper split wins.
-  if (pair_tiles >= 38) return 1;
-  if (pair_tiles >= 24 && pair_tiles * 4 <= sms && kb_total >= 4) return 2;
-  return 0;
+struct PairPlan {
+  int split, bn, nacc = 1;      // pairs per cluster (0: not this kernel), token columns of a tile, accumulators
+};
+// Estimate of the pair kernel's time in us for token tiles of bn columns, S pairs per cluster; constants fitted to 206 sweeps on B200 (N = 16 .. 50400,
+// K = 1600 .. 20480, 4 .. 8192 tokens, cold weights): the choice it leads to is 1.2 % behind the fastest of all (S, bn) on average.  A 64-column block
+// takes the longest of issuing it, its MMAs (slower the more of the chip is busy) and its share of what L2 delivers; all of it no less than memory
+// takes (token tiles of one weight tile do not all find it in L2); prologue and last epilogue grow with the tile.
+float pair_cost(int M, int N, int K, int kb_total, int sms, int bn, int S) {
+  const int tiles_m = (M + bn - 1) / bn, tiles = ((N + 2 * BM - 1) / (2 * BM)) * tiles_m;
+  const int pairs = sms / 2 > 1 ? sms / 2 : 1, rounds = S > 1 ? 1 : (tiles + pairs - 1) / pairs;
+  const float active = S > 1 ? (float)(tiles * S) : (float)((tiles + rounds - 1) / rounds);
+  const float mma = 0.00107f * bn * (1.f + 0.3f * active / pairs), l2 = active * 2.f * PCfg2::stage_bytes(bn) * (1.f / 15e6f);
+  float block = 0.15f;
+  if (mma > block) block = mma;
+  if (l2 > block) block = l2;
+  const float main_loop = (float)rounds * ((kb_total + S - 1) / S) * block;
+  const float mem = 2.f * ((float)N * K * (1.f + 0.15f * (tiles_m - 1)) + (float)M * K) * (1.f / 6.5e6f);
+  const float all = (main_loop > mem ? main_loop : mem) + (S > 1 ? 4.8f + 0.038f * bn : 3.5f + 0.025f * bn);
+  return bn == PCfg2::BN ? 0.96f * all : all;        // (fewest loads: faster than this where the whole chip is at its power limit)
+}
+// Accumulators that a tile may have.  A tensor core's sum over K is cut off at 24 bits after every 16 products, so that a 32-bit result of one chain over K = 2048
+// lies 2e-6 of its norm from 64 bits and one summed from eight stretches 5e-7.  A launch that gives every pair one tile has all of tensor memory for it,
+// others half.
+int pair_accumulators(int tiles, int bn, int sms) { return (tiles <= sms / 2 ? 512 : 256) / bn; }
+// the cheapest of all (S, bn) whose S times accumulators are at least `parts`; at most 128 features run only as two pairs per tile with narrow tiles (see pick_pair)
+PairPlan best_pair(int M, int N, int K, int kb_total, int sms, int parts, float* cost) {
+  const int pair_tiles_n = (N + 2 * BM - 1) / (2 * BM);
+  PairPlan best{0, 0, 1};
+  *cost = 0.f;
+  for (int bn = 32; bn <= PCfg2::BN && bn < M + 32; bn += 32)
+    for (int S = 1; S <= 2; ++S) {
+      if (S == 1 ? N <= BM : (kb_total < 4 || (int64_t)pair_tiles_n * ((M + bn - 1) / bn) * 4 > sms || (N <= BM && bn > 96))) continue;
+      const int n = (parts + S - 1) / S;
+      if (n > 1 && n > pair_accumulators(pair_tiles_n * ((M + bn - 1) / bn) * S, bn, sms)) continue;
+      const float c = pair_cost(M, N, K, kb_total, sms, bn, S) + (n > 1 ? 0.15f * (n - 1) * (bn / 32) : 0.f);
+      if (best.split == 0 || c < *cost) {
+        best = PairPlan{S, bn, n > 1 ? n : 1};
+        *cost = c;
+      }
+    }
+  return best;
+}
+// The pair kernel, or {0, 0}: the single-CTA kernels.  Those keep few tokens over few features, where a tile shared by up to eight CTAs is finished
+// sooner (us, single-CTA / pairs: 4 tokens 2048 x 2048 7.0 / 8.4, 4096 x 4096 11.2 / 12.1; 64 tokens 4096 x 4096 12.7 / 13.1, but 6144 x 2048
+// 16.3 / 10.4; 16 tokens 8320 x 4096 16.2 / 17.6, 50400 x 4096 69.3 / 65.5), and at most 128 features (half of each pair's MMA would be idle) unless two
+// pairs per tile fit the machine (16 x 2048: 140 tokens 11.5 / 7.8, 1200 11.9 / 9.9, 5000 15.4 / 17).  Above 64 tokens one 128-feature tile per CTA
+// loads too much: 128 tokens 6144 x 2048 21.2 / 10.7, 700 tokens 512 x 4096 46.6 / 12.0.
+PairPlan pick_pair(int M, int N, int K, int kb_total, int sms, int parts) {
+  const int mode = pair_mode() & 255, forced_bn = pair_mode() >> 8;
+  if (mode == 0) return {0, 0, 1};
+  if (mode == 1 || mode == 2 || mode == 4) {
+    if (M <= 128 && forced_bn == 0) return {0, 0, 1};
+    return {mode <= kb_total ? mode : 1, forced_bn ? forced_bn : 256, 1};
+  }
+  const int pair_tiles_n = (N + 2 * BM - 1) / (2 * BM);
+  if (M <= 16 ? pair_tiles_n < 44 : M <= 64 ? pair_tiles_n < 24 : false) return {0, 0, 1};
+  float cost;
+  return best_pair(M, N, K, kb_total, sms, parts, &cost);
 }
 
 // Largest cluster size (2..8) for which all `tiles` clusters are co-resident (one wave) and every CTA still
@@ -1967,7 +2019,7 @@ int pick_bn(int M) {
 // Profiling aid: when non-null, every CTA of the following llmss_gemm launches writes 8 globaltimer
 // stamps (entry, prologue done, last TMA issued, first stage landed, last MMA issued, first
 // accumulator ready, epilogue done, exit) to buf[cta*8 .. cta*8+7].  buf must be zeroed by the caller.
-LLMSS_API int llmss_gemm_set_pair(int mode) {
+LLMSS_API int llmss_gemm_set_pair(int mode) {          // mode | token tile << 8 also pins the width of the token tile
   g_pair_mode = mode;
   return 0;
 }
@@ -2124,26 +2176,35 @@ LLMSS_API int llmss_gemm_ex(const void* x, int64_t ldx, const void* w, int64_t l
                   ws->lam_bytes);
   }
   if (collective == 0) {
-    // token tiles of 129..256 rows: two CTAs share one 256 x 256 MMA, each loading half of the activation tile
-    const int ps = pick_pair_split(M, N, p.kb_total, max_ctas > 0 ? max_ctas : num_sms());
+    // two CTAs share one MMA of 256 features, each loading half of the token tile
+    // a 32-bit result is summed from more stretches of K than the single-CTA kernels would cut it into (above 128 tokens and 23 tiles of 256 x 256: two,
+    // and from 38 such tiles one), so that its error against 64 bits is no larger than theirs
+    const int sms = max_ctas > 0 ? max_ctas : num_sms(), wide = ((N + 2 * BM - 1) / (2 * BM)) * ((M + 255) / 256);
+    int parts = 1;
+    if (out_f32 && p.kb_total > 1) {
+      const int cut = p.split > 0 ? p.split : need_sk ? (p.grid + p.tiles - 1) / p.tiles : 1;
+      parts = M > 128 && wide >= 38 ? 1 : M > 128 && wide >= 24 ? 2 : cut > 1 ? cut + 1 : need_sk ? 2 : 1;
+      if (parts > p.kb_total) parts = p.kb_total;
+    }
+    const PairPlan pp = pick_pair(M, N, K, p.kb_total, sms, parts);
+    const int ps = pp.split;
     if (ps > 0) {
       CUtensorMap pw, px;
       if (int e = make_tmap(&pw, w, dtype, N, K, ldw, BM)) return e;
-      if (int e = make_tmap(&px, x, dtype, M, K, ldx, PCfg2::XH)) return e;
+      if (int e = make_tmap(&px, x, dtype, M, K, ldx, pp.bn / 2)) return e;
       GemmArgs a;
       memset(&a, 0, sizeof(a));
       a.M = M; a.N = N; a.K = K;
       a.tiles_n = (N + BM - 1) / BM;
-      a.tiles_m = (M + PCfg2::BN - 1) / PCfg2::BN;
+      a.bn = pp.bn;
+      a.nacc = pp.nacc;
+      a.tiles_m = (M + pp.bn - 1) / pp.bn;
       a.kb_total = p.kb_total;
       a.dtype = dtype;
       a.bias = bias; a.residual = residual; a.ldr = ldr;
       a.out = out; a.ldo = ldo; a.out_f32 = out_f32;
       a.act = act; a.act_start = act_start; a.gated = gated;
       a.epi = gated ? EPI_GATED : (out_f32 ? EPI_F32 : (act != LLMSS_ACT_NONE ? EPI_ACT : EPI_PLAIN));
-      static const int flip = getenv("LLMSS_GEMM_PAIR_FLIP") ? atoi(getenv("LLMSS_GEMM_PAIR_FLIP")) : 0;
-      a.aligned = flip;
-      { const char* d = getenv("LLMSS_GEMM_PAIR_DEBUG"); a.tm_rot = d ? atoi(d) : 0; }
       a.dbg = g_dbg;
       const int pair_tiles = ((a.tiles_n + 1) / 2) * a.tiles_m;
       // split-K: one tile per cluster; otherwise persistent pairs, as many as the machine holds (balanced over the tiles)
@@ -2227,16 +2288,27 @@ LLMSS_API int llmss_gemm_ex(const void* x, int64_t ldx, const void* w, int64_t l
 // Grouped linear layers (routed experts): rows [rows[e], rows[e + 1]) of x [P, K] times w_e [N, K] (element (n, k) of group e at
 // w + e * w_group_stride + n * ldw + k) -> the same rows of out.  groups: device table [rows[0..E] | first token tile of 256
 // rows, [0..E]] as llmss_moe_group writes it.  Nothing is read on the host.  gated: rows of w_e interleave (gate, up).
+LLMSS_API int llmss_gemm_grouped_tiles(const void* x, int64_t ldx, const void* w, int64_t ldw, int64_t w_group_stride, const int* groups, int E,
+                                       void* out, int64_t ldo, int P, int N, int K, int dtype, int out_f32, int act, int gated, int tile_rows,
+                                       cudaStream_t stream);
 LLMSS_API int llmss_gemm_grouped(const void* x, int64_t ldx, const void* w, int64_t ldw, int64_t w_group_stride, const int* groups, int E,
                                  void* out, int64_t ldo, int P, int N, int K, int dtype, int out_f32, int act, int gated,
                                  cudaStream_t stream) {
+  return llmss_gemm_grouped_tiles(x, ldx, w, ldw, w_group_stride, groups, E, out, ldo, P, N, K, dtype, out_f32, act, gated, PCfg2::BN, stream);
+}
+
+// The same with token tiles of tile_rows rows (a multiple of 32 up to 256), which `groups` counts
+LLMSS_API int llmss_gemm_grouped_tiles(const void* x, int64_t ldx, const void* w, int64_t ldw, int64_t w_group_stride, const int* groups, int E,
+                                       void* out, int64_t ldo, int P, int N, int K, int dtype, int out_f32, int act, int gated, int tile_rows,
+                                       cudaStream_t stream) {
+  LLMSS_REQUIRE(tile_rows >= 32 && tile_rows <= PCfg2::BN && tile_rows % 32 == 0, "gemm_grouped: token tiles of %d rows (32, 64 .. 256)", tile_rows);
   LLMSS_REQUIRE(dtype == LLMSS_F16 || dtype == LLMSS_BF16, "gemm_grouped: dtype must be f16/bf16");
   LLMSS_REQUIRE(P > 0 && N > 0 && K > 0 && K % 8 == 0 && E > 0 && E <= PCfg2::MAX_GROUPS, "gemm_grouped: bad shape P=%d N=%d K=%d E=%d", P, N, K, E);
   LLMSS_REQUIRE(!(gated && out_f32) && (!gated || N % 2 == 0), "gemm_grouped: a gated product has an even N and a 16-bit result");
   LLMSS_REQUIRE(((uintptr_t)w % 16) == 0 && ldw % 8 == 0 && w_group_stride % 8 == 0, "gemm_grouped: weights off the 16-byte lines");
   CUtensorMap tw, tx;
   if (int e = make_tmap_3d(&tw, w, dtype, K, N, E, ldw, w_group_stride, BM)) return e;
-  if (int e = make_tmap(&tx, x, dtype, P, K, ldx, PCfg2::XH)) return e;
+  if (int e = make_tmap(&tx, x, dtype, P, K, ldx, tile_rows / 2)) return e;
   GemmArgs a;
   memset(&a, 0, sizeof(a));
   a.M = P; a.N = N; a.K = K;
@@ -2247,13 +2319,56 @@ LLMSS_API int llmss_gemm_grouped(const void* x, int64_t ldx, const void* w, int6
   a.act = act; a.gated = gated;
   a.epi = gated ? EPI_GATED : (out_f32 ? EPI_F32 : (act != LLMSS_ACT_NONE ? EPI_ACT : EPI_PLAIN));
   a.groups = groups; a.n_groups = E;
+  a.bn = tile_rows;
+  a.nacc = 1;
   // as many persistent pairs as the machine holds; never more than there can be tiles
-  const int64_t most = (int64_t)((a.tiles_n + 1) / 2) * ((int64_t)P / PCfg2::BN + (P < E ? P : E));
+  const int64_t most = (int64_t)((a.tiles_n + 1) / 2) * ((int64_t)P / tile_rows + (P < E ? P : E));
   int clusters = num_sms() / 2;
   if (clusters > most) clusters = (int)most;
   if (clusters < 1) clusters = 1;
   return dtype == LLMSS_F16 ? launch_pair<__half, true>(tw, tx, a, clusters, 1, stream)
                             : launch_pair<__nv_bfloat16, true>(tw, tx, a, clusters, 1, stream);
+}
+
+// Token tiles of an expert with `rows` rows on average: counts spread by a binomial's deviation and a tenth of the mean.
+static float expert_tiles(float rows, int bn) {
+  const float s = sqrtf(rows) + 0.1f * rows;
+  float t = 0.f;
+  for (int i = -2; i <= 2; ++i) t += ceilf(fmaxf(rows + 0.6f * i * s, 0.f) / bn);
+  return 0.2f * t;
+}
+// Estimates, in us, of T tokens' choices of `top` of E experts (up matrices [rows, W], down [W, F]): both products over all experts for every token (dense),
+// and sorted by expert in tiles of *tile_rows rows (grouped), with the passes that sort, place and sum the rows.  Terms as in pair_cost; within 15 % of 30
+// measured blocks (4 of 16 experts of 1024, width 2048; 2 of 8 gated ones of 2048; 4 of 32 of 1536, width 4096; 64 .. 8192 tokens).
+LLMSS_API int llmss_moe_forms(int T, int top, int E, int W, int F, int rows, float* dense_us, float* grouped_us, int* tile_rows) {
+  LLMSS_REQUIRE(T > 0 && top > 0 && E > 0 && W > 0 && F > 0 && rows > 0, "moe_forms: bad sizes");
+  const int sms = num_sms(), pairs = sms / 2;
+  float dense = 4.f + (float)T * E * F * 4.f * (1.f / 4e6f), grouped = 0.f;
+  for (int i = 0; i < 2; ++i) {
+    const int64_t N = i ? W : (int64_t)E * rows, K = i ? (int64_t)E * F : W;
+    LLMSS_REQUIRE(N < (1ll << 31) && K < (1ll << 31), "moe_forms: sizes too large");
+    float best;
+    best_pair(T, (int)N, (int)K, (int)((K + BK - 1) / BK), sms, 1, &best);
+    dense += best;
+  }
+  const float mean = (float)T * top / E, used = (float)(E < (int64_t)T * top ? E : T * top);
+  for (int bn = 32; bn <= PCfg2::BN; bn += 32) {
+    float c = 0.f;
+    for (int i = 0; i < 2; ++i) {
+      const int N = i ? W : rows, K = i ? F : W;
+      const float all = expert_tiles(mean, bn) * E * ((N + 2 * BM - 1) / (2 * BM)), rounds = all <= pairs ? 1.f : ceilf(all / pairs);
+      const float active = all / rounds;
+      const float block = fmaxf(0.15f, fmaxf(0.00107f * bn * (1.f + 0.3f * active / pairs), active * 2.f * PCfg2::stage_bytes(bn) * (1.f / 15e6f)));
+      c += fmaxf(rounds * ((K + BK - 1) / BK) * block, 2.f * used * N * K * (1.f / 6.5e6f)) + 3.5f + 0.025f * bn;
+    }
+    if (grouped == 0.f || c < grouped) {
+      grouped = c;
+      *tile_rows = bn;
+    }
+  }
+  *dense_us = dense;
+  *grouped_us = grouped + 20.f + (float)T * top * W * 12.f * (1.f / 5e6f);
+  return 0;
 }
 
 // Per-head products: out(t, h, n) = scale(t, h, n) * sum_k x[t * ldx + h * sxh + k] * w[h * swh + n * ldw + k], 16-bit operands, all

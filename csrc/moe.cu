@@ -318,7 +318,6 @@ __global__ void __launch_bounds__(256) moe_combine_kernel(const float* __restric
 // ---- the same sorting without the host: per-block expert counts, then every block derives its own offsets from all counts and
 // places its pairs in pair order (the result does not depend on scheduling).  The table is what llmss_gemm_grouped reads.
 constexpr int PAIRS = 1024;      // pairs per block
-constexpr int GROUP_ROWS = 256;  // rows of a token tile of the grouped product
 
 __global__ void __launch_bounds__(256) moe_hist_kernel(const int* __restrict__ ids, int P, int E, int* __restrict__ hist) {
   __shared__ int c[256];
@@ -353,7 +352,7 @@ __device__ __forceinline__ int block_exclusive(int v, int* warps, int* total) {
 }
 
 __global__ void __launch_bounds__(256) moe_place_kernel(const int* __restrict__ ids, int P, int E, const int* __restrict__ hist,
-                                                        int* __restrict__ table, int* __restrict__ inv) {
+                                                        int* __restrict__ table, int* __restrict__ inv, int tile_rows) {
   __shared__ int warps[8];
   __shared__ int next[256];          // next free row of every expert for this block's pairs
   __shared__ int wcount[8][256];     // a round's pairs per warp and expert
@@ -369,7 +368,7 @@ __global__ void __launch_bounds__(256) moe_place_kernel(const int* __restrict__ 
   }
   int total, tiles;
   const int first = block_exclusive(all, warps, &total);
-  const int tile0 = block_exclusive((all + GROUP_ROWS - 1) / GROUP_ROWS, warps, &tiles);
+  const int tile0 = block_exclusive((all + tile_rows - 1) / tile_rows, warps, &tiles);
   if (blockIdx.x == 0) {
     if (e < E) { table[e] = first; table[E + 1 + e] = tile0; }
     if (e == 0) { table[E] = total; table[2 * E + 1] = tiles; }
@@ -546,15 +545,18 @@ LLMSS_API int llmss_moe_combine(const float* y, const int* inv, const float* wts
 }
 
 // Sorts the P = T * top (token, expert) pairs by expert on the device.  inv[pair] = row in the sorted order; table [2 * (E + 1)]:
-// first row of every expert (and P), first token tile of 256 rows of every expert (and their number); hist: scratch of
+// first row of every expert (and P), first token tile (of tile_rows rows; llmss_moe_group: of 256) of every expert (and their number); hist: scratch of
 // ceil(P / 1024) * E numbers.
-LLMSS_API int llmss_moe_group(const int* ids, int P, int E, int* hist, int* table, int* inv, cudaStream_t stream) {
-  LLMSS_REQUIRE(P > 0 && E > 0 && E <= 256, "moe_group: %d pairs, %d experts (at most 256)", P, E);
+LLMSS_API int llmss_moe_group_tiles(const int* ids, int P, int E, int* hist, int* table, int* inv, int tile_rows, cudaStream_t stream) {
+  LLMSS_REQUIRE(tile_rows > 0 && P > 0 && E > 0 && E <= 256, "moe_group: %d pairs, %d experts (at most 256)", P, E);
   const int blocks = (P + PAIRS - 1) / PAIRS;
   moe_hist_kernel<<<blocks, 256, 0, stream>>>(ids, P, E, hist);
-  moe_place_kernel<<<blocks, 256, 0, stream>>>(ids, P, E, hist, table, inv);
+  moe_place_kernel<<<blocks, 256, 0, stream>>>(ids, P, E, hist, table, inv, tile_rows);
   LLMSS_CHECK_CUDA(cudaGetLastError());
   return 0;
+}
+LLMSS_API int llmss_moe_group(const int* ids, int P, int E, int* hist, int* table, int* inv, cudaStream_t stream) {
+  return llmss_moe_group_tiles(ids, P, E, hist, table, inv, 256, stream);
 }
 
 // xs[inv[t * top + k]] = h[t] for every token and choice; h, xs 16-bit

@@ -91,8 +91,9 @@ typedef struct llmss_gemm_plan {
   int64_t sk_counters;
   int64_t ar_bytes;
 } llmss_gemm_plan;
-/* CTA-pair kernel (tcgen05 cta_group::2) for token tiles of 129..256 rows: -1 = environment (LLMSS_GEMM_PAIR =
- * off | auto | 1 | 2 | 4), 0 = off, 1 / 2 / 4 = pairs per cluster (split-K depth), 8 = automatic */
+/* CTA-pair kernel (tcgen05 cta_group::2): -1 = environment (LLMSS_GEMM_PAIR =
+ * off | auto | 1 | 2 | 4), 0 = off, 1 / 2 / 4 = pairs per cluster (split-K depth), 8 = automatic; 1 / 2 / 4 | n << 8: token tiles of n columns (32, 64 ..
+ * 256), also below 129 tokens */
 int llmss_gemm_set_pair(int mode);
 int llmss_gemm_set_debug(unsigned long long* per_cta_stamps); /* profiling aid: 8 globaltimer stamps per CTA */
 int llmss_gemm_plan_query(int M, int N, int K, int nranks, int elem_bytes, int max_ctas, llmss_gemm_plan* p);
@@ -224,12 +225,21 @@ int llmss_moe_gather_rows(const void* h, int64_t ldh, const int* perm, int top, 
 /* the same sorting without the host: inv[pair] = row in the order by expert, table [2 * (E + 1)] = first row of every expert (and P),
  * first tile of 256 rows of every expert (and their number); hist: ceil(P / 1024) * E numbers of scratch */
 int llmss_moe_group(const int* ids, int P, int E, int* hist, int* table, int* inv, llmss_stream_t stream);
+/* the same with tiles of tile_rows rows (what llmss_gemm_grouped_tiles is given) */
+int llmss_moe_group_tiles(const int* ids, int P, int E, int* hist, int* table, int* inv, int tile_rows, llmss_stream_t stream);
+/* host only: estimated us of T tokens' choices of `top` of E experts (up matrices [rows, W], down matrices [W, F]) with every expert for every token and
+ * sorted by expert, and the tile rows that suit the latter */
+int llmss_moe_forms(int T, int top, int E, int W, int F, int rows, float* dense_us, float* grouped_us, int* tile_rows);
 /* xs[inv[t * top + k]] = h[t], 16-bit rows */
 int llmss_moe_scatter_rows(const void* h, int64_t ldh, const int* inv, int top, void* xs, int T, int W, llmss_stream_t stream);
 /* rows [table[e], table[e + 1]) of x [P, K] times w_e [N, K]^T (element (n, k) at w + e * w_group_stride + n * ldw + k), 16-bit operands
  * with K, ldx, ldw and w_group_stride multiples of 8 */
 int llmss_gemm_grouped(const void* x, int64_t ldx, const void* w, int64_t ldw, int64_t w_group_stride, const int* table, int E, void* out,
                        int64_t ldo, int P, int N, int K, int dtype, int out_f32, int act, int gated, llmss_stream_t stream);
+/* the same in token tiles of tile_rows rows (a multiple of 32 up to 256; llmss_gemm_grouped: 256), counted by `table` */
+int llmss_gemm_grouped_tiles(const void* x, int64_t ldx, const void* w, int64_t ldw, int64_t w_group_stride, const int* table, int E, void* out,
+                             int64_t ldo, int P, int N, int K, int dtype, int out_f32, int act, int gated, int tile_rows,
+                             llmss_stream_t stream);
 /* per-head products out(t, h, n) = scale(t, h, n) * sum_k x[t * ldx + h * sxh + k] * w[h * swh + n * ldw + k]; llmss_bgemm_simt_ex takes it where it pays */
 int llmss_gemm_heads(const void* x, int64_t ldx, int64_t sxh, const void* w, int64_t ldw, int64_t swh, const float* scale, int64_t lds,
                      int64_t ssh, int64_t ssn, void* out, int64_t ldo, int64_t soh, int M, int N, int K, int H, int dtype, int out_f32,

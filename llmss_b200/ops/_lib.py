@@ -118,6 +118,10 @@ _SIGS = {
     "llmss_moe_permute": (c_int, [c_void_p, c_int, c_int, c_void_p, c_void_p, c_void_p, c_void_p]),
     "llmss_moe_gather_rows": (c_int, [c_void_p, c_int64, c_void_p, c_int, c_void_p, c_int, c_int, c_int, c_void_p]),
     "llmss_moe_group": (c_int, [c_void_p, c_int, c_int, c_void_p, c_void_p, c_void_p, c_void_p]),
+    "llmss_moe_group_tiles": (c_int, [c_void_p, c_int, c_int, c_void_p, c_void_p, c_void_p, c_int, c_void_p]),
+    "llmss_moe_forms": (c_int, [c_int, c_int, c_int, c_int, c_int, c_int, c_void_p, c_void_p, c_void_p]),
+    "llmss_gemm_grouped_tiles": (c_int, [c_void_p, c_int64, c_void_p, c_int64, c_int64, c_void_p, c_int, c_void_p, c_int64, c_int, c_int, c_int,
+                                         c_int, c_int, c_int, c_int, c_int, c_void_p]),
     "llmss_moe_scatter_rows": (c_int, [c_void_p, c_int64, c_void_p, c_int, c_void_p, c_int, c_int, c_void_p]),
     "llmss_gemm_grouped": (c_int, [c_void_p, c_int64, c_void_p, c_int64, c_int64, c_void_p, c_int, c_void_p, c_int64, c_int, c_int, c_int,
                                    c_int, c_int, c_int, c_int, c_void_p]),

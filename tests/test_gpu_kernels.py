@@ -139,6 +139,53 @@ def test_gemm_cta_pair_kernel(mode):
         lib.llmss_gemm_set_pair(-1)
 
 
+@pytest.mark.parametrize("split", [1, 2])
+@pytest.mark.parametrize("tile", [32, 96, 160, 224, 256])
+def test_gemm_pair_token_tiles(tile, split):
+    """Token tiles of every kind of width: one row, a row short of a tile, one over, several tiles; feature tiles without a partner; K tails and fewer
+    k-blocks than stages.  Bound (of the norm): the tensor core's sums are cut off at 24 bits once per 16 products, K / 16 x 2^-24 at most."""
+    from llmss_b200.ops import _lib
+
+    cu = _cu()
+    lib = _lib.load()
+    try:
+        lib.llmss_gemm_set_pair(split | tile << 8)
+        for M, N, K in [(1, 256, 128), (tile - 1, 640, 1096), (tile + 1, 130, 192), (3 * tile + 5, 896, 2048), (20, 20 * 256, 320)]:
+            torch.manual_seed(M + N)
+            x = torch.randn(M, K, device="cuda", dtype=torch.bfloat16)
+            w = (torch.randn(N, K, device="cuda") * K ** -0.5).to(torch.bfloat16)
+            b = torch.randn(N, device="cuda", dtype=torch.bfloat16)
+            want = x.double() @ w.double().t() + b.double()
+            got = cu.linear(x, w, b, out_dtype=torch.float32)
+            assert ((got.double() - want).norm() / want.norm()).item() < max(K, 256) / 16 * 2.0 ** -24, (M, N, K)
+            gated = cu.linear(x, w, act=R.ACT_SILU, gated=True)
+            _close(gated, R.linear(x, w, act=R.ACT_SILU, gated=True, out_dtype=torch.float32), 4e-2, 2e-2, f"gated {M} x {N} x {K}")
+    finally:
+        lib.llmss_gemm_set_pair(-1)
+
+
+@pytest.mark.parametrize("M,N,K", [(33, 6144, 2048), (65, 512, 4096), (100, 2048, 2048), (161, 2048, 2048), (300, 1000, 1032), (140, 16, 2048), (2401, 16, 320)])
+def test_gemm_32_bit_results_of_short_stretches(M, N, K):
+    """32-bit results that the library sums from several accumulators: no further from 64 bits than those of the single-CTA kernels, whose split over K they
+    replace (a tenth of that for chance)."""
+    from llmss_b200.ops import _lib
+
+    cu = _cu()
+    lib = _lib.load()
+    torch.manual_seed(M)
+    x = torch.randn(M, K, device="cuda", dtype=torch.bfloat16)
+    w = (torch.randn(N, K, device="cuda") * K ** -0.5).to(torch.bfloat16)
+    want = x.double() @ w.double().t()
+    err = {}
+    try:
+        for mode in (0, 8):
+            lib.llmss_gemm_set_pair(mode)
+            err[mode] = ((cu.linear(x, w, out_dtype=torch.float32).double() - want).norm() / want.norm()).item()
+    finally:
+        lib.llmss_gemm_set_pair(-1)
+    assert err[8] <= 1.1 * err[0], err
+
+
 # ------------------------------------------------------------------ norm
 @pytest.mark.parametrize("dtype", DT)
 @pytest.mark.parametrize("kind", [R.NORM_LAYER, R.NORM_RMS])
