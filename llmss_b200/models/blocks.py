@@ -182,10 +182,10 @@ class RotaryLatentAttention:
             return ops.linear(ctx, self.w_o, out_dtype=torch.float32)
 
 
-_GROUPED_ROWS = int(os.environ.get("LLMSS_MOE_GROUPED_MIN_ROWS", "64"))   # grouped form from this many rows per expert on average
+_GROUPED_ROWS = int(os.environ.get("LLMSS_MOE_GROUPED_MIN_ROWS", "16"))   # grouped form from this many rows per expert on average
 _FORCE_GROUPED = os.environ.get("LLMSS_MOE_FORCE_GROUPED", "0") == "1"
 _GEMM_TFLOPS, _CALL_US = 1200.0, 30.0     # sustained tensor-core rate of the expert GEMMs; host cost of issuing one GEMM
-_ROW_GBS, _GROUP_US = 5000.0, 55.0        # rate of the row passes around the grouped form; issuing its launches, fill-up
+_DENSE_HOST_US, _GROUPED_HOST_US = 70.0, 95.0   # issuing the launches of the two forms, the router's aside
 _DENSE_MIN = int(os.environ.get("LLMSS_MOE_DENSE_MIN_TOKENS", "0"))   # 0: dense as soon as token x top pairs >= experts
 
 
@@ -221,25 +221,22 @@ class RoutedExperts:
         return self.w_router
 
     def _grouped_pays(self, h) -> bool:
-        """Dense runs experts / top times the FLOPs in two launches; grouped runs the needed FLOPs, in tiles of 256 rows per
-        expert, plus the passes that sort the rows and sum a token's experts (16-bit rows out and back in, 32-bit results out and
-        back in: 12 bytes per pair and column).  Estimate both and take the cheaper.  Measured on B200, dense / grouped us: width 2048, 4
-        of 16 experts of 1024: 153 / 164 at 1024 tokens, 224 / 164 at 2048, 814 / 388 at 8192; 2 of 8 gated ones of 2048: 130 / 133 at 512,
-        171 / 133 at 700; width 4096, 4 of 32 of 1536: 210 / 229 at 256, 348 / 258 at 512.  Sizes off the tensor maps issue 2 x experts
-        GEMMs from the host.  LLMSS_MOE_GROUPED_MIN_ROWS=1 with LLMSS_MOE_FORCE_GROUPED=1 forces the grouped form."""
+        """Dense runs experts / top times the FLOPs in two launches; grouped runs the needed FLOPs, in tiles per expert, plus the
+        passes that sort the rows and sum a token's experts.  The library estimates both (llmss_moe_forms); neither is done before the host has issued its
+        launches.  Measured on B200 (device, without the router), dense / grouped us: width 2048, 4 of 16 experts of 1024: 58 / 52 at 215 tokens, 103 / 66 at
+        788, 757 / 329 at 8192; 2 of 8 gated ones of 2048: 95 / 63 at 400, 294 / 124 at 2000; width 4096, 4 of 32 of 1536: 139 / 144 at 64, 263 / 159 at
+        400.  Sizes off the tensor maps issue 2 x experts GEMMs from the host.  LLMSS_MOE_GROUPED_MIN_ROWS=1 with
+        LLMSS_MOE_FORCE_GROUPED=1 forces the grouped form."""
         if _FORCE_GROUPED:
             return True
         from ..ops import cuda_impl as cu
 
         T, W = h.shape
-        dense_us = (6.0 if self.gated else 4.0) * T * self.experts * self.ff * W / (_GEMM_TFLOPS * 1e6)
-        rows = T * self.top / self.experts
         if cu.moe_groups_on_device(h, self.w_up, self.w_down, self.gated):
-            tiles = (rows / 256 + 0.5) / max(1, -(-T // 256))          # of the dense form's token tiles
-            grouped_us = dense_us * tiles + T * self.top * W * 12 / (_ROW_GBS * 1e3) + _GROUP_US
-        else:
-            grouped_us = max(2 * self.experts * _CALL_US, dense_us * self.top / self.experts) + 150.0
-        return grouped_us < dense_us
+            dense_us, grouped_us, _ = cu.moe_forms(T, self.top, self.w_up.shape, self.ff)
+            return max(grouped_us, _GROUPED_HOST_US) < max(dense_us, _DENSE_HOST_US)
+        dense_us = (6.0 if self.gated else 4.0) * T * self.experts * self.ff * W / (_GEMM_TFLOPS * 1e6)
+        return max(2 * self.experts * _CALL_US, dense_us * self.top / self.experts) + 150.0 < dense_us
 
     def bind(self, base: int):
         self.z_off = base

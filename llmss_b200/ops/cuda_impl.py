@@ -7,6 +7,7 @@ a per-device arena allocated once.
 from __future__ import annotations
 
 import ctypes as C
+import functools
 import math
 import os
 from typing import Optional
@@ -630,11 +631,20 @@ def moe_groups_on_device(h, w_up, w_down, gated: bool = False) -> bool:
             and w_up.data_ptr() % 16 == 0 and w_down.data_ptr() % 16 == 0)
 
 
-def moe_experts_grouped(h, ids, wts, w_up, w_down, act, gated: bool = False, base=None):
+@functools.lru_cache(maxsize=1024)
+def moe_forms(T: int, top: int, up_shape, F: int):
+    """(us of the dense form, us of the grouped form, its tile rows) as the library estimates them."""
+    E, rows, W = up_shape
+    dense, grouped, tile = C.c_float(), C.c_float(), C.c_int()
+    _lib.check(_lib.load().llmss_moe_forms(T, top, E, W, F, rows, C.addressof(dense), C.addressof(grouped), C.addressof(tile)), "llmss_moe_forms")
+    return dense.value, grouped.value, tile.value
+
+
+def moe_experts_grouped(h, ids, wts, w_up, w_down, act, gated: bool = False, base=None, tile_rows: int = 0):
     """Long prompts: sort the (token, expert) pairs by expert and run every expert on its own contiguous rows -- top / experts of
     the dense form's FLOPs.  Sorting, row ranges and tiles stay on the device: one tensor-core launch per projection walks the
     experts (llmss_gemm_grouped).  Sizes that miss its tensor maps count on the host instead (one small synchronising copy) and
-    run a pair of linear layers per expert."""
+    run a pair of linear layers per expert.  ``tile_rows``: rows of a tile of the grouped products (0: chosen by the library)."""
     lib = _lib.load()
     T, W, ldh = _rows2d(h)
     E, F, _ = w_up.shape
@@ -649,13 +659,14 @@ def moe_experts_grouped(h, ids, wts, w_up, w_down, act, gated: bool = False, bas
     if moe_groups_on_device(h, w_up, w_down, gated):
         ints = torch.empty(P + 2 * (E + 1) + -(-P // 1024) * E, dtype=torch.int32, device=dev)
         inv, table, hist = ints[:P], ints[P:P + 2 * (E + 1)], ints[P + 2 * (E + 1):]
-        _lib.check(lib.llmss_moe_group(_ptr(ids), P, E, _ptr(hist), _ptr(table), _ptr(inv), _stream()), "llmss_moe_group")
-        _lib.check(lib.llmss_moe_scatter_rows(_ptr(h), ldh, _ptr(inv), top, _ptr(xs), T, W, _stream()), "llmss_moe_scatter_rows")
         rows = w_up.shape[1]
-        _lib.check(lib.llmss_gemm_grouped(_ptr(xs), W, _ptr(w_up), W, rows * W, _ptr(table), E, _ptr(a), F, P, rows, W, _DT[h.dtype], 0, act,
-                                          1 if gated else 0, _stream()), "llmss_gemm_grouped")
-        _lib.check(lib.llmss_gemm_grouped(_ptr(a), F, _ptr(w_down), w_down.stride(0), F, _ptr(table), E, _ptr(y), W, P, W, F, _DT[h.dtype], 1,
-                                          ACT_NONE, 0, _stream()), "llmss_gemm_grouped")
+        tile_rows = tile_rows or moe_forms(T, top, w_up.shape, F)[2]
+        _lib.check(lib.llmss_moe_group_tiles(_ptr(ids), P, E, _ptr(hist), _ptr(table), _ptr(inv), tile_rows, _stream()), "llmss_moe_group")
+        _lib.check(lib.llmss_moe_scatter_rows(_ptr(h), ldh, _ptr(inv), top, _ptr(xs), T, W, _stream()), "llmss_moe_scatter_rows")
+        _lib.check(lib.llmss_gemm_grouped_tiles(_ptr(xs), W, _ptr(w_up), W, rows * W, _ptr(table), E, _ptr(a), F, P, rows, W, _DT[h.dtype], 0, act,
+                                                1 if gated else 0, tile_rows, _stream()), "llmss_gemm_grouped")
+        _lib.check(lib.llmss_gemm_grouped_tiles(_ptr(a), F, _ptr(w_down), w_down.stride(0), F, _ptr(table), E, _ptr(y), W, P, W, F, _DT[h.dtype], 1,
+                                                ACT_NONE, 0, tile_rows, _stream()), "llmss_gemm_grouped")
         _count(5)
     else:
         counts = torch.empty(E, dtype=torch.int32, device=dev)

@@ -392,6 +392,22 @@ def test_experts_sorted_on_the_device(T, W, E, top, F, gated, skew):
     assert _rel(got.double() - base.double(), want.cpu()) < 1e-2
 
 
+@pytest.mark.parametrize("tile_rows", [32, 96, 224])
+@pytest.mark.parametrize("T,top,E,W,F,gated", [(5, 2, 8, 256, 192, False), (95, 3, 6, 136, 72, True), (700, 4, 16, 512, 256, False)])
+def test_grouped_tile_rows(T, top, E, W, F, gated, tile_rows):
+    """Grouped products in narrow tiles: the same bits as in tiles of 256 rows (every number is the same sum over K)."""
+    from llmss_b200.ops import cuda_impl as cu
+
+    torch.manual_seed(T)
+    dt = torch.bfloat16
+    h = torch.randn(T, W, device="cuda").to(dt)
+    up = (torch.randn(E, 2 * F if gated else F, W, device="cuda") * W ** -0.5).to(dt)
+    down = (torch.randn(W, E * F, device="cuda") * F ** -0.5).to(dt)
+    ids, wts = ops.moe_route(torch.randn(T, E, device="cuda"), E, top, 1, 1, 1.0)
+    got, want = (cu.moe_experts_grouped(h, ids, wts, up, down, ops.ACT_SILU, gated, tile_rows=r) for r in (tile_rows, 256))
+    assert torch.equal(got, want)
+
+
 @pytest.mark.parametrize("T,top,E,skew", [(1, 2, 8, False), (300, 4, 16, False), (513, 1, 5, True), (1024, 8, 256, False), (1025, 3, 3, False), (4096, 2, 200, True)])
 def test_pairs_sorted_by_expert(T, top, E, skew):
     """Places, row ranges and tile counts against a stable sort: single blocks and several, experts without pairs, a partial last block."""
