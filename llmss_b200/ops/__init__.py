@@ -13,6 +13,7 @@ from typing import Optional
 
 import torch
 
+from . import cuda_impl as cu
 from . import reference as ref
 from .reference import (DECAY_HEAD, DECAY_TOKEN_CHANNEL, DECAY_TOKEN_HEAD, GATE_NONE, GATE_SIGMOID, GATE_SILU, UNARY_NEG_EXP,
                         UNARY_TANH, distance_bias_table, rotary_frequencies, window_bias_table)
@@ -70,8 +71,6 @@ def linear(x, w, bias=None, act: int = ACT_NONE, gated: bool = False, act_start:
     bias/residual are applied once after the reduction."""
     reduce = comm is not None and not comm.single
     if _cuda(x):
-        from . import cuda_impl as cu
-
         if not reduce:
             return cu.linear(x, w, bias, act, gated, act_start, residual, out_dtype, out=out)
         assert out is None, "linear: out belongs to the unreduced form"
@@ -102,8 +101,6 @@ def linear(x, w, bias=None, act: int = ACT_NONE, gated: bool = False, act_start:
 def norm_residual(x, residual, weight, bias, eps: float, kind: int, x2=None):
     """Returns (norm(x [+x2] [+residual]), the pre-norm sum)."""
     if _cuda(x):
-        from . import cuda_impl as cu
-
         return cu.norm_residual(x, residual, weight, bias, eps, kind, x2=x2)
     if x2 is not None:
         x = (x.float() + x2.float()).to(x.dtype)
@@ -113,8 +110,6 @@ def norm_residual(x, residual, weight, bias, eps: float, kind: int, x2=None):
 def rope_kv_write(qkv, positions, slot_mapping, k_cache, v_cache, hq, hkv, d, rotary_dim, style, base,
                   q_off, k_off, v_off):
     if _cuda(qkv):
-        from . import cuda_impl as cu
-
         return cu.rope_kv_write(qkv, positions, slot_mapping, k_cache, v_cache, hq, hkv, d, rotary_dim, style, base,
                                 q_off, k_off, v_off)
     return ref.rope_kv_write(qkv, positions, slot_mapping, k_cache, v_cache, hq, hkv, d, rotary_dim, style, base,
@@ -133,8 +128,6 @@ def attention(qkv, out, batch, k_cache, v_cache, hq, hkv, d, scale, q_off, k_off
     q_view = qkv[:, q_off:q_off + hq * d]
     out_view = out[:, out_off:out_off + hq * d]
     if _cuda(qkv):
-        from . import cuda_impl as cu
-
         if d not in (64, 128, 256):
             _warn_once(f"head_dim={d} has no sm_100a attention kernel (64/128/256 do); using the generic PyTorch path")
         elif batch.is_decode:
@@ -184,8 +177,6 @@ def embed(tokens, wte, positions=None, wpe=None, pos_offset: int = 0, out_dtype=
     """``out_dtype=torch.float32``: rows summed and stored in 32-bit (32-bit residual stream); then ``scale`` multiplies the
     token row and ``out`` ([T, width] 32-bit, e.g. a plane of a layer-output history) receives the result."""
     if _cuda(wte):
-        from . import cuda_impl as cu
-
         if out_dtype == torch.float32:
             return cu.embed_f32(tokens, wte, positions, wpe, pos_offset, scale, out)
         assert scale == 1.0 and out is None, "embed: scale / out belong to the 32-bit form"
@@ -201,8 +192,6 @@ def dyt_residual(resid, alpha: float, weight, bias, a=None, scale_a=None, b=None
     (tanh(alpha x) * weight + bias): returns (normed in ``out_dtype``, new residual).  ``want_norm=False`` only
     updates the residual (before an op that is not a norm, e.g. a re-injection GEMM)."""
     if _cuda(resid):
-        from . import cuda_impl as cu
-
         return cu.dyt_residual(resid, alpha, weight, bias, a, scale_a, b, scale_b, out_dtype, want_norm)
     return ref.dyt_residual(resid, alpha, weight, bias, a, scale_a, b, scale_b, out_dtype, want_norm)
 
@@ -210,8 +199,6 @@ def dyt_residual(resid, alpha: float, weight, bias, a=None, scale_a=None, b=None
 def cast_concat(a, b, dtype):
     """[cast(a) | cast(b)] of two 32-bit [T, *] streams as one GEMM operand."""
     if _cuda(a):
-        from . import cuda_impl as cu
-
         return cu.cast_concat(a, b, dtype)
     return ref.cast_concat(a, b, dtype)
 
@@ -219,8 +206,6 @@ def cast_concat(a, b, dtype):
 # ----------------------------------------------------------------------------- latent attention
 def latent_prep(y, q_off, c_off, g_off, n_q, rank, heads, norm_w, eps, slot_mapping, cache, dtype):
     if _cuda(y):
-        from . import cuda_impl as cu
-
         return cu.latent_prep(y, q_off, c_off, g_off, n_q, rank, heads, norm_w, eps, slot_mapping, cache, dtype)
     return ref.latent_prep(y, q_off, c_off, g_off, n_q, rank, heads, norm_w, eps, slot_mapping, cache, dtype)
 
@@ -229,8 +214,6 @@ def heads_matmul(x, w, heads, k, n, w_is_kn, row_scale=None, out_dtype=None, x_h
                  out_head_stride=None):
     """Per-head product [T, heads * k] x [heads, k, n]; see ops.reference.heads_matmul for the strides and scales."""
     if _cuda(x):
-        from . import cuda_impl as cu
-
         return cu.heads_matmul(x, w, heads, k, n, w_is_kn, row_scale, out_dtype, x_head_stride, elem_scale, out, out_head_stride)
     return ref.heads_matmul(x, w, heads, k, n, w_is_kn, row_scale, out_dtype, x_head_stride, elem_scale, out, out_head_stride)
 
@@ -239,8 +222,6 @@ def latent_query_dtype(cache, heads, rank):
     """Type in which latent_attention() wants the absorbed queries: the cache's 16-bit type where it will run on the
     tcgen05 multi-query kernels, 32-bit for the generic kernel and on CPU."""
     if _cuda(cache):
-        from . import cuda_impl as cu
-
         if cu.latent_uses_tc(cache.dtype, rank, cache.shape[1], heads):
             return cache.dtype
     return torch.float32
@@ -253,8 +234,6 @@ def latent_attention(q_abs, cache, batch, heads, rank, scale, out_dtype):
     cache has their [blocks, 1, block_size, d] layout): decode batches on the split-KV decode kernel, portions of
     prompts on the paged prefill kernel.  Every other case (true 32-bit, other ranks) runs the generic kernel."""
     if _cuda(q_abs):
-        from . import cuda_impl as cu
-
         return cu.latent_attention(q_abs, cache, batch, heads, rank, scale, out_dtype)
     return ref.latent_attention(q_abs, cache, batch.block_tables, batch.seq_lens, batch.cu_q, heads, rank, scale, out_dtype)
 
@@ -262,8 +241,6 @@ def latent_attention(q_abs, cache, batch, heads, rank, scale, out_dtype):
 # ----------------------------------------------------------------------------- routed experts
 def moe_route(z, experts, top, groups, keep, route_scale, score="softmax", correction=None, group_top=1, renorm=True):
     if _cuda(z):
-        from . import cuda_impl as cu
-
         return cu.moe_route(z, experts, top, groups, keep, route_scale, score=score, correction=correction, group_top=group_top,
                             renorm=renorm)
     return ref.moe_route(z, experts, top, groups, keep, route_scale, score, correction, group_top, renorm)
@@ -272,8 +249,6 @@ def moe_route(z, experts, top, groups, keep, route_scale, score="softmax", corre
 def moe_experts(h, ids, wts, w_up, w_down, act, gated: bool = False, base=None):
     """``base`` [T, W] 32-bit: the weighted sum is added to it in place."""
     if _cuda(h):
-        from . import cuda_impl as cu
-
         return cu.moe_experts(h, ids, wts, w_up, w_down, act, gated, base)
     return ref.moe_experts(h, ids, wts, w_up, w_down, act, gated, base)
 
@@ -281,8 +256,6 @@ def moe_experts(h, ids, wts, w_up, w_down, act, gated: bool = False, base=None):
 # ----------------------------------------------------------------------------- recurrent layers, post-norm residual
 def _dispatch(name, probe, *args, **kw):
     if _cuda(probe):
-        from . import cuda_impl as cu
-
         return getattr(cu, name)(*args, **kw)
     return getattr(ref, name)(*args, **kw)
 
@@ -324,8 +297,6 @@ def attention_bias(q, k_cache, v_cache, batch, hq, hkv, dk, dv, scale, dist_bias
     maps per head, combined as rms_div(a1 - lam * a2) * factor; ``out``: view that receives [T, hq * dv].
     ``chunk``: keys outside the query's own block of ``chunk`` positions are hidden.  v_cache may be a column view of wider rows."""
     if _cuda(q):
-        from . import cuda_impl as cu
-
         return cu.attention_bias(q, k_cache, v_cache, batch, hq, hkv, dk, dv, scale, dist_bias, gate, out_dtype, bias_over_scale,
                                  window, slopes, sinks, keep_first, softcap, diff, out, chunk)
     return ref.attention_bias(q, k_cache, v_cache, batch.block_tables, batch.seq_lens, batch.cu_q, hq, hkv, dk, dv, scale,
@@ -426,8 +397,6 @@ def norm_rope_kv_write(qkv, hq, hkv, dk, dv, maps, q_w, k_w, eps, freq, mag, int
     prepares queries only.  ``v_first`` [T, hkv * dv] 32-bit: the values become (1 - v_lam) * v + v_lam * v_first.  ``batch`` and the score ``scale`` let the CUDA path lay the queries out for the attention kernel that will
     read them (attention_bias with the same ``batch``)."""
     if _cuda(qkv):
-        from . import cuda_impl as cu
-
         return cu.norm_rope_kv_write(qkv, hq, hkv, dk, dv, maps, q_w, k_w, eps, freq, mag, interleaved, positions, slot_mapping, k_cache,
                                      v_cache, batch, scale, out_dtype, v_first, v_lam)
     return ref.norm_rope_kv_write(qkv, hq, hkv, dk, dv, maps, q_w, k_w, eps, freq, mag, interleaved, positions, slot_mapping, k_cache,
@@ -436,8 +405,6 @@ def norm_rope_kv_write(qkv, hq, hkv, dk, dv, maps, q_w, k_w, eps, freq, mag, int
 
 def sample(logits, greedy, temperature, top_k, top_p, rng_state, vocab: Optional[int] = None, out=None):
     if _cuda(logits):
-        from . import cuda_impl as cu
-
         return cu.sample(logits, greedy, temperature, top_k, top_p, rng_state, vocab, out)
     tok = ref.sample(logits, greedy, temperature, top_k, top_p, rng_state, vocab).to(torch.int32)
     if out is not None:

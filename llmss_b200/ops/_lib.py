@@ -295,6 +295,9 @@ def load(build_if_missing: bool = True):
         if hasattr(lib, name):
             fn = getattr(lib, name)
             fn.restype, fn.argtypes = res, args
+    from . import calls
+
+    calls.attach(lib, lib_path().parent, {**_SIGS, **_OPTIONAL})
     _LIB, LOADED_FROM = lib, str(path)
     return lib
 

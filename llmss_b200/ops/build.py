@@ -77,8 +77,23 @@ def is_current() -> bool:
     return LIB_PATH.exists() and stamp.exists() and stamp.read_text().strip() == tree_digest()
 
 
+def _calls_current() -> bool:
+    from . import _lib, calls
+
+    return calls.module_path(LIB_DIR, {**_lib._SIGS, **_lib._OPTIONAL}).exists()
+
+
+def _build_calls():
+    """The entries as plain functions (calls.py); every call works without them."""
+    from . import _lib, calls
+
+    OBJ_DIR.mkdir(parents=True, exist_ok=True)
+    if not calls.build(LIB_DIR, OBJ_DIR, {**_lib._SIGS, **_lib._OPTIONAL}):
+        print("[build] no C compiler or Python headers: library calls go through ctypes", file=sys.stderr)
+
+
 def build_library(verbose: bool = False, force: bool = False) -> Path:
-    if not force and is_current():  # e.g. on the GPU box: the .so travelled with the tree
+    if not force and is_current() and _calls_current():  # e.g. on the GPU box: the .so files travelled with the tree
         return LIB_PATH
     LIB_DIR.mkdir(parents=True, exist_ok=True)
     # one builder at a time (torchrun starts N ranks at once); the others wait, then see a current library
@@ -87,6 +102,8 @@ def build_library(verbose: bool = False, force: bool = False) -> Path:
     with open(LIB_DIR / ".build.lock", "w") as lock:
         fcntl.flock(lock, fcntl.LOCK_EX)
         try:
+            if not _calls_current():
+                _build_calls()
             if not force and is_current():
                 return LIB_PATH
             return _build_locked(verbose, force)

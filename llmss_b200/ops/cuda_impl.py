@@ -69,8 +69,9 @@ def arena(device) -> _Arena:
 
 
 def _rows2d(x: torch.Tensor):
-    assert x.dim() == 2 and x.stride(1) == 1, "expected a 2-D tensor with contiguous last dim"
-    return x.shape[0], x.shape[1], x.stride(0)
+    shape, stride = x.shape, x.stride()
+    assert len(shape) == 2 and stride[1] == 1, "expected a 2-D tensor with contiguous last dim"
+    return shape[0], shape[1], stride[0]
 
 
 # --------------------------------------------------------------------------- GEMM
