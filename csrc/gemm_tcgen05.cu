@@ -103,6 +103,7 @@ struct GemmArgs {
   const int* groups;           // grouped pair kernel: [E + 1] first row of every group, then [E + 1] first token tile
   int n_groups;                // E
   int bn;                      // pair kernel: token columns of a tile, a multiple of 32 up to 256
+  int wide;                    // 16-bit rows of out may be stored by 8 bytes (see store_4_tokens)
   int nacc;                    // pair kernel: accumulators of a tile, each over its own stretch of K (see pair_accumulators)
   unsigned long long* dbg;  // optional per-CTA phase timestamps [grid][8] (globaltimer ns), see llmss_gemm_set_debug
   SymmWs ws;
@@ -272,11 +273,42 @@ __device__ __forceinline__ void store_chunk(const GemmArgs& a, const float (&v)[
 #undef LLMSS_SC
 }
 
+template <typename T>
+__device__ __forceinline__ uint32_t pack2(float lo, float hi) {
+  typename Vec2<T>::type p;
+  if constexpr (std::is_same<T, __half>::value) p = __floats2half2_rn(lo, hi);
+  else p = __floats2bfloat162_rn(lo, hi);
+  return *reinterpret_cast<const uint32_t*>(&p);
+}
+// Four tokens of a lane's feature, 16-bit, as 8-byte stores: four neighbouring lanes exchange until lane r of them has token r of their four features, so that
+// a warp's store covers four rows of 64 bytes (each lane storing its own column takes four instructions of one row each: per-head products of 8192 tokens
+// 33.0 us, so 31.2; the products of a 6-layer prompt pass, with GELU, 88 each, so 85).  o: row 0 at the first of the four features, 8-byte aligned with ldo a multiple of 4.  The whole warp calls it.
+template <typename T>
+__device__ __forceinline__ void store_4_tokens(T* o, int64_t ldo, float t0, float t1, float t2, float t3, int lane) {
+  const bool odd = lane & 1, upper = lane & 2;
+  const uint32_t a0 = pack2<T>(t0, t1), a1 = pack2<T>(t2, t3);
+  uint32_t got = __shfl_xor_sync(0xffffffffu, __byte_perm(a0, a1, odd ? 0x5410 : 0x7632), 1);
+  const uint32_t b0 = __byte_perm(a0, got, odd ? 0x3254 : 0x5410), b1 = __byte_perm(a1, got, odd ? 0x3276 : 0x7610);
+  got = __shfl_xor_sync(0xffffffffu, upper ? b0 : b1, 2);
+  *reinterpret_cast<uint2*>(o + (int64_t)(lane & 3) * ldo) = upper ? make_uint2(got, b1) : make_uint2(b0, got);
+}
+
 // Plain flavour (bias / residual only), all CH*8 token rows and the feature in range: one pointer walked by the row
 // stride, no per-element predicate or address arithmetic (with the generic path above the epilogue of a 128 x 256 tile took 11 us).
 template <typename T, int CH>
-__device__ __forceinline__ void store_chunk_plain_full(const GemmArgs& a, const float (&v)[CH][8], int n, int mb0, float bval) {
+__device__ __forceinline__ void store_chunk_plain_full(const GemmArgs& a, const float (&v)[CH][8], int n, int mb0, int lane, float bval) {
   T* o = reinterpret_cast<T*>(a.out) + (int64_t)mb0 * a.ldo + n;
+  if (a.wide && a.residual == nullptr) {
+    o -= lane & 3;
+#pragma unroll
+    for (int u = 0; u < CH; ++u)
+#pragma unroll
+      for (int j = 0; j < 8; j += 4) {
+        store_4_tokens<T>(o, a.ldo, v[u][j] + bval, v[u][j + 1] + bval, v[u][j + 2] + bval, v[u][j + 3] + bval, lane);
+        o += 4 * a.ldo;
+      }
+    return;
+  }
   if (a.residual != nullptr) {
     const T* r = reinterpret_cast<const T*>(a.residual) + (int64_t)mb0 * a.ldr + n;
     float rv[CH][8];
@@ -321,6 +353,26 @@ __device__ __forceinline__ void store_chunk_full_t(const GemmArgs& a, const floa
   } else {
     using TO = typename std::conditional<EPI == EPI_F32, float, T>::type;
     TO* o = reinterpret_cast<TO*>(a.out) + (int64_t)mb0 * a.ldo + n;
+    if constexpr (EPI != EPI_F32) {
+      if (a.wide && !has_res) {
+        const bool act = n >= a.act_start;
+        o -= lane & 3;
+#pragma unroll
+        for (int u = 0; u < CH; ++u)
+#pragma unroll
+          for (int j = 0; j < 8; j += 4) {
+            float y[4];
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+              const float x = v[u][j + i] + bval;
+              y[i] = act ? act_t<ACT>(x, a.act) : x;
+            }
+            store_4_tokens<T>(o, a.ldo, y[0], y[1], y[2], y[3], lane);
+            o += 4 * a.ldo;
+          }
+        return;
+      }
+    }
     const T* r = reinterpret_cast<const T*>(a.residual) + (int64_t)mb0 * a.ldr + n;
     const bool do_act = n >= a.act_start;
 #pragma unroll
@@ -339,7 +391,7 @@ __device__ __forceinline__ void store_chunk_full_t(const GemmArgs& a, const floa
 template <typename T, int CH>
 __device__ __forceinline__ void store_chunk_full(const GemmArgs& a, const float (&v)[CH][8], int n, int mb0, int lane, float bval) {
   if (a.epi == EPI_PLAIN) {
-    store_chunk_plain_full<T, CH>(a, v, n, mb0, bval);
+    store_chunk_plain_full<T, CH>(a, v, n, mb0, lane, bval);
   } else if (a.epi == EPI_ACT) {
     if (a.act == LLMSS_ACT_GELU_TANH) store_chunk_full_t<T, CH, EPI_ACT, LLMSS_ACT_GELU_TANH>(a, v, n, mb0, lane, bval);
     else if (a.act == LLMSS_ACT_SILU) store_chunk_full_t<T, CH, EPI_ACT, LLMSS_ACT_SILU>(a, v, n, mb0, lane, bval);
@@ -1213,10 +1265,14 @@ gemm_cluster_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
 // Protocol: every CTA's TMA warp fills its own ring; the loads of both CTAs report to the even CTA's `full` barrier (cta_group::2), which that CTA
 // arms with the bytes of both.  The even CTA's warp 1 issues, and frees the stage in BOTH CTAs with one multicast commit.  Accumulator hand-over: one
 // multicast commit raises `tfull` in both CTAs; the epilogue warps of both CTAs arrive on the EVEN CTA's `tempty`
-// (8 arrivals: 4 local, 4 remote) when they have drained a buffer.  All loads are plain per-CTA TMA loads of this
+// (16 arrivals: 8 local, 8 remote) when they have drained a buffer.  All loads are plain per-CTA TMA loads of this
 // GPU's own operands.
 // ======================================================================================
 struct PCfg2 {
+  // warps 0 and 1 as everywhere, 2 .. 9 the epilogue: two to a quarter of the features, alternate chunks of 32 columns.  A chunk is a chain from the load out of
+  // tensor memory to the stores, and the last tile's chunks are exposed: with one warp to a quarter 366 tokens 4096 x 4096 took 28.9 us in tiles of 256 columns,
+  // with two 27.2; per-head products of 8192 tokens, which are little else, 45.5 and 31
+  static constexpr int THREADS = 320, EPI_WARPS = 8;
   static constexpr int BN = 256;                 // most token columns of the pair's accumulator (GemmArgs::bn: those of a launch)
   static constexpr int W_BYTES = BM * BK * 2;
   static constexpr int RING_BYTES = 192 * 1024;  // the parked fp32 tile of the split-K schedule (up to 128 KB) reuses it
@@ -1253,7 +1309,7 @@ struct GroupWalk {
 };
 
 template <typename T, bool GROUPED>
-__global__ void __launch_bounds__(kNumThreads, 1)
+__global__ void __launch_bounds__(PCfg2::THREADS, 1)
 gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant__ CUtensorMap tmap_x,
                  const __grid_constant__ GemmArgs a) {
   using C = PCfg2;
@@ -1290,7 +1346,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_consta
     }
     for (int s = 0; s < 2; ++s) {
       mbar_init(&tfull_bar[s], 1);
-      mbar_init(&tempty_bar[s], 8);   // one arrive per epilogue warp of either CTA
+      mbar_init(&tempty_bar[s], 2 * C::EPI_WARPS);   // one arrive per epilogue warp of either CTA
     }
     fence_mbar_init();
   }
@@ -1306,7 +1362,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_consta
   float4* staging = reinterpret_cast<float4*>(smem);  // split-K: [NG*2][128] float4, reuses the drained TMA ring
   pdl_wait();
   if (GROUPED) {
-    for (int i = threadIdx.x; i < 2 * (a.n_groups + 1); i += kNumThreads) group_table[i] = a.groups[i];
+    for (int i = threadIdx.x; i < 2 * (a.n_groups + 1); i += C::THREADS) group_table[i] = a.groups[i];
     __syncthreads();
     n_tiles = pair_tiles_n * group_table[2 * a.n_groups + 1];
   }
@@ -1382,7 +1438,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_consta
     }
     if (lane == 0) LLMSS_STAMP(4);
   } else {
-    const int quarter = warp & 3;
+    const int quarter = warp & 3, half = (warp - 2) >> 2;
     const int f = quarter * 32 + lane;
     const T* bias = reinterpret_cast<const T*>(a.bias);
     int as = 0;
@@ -1412,7 +1468,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_consta
         // per chunk
         const bool plain_ok = tn * BM + quarter * 32 + 32 <= a.N;
 #pragma unroll 1
-        for (int cg0 = 0; cg0 < NG; cg0 += CH) {
+        for (int cg0 = half * CH; cg0 < NG; cg0 += 2 * CH) {
           float v[CH][8], rv[CH][8];
           const bool fast = plain_ok && m0 + (cg0 + CH) * 8 <= m_end;
           if (!fast) {
@@ -1439,7 +1495,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_consta
                 for (int j = 0; j < 8; ++j) v[u][j] += __uint_as_float(q[u * 8 + j]);
             }
           }
-          if (cg0 + CH >= NG) {   // accumulator fully read: hand the buffer back before the stores
+          if (cg0 + 2 * CH >= NG) {   // this warp's part fully read: hand the buffer back before the stores
             tcgen05_fence_before();
             __syncwarp();
             if (lane == 0) mbar_arrive_remote(tempty_leader + (uint32_t)(as * 8));
@@ -1450,10 +1506,11 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_consta
             __syncwarp();        // lanes past N rejoin: the next load from tensor memory is the whole warp's
           }
         }
+        if (half * CH >= NG && lane == 0) mbar_arrive_remote(tempty_leader + (uint32_t)(as * 8));       // (a tile of one chunk)
       } else {
         // ---- split-K: park the partial accumulator in shared memory: [(cg*2 + half)][feature] float4, conflict-free
 #pragma unroll 1
-        for (int cg0 = 0; cg0 < NG; cg0 += 4) {
+        for (int cg0 = half * 4; cg0 < NG; cg0 += 8) {
           uint32_t q[32];
           tmem_ld_32x32b_x32(t_addr + cg0 * 8, q);
           tmem_ld_wait();
@@ -1489,14 +1546,14 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_consta
       const T* bias = reinterpret_cast<const T*>(a.bias);
       const uint32_t stage_u32 = smem_u32(staging);
 #pragma unroll 1
-      for (int it0 = epi_tid; it0 < my_items; it0 += 256) {
-        const bool two = it0 + 128 < my_items;
+      for (int it0 = epi_tid; it0 < my_items; it0 += 512) {
+        const bool two = it0 + 256 < my_items;
         float vv[2][8];
-        dsmem_reduce_pair(stage_u32, S, p * per + it0, p * per + (two ? it0 + 128 : it0), two, vv[0], vv[1], 2, h);
+        dsmem_reduce_pair(stage_u32, S, p * per + it0, p * per + (two ? it0 + 256 : it0), two, vv[0], vv[1], 2, h);
 #pragma unroll
         for (int u = 0; u < 2; ++u) {
           if (u == 1 && !two) break;
-          const int item = p * per + it0 + u * 128;
+          const int item = p * per + it0 + u * 256;
           const int cg = item / BM, f = item % BM;
           const int n = tn * BM + f;
           float v[1][8], rv[1][8];
@@ -1553,11 +1610,11 @@ struct HeadArgs {
   int tiles_n, tiles_m, kb_total, dtype;
   const float* scale; int64_t lds, ssh, ssn;     // scale(t, h, n) = scale[t * lds + h * ssh + n * ssn], or null
   void* out; int64_t ldo, soh;
-  int out_f32;
+  int out_f32, wide;             // wide: see store_4_tokens
 };
 
 template <typename T>
-__global__ void __launch_bounds__(kNumThreads, 1)
+__global__ void __launch_bounds__(PCfg2::THREADS, 1)
 gemm_heads_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant__ CUtensorMap tmap_x, const __grid_constant__ HeadArgs a) {
   constexpr int BN = 256, NG = BN / 8;
   using C = Cfg<BN>;
@@ -1580,7 +1637,7 @@ gemm_heads_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_const
     }
     for (int s = 0; s < 2; ++s) {
       mbar_init(&tfull_bar[s], 1);
-      mbar_init(&tempty_bar[s], 4);  // one arrive per epilogue warp
+      mbar_init(&tempty_bar[s], PCfg2::EPI_WARPS);  // one arrive per epilogue warp
     }
     fence_mbar_init();
   }
@@ -1639,7 +1696,7 @@ gemm_heads_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_const
       if (++as == 2) { as = 0; aphase ^= 1; }
     }
   } else {
-    const int quarter = warp & 3, f = quarter * 32 + lane;
+    const int quarter = warp & 3, f = quarter * 32 + lane, first = (warp - 2) >> 2 ? 4 : 0;      // (alternate chunks, as in the pair kernel)
     int as = 0;
     uint32_t aphase = 0;
     for (int tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
@@ -1651,11 +1708,11 @@ gemm_heads_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_const
       // exchanges them
       const bool by_feature = sp != nullptr && a.ssn != 0;
       auto factor = [&](int cg) { return m0 + cg * 8 + lane < a.M ? __ldg(sp + (int64_t)(cg * 8 + lane) * a.lds) : 0.f; };
-      float next = sp != nullptr && !by_feature ? factor(0) : 0.f;
+      float next = sp != nullptr && !by_feature ? factor(first) : 0.f;
       mbar_wait(&tfull_bar[as], aphase, 73);
       tcgen05_fence_after();
 #pragma unroll 1
-      for (int cg0 = 0; cg0 < NG; cg0 += 4) {
+      for (int cg0 = first; cg0 < NG; cg0 += 8) {
         const int m = m0 + cg0 * 8, rows = a.M - m;      // valid token rows of this chunk (may be <= 0 or >= 32)
         float sc[32];
         if (by_feature) {
@@ -1663,19 +1720,28 @@ gemm_heads_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_const
           for (int j = 0; j < 32; ++j) sc[j] = j < rows ? __ldg(sp + (int64_t)(cg0 * 8 + j) * a.lds) : 0.f;
         } else if (sp != nullptr) {
           const float mine = next;
-          if (cg0 + 4 < NG) next = factor(cg0 + 4);
+          if (cg0 + 8 < NG) next = factor(cg0 + 8);
 #pragma unroll
           for (int j = 0; j < 32; ++j) sc[j] = __shfl_sync(0xffffffffu, mine, j);
         }
         uint32_t q[32];
         tmem_ld_32x32b_x32(t_addr + cg0 * 8, q);
         tmem_ld_wait();
-        if (cg0 + 4 >= NG) {   // accumulator fully read: hand the buffer back before the stores
+        if (cg0 + 8 >= NG) {   // this warp's part fully read: hand the buffer back before the stores
           tcgen05_fence_before();
           __syncwarp();
           if (lane == 0) mbar_arrive(&tempty_bar[as]);
         }
-        if (n < a.N) {
+        if (a.wide && rows >= 32 && tn * BM + quarter * 32 + 32 <= a.N) {
+          T* o = reinterpret_cast<T*>(a.out) + (int64_t)m * a.ldo + h * a.soh + n - (lane & 3);
+#pragma unroll
+          for (int j = 0; j < 32; j += 4, o += 4 * a.ldo) {
+            float y[4];
+#pragma unroll
+            for (int i = 0; i < 4; ++i) y[i] = __uint_as_float(q[j + i]) * (sp != nullptr ? sc[j + i] : 1.f);
+            store_4_tokens<T>(o, a.ldo, y[0], y[1], y[2], y[3], lane);
+          }
+        } else if (n < a.N) {
           float v[32];
 #pragma unroll
           for (int j = 0; j < 32; ++j) v[j] = __uint_as_float(q[j]) * (sp != nullptr ? sc[j] : 1.f);
@@ -1842,7 +1908,7 @@ int launch_pair(const CUtensorMap& tw, const CUtensorMap& tx, const GemmArgs& a,
   cudaLaunchConfig_t cfg;
   memset(&cfg, 0, sizeof(cfg));
   cfg.gridDim = dim3(clusters * 2 * split);
-  cfg.blockDim = dim3(kNumThreads);
+  cfg.blockDim = dim3(PCfg2::THREADS);
   cfg.dynamicSmemBytes = smem;
   cfg.stream = stream;
   cudaLaunchAttribute attr[2];
@@ -1892,6 +1958,7 @@ float pair_cost(int M, int N, int K, int kb_total, int sms, int bn, int S) {
   const float all = (main_loop > mem ? main_loop : mem) + (S > 1 ? 4.8f + 0.038f * bn : 3.5f + 0.025f * bn);
   return bn == PCfg2::BN ? 0.96f * all : all;        // (fewest loads: faster than this where the whole chip is at its power limit)
 }
+int wide_rows(const void* out, int64_t ldo) { return ((uintptr_t)out & 7) == 0 && ldo % 4 == 0; }
 // Accumulators that a tile may have.  A tensor core's sum over K is cut off at 24 bits after every 16 products, so that a 32-bit result of one chain over K = 2048
 // lies 2e-6 of its norm from 64 bits and one summed from eight stretches 5e-7.  A launch that gives every pair one tile has all of tensor memory for it,
 // others half.
@@ -2198,6 +2265,7 @@ LLMSS_API int llmss_gemm_ex(const void* x, int64_t ldx, const void* w, int64_t l
       a.tiles_n = (N + BM - 1) / BM;
       a.bn = pp.bn;
       a.nacc = pp.nacc;
+      a.wide = wide_rows(out, ldo);
       a.tiles_m = (M + pp.bn - 1) / pp.bn;
       a.kb_total = p.kb_total;
       a.dtype = dtype;
@@ -2321,6 +2389,7 @@ LLMSS_API int llmss_gemm_grouped_tiles(const void* x, int64_t ldx, const void* w
   a.groups = groups; a.n_groups = E;
   a.bn = tile_rows;
   a.nacc = 1;
+  a.wide = wide_rows(out, ldo);
   // as many persistent pairs as the machine holds; never more than there can be tiles
   const int64_t most = (int64_t)((a.tiles_n + 1) / 2) * ((int64_t)P / tile_rows + (P < E ? P : E));
   int clusters = num_sms() / 2;
@@ -2382,17 +2451,17 @@ LLMSS_API int llmss_gemm_heads(const void* x, int64_t ldx, int64_t sxh, const vo
   CUtensorMap tw, tx;
   if (int e = make_tmap_3d(&tw, w, dtype, K, N, H, ldw, swh, BM)) return e;
   if (int e = make_tmap_3d(&tx, x, dtype, K, M, H, ldx, sxh, 256)) return e;
-  HeadArgs a{M, N, H, (N + BM - 1) / BM, (M + 255) / 256, (K + BK - 1) / BK, dtype, scale, lds, ssh, ssn, out, ldo, soh, out_f32};
+  HeadArgs a{M, N, H, (N + BM - 1) / BM, (M + 255) / 256, (K + BK - 1) / BK, dtype, scale, lds, ssh, ssn, out, ldo, soh, out_f32, !out_f32 && wide_rows(out, ldo) && soh % 4 == 0};
   const int64_t tiles = (int64_t)a.tiles_n * a.tiles_m * H;
   LLMSS_REQUIRE(tiles < (1ll << 30), "gemm_heads: too many tiles");
   const int grid = (int)(tiles < num_sms() ? tiles : num_sms());
   static PerDeviceSmem g16, gbf;
   if (dtype == LLMSS_F16) {
     LLMSS_CHECK_CUDA(g16.ensure(gemm_heads_kernel<__half>, Cfg<256>::SMEM_BYTES));
-    LLMSS_CHECK_CUDA(launch_pdl(gemm_heads_kernel<__half>, dim3(grid), dim3(kNumThreads), (size_t)Cfg<256>::SMEM_BYTES, stream, tw, tx, a));
+    LLMSS_CHECK_CUDA(launch_pdl(gemm_heads_kernel<__half>, dim3(grid), dim3(PCfg2::THREADS), (size_t)Cfg<256>::SMEM_BYTES, stream, tw, tx, a));
   } else {
     LLMSS_CHECK_CUDA(gbf.ensure(gemm_heads_kernel<__nv_bfloat16>, Cfg<256>::SMEM_BYTES));
-    LLMSS_CHECK_CUDA(launch_pdl(gemm_heads_kernel<__nv_bfloat16>, dim3(grid), dim3(kNumThreads), (size_t)Cfg<256>::SMEM_BYTES, stream, tw, tx, a));
+    LLMSS_CHECK_CUDA(launch_pdl(gemm_heads_kernel<__nv_bfloat16>, dim3(grid), dim3(PCfg2::THREADS), (size_t)Cfg<256>::SMEM_BYTES, stream, tw, tx, a));
   }
   return 0;
 }

@@ -164,6 +164,32 @@ def test_gemm_pair_token_tiles(tile, split):
         lib.llmss_gemm_set_pair(-1)
 
 
+@pytest.mark.parametrize("off,pad", [(0, 0), (4, 4), (2, 0), (1, 3), (0, 2), (8, 8)])
+@pytest.mark.parametrize("dtype", DT)
+def test_gemm_results_into_columns(dtype, off, pad):
+    """Results stored by 8 bytes, or by one number where rows or base are off the 8-byte lines: the same bits, and nothing beside them is touched."""
+    from llmss_b200.ops import _lib
+
+    cu = _cu()
+    lib = _lib.load()
+    M, N, K = 70, 288, 256
+    torch.manual_seed(off + pad)
+    x = torch.randn(M, K, device="cuda", dtype=dtype)
+    w = (torch.randn(N, K, device="cuda") * K ** -0.5).to(dtype)
+    b = torch.randn(N, device="cuda", dtype=dtype)
+    try:
+        for mode in (1, 2):
+            lib.llmss_gemm_set_pair(mode | 96 << 8)
+            for kw in (dict(), dict(act=R.ACT_GELU_TANH, act_start=128)):
+                want = cu.linear(x, w, b, out_dtype=torch.float32, **kw).to(dtype)
+                whole = torch.full((M, off + N + pad), 7.0, device="cuda", dtype=dtype)
+                cu.linear(x, w, b, out=whole[:, off:off + N], **kw)
+                assert torch.equal(whole[:, off:off + N], want)
+                assert bool((whole[:, :off] == 7).all()) and bool((whole[:, off + N:] == 7).all())
+    finally:
+        lib.llmss_gemm_set_pair(-1)
+
+
 @pytest.mark.parametrize("M,N,K", [(33, 6144, 2048), (65, 512, 4096), (100, 2048, 2048), (161, 2048, 2048), (300, 1000, 1032), (140, 16, 2048), (2401, 16, 320)])
 def test_gemm_32_bit_results_of_short_stretches(M, N, K):
     """32-bit results that the library sums from several accumulators: no further from 64 bits than those of the single-CTA kernels, whose split over K they
