@@ -23,18 +23,24 @@ constexpr int kMaxGroupTop = 4;  // a group scores as the sum of at most this ma
 // weights are the chosen experts' s.  A group scores as the sum of its `group_top` largest c (1: its best expert).
 // renorm: weights / (their sum + 1e-20).  Experts outside the kept groups are never chosen, whatever the sign of c.
 // PL experts per lane: 32 * PL >= E
+struct RouteArgs {
+  int E, top, groups, keep;
+  float route_scale;
+  int score_kind;
+  const float* correction;
+  int group_top, renorm;
+  int* ids; float* wts; float* dense;
+};
+// one warp routes token t from its logits zr; cs: 32 * PL numbers of shared memory for the warp
 template <int PL>
-__global__ void __launch_bounds__(128) moe_route_kernel(const float* __restrict__ z, int64_t ldz, int E, int top, int groups,
-                                                        int keep, float route_scale, int score_kind,
-                                                        const float* __restrict__ correction, int group_top, int renorm,
-                                                        int* __restrict__ ids, float* __restrict__ wts,
-                                                        float* __restrict__ dense, int T) {
-  __shared__ float cs_all[4][32 * PL];
-  const int t = blockIdx.x * 4 + (threadIdx.x >> 5);
+__device__ __forceinline__ void route_token(const RouteArgs& a, const float* zr, int t, float* cs) {
   const int lane = threadIdx.x & 31;
-  if (t >= T) return;
-  float* cs = cs_all[threadIdx.x >> 5];
-  const float* zr = z + (int64_t)t * ldz;
+  const int E = a.E, top = a.top, groups = a.groups, keep = a.keep, score_kind = a.score_kind, group_top = a.group_top, renorm = a.renorm;
+  const float route_scale = a.route_scale;
+  const float* correction = a.correction;
+  int* ids = a.ids;
+  float* wts = a.wts;
+  float* dense = a.dense;
   float s[PL], c[PL];
   bool ok[PL];
   float mx = -INFINITY;
@@ -157,6 +163,75 @@ __global__ void __launch_bounds__(128) moe_route_kernel(const float* __restrict_
     __syncwarp();
     if (lane < top && mine) dense[(int64_t)t * E + myid] = myw * inv;
   }
+}
+template <int PL>
+__global__ void __launch_bounds__(128) moe_route_kernel(RouteArgs a, const float* __restrict__ z, int64_t ldz, int T) {
+  __shared__ float cs_all[4][32 * PL];
+  const int t = blockIdx.x * 4 + (threadIdx.x >> 5);
+  if (t < T) route_token<PL>(a, z + (int64_t)t * ldz, t, cs_all[threadIdx.x >> 5]);
+}
+
+// Logits and routing in one launch, for up to 32 experts: a block has 16 tokens, its 16 warps every 16th piece of 32 channels and then a token each.  A product of 16 columns has no
+// use for the tensor-memory tiles (128 features), and its result went through memory to a second launch; here the rows come straight into mma fragments.
+// The order of a sum over channels is free, so a thread's 16-byte pieces of a token's and an expert's row are two steps of k = 16 as they lie.  Two launches /
+// one, us: 8192 tokens of 2048, 16 experts 28.7 / 20.7; 2048 of 4096, 32 experts 18.2 / 11.3; 400 of 2048, 16 experts 13.6 / 7.2 (with eight warps 20.8, 15.9,
+// 11.2: a block is one chain of loads, sums and choices).  Up to 64 experts it lost (4096 of 4096: 54).
+template <typename T> __device__ __forceinline__ void mma_16816(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
+  if constexpr (std::is_same<T, __half>::value)
+    asm("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
+        : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3]) : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+  else
+    asm("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
+        : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3]) : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+}
+template <typename T, int NT>      // NT: tiles of 8 experts
+__global__ void __launch_bounds__(512) moe_router_kernel(RouteArgs a, const T* __restrict__ h, int64_t ldh, const T* __restrict__ w, int64_t ldw,
+                                                         const T* __restrict__ bias, int K, int T_) {
+  constexpr int WARPS = 16, EP = NT * 8;
+  __shared__ float part[WARPS][16][EP + 2];
+  __shared__ float z[16][EP];
+  __shared__ float cs[WARPS][32];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = lane >> 2, l = lane & 3;
+  const int t0 = blockIdx.x * 16;
+  const T* r0 = h + (int64_t)min(t0 + g, T_ - 1) * ldh;
+  const T* r1 = h + (int64_t)min(t0 + g + 8, T_ - 1) * ldh;
+  const uint4 zero = make_uint4(0u, 0u, 0u, 0u);
+  float c[NT][4];
+#pragma unroll
+  for (int n = 0; n < NT; ++n) c[n][0] = c[n][1] = c[n][2] = c[n][3] = 0.f;
+#pragma unroll 4
+  for (int k0 = warp * 32; k0 < K; k0 += WARPS * 32) {
+    const int k = k0 + l * 8;
+    const bool in = k < K;             // (K is a multiple of 8)
+    const int kk = in ? k : 0;
+    uint4 x0 = *reinterpret_cast<const uint4*>(r0 + kk), x1 = *reinterpret_cast<const uint4*>(r1 + kk), y[NT];
+#pragma unroll
+    for (int n = 0; n < NT; ++n) y[n] = *reinterpret_cast<const uint4*>(w + (int64_t)min(n * 8 + g, a.E - 1) * ldw + kk);
+    if (!in) {                         // (both operands: zeros times what may be no number)
+      x0 = x1 = zero;
+#pragma unroll
+      for (int n = 0; n < NT; ++n) y[n] = zero;
+    }
+#pragma unroll
+    for (int n = 0; n < NT; ++n) {
+      mma_16816<T>(c[n], x0.x, x1.x, x0.y, x1.y, y[n].x, y[n].y);
+      mma_16816<T>(c[n], x0.z, x1.z, x0.w, x1.w, y[n].z, y[n].w);
+    }
+  }
+#pragma unroll
+  for (int n = 0; n < NT; ++n)
+#pragma unroll
+    for (int e = 0; e < 4; ++e) part[warp][g + (e >> 1) * 8][n * 8 + 2 * l + (e & 1)] = c[n][e];
+  __syncthreads();
+  for (int i = threadIdx.x; i < 16 * EP; i += WARPS * 32) {
+    const int t = i / EP, e = i % EP;
+    float s = 0.f;
+#pragma unroll
+    for (int x = 0; x < WARPS; ++x) s += part[x][t][e];
+    z[t][e] = s + (bias != nullptr && e < a.E ? to_f32(bias[e]) : 0.f);
+  }
+  __syncthreads();
+  if (t0 + warp < T_) route_token<1>(a, z[warp], t0 + warp, cs[warp]);
 }
 
 // grid (T, top, ceil(F / 8)); 8 warps, one output feature each
@@ -455,14 +530,38 @@ LLMSS_API int llmss_moe_route_ex(const float* z, int64_t ldz, int T_, int E, int
   LLMSS_REQUIRE(score_kind == 0 || score_kind == 1, "moe_route: score kind %d (0 softmax, 1 sigmoid)", score_kind);
   LLMSS_REQUIRE(group_top >= 1 && group_top <= kMaxGroupTop, "moe_route: a group sums its %d best (1..%d)", group_top, kMaxGroupTop);
   if (T_ == 0) return 0;
+  const RouteArgs a{E, top, groups, keep, route_scale, score_kind, correction, group_top, renorm, ids, wts, dense};
 #define LLMSS_ROUTE(PL) \
-  moe_route_kernel<PL><<<(T_ + 3) / 4, 128, 0, stream>>>(z, ldz, E, top, groups, keep, route_scale, score_kind, correction, group_top, renorm, \
-                                                         ids, wts, dense, T_)
+  moe_route_kernel<PL><<<(T_ + 3) / 4, 128, 0, stream>>>(a, z, ldz, T_)
   if (E <= 32) LLMSS_ROUTE(1);
   else if (E <= 64) LLMSS_ROUTE(2);
   else if (E <= 128) LLMSS_ROUTE(4);
   else LLMSS_ROUTE(kMaxPerLane);
 #undef LLMSS_ROUTE
+  LLMSS_CHECK_CUDA(cudaGetLastError());
+  return 0;
+}
+
+// Router logits (h [T, K] times w [E, K]^T, plus bias) and routing in one launch: 16-bit operands on 16-byte lines, K, ldh and ldw multiples of 8, E <= 32
+LLMSS_API int llmss_moe_router(const void* h, int64_t ldh, const void* w, int64_t ldw, const void* bias, int K, int T_, int E, int top, int groups,
+                               int keep, float route_scale, int score_kind, const float* correction, int group_top, int renorm, int* ids, float* wts,
+                               float* dense, int dtype, cudaStream_t stream) {
+  LLMSS_REQUIRE(E > 0 && E <= 32 && K > 0 && K % 8 == 0 && ldh % 8 == 0 && ldw % 8 == 0 && (((uintptr_t)h | (uintptr_t)w) & 15) == 0,
+                "moe_router: %d experts (at most 32), width %d (a multiple of 8, rows on 16-byte lines)", E, K);
+  LLMSS_REQUIRE(dtype == LLMSS_F16 || dtype == LLMSS_BF16, "moe_router: dtype must be f16/bf16");
+  LLMSS_REQUIRE(top > 0 && top <= 32 && top <= E, "moe_router: top=%d must be in 1..min(32, experts)", top);
+  LLMSS_REQUIRE(groups > 0 && E % groups == 0 && keep > 0 && keep <= groups, "moe_router: bad groups %d / keep %d for %d experts", groups, keep, E);
+  LLMSS_REQUIRE((score_kind == 0 || score_kind == 1) && group_top >= 1 && group_top <= kMaxGroupTop, "moe_router: score kind %d, group top %d", score_kind, group_top);
+  if (T_ <= 0) return 0;
+  const RouteArgs a{E, top, groups, keep, route_scale, score_kind, correction, group_top, renorm, ids, wts, dense};
+#define LLMSS_ROUTER(T, NT) moe_router_kernel<T, NT><<<(T_ + 15) / 16, 512, 0, stream>>>(a, (const T*)h, ldh, (const T*)w, ldw, (const T*)bias, K, T_)
+#define LLMSS_ROUTER_E(T)                  \
+  if (E <= 16) LLMSS_ROUTER(T, 2);         \
+  else LLMSS_ROUTER(T, 4)
+  if (dtype == LLMSS_F16) { LLMSS_ROUTER_E(__half); }
+  else { LLMSS_ROUTER_E(__nv_bfloat16); }
+#undef LLMSS_ROUTER_E
+#undef LLMSS_ROUTER
   LLMSS_CHECK_CUDA(cudaGetLastError());
   return 0;
 }

@@ -222,6 +222,10 @@ int llmss_moe_count(const int* ids, int P, int E, int* counts, llmss_stream_t st
 int llmss_moe_permute(const int* ids, int P, int E, const int* offsets, int* perm, int* inv, llmss_stream_t stream);
 int llmss_moe_gather_rows(const void* h, int64_t ldh, const int* perm, int top, void* xs, int P, int W, int dtype,
                           llmss_stream_t stream);
+/* router logits (h [T, K] w [E, K]^T + bias, 16-bit, E <= 32) and llmss_moe_route_ex of them in one launch */
+int llmss_moe_router(const void* h, int64_t ldh, const void* w, int64_t ldw, const void* bias, int K, int T, int E, int top, int groups, int keep,
+                     float route_scale, int score_kind, const float* correction, int group_top, int renorm, int* ids, float* wts, float* dense,
+                     int dtype, llmss_stream_t stream);
 /* the same sorting without the host: inv[pair] = row in the order by expert, table [2 * (E + 1)] = first row of every expert (and P),
  * first tile of 256 rows of every expert (and their number); hist: ceil(P / 1024) * E numbers of scratch */
 int llmss_moe_group(const int* ids, int P, int E, int* hist, int* table, int* inv, llmss_stream_t stream);

@@ -14,6 +14,7 @@ import torch
 
 from .. import ops
 from ..ops import ACT_RELU2
+from ..ops.cuda_impl import moe_router_fused as _router_fused
 from ..utils.tracing import trace
 
 
@@ -265,22 +266,31 @@ class RoutedExperts:
     def _logits(self, y):
         return y[:, self.z_off:self.z_off + self.experts]
 
-    def weigh(self, a, y):
+    def _route(self, y, h=None, dense: bool = False):
+        """(ids, weights[, dense weights]) from the logits in ``y``; ``y`` None: from the rows ``h`` themselves, in one launch."""
+        from ..ops import cuda_impl as cu
+
+        sizes = self.experts, self.top, self.groups, self.keep, self.route_scale
+        with trace("experts_route"):
+            if y is None:
+                return cu.moe_router(h, self.w_router, self.b_router, *sizes, dense=dense, **self._route_kw())
+            if dense:
+                return cu.moe_route(self._logits(y), *sizes, dense=True, **self._route_kw())
+            return ops.moe_route(self._logits(y), *sizes, **self._route_kw())
+
+    def weigh(self, a, y, h=None):
         """Dense form: scale every expert's block of the hidden rows ``a`` [T, E * F] by its routing weight (0 if not chosen)."""
         from ..ops import cuda_impl as cu
 
-        with trace("experts_route"):
-            _, _, dense = cu.moe_route(self._logits(y), self.experts, self.top, self.groups, self.keep, self.route_scale, dense=True,
-                                       **self._route_kw())
+        _, _, dense = self._route(y, h, dense=True)
         with trace("experts_weigh"):
             cu.moe_scale(a, dense, self.experts, self.ff)
 
     def forward(self, h, y=None, base=None, form=None):
-        """``y``: a fused projection that holds the router logits at ``z_off`` (32-bit, bias included); without it the router runs as
-        a GEMM of its own (32-bit accumulation and output).  ``base`` [T, W] 32-bit: the result is added to it in place (gather and
-        grouped form)."""
-        E = self.experts
-        if y is None:
+        """``y``: a fused projection that holds the router logits at ``z_off`` (32-bit, bias included); without it the router runs with
+        the routing in one launch, or as a GEMM of its own (32-bit accumulation and output).  ``base`` [T, W] 32-bit: the result is added to it in
+        place (gather and grouped form)."""
+        if y is None and not (h.is_cuda and _router_fused(h, self.w_router, self.b_router, self.experts)):
             with trace("experts_router"):
                 y = ops.linear(h, self.w_router, self.b_router, out_dtype=torch.float32)
         form = form or self.form(h)
@@ -288,11 +298,10 @@ class RoutedExperts:
             assert base is None
             with trace("experts_dense_up"):
                 a = ops.linear(h, self.w_up.view(self.w_up.shape[0] * self.w_up.shape[1], -1), act=self.act, gated=self.gated)
-            self.weigh(a, y)
+            self.weigh(a, y, h)
             with trace("experts_dense_down"):
                 return ops.linear(a, self.w_down, out_dtype=torch.float32)
-        with trace("experts_route"):
-            ids, wts = ops.moe_route(self._logits(y), E, self.top, self.groups, self.keep, self.route_scale, **self._route_kw())
+        ids, wts = self._route(y, h)
         if form == "grouped":
             from ..ops import cuda_impl as cu
 

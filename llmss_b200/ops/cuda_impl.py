@@ -597,6 +597,30 @@ def moe_route(z, experts, top, groups, keep, route_scale, dense: bool = False, s
     return (ids, wts, dn) if dense else (ids, wts)
 
 
+def moe_router_fused(h, w, bias, experts: int) -> bool:
+    """Whether moe_router() takes these operands (csrc/moe.cu: logits and routing in one launch)."""
+    return (h.dtype in (torch.float16, torch.bfloat16) and w.dtype == h.dtype and experts <= 32 and h.dim() == 2 and h.stride(1) == 1 and w.stride(1) == 1
+            and not (h.shape[1] % 8 or h.stride(0) % 8 or w.stride(0) % 8 or h.data_ptr() % 16 or w.data_ptr() % 16)
+            and (bias is None or (bias.dtype == h.dtype and bias.is_contiguous())))
+
+
+def moe_router(h, w, bias, experts, top, groups, keep, route_scale, dense: bool = False, score: str = "softmax", correction=None,
+               group_top: int = 1, renorm: bool = True):
+    """moe_route() of the logits h w^T + bias."""
+    T, K, ldh = _rows2d(h)
+    assert w.shape == (experts, K) and score in ("softmax", "sigmoid")
+    assert correction is None or (correction.dtype == torch.float32 and correction.numel() == experts)
+    ids = torch.empty(T, top, dtype=torch.int32, device=h.device)
+    wts = torch.empty(T, top, dtype=torch.float32, device=h.device)
+    dn = torch.empty(T, experts, dtype=torch.float32, device=h.device) if dense else None
+    rc = _lib.load().llmss_moe_router(_ptr(h), ldh, _ptr(w), w.stride(0), _ptr(bias), K, T, experts, top, groups, keep, float(route_scale),
+                                      0 if score == "softmax" else 1, _ptr(correction), int(group_top), 1 if renorm else 0, _ptr(ids), _ptr(wts),
+                                      _ptr(dn), _DT[h.dtype], _stream())
+    _lib.check(rc, "llmss_moe_router")
+    _count()
+    return (ids, wts, dn) if dense else (ids, wts)
+
+
 def moe_experts(h, ids, wts, w_up, w_down, act, gated: bool = False, base=None):
     lib = _lib.load()
     T, W, ldh = _rows2d(h)

@@ -392,6 +392,33 @@ def test_experts_sorted_on_the_device(T, W, E, top, F, gated, skew):
     assert _rel(got.double() - base.double(), want.cpu()) < 1e-2
 
 
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("T,E,K,top,groups,keep,score,extra", [(1, 8, 8, 2, 1, 1, "softmax", False), (15, 16, 264, 4, 4, 2, "softmax", True), (17, 6, 40, 3, 3, 2, "sigmoid", True),
+                                                               (33, 32, 2048, 4, 8, 4, "sigmoid", True), (100, 20, 520, 5, 1, 1, "softmax", False), (16, 32, 4096, 8, 8, 3, "softmax", True)])
+def test_router_in_one_launch(T, E, K, top, groups, keep, score, extra, dtype):
+    """Logits and routing together against the oracle's routing of 64-bit logits: tokens and experts short of a tile, widths short of a step.  Weights: 32-bit
+    sums of K products of 16-bit numbers, 1e-5; a choice may differ only where two scores lie closer than that."""
+    from llmss_b200.ops import cuda_impl as cu, reference as R
+
+    torch.manual_seed(T + E)
+    wide = torch.randn(T, K + 8, device="cuda").to(dtype)
+    h = wide[:, 8:]
+    w = (2 * torch.randn(E, K, device="cuda") * K ** -0.5).to(dtype)
+    bias = torch.randn(E, device="cuda").to(dtype) if extra else None
+    corr = 0.1 * torch.randn(E, device="cuda") if score == "sigmoid" else None
+    z = h.double() @ w.double().t() + (bias.double() if extra else 0.0)
+    kw = dict(score=score, correction=corr, group_top=min(2, E // groups) if score == "sigmoid" else 1)
+    assert cu.moe_router_fused(h, w, bias, E)
+    ids, wts, dense = cu.moe_router(h, w, bias, E, top, groups, keep, 1.5, dense=True, **kw)
+    want_ids, want = R.moe_route(z.float().cpu(), E, top, groups, keep, 1.5, score, None if corr is None else corr.cpu(), kw["group_top"])
+    got_ids, got = ids.cpu(), wts.cpu()
+    full = torch.zeros(T, E).scatter_(1, got_ids.long(), got)
+    assert torch.equal(full, dense.cpu())
+    same = (got_ids == want_ids).all(1)
+    assert same.float().mean() > 0.98
+    assert ((got - want).abs()[same] <= 1e-5 * want.abs()[same] + 1e-6).all()
+
+
 @pytest.mark.parametrize("tile_rows", [32, 96, 224])
 @pytest.mark.parametrize("T,top,E,W,F,gated", [(5, 2, 8, 256, 192, False), (95, 3, 6, 136, 72, True), (700, 4, 16, 512, 256, False)])
 def test_grouped_tile_rows(T, top, E, W, F, gated, tile_rows):
