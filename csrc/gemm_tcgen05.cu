@@ -1988,7 +1988,7 @@ PairPlan best_pair(int M, int N, int K, int kb_total, int sms, int parts, float*
 // loads too much: 128 tokens 6144 x 2048 21.2 / 10.7, 700 tokens 512 x 4096 46.6 / 12.0.
 PairPlan pick_pair(int M, int N, int K, int kb_total, int sms, int parts) {
   const int mode = pair_mode() & 255, forced_bn = pair_mode() >> 8;
-  if (mode == 0) return {0, 0, 1};
+  if (mode == 0 || sms < 2) return {0, 0, 1};
   if (mode == 1 || mode == 2 || mode == 4) {
     if (M <= 128 && forced_bn == 0) return {0, 0, 1};
     return {mode <= kb_total ? mode : 1, forced_bn ? forced_bn : 256, 1};
@@ -2087,6 +2087,7 @@ int pick_bn(int M) {
 // stamps (entry, prologue done, last TMA issued, first stage landed, last MMA issued, first
 // accumulator ready, epilogue done, exit) to buf[cta*8 .. cta*8+7].  buf must be zeroed by the caller.
 LLMSS_API int llmss_gemm_set_pair(int mode) {          // mode | token tile << 8 also pins the width of the token tile
+  LLMSS_REQUIRE(mode < 256 || ((mode >> 8) % 32 == 0 && (mode >> 8) <= PCfg2::BN), "gemm_set_pair: token tiles of %d columns (32, 64 .. 256)", mode >> 8);
   g_pair_mode = mode;
   return 0;
 }
