@@ -84,29 +84,41 @@ def _calls_current() -> bool:
 
 
 def _build_calls():
-    """The entries as plain functions (calls.py); every call works without them."""
+    """The entries as plain functions (calls.py).  Every call works without them, so that nothing here stops the library."""
     from . import _lib, calls
 
-    OBJ_DIR.mkdir(parents=True, exist_ok=True)
-    if not calls.build(LIB_DIR, OBJ_DIR, {**_lib._SIGS, **_lib._OPTIONAL}):
-        print("[build] no C compiler or Python headers: library calls go through ctypes", file=sys.stderr)
+    try:
+        OBJ_DIR.mkdir(parents=True, exist_ok=True)
+        if not calls.build(LIB_DIR, OBJ_DIR, {**_lib._SIGS, **_lib._OPTIONAL}):
+            print("[build] no C compiler or Python headers: library calls go through ctypes", file=sys.stderr)
+    except (OSError, RuntimeError) as e:
+        print(f"[build] library calls go through ctypes: {e}", file=sys.stderr)
 
 
 def build_library(verbose: bool = False, force: bool = False) -> Path:
-    if not force and is_current() and _calls_current():  # e.g. on the GPU box: the .so files travelled with the tree
+    from . import calls
+
+    # e.g. on the GPU box: the .so files travelled with the tree.  A library that is current needs no lock where the calls' module cannot be built
+    current = not force and is_current()
+    if current and (_calls_current() or calls.compiler() is None):
         return LIB_PATH
-    LIB_DIR.mkdir(parents=True, exist_ok=True)
     # one builder at a time (torchrun starts N ranks at once); the others wait, then see a current library
     import fcntl
 
-    with open(LIB_DIR / ".build.lock", "w") as lock:
+    try:
+        LIB_DIR.mkdir(parents=True, exist_ok=True)
+        lock = open(LIB_DIR / ".build.lock", "w")
+    except OSError:
+        if current:          # a read-only installation: calls go through ctypes
+            return LIB_PATH
+        raise
+    with lock:
         fcntl.flock(lock, fcntl.LOCK_EX)
         try:
+            path = LIB_PATH if not force and is_current() else _build_locked(verbose, force)
             if not _calls_current():
                 _build_calls()
-            if not force and is_current():
-                return LIB_PATH
-            return _build_locked(verbose, force)
+            return path
         finally:
             fcntl.flock(lock, fcntl.LOCK_UN)
 

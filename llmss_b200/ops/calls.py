@@ -2,7 +2,7 @@
 
 A ctypes call converts every argument through an object of its own: 3.2 us for the 24 arguments of a linear layer, of which a decode step issues hundreds;
 through the module it is 0.4 us.  What the module does not take (a ctypes object, a wrong number or kind of arguments) it hands to the ctypes function, which
-behaves and raises as before; without a compiler or Python's headers every call goes there.
+behaves and raises as before; without the module (no compiler, no Python headers, a folder that takes no files) every call goes there.
 """
 from __future__ import annotations
 
@@ -13,6 +13,7 @@ import importlib.util
 import os
 import shutil
 import subprocess
+import sys
 import sysconfig
 from pathlib import Path
 
@@ -110,29 +111,35 @@ PyMODINIT_FUNC PyInit_NAME(void) { return PyModule_Create(&module); }
     return "\n".join(out)
 
 
-def digest(sigs: dict) -> str:
-    return hashlib.sha256((source(sigs) + sysconfig.get_config_var("SOABI")).encode()).hexdigest()[:16]
+def _abi() -> str:
+    return sysconfig.get_config_var("SOABI") or "abi"
 
 
 def module_path(lib_dir: Path, sigs: dict) -> Path:
-    """The file carries its sources' digest: one written from other signatures is never loaded."""
-    return Path(lib_dir) / f"{NAME}.{digest(sigs)}.so"
+    """The file carries its source's digest and Python's ABI: one written from other signatures, or for another Python, is never loaded."""
+    return Path(lib_dir) / f"{NAME}.{hashlib.sha256(source(sigs).encode()).hexdigest()[:16]}.{_abi()}.so"
+
+
+def compiler():
+    """(C compiler, folder of Python.h), or None where the module cannot be built."""
+    cc, include = shutil.which("gcc") or shutil.which("cc"), sysconfig.get_paths()["include"]
+    return (cc, include) if cc is not None and (Path(include) / "Python.h").exists() else None
 
 
 def build(lib_dir: Path, obj_dir: Path, sigs: dict) -> bool:
-    """Compile the module if it is not there; False where that is not possible."""
+    """Compile the module if it is not there; False without a compiler or Python's headers."""
     path = module_path(lib_dir, sigs)
     if path.exists():
         return True
-    cc, include = shutil.which("gcc") or shutil.which("cc"), sysconfig.get_paths()["include"]
-    if cc is None or not (Path(include) / "Python.h").exists():
+    tools = compiler()
+    if tools is None:
         return False
     text, tmp = Path(obj_dir) / f"{NAME}.c", path.with_suffix(f".tmp{os.getpid()}")
     text.write_text(source(sigs))
-    r = subprocess.run([cc, "-O2", "-shared", "-fPIC", "-I", include, str(text), "-o", str(tmp)], capture_output=True, text=True)
+    r = subprocess.run([tools[0], "-O2", "-shared", "-fPIC", "-I", tools[1], str(text), "-o", str(tmp)], capture_output=True, text=True)
     if r.returncode != 0:
-        return False
-    for old in Path(lib_dir).glob(f"{NAME}.*.so"):
+        raise RuntimeError(f"{tools[0]} failed for {text}:\n{r.stderr}")
+    for old in Path(lib_dir).glob(f"{NAME}.*.{_abi()}.so"):       # (another Python's stay)
         old.unlink()
     os.replace(tmp, path)
     return True
@@ -147,7 +154,8 @@ def attach(lib, lib_dir: Path, sigs: dict) -> int:
         spec = importlib.util.spec_from_loader(NAME, importlib.machinery.ExtensionFileLoader(NAME, str(path)))
         mod = importlib.util.module_from_spec(spec)
         spec.loader.exec_module(mod)
-    except ImportError:
+    except ImportError as e:
+        print(f"[llmss_b200] library calls go through ctypes: {e}", file=sys.stderr)
         return 0
     names = wrappable(sigs)
     for k, name in enumerate(names):
