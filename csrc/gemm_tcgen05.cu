@@ -1963,11 +1963,11 @@ int wide_rows(const void* out, int64_t ldo) { return ((uintptr_t)out & 7) == 0 &
 // lies 2e-6 of its norm from 64 bits and one summed from eight stretches 5e-7.  A launch that gives every pair one tile has all of tensor memory for it,
 // others half.
 int pair_accumulators(int tiles, int bn, int sms) { return (tiles <= sms / 2 ? 512 : 256) / bn; }
-// the cheapest of all (S, bn) whose S times accumulators are at least `parts`; at most 128 features run only as two pairs per tile with narrow tiles (see pick_pair)
+// The cheapest of all (S, bn) whose S times accumulators are at least `parts`, and its cost; split 0 and no cost where none fits.  At most 128 features run
+// only as two pairs per tile with narrow tiles (see pick_pair).
 PairPlan best_pair(int M, int N, int K, int kb_total, int sms, int parts, float* cost) {
   const int pair_tiles_n = (N + 2 * BM - 1) / (2 * BM);
   PairPlan best{0, 0, 1};
-  *cost = 0.f;
   for (int bn = 32; bn <= PCfg2::BN && bn < M + 32; bn += 32)
     for (int S = 1; S <= 2; ++S) {
       if (S == 1 ? N <= BM : (kb_total < 4 || (int64_t)pair_tiles_n * ((M + bn - 1) / bn) * 4 > sms || (N <= BM && bn > 96))) continue;
@@ -2417,9 +2417,16 @@ LLMSS_API int llmss_moe_forms(int T, int top, int E, int W, int F, int rows, flo
   for (int i = 0; i < 2; ++i) {
     const int64_t N = i ? W : (int64_t)E * rows, K = i ? (int64_t)E * F : W;
     LLMSS_REQUIRE(N < (1ll << 31) && K < (1ll << 31), "moe_forms: sizes too large");
-    float best;
-    best_pair(T, (int)N, (int)K, (int)((K + BK - 1) / BK), sms, 1, &best);
-    dense += best;
+    const int kb = (int)((K + BK - 1) / BK);
+    float us;
+    if (best_pair(T, (int)N, (int)K, kb, sms, 1, &us).split == 0) {
+      // at most 128 columns in the single-CTA kernels, few CTAs each of which has the whole of its rows to load; stream-K also exchanges partial tiles.  Within
+      // a fifth of 128 x 1024, 4096 and 16384 at 2000 .. 16384 tokens (the longest 116 us, stream-K 40 .. 67)
+      llmss_gemm_plan p;
+      gemm_plan_impl(T, (int)N, (int)K, 1, 2, 0, LLMSS_BF16, 0, &p);
+      us = 10.f + 2.f * ((float)N * K + (float)T * K) * (1.f / 5e6f) + (p.split == 0 ? 30.f : 0.f);
+    }
+    dense += us;
   }
   const float mean = (float)T * top / E, used = (float)(E < (int64_t)T * top ? E : T * top);
   for (int bn = 32; bn <= PCfg2::BN; bn += 32) {
