@@ -1924,15 +1924,25 @@ int launch_pair(const CUtensorMap& tw, const CUtensorMap& tx, const GemmArgs& a,
   return 0;
 }
 
-// CTA-pair kernel: -1 = environment (LLMSS_GEMM_PAIR: off | auto (default) | 1 | 2 | 4), 0 = off, 1 / 2 / 4 = pairs per
-// cluster (1 = persistent, 2 / 4 = split-K depth), 8 = auto.  llmss_gemm_set_pair() overrides the environment (A/B measurements inside one process).
+// LLMSS_GEMM_MODE: 1 = streamk, 2 = cluster, 0 = unset
+int forced_single_mode() {
+  static const int mode = [] {
+    const char* e = getenv("LLMSS_GEMM_MODE");
+    return e == nullptr ? 0 : strcmp(e, "streamk") == 0 ? 1 : strcmp(e, "cluster") == 0 ? 2 : 0;
+  }();
+  return mode;
+}
+
+// CTA-pair kernel: -1 = environment (LLMSS_GEMM_PAIR: off | auto | 1 | 2 | 4), 0 = off, 1 / 2 / 4 = pairs per
+// cluster (1 = persistent, 2 / 4 = split-K depth), 8 = auto.  Without it auto, but off where LLMSS_GEMM_MODE asks for one of the single-CTA kernels.
+// llmss_gemm_set_pair() overrides the environment (A/B measurements inside one process).
 int g_pair_mode = -1;
 int pair_mode() {
   if (g_pair_mode >= 0) return g_pair_mode;
   static int env_mode = -1;
   if (env_mode < 0) {
     const char* e = getenv("LLMSS_GEMM_PAIR");
-    env_mode = 8;  // default: automatic (pick_pair)
+    env_mode = forced_single_mode() != 0 ? 0 : 8;
     if (e != nullptr) env_mode = strcmp(e, "off") == 0 ? 0 : strcmp(e, "auto") == 0 ? 8 : atoi(e);
     if (env_mode != 0 && env_mode != 1 && env_mode != 2 && env_mode != 4 && env_mode != 8) env_mode = 8;
   }
@@ -2044,11 +2054,9 @@ int clusters_for(int dtype, int bn, int split) {
 }
 
 int pick_cluster_split(int tiles, int kb_total, int bn, int sms, int dtype) {
-  static int forced = -1;
+  const int forced = forced_single_mode();
   static int min_kb = -1;  // k-blocks (64 x 16-bit columns, 16 KB of weights) every CTA of a split must at least stream
-  if (forced < 0) {
-    const char* e = getenv("LLMSS_GEMM_MODE");
-    forced = (e == nullptr) ? 0 : (strcmp(e, "streamk") == 0 ? 1 : (strcmp(e, "cluster") == 0 ? 2 : 0));
+  if (min_kb < 0) {
     const char* m = getenv("LLMSS_GEMM_MIN_KB_PER_CTA");
     min_kb = (m != nullptr) ? atoi(m) : 2;
     if (min_kb < 1) min_kb = 1;

@@ -567,6 +567,33 @@ print('MODES_OK' if bad == 0 else 'MODES_FAILED')
     assert "MODES_OK" in r.stdout, r.stdout[-3000:] + r.stderr[-2000:]
 
 
+@pytest.mark.parametrize("mode", ["streamk", "cluster"])
+def test_gemm_mode_forces_its_kernel(mode):
+    """LLMSS_GEMM_MODE leaves the pair kernel out, also above 64 tokens: the 32-bit results have the bits of the single-CTA kernels and not those of the pair
+    kernel, which sums other stretches of K."""
+    import os
+    import subprocess
+    import sys
+
+    code = r"""
+import torch
+from llmss_b200.ops import _lib, cuda_impl as cu
+lib = _lib.load()
+torch.manual_seed(0)
+for (M, N, K) in [(128, 2048, 1024), (256, 4096, 4096), (300, 12288, 1024)]:
+    x = torch.randn(M, K, device='cuda', dtype=torch.bfloat16); w = torch.randn(N, K, device='cuda', dtype=torch.bfloat16)
+    y = {}
+    for pair in (-1, 0, 8):
+        lib.llmss_gemm_set_pair(pair)
+        y[pair] = cu.linear(x, w, out_dtype=torch.float32)
+    print('FORCED' if torch.equal(y[-1], y[0]) else 'OTHER', M, N, K, 'pair kernel differs' if not torch.equal(y[-1], y[8]) else 'as pair kernel')
+"""
+    env = dict(os.environ, LLMSS_GEMM_MODE=mode, PYTHONPATH=os.path.dirname(os.path.dirname(os.path.abspath(__file__))))
+    env.pop("LLMSS_GEMM_PAIR", None)
+    r = subprocess.run([sys.executable, "-c", code], capture_output=True, text=True, timeout=300, env=env)
+    assert r.stdout.count("FORCED") == 3 and r.stdout.count("pair kernel differs") >= 2, r.stdout[-3000:] + r.stderr[-2000:]
+
+
 # ------------------------------------------------------------------ prefill attention (tcgen05)
 @pytest.mark.parametrize("dtype", DT)
 @pytest.mark.parametrize("hq,hkv,d", [(4, 4, 256), (8, 8, 128), (6, 6, 64), (8, 2, 128), (6, 1, 128)])
