@@ -2254,13 +2254,17 @@ LLMSS_API int llmss_gemm_ex(const void* x, int64_t ldx, const void* w, int64_t l
   if (collective == 0) {
     // two CTAs share one MMA of 256 features, each loading half of the token tile
     // a 32-bit result is summed from more stretches of K than the single-CTA kernels would cut it into (above 128 tokens and 23 tiles of 256 x 256: two,
-    // and from 38 such tiles one), so that its error against 64 bits is no larger than theirs
+    // and from 38 such tiles one), so that its error against 64 bits is no larger than theirs.  An fp16 result from as many, as far as its stretches come to
+    // more than 4096 products: its rounding is 2.1e-4 of the norm, to which one chain over K = 20480 adds 0.16 %, over 4096 0.02 % (bf16: nothing that can be
+    // measured).  Times are the same within 1 us (4096 x 4096 .. 20480, 65 .. 900 tokens), while as many stretches as a 32-bit result takes cost
+    // 512 x 20480 43.8 -> 65 us.
     const int sms = max_ctas > 0 ? max_ctas : num_sms(), wide = ((N + 2 * BM - 1) / (2 * BM)) * ((M + 255) / 256);
     int parts = 1;
-    if (out_f32 && p.kb_total > 1) {
+    if ((out_f32 || dtype == LLMSS_F16) && p.kb_total > 1) {
       const int cut = p.split > 0 ? p.split : need_sk ? (p.grid + p.tiles - 1) / p.tiles : 1;
       parts = M > 128 && wide >= 38 ? 1 : M > 128 && wide >= 24 ? 2 : cut > 1 ? cut + 1 : need_sk ? 2 : 1;
-      if (parts > p.kb_total) parts = p.kb_total;
+      const int most = out_f32 ? p.kb_total : (p.kb_total + 63) / 64;
+      if (parts > most) parts = most;
     }
     const PairPlan pp = pick_pair(M, N, K, p.kb_total, sms, parts);
     const int ps = pp.split;

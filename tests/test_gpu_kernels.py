@@ -212,6 +212,28 @@ def test_gemm_32_bit_results_of_short_stretches(M, N, K):
     assert err[8] <= 1.1 * err[0], err
 
 
+@pytest.mark.parametrize("M,N,K", [(65, 4096, 20480), (200, 4096, 20480), (128, 512, 20480), (900, 512, 20480), (100, 4096, 16384)])
+def test_gemm_fp16_results_of_long_sums(M, N, K):
+    """fp16 results over a long K, which the single-CTA kernels sum from several stretches: no further from 64 bits than theirs, but for what a chain of 4096
+    products adds.  It is cut off at 24 bits once per 16 products, half a unit on average: 4096 / 16 x 2^-25 of the norm, beside the rounding of the result."""
+    from llmss_b200.ops import _lib
+
+    cu = _cu()
+    lib = _lib.load()
+    torch.manual_seed(M)
+    x = torch.randn(M, K, device="cuda", dtype=torch.float16)
+    w = (torch.randn(N, K, device="cuda") * K ** -0.5).to(torch.float16)
+    want = x.double() @ w.double().t()
+    err = {}
+    try:
+        for mode in (0, 8):
+            lib.llmss_gemm_set_pair(mode)
+            err[mode] = ((cu.linear(x, w).double() - want).norm() / want.norm()).item()
+    finally:
+        lib.llmss_gemm_set_pair(-1)
+    assert err[8] <= math.hypot(err[0], 4096 / 16 * 2.0 ** -25), err
+
+
 # ------------------------------------------------------------------ norm
 @pytest.mark.parametrize("dtype", DT)
 @pytest.mark.parametrize("kind", [R.NORM_LAYER, R.NORM_RMS])
