@@ -100,10 +100,14 @@ def test_gemm_gated_and_f32_out_and_strided_input():
     _close(z, R.linear(x, w, out_dtype=torch.float32), 5e-3, 1e-2, "f32 out")
 
 
+# products whose K the automatic choice splits over two pairs
+PAIR_SPLIT = [(100, 2048, 2048), (65, 512, 4096), (200, 130, 2048)]
+
+
 @pytest.mark.parametrize("mode", [8, 1, 2, 4])
 def test_gemm_cta_pair_kernel(mode):
-    """tcgen05 cta_group::2 kernel (two CTAs share one 256 x 256 MMA): the automatic choice (persistent pairs from 40
-    pair tiles upwards) and the forced schedules (1 = persistent, 2 / 4 = split-K over 2 / 4 pairs per cluster), every
+    """tcgen05 cta_group::2 kernel (two CTAs share one MMA of 256 features): the automatic choice (the cheapest token tile and
+    schedule by an estimate) and the forced schedules (1 = persistent, 2 / 4 = split-K over 2 / 4 pairs per cluster), every
     epilogue flavour, ragged rows / odd feature-tile counts / K tails, against the fp32 oracle and the single-CTA kernels."""
     from llmss_b200.ops import _lib
 
@@ -113,7 +117,8 @@ def test_gemm_cta_pair_kernel(mode):
     if mode != 8:
         cases += [(256, 512, 512, torch.bfloat16), (200, 4224, 4160, torch.bfloat16)]
     else:
-        cases += [(256, 6144, 512, torch.bfloat16)]     # 24 pair tiles: the automatic choice splits K over two pairs
+        # many tiles, persistent pairs; few tiles and a long K, split over two pairs each (test_gemm_pair_automatic_split: that it is so)
+        cases += [(256, 6144, 512, torch.bfloat16)] + [(*c, dt) for c in PAIR_SPLIT for dt in DT]
     try:
         for M, N, K, dt in cases:
             torch.manual_seed(M + N + K + mode)
@@ -137,6 +142,26 @@ def test_gemm_cta_pair_kernel(mode):
                 assert (y.float() - y_single.float()).abs().max().item() <= 0.05 * max(1.0, ref.abs().max().item()), tag
     finally:
         lib.llmss_gemm_set_pair(-1)
+
+
+@pytest.mark.parametrize("M,N,K", PAIR_SPLIT)
+def test_gemm_pair_automatic_split(M, N, K):
+    """The bits of the automatic choice are those of two pairs per tile (whatever its width) and not those of one chain over K."""
+    from llmss_b200.ops import _lib
+
+    cu = _cu()
+    lib = _lib.load()
+    torch.manual_seed(M)
+    x = torch.randn(M, K, device="cuda", dtype=torch.bfloat16)
+    w = torch.randn(N, K, device="cuda", dtype=torch.bfloat16)
+    y = {}
+    try:
+        for mode in (8, 2 | 32 << 8, 1 | 32 << 8):
+            lib.llmss_gemm_set_pair(mode)
+            y[mode] = cu.linear(x, w)
+    finally:
+        lib.llmss_gemm_set_pair(-1)
+    assert torch.equal(y[8], y[2 | 32 << 8]) and not torch.equal(y[8], y[1 | 32 << 8])
 
 
 @pytest.mark.parametrize("split", [1, 2])
@@ -210,6 +235,33 @@ def test_gemm_32_bit_results_of_short_stretches(M, N, K):
     finally:
         lib.llmss_gemm_set_pair(-1)
     assert err[8] <= 1.1 * err[0], err
+
+
+@pytest.mark.parametrize("M,N,K", [(64, 20480 + 130, 1032), (40, 50257, 256), (17, 30000, 200)])
+def test_gemm_several_accumulators_over_several_tiles(M, N, K):
+    """32-bit results of pairs that walk several tiles with two accumulators each, of which both are buffered twice in tensor memory: every number has the
+    bits of the two stretches' products added, then the bias."""
+    from llmss_b200.ops import _lib
+
+    cu = _cu()
+    lib = _lib.load()
+    torch.manual_seed(M)
+    x = torch.randn(M, K, device="cuda", dtype=torch.bfloat16)
+    w = (torch.randn(N, K, device="cuda") * K ** -0.5).to(torch.bfloat16)
+    b = torch.randn(N, device="cuda", dtype=torch.bfloat16)
+    blocks = -(-K // 64)
+    cut = (blocks + 1) // 2 * 64
+    got = cu.linear(x, w, b, out_dtype=torch.float32)
+    try:
+        lib.llmss_gemm_set_pair(1 | 64 << 8)       # one chain per tile
+        parts = [cu.linear(x[:, a:e], w[:, a:e], out_dtype=torch.float32) for a, e in ((0, cut), (cut, K))]
+        chain = cu.linear(x, w, b, out_dtype=torch.float32)
+    finally:
+        lib.llmss_gemm_set_pair(-1)
+    assert torch.equal(got, parts[0] + parts[1] + b.float())
+    assert not torch.equal(got, chain)
+    want = x.double() @ w.double().t() + b.double()
+    assert ((got.double() - want).norm() / want.norm()).item() < max(K, 256) / 16 * 2.0 ** -24
 
 
 @pytest.mark.parametrize("M,N,K", [(65, 4096, 20480), (200, 4096, 20480), (128, 512, 20480), (900, 512, 20480), (100, 4096, 16384)])
