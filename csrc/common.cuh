@@ -394,6 +394,18 @@ __device__ __forceinline__ void umma_ss_pair(uint32_t d, uint32_t a_lo, uint32_t
 
 }  // namespace umma_lo
 
+// ---------------------------------------------------------------- warp-level tensor-core product
+// c (16 x 8, 32-bit) += a (16 x 16) b (16 x 8) of one warp, 16-bit operands in the instruction's fragments; for products too small for a tcgen05 tile
+template <typename T>
+__device__ __forceinline__ void mma_16816(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
+  if constexpr (std::is_same<T, __half>::value)
+    asm("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
+        : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3]) : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+  else
+    asm("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
+        : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3]) : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+}
+
 // ---------------------------------------------------------------- visible keys
 // first key position that query position p sees through a sliding window (0: none) and / or a chunked mask (0: none; p sees its own
 // block of `chunk` positions, counted from the sequence's start)

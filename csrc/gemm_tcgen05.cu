@@ -280,9 +280,10 @@ __device__ __forceinline__ uint32_t pack2(float lo, float hi) {
   else p = __floats2bfloat162_rn(lo, hi);
   return *reinterpret_cast<const uint32_t*>(&p);
 }
-// Four tokens of a lane's feature, 16-bit, as 8-byte stores: four neighbouring lanes exchange until lane r of them has token r of their four features, so that
-// a warp's store covers four rows of 64 bytes (each lane storing its own column takes four instructions of one row each: per-head products of 8192 tokens
-// 33.0 us, so 31.2; the products of a 6-layer prompt pass, with GELU, 88 each, so 85).  o: row 0 at the first of the four features, 8-byte aligned with ldo a multiple of 4.  The whole warp calls it.
+// Four tokens of a lane's feature, 16-bit, as 8-byte stores: four neighbouring lanes exchange until lane r of them has token r of their four features, so
+// that a warp's store covers four rows of 64 bytes (each lane storing its own column takes four instructions of one row each: per-head products of 8192
+// tokens 33.0 us, so 31.2; the products of a 6-layer prompt pass, with GELU, 88 each, so 85).  o: row 0 at the first of the four features, 8-byte aligned
+// with ldo a multiple of 4.  The whole warp calls it.
 template <typename T>
 __device__ __forceinline__ void store_4_tokens(T* o, int64_t ldo, float t0, float t1, float t2, float t3, int lane) {
   const bool odd = lane & 1, upper = lane & 2;
@@ -1241,7 +1242,8 @@ gemm_cluster_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
 }
 
 // ======================================================================================
-// CTA-pair kernel (tcgen05 cta_group::2): every product of more than 64 tokens, and fewer tokens over many features.
+// CTA-pair kernel (tcgen05 cta_group::2): products of more than 64 tokens and more than 128 features, fewer tokens over many features (pick_pair has the
+// lines and what else stays with the single-CTA kernels).
 //
 // With 128-feature tiles every CTA re-reads the whole 256-token activation tile per k-block: 32 KB of activations from
 // L2 for 16 KB of weights, and from M = 256 upwards the L2 -> SM traffic and the bytes a 4-stage ring can keep in
@@ -1249,10 +1251,10 @@ gemm_cluster_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
 // 256 x 256 x 16 MMA: each CTA loads its own 128 weight rows and HALF of the token rows (both at the same shared-memory
 // offsets), the even CTA issues `tcgen05.mma.cta_group::2`, the tensor cores of both SMs read both halves of the
 // activation tile, and each CTA's tensor memory receives the accumulator of its own 128 features.  Activation traffic per
-// weight byte halves and the ring holds 6 stages instead of 4 (measured: 313 ns per k-block of 256 x 256 x 64, against
-// ~410 ns for two single-CTA tiles at M = 8192).  The token tile is 32 .. 256 columns wide, chosen per launch (pick_pair): fewer tokens, or few feature
-// tiles, take narrower ones, whose k-blocks take as much less time down to 128 columns.  Against tiles of 256 columns only (us): 366 tokens 4096 x 4096
-// 24.5 -> 18, 526 tokens 4096 x 11008 62 -> 45, 827 tokens 2048 x 2048 19.1 -> 12.2, 64 tokens 28672 x 4096 45.1 -> 42 (from the single-CTA kernel).
+// weight byte halves and the ring holds 6 stages of 256 columns instead of 4, up to 10 of narrower tiles (measured: 313 ns per k-block of 256 x 256 x 64,
+// against ~410 ns for two single-CTA tiles at M = 8192).  The token tile is 32 .. 256 columns wide, chosen per launch (pick_pair): fewer tokens, or few
+// feature tiles, take narrower ones, whose k-blocks take as much less time down to 128 columns.  Tiles of 256 columns / as chosen, us: 366 tokens
+// 4096 x 4096 27.1 / 17.1, 526 tokens 4096 x 11008 62.4 / 45.1, 827 tokens 2048 x 2048 18.4 / 12.2; 64 tokens 28672 x 4096 46.5 (single-CTA kernel) / 41.7.
 //
 // Two schedules, chosen on the host:
 //  * persistent (clusters of 2, S = 1): every pair walks tiles p, p + P, p + 2P, ... with TWO accumulators of 256 columns
@@ -1269,9 +1271,9 @@ gemm_cluster_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
 // GPU's own operands.
 // ======================================================================================
 struct PCfg2 {
-  // warps 0 and 1 as everywhere, 2 .. 9 the epilogue: two to a quarter of the features, alternate chunks of 32 columns.  A chunk is a chain from the load out of
-  // tensor memory to the stores, and the last tile's chunks are exposed: with one warp to a quarter 366 tokens 4096 x 4096 took 28.9 us in tiles of 256 columns,
-  // with two 27.2; per-head products of 8192 tokens, which are little else, 45.5 and 31
+  // warps 0 and 1 as everywhere, 2 .. 9 the epilogue: two to a quarter of the features, alternate chunks of 32 columns.  A chunk is a chain from the load
+  // out of tensor memory to the stores, and the last tile's chunks are exposed: with one warp to a quarter 366 tokens 4096 x 4096 took 28.9 us in tiles of
+  // 256 columns, with two 27.2; per-head products of 8192 tokens, which are little else, 45.5 and 31
   static constexpr int THREADS = 320, EPI_WARPS = 8;
   static constexpr int BN = 256;                 // most token columns of the pair's accumulator (GemmArgs::bn: those of a launch)
   static constexpr int W_BYTES = BM * BK * 2;
@@ -1951,9 +1953,9 @@ int pair_mode() {
 struct PairPlan {
   int split, bn, nacc = 1;      // pairs per cluster (0: not this kernel), token columns of a tile, accumulators
 };
-// Estimate of the pair kernel's time in us for token tiles of bn columns, S pairs per cluster; constants fitted to 206 sweeps on B200 (N = 16 .. 50400,
-// K = 1600 .. 20480, 4 .. 8192 tokens, cold weights): the choice it leads to is 1.2 % behind the fastest of all (S, bn) on average.  A 64-column block
-// takes the longest of issuing it, its MMAs (slower the more of the chip is busy) and its share of what L2 delivers; all of it no less than memory
+// Estimate of the pair kernel's time in us for token tiles of bn columns, S pairs per cluster; constants fitted to sweeps of (S, bn) on B200 (N = 16 ..
+// 50400, K = 1600 .. 20480, 4 .. 8192 tokens, cold weights).  Over 175 such products the choice that it leads to is 1.8 % behind the fastest on average
+// (worst: 34 clusters of four at 526 tokens 512 x 4096, probably more than fit at once, 20.2 / 11.8 us).  A 64-column block takes the longest of issuing it, its MMAs (slower the more of the chip is busy) and its share of what L2 delivers; all of it no less than memory
 // takes (token tiles of one weight tile do not all find it in L2); prologue and last epilogue grow with the tile.
 float pair_cost(int M, int N, int K, int kb_total, int sms, int bn, int S) {
   const int tiles_m = (M + bn - 1) / bn, tiles = ((N + 2 * BM - 1) / (2 * BM)) * tiles_m;
@@ -1969,9 +1971,9 @@ float pair_cost(int M, int N, int K, int kb_total, int sms, int bn, int S) {
   return bn == PCfg2::BN ? 0.96f * all : all;        // (fewest loads: faster than this where the whole chip is at its power limit)
 }
 int wide_rows(const void* out, int64_t ldo) { return ((uintptr_t)out & 7) == 0 && ldo % 4 == 0; }
-// Accumulators that a tile may have.  A tensor core's sum over K is cut off at 24 bits after every 16 products, so that a 32-bit result of one chain over K = 2048
-// lies 2e-6 of its norm from 64 bits and one summed from eight stretches 5e-7.  A launch that gives every pair one tile has all of tensor memory for it,
-// others half.
+// Accumulators that a tile may have.  A tensor core's sum over K is cut off at 24 bits after every 16 products, so that a 32-bit result of one chain over
+// K = 2048 lies 2.1e-6 of its norm from 64 bits and one summed from eight stretches 2.4e-7.  A launch that gives every pair one tile has all of tensor
+// memory for it, others half.
 int pair_accumulators(int tiles, int bn, int sms) { return (tiles <= sms / 2 ? 512 : 256) / bn; }
 // The cheapest of all (S, bn) whose S times accumulators are at least `parts`, and its cost; split 0 and no cost where none fits.  At most 128 features run
 // only as two pairs per tile with narrow tiles (see pick_pair).
@@ -1991,11 +1993,12 @@ PairPlan best_pair(int M, int N, int K, int kb_total, int sms, int parts, float*
     }
   return best;
 }
-// The pair kernel, or {0, 0}: the single-CTA kernels.  Those keep few tokens over few features, where a tile shared by up to eight CTAs is finished
-// sooner (us, single-CTA / pairs: 4 tokens 2048 x 2048 7.0 / 8.4, 4096 x 4096 11.2 / 12.1; 64 tokens 4096 x 4096 12.7 / 13.1, but 6144 x 2048
-// 16.3 / 10.4; 16 tokens 8320 x 4096 16.2 / 17.6, 50400 x 4096 69.3 / 65.5), and at most 128 features (half of each pair's MMA would be idle) unless two
-// pairs per tile fit the machine (16 x 2048: 140 tokens 11.5 / 7.8, 1200 11.9 / 9.9, 5000 15.4 / 17).  Above 64 tokens one 128-feature tile per CTA
-// loads too much: 128 tokens 6144 x 2048 21.2 / 10.7, 700 tokens 512 x 4096 46.6 / 12.0.
+// The pair kernel, or {0, 0}: the single-CTA kernels.  Those keep few tokens over few features (up to 16 tokens below 44 tiles of 256 features, 11009
+// features; up to 64 below 24, 5889 features), where a tile shared by up to eight CTAs is finished sooner (us, single-CTA / pairs: 4 tokens 2048 x 2048
+// 7.3 / 8.6, 4096 x 4096 11.1 / 12.1; 64 tokens 4096 x 4096 12.4 / 12.6, but 6144 x 2048 16.3 / 10.5; 16 tokens 8320 x 4096 16.2 / 17.6, 50400 x 4096
+// 70.4 / 64.8), and at most 128 features (half of each pair's MMA would be idle) unless two pairs per tile fit the machine and K has four blocks (16 x 2048:
+// 128 tokens 9.0 / 8.0, 1500 12.1 / 10.7, 8192 15.8 / 17.8).  The same goes for results that need more accumulators than fit.  Above 64 tokens one
+// 128-feature tile per CTA loads too much: 128 tokens 6144 x 2048 20.9 / 10.6, 827 tokens 512 x 4096 40.1 / 12.0.
 PairPlan pick_pair(int M, int N, int K, int kb_total, int sms, int parts) {
   const int mode = pair_mode() & 255, forced_bn = pair_mode() >> 8;
   if (mode == 0 || sms < 2) return {0, 0, 1};
@@ -2010,7 +2013,7 @@ PairPlan pick_pair(int M, int N, int K, int kb_total, int sms, int parts) {
 }
 
 // Largest cluster size (2..8) for which all `tiles` clusters are co-resident (one wave) and every CTA still
-// streams >= 2 k-blocks; 0 = use the stream-K persistent kernel.  LLMSS_GEMM_MODE=streamk|cluster forces one.
+// streams >= 2 k-blocks; 0 = use the stream-K persistent kernel.  LLMSS_GEMM_MODE=streamk|cluster forces one (and leaves the pair kernel out).
 template <typename T, int BN>
 int max_active_clusters(int split) {
   static int cache[9] = {-1, -1, -1, -1, -1, -1, -1, -1, -1};
@@ -2091,9 +2094,9 @@ int pick_bn(int M) {
 
 }  // namespace
 
-// Profiling aid: when non-null, every CTA of the following llmss_gemm launches writes 8 globaltimer
-// stamps (entry, prologue done, last TMA issued, first stage landed, last MMA issued, first
-// accumulator ready, epilogue done, exit) to buf[cta*8 .. cta*8+7].  buf must be zeroed by the caller.
+// Profiling aid: when non-null, every CTA of the following llmss_gemm launches writes globaltimer stamps to buf[cta*8 .. cta*8+7]: 0 entry, 1 prologue
+// done, 2 partial sums of the cluster or of other CTAs ready (split K only), 3 first stage landed (not the pair kernel), 4 last MMA issued (pair kernel: the
+// even CTA's), 5 accumulator ready, 6 epilogue done, 7 exit.  buf must be zeroed by the caller.
 LLMSS_API int llmss_gemm_set_pair(int mode) {          // mode | token tile << 8 also pins the width of the token tile
   LLMSS_REQUIRE(mode < 256 || ((mode >> 8) % 32 == 0 && (mode >> 8) <= PCfg2::BN), "gemm_set_pair: token tiles of %d columns (32, 64 .. 256)", mode >> 8);
   g_pair_mode = mode;
@@ -2420,8 +2423,9 @@ static float expert_tiles(float rows, int bn) {
   return 0.2f * t;
 }
 // Estimates, in us, of T tokens' choices of `top` of E experts (up matrices [rows, W], down [W, F]): both products over all experts for every token (dense),
-// and sorted by expert in tiles of *tile_rows rows (grouped), with the passes that sort, place and sum the rows.  Terms as in pair_cost; within 15 % of 30
-// measured blocks (4 of 16 experts of 1024, width 2048; 2 of 8 gated ones of 2048; 4 of 32 of 1536, width 4096; 64 .. 8192 tokens).
+// and sorted by expert in tiles of *tile_rows rows (grouped), with the passes that sort, place and sum the rows.  Terms as in pair_cost; both within 17 % of
+// 30 measured blocks (4 of 16 experts of 1024, width 2048; 2 of 8 gated ones of 2048; 4 of 32 of 1536, width 4096; 64 .. 8192 tokens), also where the
+// single-CTA kernels take a product of the dense form (up to 64 tokens over few features, within 5 % of the pair kernel's there).
 LLMSS_API int llmss_moe_forms(int T, int top, int E, int W, int F, int rows, float* dense_us, float* grouped_us, int* tile_rows) {
   LLMSS_REQUIRE(T > 0 && top > 0 && E > 0 && W > 0 && F > 0 && rows > 0, "moe_forms: bad sizes");
   const int sms = num_sms(), pairs = sms / 2;
@@ -2471,7 +2475,8 @@ LLMSS_API int llmss_gemm_heads(const void* x, int64_t ldx, int64_t sxh, const vo
   CUtensorMap tw, tx;
   if (int e = make_tmap_3d(&tw, w, dtype, K, N, H, ldw, swh, BM)) return e;
   if (int e = make_tmap_3d(&tx, x, dtype, K, M, H, ldx, sxh, 256)) return e;
-  HeadArgs a{M, N, H, (N + BM - 1) / BM, (M + 255) / 256, (K + BK - 1) / BK, dtype, scale, lds, ssh, ssn, out, ldo, soh, out_f32, !out_f32 && wide_rows(out, ldo) && soh % 4 == 0};
+  const int wide = !out_f32 && wide_rows(out, ldo) && soh % 4 == 0;
+  HeadArgs a{M, N, H, (N + BM - 1) / BM, (M + 255) / 256, (K + BK - 1) / BK, dtype, scale, lds, ssh, ssn, out, ldo, soh, out_f32, wide};
   const int64_t tiles = (int64_t)a.tiles_n * a.tiles_m * H;
   LLMSS_REQUIRE(tiles < (1ll << 30), "gemm_heads: too many tiles");
   const int grid = (int)(tiles < num_sms() ? tiles : num_sms());

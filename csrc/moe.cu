@@ -171,19 +171,11 @@ __global__ void __launch_bounds__(128) moe_route_kernel(RouteArgs a, const float
   if (t < T) route_token<PL>(a, z + (int64_t)t * ldz, t, cs_all[threadIdx.x >> 5]);
 }
 
-// Logits and routing in one launch, for up to 32 experts: a block has 16 tokens, its 16 warps every 16th piece of 32 channels and then a token each.  A product of 16 columns has no
-// use for the tensor-memory tiles (128 features), and its result went through memory to a second launch; here the rows come straight into mma fragments.
-// The order of a sum over channels is free, so a thread's 16-byte pieces of a token's and an expert's row are two steps of k = 16 as they lie.  Two launches /
-// one, us: 8192 tokens of 2048, 16 experts 28.7 / 20.7; 2048 of 4096, 32 experts 18.2 / 11.3; 400 of 2048, 16 experts 13.6 / 7.2 (with eight warps 20.8, 15.9,
-// 11.2: a block is one chain of loads, sums and choices).  Up to 64 experts it lost (4096 of 4096: 54).
-template <typename T> __device__ __forceinline__ void mma_16816(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
-  if constexpr (std::is_same<T, __half>::value)
-    asm("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
-        : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3]) : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
-  else
-    asm("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
-        : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3]) : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
-}
+// Logits and routing in one launch, for up to 32 experts: a block has 16 tokens, its 16 warps every 16th piece of 32 channels and then a token each.  A
+// product of 16 columns has no use for the tensor-memory tiles (128 features), and its result went through memory to a second launch; here the rows come
+// straight into mma fragments.  The order of a sum over channels is free, so a thread's 16-byte pieces of a token's and an expert's row are two steps of
+// k = 16 as they lie.  Two launches / one, us: 8192 tokens of 2048, 16 experts 28.7 / 20.7; 2048 of 4096, 32 experts 18.2 / 11.3; 400 of 2048, 16 experts
+// 13.6 / 7.2 (with eight warps 20.8, 15.9, 11.2: a block is one chain of loads, sums and choices).  Up to 64 experts it lost (4096 of 4096: 54).
 template <typename T, int NT>      // NT: tiles of 8 experts
 __global__ void __launch_bounds__(512) moe_router_kernel(RouteArgs a, const T* __restrict__ h, int64_t ldh, const T* __restrict__ w, int64_t ldw,
                                                          const T* __restrict__ bias, int K, int T_) {
@@ -554,7 +546,8 @@ LLMSS_API int llmss_moe_router(const void* h, int64_t ldh, const void* w, int64_
   LLMSS_REQUIRE((score_kind == 0 || score_kind == 1) && group_top >= 1 && group_top <= kMaxGroupTop, "moe_router: score kind %d, group top %d", score_kind, group_top);
   if (T_ <= 0) return 0;
   const RouteArgs a{E, top, groups, keep, route_scale, score_kind, correction, group_top, renorm, ids, wts, dense};
-#define LLMSS_ROUTER(T, NT) moe_router_kernel<T, NT><<<(T_ + 15) / 16, 512, 0, stream>>>(a, (const T*)h, ldh, (const T*)w, ldw, (const T*)bias, K, T_)
+#define LLMSS_ROUTER(T, NT) \
+  moe_router_kernel<T, NT><<<(T_ + 15) / 16, 512, 0, stream>>>(a, (const T*)h, ldh, (const T*)w, ldw, (const T*)bias, K, T_)
 #define LLMSS_ROUTER_E(T)                  \
   if (E <= 16) LLMSS_ROUTER(T, 2);         \
   else LLMSS_ROUTER(T, 4)

@@ -122,20 +122,6 @@ __global__ void __launch_bounds__(NT) bgemm_kernel(BgArgs a) {
 // fragment layouts of the instruction); 8 warps, each 16 rows x (64 / warps-per-row) columns.  No bias / activation.
 constexpr int MK = 32, MN = 64, MPAD = 8;
 
-template <typename T> struct MmaOp;
-template <> struct MmaOp<__nv_bfloat16> {
-  static __device__ __forceinline__ void run(float (&c)[4], const uint32_t (&a)[4], const uint32_t (&b)[2]) {
-    asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
-                 : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3]) : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b[0]), "r"(b[1]));
-  }
-};
-template <> struct MmaOp<__half> {
-  static __device__ __forceinline__ void run(float (&c)[4], const uint32_t (&a)[4], const uint32_t (&b)[2]) {
-    asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
-                 : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3]) : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b[0]), "r"(b[1]));
-  }
-};
-
 template <typename T, bool OUT_F32, int TM>
 __global__ void __launch_bounds__(NT) bgemm_mma_kernel(BgArgs a) {
   constexpr int WM = TM / 16, WN = 8 / WM, NW = MN / WN, NF = NW / 8;   // warps along m / n, columns and n-fragments per warp
@@ -210,7 +196,7 @@ __global__ void __launch_bounds__(NT) bgemm_mma_kernel(BgArgs a) {
         const T* br = &Bs[wn * NW + f * 8 + gid][kk + tig * 2];
         bf[0] = *reinterpret_cast<const uint32_t*>(br);
         bf[1] = *reinterpret_cast<const uint32_t*>(br + 8);
-        MmaOp<T>::run(acc[f], af, bf);
+        mma_16816<T>(acc[f], af[0], af[1], af[2], af[3], bf[0], bf[1]);
       }
     }
     __syncthreads();
