@@ -186,7 +186,7 @@ class RotaryLatentAttention:
 _GROUPED_ROWS = int(os.environ.get("LLMSS_MOE_GROUPED_MIN_ROWS", "16"))   # grouped form from this many rows per expert on average
 _FORCE_GROUPED = os.environ.get("LLMSS_MOE_FORCE_GROUPED", "0") == "1"
 _GEMM_TFLOPS, _CALL_US = 1200.0, 30.0     # sustained tensor-core rate of the expert GEMMs; host cost of issuing one GEMM
-_DENSE_HOST_US, _GROUPED_HOST_US = 45.0, 65.0   # issuing the launches of the two forms, the router's aside
+_DENSE_HOST_US, _GROUPED_HOST_US = 45.0, 65.0   # issuing the launches of the two forms, the router's aside (39 .. 41 / 53 .. 54; through ctypes 48 .. 51 / 64 .. 65)
 _DENSE_MIN = int(os.environ.get("LLMSS_MOE_DENSE_MIN_TOKENS", "0"))   # 0: dense as soon as token x top pairs >= experts
 
 
